@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/hero_gpu.h"
+#include "hero_band.cuh"
 #include "hero_internal.cuh"
 
 using namespace hero;
@@ -75,6 +76,10 @@ struct hero_ctx {
     uint64_t vote_ext_bytes = 0;
     DBuf wcache;                    // per batch: the table slot each probe window found
     DBuf map_hist, map_max;
+    // the window DP's buffers: without room for them the whole-matrix kernels do all the work
+    DBuf q_pack, s_pack;            // 2-bit codes of the reads, kPackPad words of room on both sides
+    DBuf w_key, w_order, w_rest, w_bin, w_codes;
+    bool window = true;             // off from an allocation that did not fit until the next query set
     bool consensus_done = false;  // out_seq holds the consensus of the current votes
     std::vector<uint8_t> aln_host;  // .aln text of every subject aligned since the last take
     // index build temporaries (kept between builds)
@@ -112,7 +117,8 @@ struct hero_ctx {
                         &x_klo, &x_khi, &x_kval, &x_owner, &x_count, &x_slot_of, &x_start,
                         &x_fill, &x_tmp, &q_job, &win_sorted, &win_bins, &a_list, &a_n,
                         &a_roff, &a_unit, &a_len, &a_pre, &a_cig, &a_uoff, &a_text, &q_ext,
-                        &m_seq, &m_len, &map_hist, &map_max, &wcache};
+                        &m_seq, &m_len, &map_hist, &map_max, &wcache, &q_pack, &s_pack,
+                        &w_key, &w_order, &w_rest, &w_bin, &w_codes};
         for (DBuf *b : list) all.push_back(b);
     }
 
@@ -147,8 +153,34 @@ struct hero_ctx {
         b.external = false;
         b.pooled = false;
     }
+    // gives the window DP's buffers back (work that reads them is queued before
+    // the stream-ordered frees); false when there are none
+    bool shed() {
+        bool any = false;
+        for (DBuf *b : {&q_pack, &s_pack, &w_key, &w_order, &w_rest, &w_bin, &w_codes}) {
+            any = any || b->p;
+            release(*b);
+        }
+        window = false;
+        if (any) plan_ok = false;  // a captured round reads them
+        return any;
+    }
+    // a buffer of the window DP: one that does not fit turns the window off
+    bool optional(DBuf &b, size_t need, const char *what) {
+        if (!window) return false;
+        const std::string before = err;
+        if (grow(b, need, what) == HERO_OK) return true;
+        err = before;
+        shed();
+        return false;
+    }
     // grows a device buffer to at least `need` bytes (contents are not kept)
     int ensure(DBuf &b, size_t need, const char *what) {
+        int r = grow(b, need, what);
+        if (r == HERO_E_OOM && shed()) r = grow(b, need, what);
+        return r;
+    }
+    int grow(DBuf &b, size_t need, const char *what) {
         if (need == 0) need = 16;
         if (b.cap >= need) return HERO_OK;
         if (b.external) return fail(HERO_E_INPUT, std::string("caller's buffer too small for ") + what);
@@ -211,9 +243,13 @@ static T *P_(DBuf &b) {
 
 static const uint32_t *job_tags(hero_ctx *c) { return c->tagged ? P_<uint32_t>(c->q_job) : nullptr; }
 
+// packed codes, behind their room; NULL without the buffer
+static uint32_t *pack_words(const DBuf &b) { return b.p ? static_cast<uint32_t *>(b.p) + kPackPad : nullptr; }
+static size_t pack_bytes(uint64_t nb) { return size_t((nb + 15) / 16 + 2 * kPackPad) * 4; }
+
 static ReadsView query_view(hero_ctx *c) {
     return ReadsView{P_<uint8_t>(c->q_code), P_<uint64_t>(c->q_off), P_<uint32_t>(c->q_len),
-                     P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_good), c->nq, job_tags(c)};
+                     P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_good), c->nq, job_tags(c), pack_words(c->q_pack)};
 }
 
 // kernel shape of a DP launch from the tuning table (first class covering rmax)
@@ -322,7 +358,7 @@ extern "C" const char *hero_last_error(const hero_ctx *ctx) {
 
 // uploads reads and derives codes, lengths and good flags on the device
 static int upload_reads(hero_ctx *c, const uint8_t *seq, const uint64_t *off, const int64_t *uid,
-                        uint64_t n, DBuf &raw, DBuf &code, DBuf &doff, DBuf &len, DBuf &duid,
+                        uint64_t n, DBuf &raw, DBuf &code, DBuf &pack, DBuf &doff, DBuf &len, DBuf &duid,
                         DBuf *gq, DBuf *gs, DBuf *gc) {
     const uint64_t nb = n ? off[n] : 0;
     HERO_TRY(c->ensure(raw, nb, "reads"));
@@ -339,10 +375,11 @@ static int upload_reads(hero_ctx *c, const uint8_t *seq, const uint64_t *off, co
         const uint64_t z = 0;
         return c->cuda(cudaMemcpy(doff.p, &z, 8, cudaMemcpyHostToDevice), "upload");
     }
+    c->optional(pack, pack_bytes(nb), "packed codes");
     HERO_TRY(c->cuda(cudaMemcpyAsync(raw.p, seq, nb, cudaMemcpyHostToDevice, c->st), "upload"));
     HERO_TRY(c->cuda(cudaMemcpyAsync(doff.p, off, (n + 1) * 8, cudaMemcpyHostToDevice, c->st), "upload"));
     HERO_TRY(c->cuda(cudaMemcpyAsync(duid.p, uid, n * 8, cudaMemcpyHostToDevice, c->st), "upload"));
-    launch_prep_reads(P_<uint8_t>(raw), nb, P_<uint8_t>(code), P_<uint64_t>(doff), n,
+    launch_prep_reads(P_<uint8_t>(raw), nb, P_<uint8_t>(code), pack_words(pack), P_<uint64_t>(doff), n,
                       P_<uint32_t>(len), gq ? P_<uint8_t>(*gq) : nullptr,
                       gs ? P_<uint8_t>(*gs) : nullptr, gc ? P_<double>(*gc) : nullptr, c->p.l, c->st);
     return c->check_launch("prep reads");
@@ -376,7 +413,8 @@ extern "C" int hero_set_queries(hero_ctx *c, const uint8_t *seq, const uint64_t 
     c->have_index = false;
     c->consensus_done = false;
     c->tagged = false;
-    HERO_TRY(upload_reads(c, seq, n ? off : nullptr, uid, n, c->q_raw, c->q_code, c->q_off,
+    c->window = true;
+    HERO_TRY(upload_reads(c, seq, n ? off : nullptr, uid, n, c->q_raw, c->q_code, c->q_pack, c->q_off,
                           c->q_len, c->q_uid, &c->q_good, &c->q_sgood, &c->q_gc));
     HERO_TRY(c->ensure(c->fp, 8, "fingerprint"));
     launch_fingerprint(P_<uint8_t>(c->q_raw), c->nqb, P_<uint64_t>(c->q_off), P_<int64_t>(c->q_uid), n,
@@ -537,6 +575,44 @@ extern "C" int hero_build_index(hero_ctx *c) {
     return r;
 }
 
+struct DpBufs {
+    DBuf &bins, &bin_off, &perm, &tasks, &key, &order, &rest, &bin, &codes, &scan;
+};
+
+// The DP of a.nd segments: the window kernels, then the whole-matrix kernels on
+// what they leave.  a.n_rest must be zero.  Without the window's buffers every
+// segment goes to the whole-matrix kernels (their list then lies in the op
+// words, which nothing has written yet).
+static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
+    if (!a.nd) return HERO_OK;
+    BandWork w{};
+    w.warps = band_warps(c->dev, a.nd);
+    w.code_words = band_code_words(cmax, a.affine != 0);
+    const size_t table = kBandBins * (sizeof(BandBin) + 4) + 16;
+    w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 4, "DP windows") &&
+           c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 4, "DP windows") &&
+           c->optional(b.bin, table, "DP windows") &&
+           c->optional(b.codes, size_t(w.warps) * w.code_words * 4, "DP windows");
+    a.bins = P_<uint32_t>(b.bins);
+    a.rest = w.on ? P_<uint32_t>(b.rest) : a.ops;
+    a.perm = P_<uint32_t>(b.perm);
+    if (w.on) {
+        w.key = P_<uint32_t>(b.key);
+        w.order = P_<uint32_t>(b.order);
+        w.bin = P_<BandBin>(b.bin);
+        w.cursor = reinterpret_cast<uint32_t *>(w.bin + kBandBins);
+        w.head = w.cursor + kBandBins;
+        w.codes = P_<uint32_t>(b.codes);
+        w.count = a.bins + kDpBins;
+    }
+    HERO_TRY(c->cuda(cudaMemsetAsync(b.bins.p, 0, (kDpBins + kBandBins) * 4, c->st), "DP bins"));
+    apply_tuning(c, a);
+    launch_band(a, w, c->st);
+    launch_dp_sort(a, P_<uint32_t>(b.perm), P_<uint64_t>(b.bin_off), b.scan.p, c->st);
+    launch_dp(a, P_<uint64_t>(b.bin_off), P_<uint64_t>(b.tasks), cmax, c->st);
+    return HERO_OK;
+}
+
 // Alignment output of one batch (after the records are scored): the kept
 // records per subject (SubjectRead::addAlignment by query uniqueId), the text
 // units, their sizes, a scan, the text; appended to the context's host text.
@@ -609,8 +685,8 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         if ((r = c->ensure(c->scan_tmp, scan_tmp_bytes(std::max<uint64_t>(nseg + 1, kDpBins + 1)), "scan"))) break;
         // zero the per-batch counters that size buffers (keep the running totals)
         if ((r = c->cuda(cudaMemsetAsync(ctr + C_NC, 0, sizeof(unsigned long long) * (C_MAXC - C_NC + 1), c->st), "batch: counters"))) break;
-        static_assert(C_WIN == C_OVERFLOW + 1, "overflow flag and winner count are cleared together");
-        if ((r = c->cuda(cudaMemsetAsync(ctr + C_OVERFLOW, 0, 2 * sizeof(unsigned long long), c->st), "batch: counters"))) break;
+        static_assert(C_WIN == C_OVERFLOW + 1 && C_REST == C_WIN + 1, "cleared together");
+        if ((r = c->cuda(cudaMemsetAsync(ctr + C_OVERFLOW, 0, 3 * sizeof(unsigned long long), c->st), "batch: counters"))) break;
         // the count pass leaves the slot of every window (2 x 8 bytes a subject base) for the emit pass
         if ((r = c->ensure(c->wcache, std::max<uint64_t>(nbases, 1) * 16, "probe windows"))) break;
         uint2 *wc = P_<uint2>(c->wcache);
@@ -680,16 +756,14 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         if ((r = c->ensure(c->cells, NDc * 4, "DP cells"))) break;
         if ((r = c->ensure(c->perm, NDc * 4, "DP order"))) break;
         if ((r = c->ensure(c->ops, NDc * stride * 4, "DP ops"))) break;
-        if ((r = c->ensure(c->bins, kDpBins * 4, "DP bins"))) break;
+        if ((r = c->ensure(c->bins, (kDpBins + kBandBins) * 4, "DP bins"))) break;
         if ((r = c->ensure(c->bin_off, (kDpBins + 1) * 8, "DP bins"))) break;
         const int32_t nst = (cmax + kStripW - 1) / kStripW;
-        if ((r = c->ensure(c->dp_tasks, 128 * 8, "DP tasks"))) break;
+        if ((r = c->ensure(c->dp_tasks, kDpTaskWords * 8, "DP tasks"))) break;
         if (dp_needs_scratch(rmax, cmax)) {
             if ((r = c->ensure(c->tb, size_t(c->dp_T) * size_t(rmax) * size_t(nst) * 2, "DP traceback scratch"))) break;
             if ((r = c->ensure(c->bnd, size_t(c->dp_T) * size_t(rmax + 1) * 3 * 4, "DP boundary scratch"))) break;
         }
-        launch_dp_sort(P_<DpSeg>(c->segs), ND, P_<uint32_t>(c->bins), P_<uint32_t>(c->perm),
-                       P_<uint64_t>(c->bin_off), c->scan_tmp.p, c->st);
         rec(3);
         if (cap) launch_stamp(P_<unsigned long long>(c->stamps) + 2 * c->batch_idx, c->st);
         DpLaunch a{P_<DpSeg>(c->segs), P_<uint32_t>(c->perm), ND, subj.code, subj.off, subj.len,
@@ -698,8 +772,11 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
                    c->p.affine, 1,  // reads with a non-ACGT base never reach the DP
                    0u, 0u, kStripsAll, 4, ctr + C_CELLS_PAIR};
         a.staged = ctr + C_STAGED;
-        apply_tuning(c, a);
-        launch_dp(a, P_<uint64_t>(c->bin_off), P_<uint64_t>(c->dp_tasks), cmax, c->st);
+        a.spack = subj.pack;
+        a.qpack = q.pack;
+        a.n_rest = ctr + C_REST;
+        if ((r = run_dp(c, a, cmax, DpBufs{c->bins, c->bin_off, c->perm, c->dp_tasks, c->w_key, c->w_order,
+                                           c->w_rest, c->w_bin, c->w_codes, c->scan_tmp}))) break;
         if ((r = c->check_launch("dp"))) break;
         rec(4);
         if (cap) launch_stamp(P_<unsigned long long>(c->stamps) + 2 * c->batch_idx + 1, c->st);
@@ -761,7 +838,7 @@ static int align_reads(hero_ctx *c, const ReadsView &all, uint64_t n, const uint
         c->batch_idx = size_t(b / B);
         // a batch is a window of the read arrays: shift the per-read pointers
         ReadsView v{all.code, all.off + b,  all.len + b, all.uid + b, all.good + b,
-                    nb,       all.job ? all.job + b : nullptr};
+                    nb,       all.job ? all.job + b : nullptr, all.pack};
         HERO_TRY(align_batch(c, v, nb, off_h[b + nb] - off_h[b], ms));
     }
     if (c->capturing) return HERO_OK;
@@ -785,7 +862,7 @@ extern "C" int hero_align_self(hero_ctx *c) {
     if (!c->have_index) return c->fail(HERO_E_STATE, "index not built");
     cudaSetDevice(c->dev);
     ReadsView v{P_<uint8_t>(c->q_code), P_<uint64_t>(c->q_off), P_<uint32_t>(c->q_len),
-                P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_sgood), c->nq, job_tags(c)};
+                P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_sgood), c->nq, job_tags(c), pack_words(c->q_pack)};
     return align_reads(c, v, c->nq, c->q_off_h.data());
 }
 
@@ -798,7 +875,7 @@ extern "C" int hero_align_self_range(hero_ctx *c, uint64_t first, uint64_t count
     const uint32_t *job = job_tags(c);
     ReadsView v{P_<uint8_t>(c->q_code), P_<uint64_t>(c->q_off) + first, P_<uint32_t>(c->q_len) + first,
                 P_<int64_t>(c->q_uid) + first, P_<uint8_t>(c->q_sgood) + first, count,
-                job ? job + first : nullptr};
+                job ? job + first : nullptr, pack_words(c->q_pack)};
     return align_reads(c, v, count, c->q_off_h.data() + first);
 }
 
@@ -908,7 +985,7 @@ extern "C" int hero_align_subjects(hero_ctx *c, const uint8_t *seq, const uint64
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, c->st);
-    HERO_TRY(upload_reads(c, seq, off, uid, n, c->s_raw, c->s_code, c->s_off, c->s_len, c->s_uid,
+    HERO_TRY(upload_reads(c, seq, off, uid, n, c->s_raw, c->s_code, c->s_pack, c->s_off, c->s_len, c->s_uid,
                           nullptr, &c->s_good, nullptr));
     cudaEventRecord(e1, c->st);
     HERO_TRY(c->cuda(cudaStreamSynchronize(c->st), "upload subjects"));
@@ -916,7 +993,7 @@ extern "C" int hero_align_subjects(hero_ctx *c, const uint8_t *seq, const uint64
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ReadsView v{P_<uint8_t>(c->s_code), P_<uint64_t>(c->s_off), P_<uint32_t>(c->s_len),
-                P_<int64_t>(c->s_uid), P_<uint8_t>(c->s_good), n};
+                P_<int64_t>(c->s_uid), P_<uint8_t>(c->s_good), n, nullptr, pack_words(c->s_pack)};
     return align_reads(c, v, n, off);
 }
 
@@ -999,7 +1076,7 @@ static int round_body(hero_ctx *c) {
         HERO_TRY(c->cuda(cudaMemsetAsync(c->q_ext.p, 0, c->nq * kOverhang * 16, c->st), "round: clear votes"));
     HERO_TRY(hero_build_index(c));
     ReadsView v{P_<uint8_t>(c->q_code), P_<uint64_t>(c->q_off), P_<uint32_t>(c->q_len),
-                P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_sgood), c->nq, job_tags(c)};
+                P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_sgood), c->nq, job_tags(c), pack_words(c->q_pack)};
     HERO_TRY(align_reads(c, v, c->nq, c->q_off_h.data()));
     return consensus_device(c);
 }
@@ -1253,20 +1330,20 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
     bool acgt = true;
     for (const auto &rd : {std::make_pair(subj, subj_off[n_subj]), std::make_pair(query, query_off[n_query])})
         for (uint64_t k = 0; k < rd.second && acgt; k++) acgt = base_code(rd.first[k]) < 4;
-    DBuf sraw, scode, soff, slen, suid, qraw, qcode, qoff, qlen, quid, dsegs, dsums, dops, dtb, dbnd,
-        doo, dout, dn, dperm, dbins, dbinoff, dtasks, dtmp;
+    DBuf sraw, scode, spack, soff, slen, suid, qraw, qcode, qpack, qoff, qlen, quid, dsegs, dsums, dops, dtb,
+        dbnd, doo, dout, dn, dperm, dbins, dbinoff, dtasks, dtmp, dkey, dorder, drest, dbin, dcodes;
     auto cleanup = [&]() {
         for (DBuf *b : {&sraw, &scode, &soff, &slen, &suid, &qraw, &qcode, &qoff, &qlen, &quid,
                         &dsegs, &dsums, &dops, &dtb, &dbnd, &doo, &dout, &dn, &dperm, &dbins,
-                        &dbinoff, &dtasks, &dtmp})
+                        &dbinoff, &dtasks, &dtmp, &spack, &qpack, &dkey, &dorder, &drest, &dbin, &dcodes})
             c->release(*b);
     };
     int r = HERO_OK;
     do {
-        if ((r = upload_reads(c, subj, subj_off, no_uid.data(), n_subj, sraw, scode, soff, slen, suid,
+        if ((r = upload_reads(c, subj, subj_off, no_uid.data(), n_subj, sraw, scode, spack, soff, slen, suid,
                               nullptr, nullptr, nullptr)))
             break;
-        if ((r = upload_reads(c, query, query_off, no_uid.data(), n_query, qraw, qcode, qoff, qlen,
+        if ((r = upload_reads(c, query, query_off, no_uid.data(), n_query, qraw, qcode, qpack, qoff, qlen,
                               quid, nullptr, nullptr, nullptr)))
             break;
         const int32_t nst = (cmax + kStripW - 1) / kStripW;
@@ -1278,23 +1355,24 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
             if ((r = c->ensure(dbnd, size_t(c->dp_T) * (rmax + 1) * 3 * 4, "scratch"))) break;
         }
         if ((r = c->ensure(dperm, n_seg * 4, "order"))) break;
-        if ((r = c->ensure(dbins, kDpBins * 4, "bins"))) break;
+        if ((r = c->ensure(dbins, (kDpBins + kBandBins) * 4, "bins"))) break;
         if ((r = c->ensure(dbinoff, (kDpBins + 1) * 8, "bins"))) break;
-        if ((r = c->ensure(dtasks, 128 * 8, "tasks"))) break;
+        if ((r = c->ensure(dtasks, (kDpTaskWords + 1) * 8, "tasks"))) break;
         if ((r = c->ensure(dtmp, scan_tmp_bytes(kDpBins + 1), "scan"))) break;
         if ((r = c->ensure(doo, (n_seg + 1) * 8, "ops"))) break;
         if ((r = c->ensure(dout, ops_off[n_seg], "ops"))) break;
         if ((r = c->ensure(dn, n_seg * 4, "ops"))) break;
         cudaMemcpyAsync(dsegs.p, h.data(), n_seg * sizeof(DpSeg), cudaMemcpyHostToDevice, c->st);
         cudaMemcpyAsync(doo.p, ops_off, (n_seg + 1) * 8, cudaMemcpyHostToDevice, c->st);
-        launch_dp_sort(P_<DpSeg>(dsegs), n_seg, P_<uint32_t>(dbins), P_<uint32_t>(dperm),
-                       P_<uint64_t>(dbinoff), dtmp.p, c->st);
         DpLaunch a{P_<DpSeg>(dsegs), P_<uint32_t>(dperm), n_seg, P_<uint8_t>(scode), P_<uint64_t>(soff),
                    P_<uint32_t>(slen), P_<uint8_t>(qcode), P_<uint64_t>(qoff), P_<uint32_t>(dops),
                    stride, P_<DpSum>(dsums), nullptr, P_<uint16_t>(dtb), P_<int32_t>(dbnd),
                    c->dp_T, rmax, affine ? 1 : 0, acgt ? 1 : 0, 0u, 0u, kStripsAll, 4};
-        apply_tuning(c, a);
-        launch_dp(a, P_<uint64_t>(dbinoff), P_<uint64_t>(dtasks), cmax, c->st);
+        a.spack = pack_words(spack);
+        a.qpack = pack_words(qpack);
+        a.n_rest = P_<unsigned long long>(dtasks) + kDpTaskWords;
+        if ((r = c->cuda(cudaMemsetAsync(a.n_rest, 0, 8, c->st), "tasks"))) break;
+        if ((r = run_dp(c, a, cmax, DpBufs{dbins, dbinoff, dperm, dtasks, dkey, dorder, drest, dbin, dcodes, dtmp}))) break;
         launch_unpack_ops(P_<uint32_t>(dops), stride, P_<DpSum>(dsums), n_seg, P_<uint64_t>(doo),
                           P_<uint8_t>(dout), P_<int32_t>(dn), c->st);
         if ((r = c->check_launch("align segments"))) break;

@@ -1,0 +1,351 @@
+// hero_band.cu -- kernels of the window DP (hero_band.cuh): which segments take
+// it, their order, the fill and traceback.  What it cannot certify goes to the
+// whole-matrix kernels of hero_kernels.cu.
+#include <cuda_runtime.h>
+
+#include "hero_band.cuh"
+#include "hero_internal.cuh"
+
+namespace hero {
+
+namespace {
+
+__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
+
+// segment as the window reads it; R and C of the longer and shorter side
+__device__ __forceinline__ BandSeg band_seg(const DpLaunch &a, const DpSeg &g, bool &reversed) {
+    const uint32_t orient = (g.flags >> kSegOrientShift) & 1u, qrc = (g.flags >> kSegQrcShift) & 1u;
+    const int64_t so = int64_t(a.soff[g.subj]), qo = int64_t(a.qoff[g.query]);
+    PackSeq s{a.spack, orient ? so + int64_t(a.slen[g.subj]) - 1 - g.s0 : so + g.s0, orient ? -1 : 1};
+    PackSeq q{a.qpack, qo + g.q0, 1};
+    if (qrc) q = PackSeq{a.qpack, int64_t(a.qoff[g.query + 1]) - 1 - g.q0, -1};
+    const int32_t ls = g.s1 - g.s0, lq = g.q1 - g.q0;
+    reversed = lq > ls;
+    BandSeg b;
+    b.row = reversed ? q : s;
+    b.col = reversed ? s : q;
+    b.R = reversed ? lq : ls;
+    b.C = reversed ? ls : lq;
+    b.base = 0;
+    b.m = g.band > b.R - b.C ? g.band : b.R - b.C;  // the aligner widens its band (BandAligner.cpp:59-62)
+    return b;
+}
+
+__device__ __forceinline__ int band_type(const DpSeg &g) {
+    return (g.flags & DPF_RIGHT) ? BT_RIGHT : ((g.flags & DPF_LEFT) ? BT_LEFT : BT_NONE);
+}
+
+// Window classes, widest first: 0..3 whole-band segments, 4..5 segments whose
+// band cuts the matrix.  A segment's mismatches on the main diagonal, e, bound
+// its deficit by 5 e, so few mismatches need only a narrow window (the limits
+// of 8, 16, 24 and 40 diagonals are 8, 13, 18 and 29 for the affine aligner, of
+// 8 and 16 diagonals 19 and 35 for the global one); from four on the cause is
+// mostly a gap, whose own deficit is small.
+template <bool AFFINE, int CLS>
+__host__ __device__ constexpr int band_width() {
+    return AFFINE ? (CLS == 0 ? 40 : CLS == 1 || CLS == 4 ? 24 : CLS == 2 || CLS == 5 ? 16 : 8)
+                  : (CLS == 0 || CLS == 4 || CLS == 5 ? 16 : 8);
+}
+__device__ __forceinline__ int band_class(bool affine, bool masked, int32_t e) {
+    if (masked) return affine && e > 2 ? 4 : 5;
+    if (affine) return e > 3 ? 0 : (e == 3 ? 1 : (e == 2 ? 2 : 3));
+    return e > 3 ? 0 : 3;
+}
+
+// appends the lanes with `on` to the whole-matrix list and counts their shape
+__device__ __forceinline__ void rest_append(const DpLaunch &a, bool on, uint32_t si, const DpSeg &g) {
+    const uint32_t m = __ballot_sync(0xffffffffu, on);
+    if (!m) return;
+    const uint32_t lane = lane_id(), leader = uint32_t(__ffs(int(m))) - 1u;
+    unsigned long long at = 0;
+    if (lane == leader) at = atomicAdd(a.n_rest, (unsigned long long)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, int(leader));
+    const uint32_t key = on ? shape_key(g) : 0xffffffffu;
+    const uint32_t same = __match_any_sync(0xffffffffu, key);
+    if (on) {
+        a.rest[at + __popc(m & ((1u << lane) - 1u))] = si;
+        if (lane == uint32_t(__ffs(int(same))) - 1u) atomicAdd(&a.bins[key], uint32_t(__popc(same)));
+    }
+}
+
+// One thread a segment: its reference cells; segments without a mismatch on
+// their main diagonal are done here (deficit 0: nothing can equal it), the
+// others are counted by window class, type and columns, or listed for the
+// whole-matrix kernels.  Bound by the scattered reads of the packed bases and
+// the op words written; it replaces the whole matrix for the third (150 bp,
+// affine) to half (100 bp) of the segments.
+__global__ void __launch_bounds__(256) k_band_screen(DpLaunch a, BandWork w) {
+    const uint32_t lane = lane_id();
+    for (uint64_t b0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b0 < a.nd;
+         b0 += uint64_t(gridDim.x) * blockDim.x) {
+        const uint64_t i = b0 + lane;
+        const bool has = i < a.nd;
+        DpSeg g{};
+        uint32_t key = kBandNoKey;
+        bool rest = false;
+        if (has) {
+            g = a.segs[i];
+            bool reversed;
+            BandSeg s = band_seg(a, g, reversed);
+            if (a.cells) {
+                const uint64_t cl = band_cells(s.R, s.C, s.m);
+                a.cells[i] = uint32_t(cl > 0xffffffffull ? 0xffffffffull : cl);
+            }
+            const int type = band_type(g);
+            const int32_t d = s.R - s.C;
+            const bool masked = s.m < s.R, affine = a.affine != 0;
+            // both ends anchored on different diagonals: the widest window must hold both
+            const int32_t most_d = affine ? (masked ? 12 : 24) : 8;
+            rest = !w.on || (g.flags & 3u) == 3u || s.C > kBandMaxC || (type == BT_NONE && d > most_d);
+            if (!rest) {
+                const int32_t e = type == BT_NONE && d > 0 ? 4 : main_mismatches(s.row, s.col, main_row(type, s.R, s.C), s.C, 4);
+                if (e == 0) {
+                    DpSum sum;
+                    straight_ops(s.row, s.col, type, s.R, s.C, reversed ? uint32_t(OP_I) : uint32_t(OP_D),
+                                 a.ops + i * a.stride, a.stride, sum);
+                    a.sums[i] = sum;
+                } else {
+                    key = (uint32_t(band_class(affine, masked, e) * 3 + type) << kBandColBits) | uint32_t(kBandMaxC - s.C);
+                }
+            }
+        }
+        if (has && w.on) w.key[i] = key;
+        const uint32_t same = __match_any_sync(0xffffffffu, key);
+        if (key != kBandNoKey && lane == uint32_t(__ffs(int(same))) - 1u) atomicAdd(&w.count[key], uint32_t(__popc(same)));
+        rest_append(a, rest, uint32_t(i), g);
+    }
+}
+
+// One block: first position and first task (64 segments) of every non-empty
+// bin, in key order -- the widest windows and longest segments first.
+constexpr int kTaskSegs = 64;
+__global__ void __launch_bounds__(1024) k_band_tasks(BandWork w) {
+    __shared__ uint32_t tot[32][3];
+    constexpr int per = (kBandBins + 1023) / 1024;
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+    uint32_t n = 0, t = 0, b = 0;  // segments, tasks, bins of this thread's keys
+    for (int k = 0; k < per; k++) {
+        const uint32_t key = threadIdx.x * per + k;
+        const uint32_t c = key < kBandBins ? w.count[key] : 0u;
+        n += c;
+        t += (c + kTaskSegs - 1) / kTaskSegs;
+        b += c != 0u;
+    }
+    uint32_t v[3] = {n, t, b}, ex[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        uint32_t x = v[q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (int(lane) >= o) x += y;
+        }
+        ex[q] = x - v[q];
+        if (lane == 31) tot[wid][q] = x;
+    }
+    __syncthreads();
+    uint32_t all[3] = {0, 0, 0};
+    for (int k = 0; k < 32; k++)
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            if (k < int(wid)) ex[q] += tot[k][q];
+            all[q] += tot[k][q];
+        }
+    for (int k = 0; k < per; k++) {
+        const uint32_t key = threadIdx.x * per + k;
+        const uint32_t c = key < kBandBins ? w.count[key] : 0u;
+        if (!c) continue;
+        w.cursor[key] = ex[0];
+        w.bin[ex[2]] = BandBin{key, ex[1], ex[0], c};
+        ex[0] += c;
+        ex[1] += (c + kTaskSegs - 1) / kTaskSegs;
+        ex[2]++;
+    }
+    if (threadIdx.x == 0) {
+        w.head[0] = all[2];  // bins
+        w.head[1] = all[1];  // tasks
+        w.head[2] = 0;       // next task
+    }
+}
+
+__global__ void __launch_bounds__(256) k_band_scatter(uint64_t nd, BandWork w) {
+    const uint32_t lane = lane_id();
+    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < nd;
+         b += uint64_t(gridDim.x) * blockDim.x) {
+        const uint64_t i = b + lane;
+        const uint32_t key = i < nd ? w.key[i] : kBandNoKey;
+        const uint32_t same = __match_any_sync(0xffffffffu, key);
+        const uint32_t leader = uint32_t(__ffs(int(same))) - 1u;
+        uint32_t at = 0;
+        if (key != kBandNoKey && lane == leader) at = atomicAdd(&w.cursor[key], uint32_t(__popc(same)));
+        at = __shfl_sync(0xffffffffu, at, int(leader));
+        if (key != kBandNoKey) w.order[at + __popc(same & ((1u << lane) - 1u))] = uint32_t(i);
+    }
+}
+
+// a warp's traceback codes in global memory: word k of column j, 32 lanes wide
+template <int WORDS>
+struct WarpStore {
+    uint32_t *base, *p;
+    __device__ __forceinline__ void column(int32_t j) { p = base + size_t(j - 1) * (WORDS * 32); }
+    __device__ __forceinline__ void put(int k, uint32_t bits) { p[k * 32] = bits; }
+};
+template <int WORDS>
+struct WarpCodes {
+    const uint32_t *base;  // + lane of the segment
+    uint32_t shift;        // 16 for the high halves
+    __device__ __forceinline__ uint32_t get(int32_t j, int32_t k) const {
+        return (base[(size_t(j - 1) * WORDS + k) * 32] >> shift) & 0xffffu;
+    }
+};
+
+// One task: up to 64 segments of one class, type and column count, two a lane
+// (positions lane and lane + 32).  Registers hold the window (M and IY of every
+// diagonal, the row selectors), so a cell costs six ALU instructions and a
+// column touches memory only for its code words.
+template <bool AFFINE, int NB, int TYPE, bool MASK>
+__device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order, uint32_t n, int32_t C,
+                                       uint32_t *codes) {
+    constexpr int WORDS = (NB + 7) / 8;
+    const uint32_t lane = lane_id();
+    BandSeg s[2];
+    uint32_t si[2];
+    bool rev[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t k = lane + 32u * h;
+        si[h] = order[k < n ? k : 0u];
+        s[h] = band_seg(a, a.segs[si[h]], rev[h]);
+        s[h].base = band_base<AFFINE, NB, TYPE>(s[h].R - s[h].C);
+    }
+    int32_t jp = -s[0].base > -s[1].base ? -s[0].base : -s[1].base;
+    jp = __reduce_max_sync(0xffffffffu, jp);
+    WarpStore<WORDS> st{codes + lane, codes + lane};
+    BandEnd e[2];
+    band_fill<AFFINE, NB, TYPE, MASK>(s[0], s[1], C, jp, st, e[0], e[1]);
+    uint32_t walk[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const bool has = lane + 32u * h < n;
+        const bool sure = has && C - e[h].v <= band_limit<AFFINE, NB, TYPE>(s[h]);
+        if (sure && e[h].straight) {
+            DpSum sum;
+            straight_ops(s[h].row, s[h].col, TYPE, s[h].R, C, rev[h] ? uint32_t(OP_I) : uint32_t(OP_D),
+                         a.ops + uint64_t(si[h]) * a.stride, a.stride, sum);
+            a.sums[si[h]] = sum;
+        }
+        walk[h] = __ballot_sync(0xffffffffu, sure && !e[h].straight);
+        rest_append(a, has && !sure, si[h], a.segs[si[h]]);
+    }
+    __syncwarp();  // the codes of every lane are written
+    // the paths with gaps, one a lane: lane l traces the l-th of them
+    const uint32_t nw0 = __popc(walk[0]), nw = nw0 + __popc(walk[1]);
+    for (uint32_t r = lane; r < nw; r += 32u) {
+        const int h = r >= nw0;
+        const uint32_t at = __fns(h ? walk[1] : walk[0], 0, int(r - (h ? nw0 : 0u)) + 1);
+        const uint32_t sj = order[at + 32u * h];
+        bool reversed;
+        const DpSeg g = a.segs[sj];
+        BandSeg t = band_seg(a, g, reversed);
+        t.base = band_base<AFFINE, NB, TYPE>(t.R - t.C);
+        OpsPut put{a.ops + uint64_t(sj) * a.stride, int32_t(a.stride * 16u)};
+        DpSum sum;
+        band_walk<AFFINE, NB, TYPE>(t, WarpCodes<WORDS>{codes + at, h ? 16u : 0u},
+                                    reversed ? uint32_t(OP_I) : uint32_t(OP_D),
+                                    reversed ? uint32_t(OP_D) : uint32_t(OP_I), put);
+        put.finish(sum);
+        a.sums[sj] = sum;
+    }
+    __syncwarp();
+}
+
+template <bool AFFINE, int CLS>
+__device__ __forceinline__ void band_dispatch(int type, const DpLaunch &a, const uint32_t *order, uint32_t n,
+                                              int32_t C, uint32_t *codes) {
+    constexpr int NB = band_width<AFFINE, CLS>();
+    constexpr bool MASK = CLS >= 4;
+    if (type == BT_RIGHT) {
+        band_task<AFFINE, NB, BT_RIGHT, MASK>(a, order, n, C, codes);
+    } else if (type == BT_LEFT) {
+        band_task<AFFINE, NB, BT_LEFT, MASK>(a, order, n, C, codes);
+    } else {
+        band_task<AFFINE, NB, BT_NONE, MASK>(a, order, n, C, codes);
+    }
+}
+
+// Persistent warps fed by a queue of tasks.  Measured, DP stage of one
+// correction before (every matrix whole) and with the window: 5 Mbp affine,
+// 1.67 M x 150 bp, 109 M segments, 358 -> 78 ms; 1 Mbp global, 300 k x 100 bp,
+// 7.3 -> 2.5 ms; 300 kbp affine with -i 2 (bands of a few diagonals), 80 k x
+// 150 bp, 34.5 -> 3.0 ms.
+constexpr int kBandWarps = 4, kBandBlocks = 3;  // 12 warps an SM: 168 registers hold the widest window
+
+template <bool AFFINE>
+__global__ void __launch_bounds__(kBandWarps * 32, kBandBlocks) k_band(DpLaunch a, BandWork w) {
+    const uint32_t lane = lane_id();
+    uint32_t *codes = w.codes + size_t(blockIdx.x * kBandWarps + (threadIdx.x >> 5)) * w.code_words;
+    const uint32_t nbin = w.head[0], ntask = w.head[1];
+    for (;;) {
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(&w.head[2], 1u);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= ntask) break;
+        uint32_t lo = 0, hi = nbin;  // the last bin whose first task is at most q
+        while (hi - lo > 1u) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (w.bin[mid].task <= q) lo = mid; else hi = mid;
+        }
+        const BandBin b = w.bin[lo];
+        const uint32_t first = (q - b.task) * kTaskSegs;
+        const uint32_t n = b.count - first < kTaskSegs ? b.count - first : kTaskSegs;
+        const uint32_t *order = w.order + b.first + first;
+        const int32_t C = kBandMaxC - int32_t(b.key & ((1u << kBandColBits) - 1u));
+        const uint32_t ct = b.key >> kBandColBits;
+        const int type = int(ct % 3u);
+        switch (ct / 3u) {
+            case 0: band_dispatch<AFFINE, 0>(type, a, order, n, C, codes); break;
+            case 1: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 1 : 0>(type, a, order, n, C, codes); break;
+            case 2: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 2 : 0>(type, a, order, n, C, codes); break;
+            case 3: band_dispatch<AFFINE, 3>(type, a, order, n, C, codes); break;
+            case 4: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 4 : 5>(type, a, order, n, C, codes); break;
+            default: band_dispatch<AFFINE, 5>(type, a, order, n, C, codes); break;
+        }
+    }
+}
+
+}  // namespace
+
+uint64_t band_warps(int device, uint64_t nd) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const uint64_t full = uint64_t(sms) * kBandBlocks;
+    const uint64_t need = (nd + kBandWarps - 1) / kBandWarps;  // a task holds one segment at least
+    return kBandWarps * (need < full ? (need ? need : 1) : full);
+}
+
+uint32_t band_code_words(int32_t cmax, bool affine) {
+    const uint32_t c = uint32_t(cmax < kBandMaxC ? cmax : kBandMaxC);
+    return c * 32u * (affine ? 5u : 2u);
+}
+
+void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
+    if (!a.nd) return;
+    const uint64_t g = (a.nd + 255) / 256;
+    const unsigned grid = unsigned(g < 148u * 64u ? g : 148u * 64u);
+    count_launch();
+    k_band_screen<<<grid, 256, 0, st>>>(a, w);
+    if (!w.on) return;
+    count_launch();
+    k_band_tasks<<<1, 1024, 0, st>>>(w);
+    count_launch();
+    k_band_scatter<<<grid, 256, 0, st>>>(a.nd, w);
+    count_launch();
+    const unsigned blocks = unsigned(w.warps / kBandWarps);
+    if (a.affine) {
+        k_band<true><<<blocks, kBandWarps * 32, 0, st>>>(a, w);
+    } else {
+        k_band<false><<<blocks, kBandWarps * 32, 0, st>>>(a, w);
+    }
+}
+
+}  // namespace hero

@@ -1,0 +1,520 @@
+// hero_band.cuh -- banded DP of a segment inside a window of diagonals, with a
+// certificate that the window's path is the whole matrix's path.
+//
+// Segments join two reads at a shared k-mer, so the true path almost always
+// runs a few diagonals from the main one.  The window DP computes NB adjacent
+// diagonals only.  Let a path's deficit at column j be j minus its score: a
+// match adds nothing, a mismatch 5, a base skipped on the columns 5 (2 in an
+// extension), one skipped on the rows 4 (1 in an extension; none in column 0
+// of an align-right or column C of an align-left segment).  Deficits never
+// fall along a path, and never rise along the traceback (every move leads to a
+// cell whose best deficit is no larger), so every cell of the traceback has at
+// most the deficit D of the end cell.  A path that leaves the window pays for
+// the diagonals it crosses; band_limit() gives the largest D that is below
+// every such path's deficit at every cell the traceback can visit.  If the
+// window's own D is within the limit, no path outside the window can equal or
+// beat the values the traceback reads, so the moves -- ties included -- are the
+// whole matrix's.  Segments that miss the limit are computed in full.
+//
+// Two segments run in the 16-bit halves of each register, as dp_pair_row does.
+// Values are 4 (v + potential) + tag (tags as in dp_pair_row).  The potential
+// grows with the row and the column so that a gap extension costs nothing:
+// each of the two gap states is then one add-max a cell.
+#pragma once
+#include "hero_core.cuh"
+
+namespace hero {
+
+enum : int { BT_NONE = 0, BT_RIGHT = 1, BT_LEFT = 2 };  // anchored at both ends, at the end, at the start
+
+constexpr int32_t kBandMaxC = 1023;   // columns of a window segment: 16-bit values hold 4 * 5 * C
+constexpr int kBandStep = 4;          // columns an unrolled block computes
+constexpr int32_t kBandDead = -12000; // outside the matrix or the aligner's band: 3000 below any value
+                                      // the certificate accepts, at every column
+constexpr int kPackPad = 8;           // words (128 bases) before and after packed reads that fetches may touch
+
+// ---------------------------------------------------------------------------
+// packed reads: 2 bits a base, base g of the read array at bits 2 (g % 16) of
+// word g / 16
+// ---------------------------------------------------------------------------
+struct PackSeq {          // a stretch of a read, oriented: base t is at + dir * t, complemented when dir < 0
+    const uint32_t *w;
+    int64_t at;
+    int32_t dir;
+};
+
+HERO_HD uint32_t reverse_fields(uint32_t x) {  // the sixteen 2-bit fields in reverse order
+#if defined(__CUDA_ARCH__)
+    x = __brev(x);
+    return ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
+#else
+    uint32_t r = 0;
+    for (int i = 0; i < 16; i++) r |= ((x >> (2 * i)) & 3u) << (2 * (15 - i));
+    return r;
+#endif
+}
+
+// bases t .. t + 15, base t in the lowest bits
+HERO_HD uint32_t pack16(const PackSeq &s, int32_t t) {
+    const int64_t p = s.dir > 0 ? s.at + t : s.at - t - 15;
+    const int64_t k = p >> 4;
+    const uint32_t sh = uint32_t(p & 15) * 2u;
+    const uint32_t lo = s.w[k], hi = s.w[k + 1];
+#if defined(__CUDA_ARCH__)
+    const uint32_t x = __funnelshift_r(lo, hi, sh);
+#else
+    const uint32_t x = uint32_t(((uint64_t(hi) << 32) | lo) >> sh);
+#endif
+    return s.dir > 0 ? x : reverse_fields(x) ^ 0xaaaaaaaau;
+}
+
+// 01 in every field where two packed words differ: OP_X there, OP_M elsewhere
+HERO_HD uint32_t mismatch16(uint32_t a, uint32_t b) {
+    const uint32_t x = a ^ b;
+    return (x | (x >> 1)) & 0x55555555u;
+}
+
+struct BandSeg {  // a segment as the window DP reads it (rows = longer side)
+    PackSeq row, col;
+    int32_t R, C;
+    int32_t base;   // offset (row - column) of the window's first diagonal
+    int32_t m;      // the aligner's band: cells with |row - column| > m do not exist
+};
+
+// window shape: the side on which leaving costs less a diagonal is the longer
+template <bool AFFINE, int NB>
+struct BandWin {
+    static constexpr int near = AFFINE ? (NB - 1) / 3 : (NB - 1) / 2;
+    static constexpr int far = NB - 1 - near;
+};
+// window position of the main diagonal (the one the anchored end lies on; both
+// ends of a BT_NONE segment of equal sides)
+template <bool AFFINE, int NB, int TYPE>
+HERO_HD constexpr int band_main() {
+    return TYPE == BT_RIGHT ? BandWin<AFFINE, NB>::far : TYPE == BT_LEFT ? BandWin<AFFINE, NB>::near : (NB - 1) / 2;
+}
+template <bool AFFINE, int NB, int TYPE>
+HERO_HD int32_t band_base(int32_t d) {
+    return TYPE == BT_RIGHT ? d - BandWin<AFFINE, NB>::far
+         : TYPE == BT_LEFT ? -BandWin<AFFINE, NB>::near : -((NB - 1 - d) / 2);
+}
+
+// The largest end deficit at which no path through cells outside the window
+// [base, base + NB) can match the values of the traceback.  Below the window a
+// path has skipped columns (and must skip rows to return), or, aligned right,
+// started on an earlier row of column 0 (and must skip rows to reach the end's
+// diagonal); above it the reverse.  The affine column 0 and row 0 let a gap
+// turn without a second opening cost, so only one opening is counted.  An
+// align-left path may also reach column C outside the window: above it the
+// moves there are still up while its deficit is no smaller than D (a tie goes
+// up for the affine aligner, not for the global one), below it the free climb
+// would carry its score to the cells of the traceback.  The limits are the
+// deficits of those paths, less one where a tie would change a move.
+template <bool AFFINE, int NB, int TYPE>
+HERO_HD int32_t band_limit(const BandSeg &s) {
+    constexpr int32_t kNone = 1 << 20;
+    const int32_t d = s.R - s.C, lo = s.base, hi = s.base + NB - 1;
+    const int32_t v1 = AFFINE ? 1 : 4, h1 = AFFINE ? 2 : 5, open = AFFINE ? 3 : 0;
+    int32_t below = kNone, above = kNone;
+    if (lo > -s.m && lo > -s.C) {
+        const int32_t h = lo > 0 ? 0 : 1 - lo;  // columns skipped to get below the window
+        if (TYPE == BT_RIGHT) below = open + h * h1 + (d - lo + 1) * v1 - 1;
+        if (TYPE == BT_LEFT) below = open + h * h1 - 1;
+        if (TYPE == BT_NONE) below = open + h * h1 + (h + d) * v1 - 1;
+    }
+    if (hi < s.m && hi < s.R) {
+        if (TYPE == BT_RIGHT) above = open + (hi - d + 1) * h1 - 1;
+        if (TYPE == BT_LEFT) above = open + (hi + 1) * v1 + (hi < d ? (AFFINE ? 0 : -1) : h1 - 1);
+        if (TYPE == BT_NONE) above = open + (hi + 1) * v1 + (hi + 1 - d) * h1 - 1;
+    }
+    return below < above ? below : above;
+}
+
+// byte select with sign replication, as PRMT: nibble n of sel picks byte n & 7
+// of {a, b}, or its sign byte when bit 3 is set
+HERO_HD uint32_t byte_sel(uint32_t a, uint32_t b, uint32_t sel) {
+#if defined(__CUDA_ARCH__)
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+#else
+    const uint64_t ab = (uint64_t(b) << 32) | a;
+    uint32_t r = 0;
+    for (int i = 0; i < 4; i++) {
+        const uint32_t n = (sel >> (4 * i)) & 15u;
+        uint32_t v = uint32_t(ab >> (8 * (n & 7u))) & 0xffu;
+        if (n & 8u) v = (v & 0x80u) ? 0xffu : 0u;
+        r |= v << (8 * i);
+    }
+    return r;
+#endif
+}
+
+HERO_HD uint32_t min_2(uint32_t a, uint32_t b) {  // per half, signed
+#if defined(__CUDA_ARCH__)
+    return __vmins2(a, b);
+#else
+    const int32_t l = half_lo(a) < half_lo(b) ? half_lo(a) : half_lo(b);
+    const int32_t h = half_hi(a) < half_hi(b) ? half_hi(a) : half_hi(b);
+    return pack2(l, h);
+#endif
+}
+
+HERO_HD constexpr uint32_t band_half2(int32_t v) { return (uint32_t(v) & 0xffffu) * 0x10001u; }
+
+// the costs in window values
+template <bool AFFINE>
+struct BandCost {
+    using T = PairTags<AFFINE>;
+    static constexpr int32_t pot = AFFINE ? 1 : 2;  // potential a row and a column
+    static constexpr int32_t match = 4 * (kHIT + 2 * pot) + T::diag, miss = 4 * (kMISS + 2 * pot) + T::diag;
+    // score bytes by the column's base: `miss` everywhere, `match` at byte `code`
+    static constexpr uint32_t table = (uint32_t(miss) & 0xffu) * 0x01010101u;
+    static constexpr uint32_t flip = (uint32_t(miss) ^ uint32_t(match)) & 0xffu;
+    static constexpr uint32_t down = band_half2(AFFINE ? 4 * (kDX + pot) + T::up - T::diag : 4 * (kDX + pot) + T::up);
+    static constexpr uint32_t right = band_half2(AFFINE ? 4 * (kDY + pot) + T::left - T::diag : 4 * (kDY + pot) + T::left);
+    // column C of an align-left segment: rows there cost sx = 0
+    static constexpr uint32_t free_open = band_half2(AFFINE ? 4 * (kSX + pot) + T::up - T::diag : 4 * (kSX + pot) + T::up);
+    static constexpr uint32_t free_more = band_half2(4 * (kSX + pot));
+};
+
+struct BandEnd {
+    int32_t v;      // score at (R, C)
+    bool straight;  // the path is the main diagonal (and the free run of an anchored segment)
+};
+
+// selector of a row's two bases for byte_sel on the column's two score tables:
+// the low half takes segment A's score byte, sign-extended, the high half B's
+HERO_HD uint32_t band_sel(uint32_t a, uint32_t b) { return a * 0x11u + b * 0x1100u + 0xc480u; }
+
+template <bool AFFINE>
+HERO_HD uint32_t band_table(uint32_t code) { return BandCost<AFFINE>::table ^ (BandCost<AFFINE>::flip << (8u * code)); }
+
+// M of column 0 at row i, and IY of (i, 1) (affine), as plain scores
+template <bool AFFINE, int TYPE>
+HERO_HD int32_t band_col0(int32_t i) {
+    if (i == 0 || TYPE == BT_RIGHT) return 0;
+    return AFFINE ? kDX - kEX + i * kEX : i * kDX;
+}
+template <int TYPE>
+HERO_HD int32_t band_col0_right(int32_t i) {
+    return (i == 0 || TYPE == BT_RIGHT) ? kDY : kDX - kEX + (i + 1) * kEX;
+}
+
+// One column of the window.  M: clean M of the column before, then of this one
+// (global: F); L (affine): IY of this column's cell one diagonal below, then of
+// the next column's.  sel[c]: the selector of cell c's row.  INJECT (affine):
+// z{a,b} is the window position of row 0, whose IX equals its IY.  Codes (two
+// bits a cell, eight cells a word) go to st.put(word, bits); the tags of the
+// main diagonal are and-ed into `straight`.
+template <bool AFFINE, int NB, int TYPE, bool MASK, bool INJECT, class Store>
+HERO_HD void band_column(uint32_t (&M)[NB], uint32_t (&L)[AFFINE ? NB : 1], const uint32_t (&P)[MASK ? NB : 1],
+                         const uint32_t *sel, uint32_t ta, uint32_t tb, int32_t za, int32_t zb,
+                         uint32_t &straight, Store &st) {
+    using K = BandCost<AFFINE>;
+    constexpr int main_c = band_main<AFFINE, NB, TYPE>();
+    const uint32_t dead = band_half2(kBandDead);
+    uint32_t x = dead, acc = 0;  // IX of the cell (affine), M of the cell above (global)
+#pragma unroll
+    for (int c = 0; c < NB; c++) {
+        const uint32_t f = add2(M[c], byte_sel(ta, tb, sel[c]));
+        uint32_t y = c + 1 < NB ? (AFFINE ? L[c + 1 < NB && AFFINE ? c + 1 : 0] : M[c + 1 < NB ? c + 1 : 0]) : dead;
+        uint32_t mt;
+        if (AFFINE) {
+            if (MASK) {
+                y = min_2(y, P[MASK ? c : 0]);
+                x = min_2(x, P[MASK ? c : 0]);
+            }
+            if (INJECT) {
+                const uint32_t on = (za == c ? 0xffffu : 0u) | (zb == c ? 0xffff0000u : 0u);
+                x = (x & ~on) | ((y + 0x00020002u) & on);
+            }
+            mt = max3_2(f, x, y);
+            L[AFFINE ? c : 0] = add_max2(f, K::right, y);
+            x = add_max2(f, K::down, x);
+        } else {
+            if (MASK) {
+                y = min_2(y, P[MASK ? c : 0]);
+                x = min_2(x, P[MASK ? c : 0]);
+            }
+            mt = add_max2(y, K::right, add_max2(x, K::down, f));
+        }
+        const uint32_t tg = mt & kTagMask2;
+        M[c] = mt & ~kTagMask2;
+        if (!AFFINE) x = M[c];
+        if (c == main_c) straight &= tg;
+        acc += tg << (2 * (c & 7));
+        if ((c & 7) == 7 || c == NB - 1) {
+            st.put(c >> 3, acc);
+            acc = 0;
+        }
+    }
+}
+
+// The window of two segments of the same type and columns (C).  jp: columns in
+// which any segment of the warp has row 0 in its window (affine).  Store:
+// column(j) before each column's puts.
+template <bool AFFINE, int NB, int TYPE, bool MASK, class Store>
+HERO_HD void band_fill(const BandSeg &a, const BandSeg &b, int32_t C, int32_t jp, Store &st, BandEnd &ea,
+                       BandEnd &eb) {
+    using K = BandCost<AFFINE>;
+    using T = PairTags<AFFINE>;
+    constexpr int main_c = band_main<AFFINE, NB, TYPE>();
+    uint32_t M[NB], L[AFFINE ? NB : 1], P[MASK ? NB : 1], sel[NB - 1 + kBandStep];
+    // column 0
+#pragma unroll
+    for (int c = 0; c < NB; c++) {
+        const int32_t ia = a.base + c, ib = b.base + c;
+        const bool oka = ia >= 0 && (!MASK || ia <= a.m), okb = ib >= 0 && (!MASK || ib <= b.m);
+        M[c] = pack2(oka ? 4 * (band_col0<AFFINE, TYPE>(ia) + K::pot * c) : kBandDead,
+                     okb ? 4 * (band_col0<AFFINE, TYPE>(ib) + K::pot * c) : kBandDead);
+        if (AFFINE)
+            L[AFFINE ? c : 0] = pack2(oka ? 4 * (band_col0_right<TYPE>(ia) + c + 1) : kBandDead,
+                                      okb ? 4 * (band_col0_right<TYPE>(ib) + c + 1) : kBandDead);
+        if (MASK)
+            P[MASK ? c : 0] = pack2(ia >= -a.m && ia <= a.m ? 0x7fff : kBandDead,
+                                    ib >= -b.m && ib <= b.m ? 0x7fff : kBandDead);
+    }
+    // selectors of rows 1 + base .. base + NB - 1 (the last NB-th row joins with each column)
+#pragma unroll
+    for (int c0 = 0; c0 < NB - 1; c0 += 16) {
+        const uint32_t wa = pack16(a.row, a.base + c0), wb = pack16(b.row, b.base + c0);
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+            if (c0 + c < NB - 1) sel[c0 + c] = band_sel((wa >> (2 * c)) & 3u, (wb >> (2 * c)) & 3u);
+    }
+    uint32_t ra = 0, rb = 0, ca = 0, cb = 0, straight = 0xffffffffu;
+    const int32_t last = TYPE == BT_LEFT ? C - 1 : C;  // column C of an align-left segment follows the loop
+#pragma unroll 1
+    for (int32_t j0 = 1; j0 <= last; j0 += kBandStep) {
+        if (((j0 - 1) & 15) == 0) {  // sixteen more rows and columns
+            ra = pack16(a.row, a.base + NB - 2 + j0);
+            rb = pack16(b.row, b.base + NB - 2 + j0);
+            ca = pack16(a.col, j0 - 1);
+            cb = pack16(b.col, j0 - 1);
+        }
+#pragma unroll
+        for (int u = 0; u < kBandStep; u++) {
+            sel[NB - 1 + u] = band_sel(ra & 3u, rb & 3u);
+            ra >>= 2;
+            rb >>= 2;
+        }
+        if (AFFINE && j0 <= jp) {
+#pragma unroll
+            for (int u = 0; u < kBandStep; u++) {
+                const int32_t j = j0 + u;
+                if (j <= last) {
+                    st.column(j);
+                    band_column<AFFINE, NB, TYPE, MASK, true>(M, L, P, sel + u, band_table<AFFINE>(ca & 3u),
+                                                              band_table<AFFINE>(cb & 3u), -a.base - j,
+                                                              -b.base - j, straight, st);
+                }
+                ca >>= 2;
+                cb >>= 2;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kBandStep; u++) {
+                const int32_t j = j0 + u;
+                if (j <= last) {
+                    st.column(j);
+                    band_column<AFFINE, NB, TYPE, MASK, false>(M, L, P, sel + u, band_table<AFFINE>(ca & 3u),
+                                                               band_table<AFFINE>(cb & 3u), 0, 0, straight, st);
+                }
+                ca >>= 2;
+                cb >>= 2;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NB - 1; c++) sel[c] = sel[c + kBandStep];
+    }
+    const int32_t da = a.R - a.C, db = b.R - b.C;
+    if (TYPE != BT_LEFT) {
+        const int32_t cea = TYPE == BT_RIGHT ? main_c : da - a.base, ceb = TYPE == BT_RIGHT ? main_c : db - b.base;
+        int32_t va = 0, vb = 0;
+#pragma unroll
+        for (int c = 0; c < NB; c++) {
+            if (c == cea) va = (half_lo(M[c]) >> 2) - K::pot * (2 * C + c);
+            if (c == ceb) vb = (half_hi(M[c]) >> 2) - K::pot * (2 * C + c);
+        }
+        const bool eqa = TYPE == BT_RIGHT || (da == 0 && cea == main_c), eqb = TYPE == BT_RIGHT || (db == 0 && ceb == main_c);
+        ea = BandEnd{va, eqa && (straight & uint32_t(T::diag)) != 0u};
+        eb = BandEnd{vb, eqb && (straight & (uint32_t(T::diag) << 16)) != 0u};
+        return;
+    }
+    // column C of align-left segments: rows cost nothing there
+    st.column(C);
+    const uint32_t ta = band_table<AFFINE>(pack16(a.col, C - 1) & 3u), tb = band_table<AFFINE>(pack16(b.col, C - 1) & 3u);
+    const uint32_t dead = band_half2(kBandDead);
+    const int32_t cea = main_c + da < NB - 1 ? main_c + da : NB - 1, ceb = main_c + db < NB - 1 ? main_c + db : NB - 1;
+    uint32_t x = dead, acc = 0, wa = 0, wb = 0;
+    int32_t va = 0, vb = 0;
+    bool sa = (straight & uint32_t(T::diag)) != 0u, sb = (straight & (uint32_t(T::diag) << 16)) != 0u;
+#pragma unroll
+    for (int c = 0; c < NB; c++) {
+        if ((c & 15) == 0) {
+            wa = pack16(a.row, C - 1 + a.base + c);
+            wb = pack16(b.row, C - 1 + b.base + c);
+        }
+        const uint32_t f = add2(M[c], byte_sel(ta, tb, band_sel(wa & 3u, wb & 3u)));
+        wa >>= 2;
+        wb >>= 2;
+        uint32_t y = c + 1 < NB ? (AFFINE ? L[c + 1 < NB && AFFINE ? c + 1 : 0] : M[c + 1 < NB ? c + 1 : 0]) : dead;
+        if (MASK) {
+            y = min_2(y, P[MASK ? c : 0]);
+            x = min_2(x, P[MASK ? c : 0]);
+        }
+        uint32_t mt, fx;  // fx: the states a further row's free move reads
+        if (AFFINE) {
+            const uint32_t on = (C + a.base + c == 0 ? 0xffffu : 0u) | (C + b.base + c == 0 ? 0xffff0000u : 0u);
+            x = (x & ~on) | ((y + 0x00020002u) & on);
+            mt = max3_2(f, x, y);
+            fx = max3_2(f, x, x);
+            x = add_max2(f, K::free_open, add2(x, K::free_more));
+        } else {
+            mt = add_max2(y, K::right, add_max2(x, c == 0 ? K::down : K::free_open, f));
+            fx = mt;
+            x = mt & ~kTagMask2;
+        }
+        const uint32_t tg = mt & kTagMask2;
+        const int32_t p = K::pot * (2 * C + c);
+        if (c == cea) va = (half_lo(c == NB - 1 && main_c + da > c ? fx : mt) >> 2) - p;
+        if (c == ceb) vb = (half_hi(c == NB - 1 && main_c + db > c ? fx : mt) >> 2) - p;
+        if (c == main_c) {
+            sa = sa && (tg & 3u) == uint32_t(T::diag);
+            sb = sb && (tg >> 16) == uint32_t(T::diag);
+        } else if (c > main_c) {
+            sa = sa && (c > cea || (tg & 3u) == uint32_t(T::up));
+            sb = sb && (c > ceb || (tg >> 16) == uint32_t(T::up));
+        }
+        acc += tg << (2 * (c & 7));
+        if ((c & 7) == 7 || c == NB - 1) {
+            st.put(c >> 3, acc);
+            acc = 0;
+        }
+    }
+    ea = BandEnd{va, sa};
+    eb = BandEnd{vb, sb};
+}
+
+// Packed ops written last to first at descending positions, with the run
+// tracking a DpSum needs (the first run put is the path's last).
+struct OpsPut {
+    uint32_t *w;
+    int32_t p;          // position of the op put last
+    uint32_t acc = 0;
+    uint32_t cur = 4u, cnt = 0, lt = 0, lc = 0, n = 0, tot[4] = {0, 0, 0, 0};
+    bool more = false;  // two or more runs
+
+    HERO_HD void put(uint32_t op, uint32_t k) {
+        if (k == 0) return;
+        n += k;
+        tot[0] += op == 0u ? k : 0u;
+        tot[1] += op == 1u ? k : 0u;
+        tot[2] += op == 2u ? k : 0u;
+        tot[3] += op == 3u ? k : 0u;
+        if (op == cur) {
+            cnt += k;
+        } else {
+            if (cur != 4u && !more) {
+                lt = cur;
+                lc = cnt;
+                more = true;
+            }
+            cur = op;
+            cnt = k;
+        }
+        while (k > 0) {  // fields of one word at a time
+            const uint32_t room = uint32_t((p - 1) & 15) + 1u, take = k < room ? k : room;
+            const uint32_t lo = room - take;
+            acc |= op * ops_mask(lo, room - 1u);
+            p -= int32_t(take);
+            k -= take;
+            if ((p & 15) == 0) {
+                w[p >> 4] = acc;
+                acc = 0;
+            }
+        }
+    }
+    HERO_HD void finish(DpSum &s) {
+        if (p & 15) w[p >> 4] = acc;
+        for (int i = 0; i < 4; i++) s.tot[i] = uint16_t(tot[i]);
+        s.ft = uint8_t(n ? cur : 0u);
+        s.fc = uint16_t(cnt);
+        s.lt = uint8_t(more ? lt : (n ? cur : 0u));
+        s.lc = uint16_t(more ? lc : cnt);
+        s.nruns = more ? 2 : 1;
+        s.pad = 0;
+    }
+};
+
+// Traceback inside the window (dp_walk's moves; codes.get(column, word) holds
+// eight cells of a segment).  gap_up / gap_left: the op of a row / column
+// skipped.  False if it leaves the window (not reached below band_limit).
+template <bool AFFINE, int NB, int TYPE, class Codes>
+HERO_HD bool band_walk(const BandSeg &s, const Codes &codes, uint32_t gap_up, uint32_t gap_left, OpsPut &out) {
+    using T = PairTags<AFFINE>;
+    int32_t i = s.R, j = s.C;
+    if (TYPE == BT_LEFT && i - j > s.base + NB - 1) {  // rows of column C above the window
+        const int32_t k = i - j - (s.base + NB - 1);
+        out.put(gap_up, uint32_t(k));
+        i -= k;
+    }
+    while (i > 0 && j > 0) {
+        const int32_t c = i - j - s.base;
+        if (uint32_t(c) >= uint32_t(NB)) return false;
+        const uint32_t code = (codes.get(j, c >> 3) >> (2 * (c & 7))) & 3u;
+        if (code == uint32_t(T::diag)) {
+            out.put((pack16(s.row, i - 1) ^ pack16(s.col, j - 1)) & 3u ? uint32_t(OP_X) : uint32_t(OP_M), 1u);
+            i--;
+            j--;
+        } else if (code == uint32_t(T::up)) {
+            out.put(gap_up, 1u);
+            i--;
+        } else {
+            out.put(gap_left, 1u);
+            j--;
+        }
+    }
+    out.put(gap_up, uint32_t(i));
+    out.put(gap_left, uint32_t(j));
+    return true;
+}
+
+// row (0-based) at which the main diagonal starts: the free run of an
+// align-right segment lies before it, that of an align-left one behind it
+HERO_HD int32_t main_row(int type, int32_t R, int32_t C) { return type == BT_RIGHT ? R - C : 0; }
+
+// mismatches on the main diagonal, counted up to `most`
+HERO_HD int32_t main_mismatches(const PackSeq &row, const PackSeq &col, int32_t r0, int32_t C, int32_t most) {
+    int32_t e = 0;
+    for (int32_t t = 0; t < C && e < most; t += 16) {
+        uint32_t x = mismatch16(pack16(row, r0 + t), pack16(col, t));
+        if (C - t < 16) x &= ops_mask(0, uint32_t(C - t - 1));
+        e += popc32(x);
+    }
+    return e;
+}
+
+// Ops of the straight path, right-aligned in `stride` words: the main diagonal's
+// matches and mismatches with the free run of R - C rows before (align-right)
+// or after (align-left) it, and their DpSum.
+HERO_HD void straight_ops(const PackSeq &row, const PackSeq &col, int type, int32_t R, int32_t C, uint32_t gap_up,
+                          uint32_t *w, uint32_t stride, DpSum &sum) {
+    const int32_t d = R - C, r0 = main_row(type, R, C);
+    const int32_t end = int32_t(stride) * 16, first = end - R;  // R = d + C ops
+    const int32_t ds = type == BT_RIGHT ? first + d : first, de = ds + C;
+    const int32_t gs = type == BT_RIGHT ? first : de;           // the gap's range [gs, gs + d)
+    for (int32_t k = first >> 4; k < int32_t(stride); k++) {
+        const int32_t p0 = k * 16;
+        uint32_t x = 0;
+        const int32_t a = ds > p0 ? ds - p0 : 0, b = de - p0 < 16 ? de - p0 : 16;  // the diagonal's fields [a, b)
+        if (a < b) x = mismatch16(pack16(row, r0 + p0 - ds), pack16(col, p0 - ds)) & ops_mask(uint32_t(a), uint32_t(b - 1));
+        const int32_t g = gs > p0 ? gs - p0 : 0, h = gs + d - p0 < 16 ? gs + d - p0 : 16;
+        if (g < h) x |= gap_up * ops_mask(uint32_t(g), uint32_t(h - 1));
+        w[k] = x;
+    }
+    ops_summary(w, uint32_t(first), uint32_t(R), sum);
+}
+
+}  // namespace hero

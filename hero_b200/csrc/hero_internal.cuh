@@ -49,6 +49,7 @@ struct ReadsView {
     const uint8_t *good;
     uint64_t n;
     const uint32_t *job;  // job of each read when jobs share a table; NULL: one job
+    const uint32_t *pack = nullptr;  // 2-bit codes, sixteen a word from base 0 of `code` (NULL: none)
 };
 
 struct TableView {
@@ -76,6 +77,7 @@ enum Counter : int {
     C_ANOMALY,
     C_OVERFLOW,
     C_WIN,          // winners of the current batch (compacted list length)
+    C_REST,         // DP segments of the current batch the window DP left to the whole-matrix kernels
     C_OVERFLOW_ALL, // overflows over the context's life (C_OVERFLOW is cleared per batch)
     C_CELLS_PAIR,   // band cells computed in 16-bit pairs (of C_CELLS_ALL's)
     C_STAGED,       // wavefront tasks whose row bases were staged by the bulk copy engine
@@ -105,11 +107,13 @@ struct ChainScratch {
 
 // kernels launched through the launchers below since the library was loaded
 uint64_t kernel_launches();
+void count_launch();
 
 // ---------------------------------------------------------------------------
 // launchers (hero_kernels.cu); all asynchronous on `st`
 // ---------------------------------------------------------------------------
-void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, const uint64_t *off,
+// pack (may be NULL): the 2-bit codes, as ReadsView::pack
+void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, uint32_t *pack, const uint64_t *off,
                        uint64_t n, uint32_t *len, uint8_t *good_query, uint8_t *good_subject,
                        double *gc, int32_t l, cudaStream_t st);
 // exclusive scan of n uint32 counts into n+1 uint64 offsets; tmp sized by scan_tmp_bytes
@@ -145,14 +149,11 @@ void launch_chain(const Params &p, uint64_t nseg, ReadsView subj, ReadsView q,
                   uint32_t *keys, DpSeg *segs, uint64_t cap_chains, uint64_t cap_keys,
                   uint64_t cap_segs, unsigned long long *counters, cudaStream_t st);
 
-// DP: shape sort then the strip kernel
-void launch_dp_sort(const DpSeg *segs, uint64_t nd, uint32_t *bins, uint32_t *perm,
-                    uint64_t *bin_off, void *scan_tmp, cudaStream_t st);
 constexpr uint32_t kShapeStripShift = 14;  // shape key: strips << 14 | align-left column << 10 | rows
 constexpr uint32_t kDpBins = 1u << 20;
 struct DpLaunch {
     const DpSeg *segs;
-    const uint32_t *perm;   // processing order; NULL = identity
+    const uint32_t *perm;   // processing order (of the n_rest listed segments)
     uint64_t nd;
     const uint8_t *scode;   // subject codes + offsets + lengths of the batch
     const uint64_t *soff;
@@ -177,11 +178,58 @@ struct DpLaunch {
     int32_t regs;           // registers a thread of the wavefront kernel: 128 (0 too) or 168
     unsigned long long *staged = nullptr;  // counters: C_STAGED, then C_STAGE_FAIL (may be NULL)
     uint32_t stage_extra = 0;  // bytes a warp's code area has past its rmax rows (set by launch_dp)
+    // the window DP (launch_band) and what it leaves to the whole-matrix kernels
+    const uint32_t *spack = nullptr, *qpack = nullptr;  // 2-bit codes of subjects and queries
+    uint32_t *rest = nullptr;                // segments for the whole-matrix kernels, in any order
+    unsigned long long *n_rest = nullptr;    // how many
+    uint32_t *bins = nullptr;                // kDpBins counts of their shapes
 };
 constexpr int kStripW = 8;
 constexpr uint32_t kStripsAll = 0xfffffffeu;  // every strip count 1..31 (bit n: n strips)
-// needs the shape sort (perm, bin_off); tasks: 128 uint64 of device scratch.
+
+#if defined(__CUDACC__)
+// (strips, align-left column, rows): a warp of the wavefront kernel takes
+// segments with equal strips, so they are grouped first; the align-left column
+// (1 + position of column C in the last strip, 0 when not aligned left) and the
+// row count keep the warps uniform
+__device__ __forceinline__ uint32_t shape_key(const DpSeg &g) {
+    const int32_t ls = g.s1 - g.s0, lq = g.q1 - g.q0;
+    const int32_t r = ls > lq ? ls : lq, c = ls > lq ? lq : ls;
+    int32_t nst = (c + kStripW - 1) / kStripW;
+    if (nst > 63) nst = 63;
+    const uint32_t wl = (g.flags & DPF_LEFT) ? 1u + uint32_t((c - 1) % kStripW) : 0u;
+    return (uint32_t(nst) << kShapeStripShift) | (wl << 10) | uint32_t(r > 1023 ? 1023 : r);
+}
+#endif
+
+// The window DP of a batch: six classes of windows, three segment types, up to
+// 1023 columns make a key; segments are counted, placed and run in key order.
+constexpr uint32_t kBandColBits = 10, kBandBins = 18u << kBandColBits, kBandNoKey = 0xffffffffu;
+struct BandBin {
+    uint32_t key, task, first, count;  // a non-empty key: its first task, first position and segments
+};
+struct BandWork {
+    bool on;           // false: every segment goes to the whole-matrix kernels
+    uint32_t *key;     // a segment's key (kBandNoKey: done, or not for the window)
+    uint32_t *order;   // segments by key
+    uint32_t *count;   // kBandBins segment counts (zeroed before launch_band)
+    uint32_t *cursor;  // kBandBins next positions
+    BandBin *bin;      // the non-empty keys
+    uint32_t *head;    // their number, the number of tasks, the next task
+    uint32_t *codes;   // traceback codes, code_words a warp
+    uint32_t code_words;
+    uint64_t warps;
+};
+uint64_t band_warps(int device, uint64_t nd);              // resident warps for nd segments
+uint32_t band_code_words(int32_t cmax, bool affine);       // code words a warp
+// fills ops, sums and cells of the segments it certifies; a.rest, a.n_rest (zeroed
+// before) and a.bins (zeroed before) get the others
+void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st);
+// order (a.nd entries) and bin offsets of the listed segments, for launch_dp
+void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void *scan_tmp, cudaStream_t st);
+// needs the shape sort (perm, bin_off); tasks: kDpTaskWords uint64 of device scratch.
 // The per-thread scratch (tb, bnd) is only used when dp_needs_scratch().
+constexpr uint32_t kDpTaskWords = 128;
 void launch_dp(const DpLaunch &a, const uint64_t *bin_off, uint64_t *tasks, int32_t cmax,
                cudaStream_t st);
 bool dp_wave_fits(int32_t rmax);

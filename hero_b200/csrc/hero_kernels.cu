@@ -7,7 +7,8 @@
 //   SubjectReadAligner::searchHashTable2 (+ sort)     k_probe, k_sort_hits
 //   processOneSubjectRead2 chaining + getAlignment2
 //   segment layout                                    k_chain
-//   BandAligner::calculateAlignment                   k_dp_hist/scatter, k_dp
+//   BandAligner::calculateAlignment                   k_band_* (hero_band.cu), then for the
+//                                                     segments they leave: k_dp_scatter, k_dp*
 //   AlignmentRecord scoring + early exits             k_assemble
 //   SubjectRead::addAlignment                         k_dedupe
 //   SubjectRead::updateQueryCoverage                  k_vote
@@ -78,10 +79,29 @@ __device__ __forceinline__ T warp_exclusive(T v, T *total) {
 // ---------------------------------------------------------------------------
 // reads
 // ---------------------------------------------------------------------------
-__global__ void k_codes(const uint8_t *raw, uint64_t n, uint8_t *code) {
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += uint64_t(gridDim.x) * blockDim.x)
-        code[i] = base_code(raw[i]);
+// One thread sixteen bases: one 16-byte load and store, and a word of 2-bit codes
+// (the code buffer holds 16 bytes past its last base).
+__global__ void k_codes(const uint8_t *raw, uint64_t n, uint8_t *code, uint32_t *pack) {
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i * 16 < n;
+         i += uint64_t(gridDim.x) * blockDim.x) {
+        union {
+            uint4 v;
+            uint8_t b[16];
+        } x, y;
+        if (i * 16 + 16 <= n) {
+            x.v = reinterpret_cast<const uint4 *>(raw)[i];
+        } else {
+            for (int k = 0; k < 16; k++) x.b[k] = i * 16 + k < n ? raw[i * 16 + k] : uint8_t(0);
+        }
+        uint32_t w = 0;
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            y.b[k] = base_code(x.b[k]);
+            w |= uint32_t(y.b[k] & 3u) << (2 * k);
+        }
+        reinterpret_cast<uint4 *>(code)[i] = y.v;
+        if (pack) pack[i] = w;
+    }
 }
 
 // QueryDataset::qualityFilter (QueryDataset.cpp:60-75), the good-read tests of
@@ -783,48 +803,25 @@ struct OpsWriter {
     }
 };
 
-// (strips, align-left column, rows): a warp of the wavefront kernel takes
-// segments with equal strips, so they are grouped first; the align-left column
-// (1 + position of column C in the last strip, 0 when not aligned left) and the
-// row count keep the warps uniform
-__device__ __forceinline__ uint32_t shape_key(const DpSeg &g) {
-    const int32_t ls = g.s1 - g.s0, lq = g.q1 - g.q0;
-    const int32_t r = ls > lq ? ls : lq, c = ls > lq ? lq : ls;
-    int32_t nst = (c + kStripW - 1) / kStripW;
-    if (nst > 63) nst = 63;
-    const uint32_t wl = (g.flags & DPF_LEFT) ? 1u + uint32_t((c - 1) % kStripW) : 0u;
-    return (uint32_t(nst) << kShapeStripShift) | (wl << 10) | uint32_t(r > 1023 ? 1023 : r);
-}
-
-// Counting sort by shape.  Segments of a chain mostly share a few shapes, so
-// the lanes of a warp with equal keys (__match_any_sync) add their count with
-// one atomic by the lowest of them; in the scatter each lane then takes its
-// rank among them.  The order inside a bin is free: every segment writes its
+// Counting sort by shape of the segments the window DP left (their shapes are
+// counted as they are listed).  Segments of a chain mostly share a few shapes,
+// so the lanes of a warp with equal keys (__match_any_sync) take their places
+// with one atomic by the lowest of them, each at its rank among them.  The order inside a bin is free: every segment writes its
 // results to its own slot.
-__global__ void k_dp_hist(const DpSeg *segs, uint64_t nd, uint32_t *bins) {
+__global__ void k_dp_scatter(DpLaunch a, uint32_t *cursor, const uint64_t *bin_off, uint32_t *perm) {
     const uint32_t lane = lane_id();
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < nd;
+    const uint64_t n = *a.n_rest;
+    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < n;
          b += uint64_t(gridDim.x) * blockDim.x) {
         const uint64_t i = b + lane;
-        const uint32_t key = i < nd ? shape_key(segs[i]) : 0xffffffffu;
-        const uint32_t same = __match_any_sync(0xffffffffu, key);
-        if (i < nd && lane == uint32_t(__ffs(int(same))) - 1u) atomicAdd(&bins[key], uint32_t(__popc(same)));
-    }
-}
-
-__global__ void k_dp_scatter(const DpSeg *segs, uint64_t nd, uint32_t *cursor,
-                             const uint64_t *bin_off, uint32_t *perm) {
-    const uint32_t lane = lane_id();
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < nd;
-         b += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t i = b + lane;
-        const uint32_t key = i < nd ? shape_key(segs[i]) : 0xffffffffu;
+        const uint32_t si = i < n ? a.rest[i] : 0u;
+        const uint32_t key = i < n ? shape_key(a.segs[si]) : 0xffffffffu;
         const uint32_t same = __match_any_sync(0xffffffffu, key);
         const uint32_t leader = uint32_t(__ffs(int(same))) - 1u;
         uint32_t base = 0;
-        if (i < nd && lane == leader) base = atomicAdd(&cursor[key], uint32_t(__popc(same)));
+        if (i < n && lane == leader) base = atomicAdd(&cursor[key], uint32_t(__popc(same)));
         base = __shfl_sync(0xffffffffu, base, int(leader));
-        if (i < nd) perm[bin_off[key] + base + __popc(same & ((1u << lane) - 1u))] = uint32_t(i);
+        if (i < n) perm[bin_off[key] + base + __popc(same & ((1u << lane) - 1u))] = si;
     }
 }
 
@@ -835,8 +832,9 @@ __global__ void __launch_bounds__(kDpThreads) k_dp(DpLaunch a) {
     const uint64_t T = uint64_t(gridDim.x) * blockDim.x;
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     DevScratch sc{a.tb, a.bnd, T, a.rmax, t};
-    for (uint64_t idx = t; idx < a.nd; idx += T) {
-        const uint32_t si = a.perm ? a.perm[idx] : uint32_t(idx);
+    const uint64_t n = *a.n_rest;
+    for (uint64_t idx = t; idx < n; idx += T) {
+        const uint32_t si = a.perm[idx];
         const DpSeg g = a.segs[si];
         const SegView v = dpseg_view(g, a.scode, a.soff, a.slen, a.qcode, a.qoff);
         dp_fill<kStripW, AFFINE>(v, sc);
@@ -845,10 +843,6 @@ __global__ void __launch_bounds__(kDpThreads) k_dp(DpLaunch a) {
         dp_traceback<kStripW>(v, sc, w, sum);
         w.flush();
         a.sums[si] = sum;
-        if (a.cells) {
-            const uint64_t cl = band_cells(v.R, v.C, v.band);
-            a.cells[si] = uint32_t(cl > 0xffffffffull ? 0xffffffffull : cl);
-        }
     }
 }
 
@@ -1109,10 +1103,6 @@ __device__ __forceinline__ void group_traceback(const DpLaunch &a, const Codes &
         ops_summary(staged ? stage : a.ops + uint64_t(si) * a.stride, a.stride * 16u - uint32_t(n),
                     uint32_t(n), sum);
         a.sums[si] = sum;
-        if (a.cells) {
-            const uint64_t cl = band_cells(v.R, v.C, v.band);
-            a.cells[si] = uint32_t(cl > 0xffffffffull ? 0xffffffffull : cl);
-        }
     }
     if (staged && active) {  // the group's lanes copy the ops out together
         uint32_t *out = a.ops + uint64_t(si) * a.stride;
@@ -1487,7 +1477,8 @@ __global__ void __launch_bounds__(kDpThreads) k_dp_wide(DpLaunch a, const uint64
     const uint64_t T = uint64_t(gridDim.x) * blockDim.x;
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     DevScratch sc{a.tb, a.bnd, T, a.rmax, t};
-    for (uint64_t idx = tasks[0] + t; idx < a.nd; idx += T) {
+    const uint64_t n = *a.n_rest;
+    for (uint64_t idx = tasks[0] + t; idx < n; idx += T) {
         const uint32_t si = a.perm[idx];
         const DpSeg g = a.segs[si];
         const SegView v = dpseg_view(g, a.scode, a.soff, a.slen, a.qcode, a.qoff);
@@ -1497,10 +1488,6 @@ __global__ void __launch_bounds__(kDpThreads) k_dp_wide(DpLaunch a, const uint64
         dp_traceback<kStripW>(v, sc, w, sum);
         w.flush();
         a.sums[si] = sum;
-        if (a.cells) {
-            const uint64_t cl = band_cells(v.R, v.C, v.band);
-            a.cells[si] = uint32_t(cl > 0xffffffffull ? 0xffffffffull : cl);
-        }
     }
 }
 
@@ -2258,12 +2245,12 @@ __global__ void k_unpack_ops(const uint32_t *ops, uint32_t stride, const DpSum *
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, const uint64_t *off,
+void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, uint32_t *pack, const uint64_t *off,
                        uint64_t n, uint32_t *len, uint8_t *good_query, uint8_t *good_subject,
                        double *gc, int32_t l, cudaStream_t st) {
     if (nbases) {
         counted();
-        k_codes<<<grid_1d(nbases, 256), 256, 0, st>>>(raw, nbases, code);
+        k_codes<<<grid_1d((nbases + 15) / 16, 256), 256, 0, st>>>(raw, nbases, code, pack);
     }
     if (n) {
         counted();
@@ -2273,6 +2260,7 @@ void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, const
 
 size_t scan_tmp_bytes(uint64_t n) { return scan_levels_bytes(n); }
 
+void count_launch() { counted(); }
 uint64_t kernel_launches() { return g_launches.load(std::memory_order_relaxed); }
 
 void launch_scan_u32(const uint32_t *in, uint64_t *out, uint64_t n, void *tmp, cudaStream_t st) {
@@ -2350,16 +2338,12 @@ void launch_chain(const Params &p, uint64_t nseg, ReadsView subj, ReadsView q,
                                                         counters);
 }
 
-void launch_dp_sort(const DpSeg *segs, uint64_t nd, uint32_t *bins, uint32_t *perm,
-                    uint64_t *bin_off, void *scan_tmp, cudaStream_t st) {
-    cudaMemsetAsync(bins, 0, sizeof(uint32_t) * kDpBins, st);
-    if (!nd) return;
+void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void *scan_tmp, cudaStream_t st) {
+    if (!a.nd) return;
+    launch_scan_u32(a.bins, bin_off, kDpBins, scan_tmp, st);
+    cudaMemsetAsync(a.bins, 0, sizeof(uint32_t) * kDpBins, st);
     counted();
-    k_dp_hist<<<grid_1d(nd, 256), 256, 0, st>>>(segs, nd, bins);
-    launch_scan_u32(bins, bin_off, kDpBins, scan_tmp, st);
-    cudaMemsetAsync(bins, 0, sizeof(uint32_t) * kDpBins, st);
-    counted();
-    k_dp_scatter<<<grid_1d(nd, 256), 256, 0, st>>>(segs, nd, bins, bin_off, perm);
+    k_dp_scatter<<<grid_1d(a.nd, 256), 256, 0, st>>>(a, a.bins, bin_off, order);
 }
 
 uint64_t dp_threads(int device) {

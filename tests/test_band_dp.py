@@ -1,0 +1,106 @@
+"""The window DP (hero_band.cuh): whatever its certificate accepts is the
+whole-matrix path, move for move.
+
+On the CPU the header's item logic runs beside hero_core.cuh's whole-matrix DP
+on every pair of short strings and on random segments of the kinds that strain
+the certificate (tandem repeats, two-letter strings, indels, narrow bands); on
+the GPU the kernels run on segments at the edges of their classes against the
+oracle."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+from hero_testlib import ROOT
+
+SRC = os.path.join(ROOT, "tests", "emu", "band_emu.cpp")
+LIB = os.path.join(ROOT, "_build", "libband_emu.so")
+HDRS = [os.path.join(ROOT, "hero_b200", "csrc", h) for h in ("hero_band.cuh", "hero_core.cuh")]
+ACGT = np.frombuffer(b"ACGT", np.uint8)
+
+
+@pytest.fixture(scope="module")
+def band():
+    if not os.path.exists(LIB) or any(os.path.getmtime(s) > os.path.getmtime(LIB) for s in [SRC] + HDRS):
+        os.makedirs(os.path.dirname(LIB), exist_ok=True)
+        subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-o", LIB, SRC], check=True)
+    return C.CDLL(LIB)
+
+
+def _clean(counts):
+    segments, certified, straight, ops, sums, straight_ops = counts
+    assert (ops, sums, straight_ops) == (0, 0, 0), counts
+    return segments, certified, straight
+
+
+@pytest.mark.parametrize("affine,nb", [(1, 4), (1, 8), (1, 16), (0, 4), (0, 8)])
+@pytest.mark.parametrize("kind", [0, 1, 2], ids=["both", "right", "left"])
+def test_every_short_segment(band, affine, nb, kind):
+    n = np.zeros(3, np.int64)
+    for letters, total in ((2, 11), (3, 7), (4, 6)):
+        for rows in range(1, total):
+            for cols in range(1, min(rows, total - rows) + 1):
+                for mask, m in ((0, 65535), (1, 0), (1, 1), (1, 3)):
+                    c = (C.c_uint64 * 6)()
+                    band.band_exhaustive(affine, nb, kind, mask, letters, rows, cols, C.c_int64(m), c)
+                    n += _clean(list(c))
+    assert n[0] > n[2] > 0 and n[1] > n[0] // 4  # the certificate accepts, and not only straight paths
+
+
+@pytest.mark.parametrize("affine,nb", [(1, 8), (1, 16), (1, 24), (1, 40), (0, 8), (0, 16)])
+@pytest.mark.parametrize("cmax", [5, 40, 250, 1023])
+def test_random_segments(band, affine, nb, cmax):
+    for mask, m in ((0, 0), (1, 4), (1, 30)):
+        c = (C.c_uint64 * 6)()
+        band.band_random(affine, nb, mask, C.c_uint64(nb * 1000 + cmax), C.c_uint64(200000 // (cmax + 100)), cmax,
+                         C.c_int64(m), c)
+        segments, certified, straight = _clean(list(c))
+        assert segments and certified > straight
+
+
+def _segments(rng, n):
+    """(subject, query, band, flags): copies with e substitutions and at times an
+    indel, on either side, with a free run on the anchored side's far end."""
+    out = []
+    sizes = [1, 2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 47, 48, 49, 64, 111, 211, 255, 256, 257]
+    for i in range(n):
+        c = int(sizes[i % len(sizes)])
+        e = i // len(sizes) % 7
+        kind = int(rng.integers(0, 3))
+        col = ACGT[rng.integers(0, 4, c)]
+        row = col.copy()
+        for p in rng.integers(0, c, e):
+            row[p] = ACGT[rng.integers(0, 4)]
+        if rng.random() < 0.3:
+            p, k = int(rng.integers(0, c)), int(rng.integers(1, 4))
+            row = np.concatenate([row[:p], ACGT[rng.integers(0, 4, k)], row[p:]]) if rng.random() < 0.5 or c < 8 \
+                else np.delete(row, slice(p, p + k))
+        d = int(rng.integers(0, 70)) if kind else 0
+        free = ACGT[rng.integers(0, 4, d)] if rng.random() < 0.7 else np.resize(col, d)
+        row = np.concatenate([free, row] if kind == 1 else [row, free])
+        s, q = (row, col) if rng.random() < 0.5 else (col, row)
+        out.append((bytes(s), bytes(q), int(rng.choice([2, 5, 9, 300])), kind))
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("affine", [0, 1])
+def test_gpu_segments_at_the_edges_of_the_classes(gpu_lib, oracle, affine):
+    from hero_b200 import Hero
+    seg = _segments(np.random.default_rng(40 + affine), 5000)
+    n = len(seg)
+    off = [np.zeros(n + 1, np.uint64) for _ in range(2)]
+    for h in range(2):
+        off[h][1:] = np.cumsum([len(x[h]) for x in seg])
+    seq = [np.frombuffer(b"".join(x[h] for x in seg), np.uint8) for h in range(2)]
+    idx, zeros = np.arange(n, dtype=np.uint32), np.zeros(n, np.int32)
+    with Hero() as h:
+        ops, oo, nops = h.align_segments(affine, seq[0], off[0], seq[1], off[1], idx, np.zeros(n, np.uint8), idx,
+                                         zeros, np.diff(off[0]).astype(np.int32), zeros,
+                                         np.diff(off[1]).astype(np.int32), np.array([x[3] for x in seg], np.uint8),
+                                         np.array([x[2] for x in seg], np.int64))
+    for i, (s, q, m, kind) in enumerate(seg):
+        want, _ = oracle.align(affine, s, q, m, kind == 1, kind == 2)
+        got = ops[int(oo[i]):int(oo[i]) + int(nops[i])]
+        assert np.array_equal(got, want), (i, len(s), len(q), m, kind)
