@@ -69,11 +69,11 @@ __device__ __forceinline__ void rest_append(const DpLaunch &a, bool on, uint32_t
 }
 
 // One thread a segment: its reference cells; segments without a mismatch on
-// their main diagonal are done here (deficit 0: nothing can equal it), the
-// others are counted by window class, type and columns, or listed for the
-// whole-matrix kernels.  Bound by the scattered reads of the packed bases and
-// the op words written; it replaces the whole matrix for the third (150 bp,
-// affine) to half (100 bp) of the segments.
+// their main diagonal (deficit 0: nothing can equal it), and nearly all of those
+// with one, are done here, the others are counted by window class, type and
+// columns, or listed for the whole-matrix kernels.  Bound by the scattered reads
+// of the packed bases and the op words written; it replaces the whole matrix for
+// 61 % (150 bp, affine) to 85 % (100 bp) of the segments.
 __global__ void __launch_bounds__(256) k_band_screen(DpLaunch a, BandWork w) {
     const uint32_t lane = lane_id();
     for (uint64_t b0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b0 < a.nd;
@@ -98,8 +98,10 @@ __global__ void __launch_bounds__(256) k_band_screen(DpLaunch a, BandWork w) {
             const int32_t most_d = affine ? (masked ? 12 : 24) : 8;
             rest = !w.on || (g.flags & 3u) == 3u || s.C > kBandMaxC || (type == BT_NONE && d > most_d);
             if (!rest) {
-                const int32_t e = type == BT_NONE && d > 0 ? 4 : main_mismatches(s.row, s.col, main_row(type, s.R, s.C), s.C, 4);
-                if (e == 0) {
+                int32_t f = 0, e = 4;
+                if (type != BT_NONE || d == 0) e = main_mismatches(s.row, s.col, main_row(type, s.R, s.C), s.C, 4, f);
+                if (e == 0 || (e == 1 && (affine ? one_mismatch_straight<true>(s.row, s.col, type, s.R, s.C, f)
+                                                 : one_mismatch_straight<false>(s.row, s.col, type, s.R, s.C, f)))) {
                     DpSum sum;
                     straight_ops(s.row, s.col, type, s.R, s.C, reversed ? uint32_t(OP_I) : uint32_t(OP_D),
                                  a.ops + i * a.stride, a.stride, sum);
@@ -250,10 +252,10 @@ __device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order,
         t.base = band_base<AFFINE, NB, TYPE>(t.R - t.C);
         OpsPut put{a.ops + uint64_t(sj) * a.stride, int32_t(a.stride * 16u)};
         DpSum sum;
-        band_walk<AFFINE, NB, TYPE>(t, WarpCodes<WORDS>{codes + at, h ? 16u : 0u},
-                                    reversed ? uint32_t(OP_I) : uint32_t(OP_D),
-                                    reversed ? uint32_t(OP_D) : uint32_t(OP_I), put);
-        put.finish(sum);
+        const int32_t np = band_walk<AFFINE, NB, TYPE>(t, WarpCodes<WORDS>{codes + at, h ? 16u : 0u},
+                                                       reversed ? uint32_t(OP_I) : uint32_t(OP_D),
+                                                       reversed ? uint32_t(OP_D) : uint32_t(OP_I), put);
+        ops_summary(put.w, a.stride * 16u - uint32_t(np), uint32_t(np), sum);
         a.sums[sj] = sum;
     }
     __syncwarp();
@@ -275,9 +277,9 @@ __device__ __forceinline__ void band_dispatch(int type, const DpLaunch &a, const
 
 // Persistent warps fed by a queue of tasks.  Measured, DP stage of one
 // correction before (every matrix whole) and with the window: 5 Mbp affine,
-// 1.67 M x 150 bp, 109 M segments, 358 -> 78 ms; 1 Mbp global, 300 k x 100 bp,
-// 7.3 -> 2.5 ms; 300 kbp affine with -i 2 (bands of a few diagonals), 80 k x
-// 150 bp, 34.5 -> 3.0 ms.
+// 1.67 M x 150 bp, 109 M segments, 358 -> 55 ms; 1 Mbp global, 300 k x 100 bp,
+// 7.3 -> 1.6 ms; 300 kbp affine with -i 2 (bands of a few diagonals), 80 k x
+// 150 bp, 34.5 -> 1.8 ms.
 constexpr int kBandWarps = 4, kBandBlocks = 3;  // 12 warps an SM: 168 registers hold the widest window
 
 template <bool AFFINE>

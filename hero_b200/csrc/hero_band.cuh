@@ -28,7 +28,6 @@ namespace hero {
 enum : int { BT_NONE = 0, BT_RIGHT = 1, BT_LEFT = 2 };  // anchored at both ends, at the end, at the start
 
 constexpr int32_t kBandMaxC = 1023;   // columns of a window segment: 16-bit values hold 4 * 5 * C
-constexpr int kBandStep = 4;          // columns an unrolled block computes
 constexpr int32_t kBandDead = -12000; // outside the matrix or the aligner's band: 3000 below any value
                                       // the certificate accepts, at every column
 constexpr int kPackPad = 8;           // words (128 bases) before and after packed reads that fetches may touch
@@ -209,7 +208,7 @@ HERO_HD int32_t band_col0_right(int32_t i) {
 // main diagonal are and-ed into `straight`.
 template <bool AFFINE, int NB, int TYPE, bool MASK, bool INJECT, class Store>
 HERO_HD void band_column(uint32_t (&M)[NB], uint32_t (&L)[AFFINE ? NB : 1], const uint32_t (&P)[MASK ? NB : 1],
-                         const uint32_t *sel, uint32_t ta, uint32_t tb, int32_t za, int32_t zb,
+                         const uint32_t (&sel)[NB], uint32_t ta, uint32_t tb, int32_t za, int32_t zb,
                          uint32_t &straight, Store &st) {
     using K = BandCost<AFFINE>;
     constexpr int main_c = band_main<AFFINE, NB, TYPE>();
@@ -260,7 +259,7 @@ HERO_HD void band_fill(const BandSeg &a, const BandSeg &b, int32_t C, int32_t jp
     using K = BandCost<AFFINE>;
     using T = PairTags<AFFINE>;
     constexpr int main_c = band_main<AFFINE, NB, TYPE>();
-    uint32_t M[NB], L[AFFINE ? NB : 1], P[MASK ? NB : 1], sel[NB - 1 + kBandStep];
+    uint32_t M[NB], L[AFFINE ? NB : 1], P[MASK ? NB : 1], sel[NB];
     // column 0
 #pragma unroll
     for (int c = 0; c < NB; c++) {
@@ -285,48 +284,31 @@ HERO_HD void band_fill(const BandSeg &a, const BandSeg &b, int32_t C, int32_t jp
     }
     uint32_t ra = 0, rb = 0, ca = 0, cb = 0, straight = 0xffffffffu;
     const int32_t last = TYPE == BT_LEFT ? C - 1 : C;  // column C of an align-left segment follows the loop
+    // One column an iteration: the loop's code then stays near the instructions a
+    // scheduler caches (four columns an iteration waited for instructions: 34 ms
+    // of window kernels against 31 on the 1.67 M x 150 bp workload).
 #pragma unroll 1
-    for (int32_t j0 = 1; j0 <= last; j0 += kBandStep) {
-        if (((j0 - 1) & 15) == 0) {  // sixteen more rows and columns
-            ra = pack16(a.row, a.base + NB - 2 + j0);
-            rb = pack16(b.row, b.base + NB - 2 + j0);
-            ca = pack16(a.col, j0 - 1);
-            cb = pack16(b.col, j0 - 1);
+    for (int32_t j = 1; j <= last; j++) {
+        if (((j - 1) & 15) == 0) {  // sixteen more rows and columns
+            ra = pack16(a.row, a.base + NB - 2 + j);
+            rb = pack16(b.row, b.base + NB - 2 + j);
+            ca = pack16(a.col, j - 1);
+            cb = pack16(b.col, j - 1);
         }
-#pragma unroll
-        for (int u = 0; u < kBandStep; u++) {
-            sel[NB - 1 + u] = band_sel(ra & 3u, rb & 3u);
-            ra >>= 2;
-            rb >>= 2;
-        }
-        if (AFFINE && j0 <= jp) {
-#pragma unroll
-            for (int u = 0; u < kBandStep; u++) {
-                const int32_t j = j0 + u;
-                if (j <= last) {
-                    st.column(j);
-                    band_column<AFFINE, NB, TYPE, MASK, true>(M, L, P, sel + u, band_table<AFFINE>(ca & 3u),
-                                                              band_table<AFFINE>(cb & 3u), -a.base - j,
-                                                              -b.base - j, straight, st);
-                }
-                ca >>= 2;
-                cb >>= 2;
-            }
+        sel[NB - 1] = band_sel(ra & 3u, rb & 3u);
+        const uint32_t ta = band_table<AFFINE>(ca & 3u), tb = band_table<AFFINE>(cb & 3u);
+        ra >>= 2;
+        rb >>= 2;
+        ca >>= 2;
+        cb >>= 2;
+        st.column(j);
+        if (AFFINE && j <= jp) {
+            band_column<AFFINE, NB, TYPE, MASK, true>(M, L, P, sel, ta, tb, -a.base - j, -b.base - j, straight, st);
         } else {
-#pragma unroll
-            for (int u = 0; u < kBandStep; u++) {
-                const int32_t j = j0 + u;
-                if (j <= last) {
-                    st.column(j);
-                    band_column<AFFINE, NB, TYPE, MASK, false>(M, L, P, sel + u, band_table<AFFINE>(ca & 3u),
-                                                               band_table<AFFINE>(cb & 3u), 0, 0, straight, st);
-                }
-                ca >>= 2;
-                cb >>= 2;
-            }
+            band_column<AFFINE, NB, TYPE, MASK, false>(M, L, P, sel, ta, tb, 0, 0, straight, st);
         }
 #pragma unroll
-        for (int c = 0; c < NB - 1; c++) sel[c] = sel[c + kBandStep];
+        for (int c = 0; c < NB - 1; c++) sel[c] = sel[c + 1];
     }
     const int32_t da = a.R - a.C, db = b.R - b.C;
     if (TYPE != BT_LEFT) {
@@ -397,103 +379,138 @@ HERO_HD void band_fill(const BandSeg &a, const BandSeg &b, int32_t C, int32_t jp
     eb = BandEnd{vb, sb};
 }
 
-// Packed ops written last to first at descending positions, with the run
-// tracking a DpSum needs (the first run put is the path's last).
+// Packed ops written last to first at descending positions.
 struct OpsPut {
     uint32_t *w;
-    int32_t p;          // position of the op put last
+    int32_t p;  // position of the op put last
     uint32_t acc = 0;
-    uint32_t cur = 4u, cnt = 0, lt = 0, lc = 0, n = 0, tot[4] = {0, 0, 0, 0};
-    bool more = false;  // two or more runs
 
-    HERO_HD void put(uint32_t op, uint32_t k) {
-        if (k == 0) return;
-        n += k;
-        tot[0] += op == 0u ? k : 0u;
-        tot[1] += op == 1u ? k : 0u;
-        tot[2] += op == 2u ? k : 0u;
-        tot[3] += op == 3u ? k : 0u;
-        if (op == cur) {
-            cnt += k;
+    // k <= 16 ops: the low k fields of `bits`, the lowest first in path order
+    HERO_HD void fields(uint32_t bits, uint32_t k) {
+        const uint32_t room = uint32_t((p - 1) & 15) + 1u;  // fields left in the current word
+        if (k < room) {
+            acc |= bits << (2u * (room - k));
         } else {
-            if (cur != 4u && !more) {
-                lt = cur;
-                lc = cnt;
-                more = true;
-            }
-            cur = op;
-            cnt = k;
+            w[(p - 1) >> 4] = acc | (bits >> (2u * (k - room)));
+            acc = k == room ? 0u : bits << (32u - 2u * (k - room));
         }
-        while (k > 0) {  // fields of one word at a time
-            const uint32_t room = uint32_t((p - 1) & 15) + 1u, take = k < room ? k : room;
-            const uint32_t lo = room - take;
-            acc |= op * ops_mask(lo, room - 1u);
-            p -= int32_t(take);
+        p -= int32_t(k);
+    }
+    HERO_HD void run(uint32_t op, uint32_t k) {
+        for (; k > 0;) {
+            const uint32_t take = k < 16u ? k : 16u;
+            fields(op * ops_mask(0, take - 1u), take);
             k -= take;
-            if ((p & 15) == 0) {
-                w[p >> 4] = acc;
-                acc = 0;
-            }
         }
     }
-    HERO_HD void finish(DpSum &s) {
+    HERO_HD void flush() {
         if (p & 15) w[p >> 4] = acc;
-        for (int i = 0; i < 4; i++) s.tot[i] = uint16_t(tot[i]);
-        s.ft = uint8_t(n ? cur : 0u);
-        s.fc = uint16_t(cnt);
-        s.lt = uint8_t(more ? lt : (n ? cur : 0u));
-        s.lc = uint16_t(more ? lc : cnt);
-        s.nruns = more ? 2 : 1;
-        s.pad = 0;
     }
 };
 
 // Traceback inside the window (dp_walk's moves; codes.get(column, word) holds
-// eight cells of a segment).  gap_up / gap_left: the op of a row / column
-// skipped.  False if it leaves the window (not reached below band_limit).
+// eight cells of a segment).  Diagonal runs are found eight columns at a time:
+// their codes are loaded together, since the cell's place in the window stays.
+// gap_up / gap_left: the op of a row / column skipped.  Returns the ops put, or
+// -1 if the path leaves the window (not reached within band_limit).
 template <bool AFFINE, int NB, int TYPE, class Codes>
-HERO_HD bool band_walk(const BandSeg &s, const Codes &codes, uint32_t gap_up, uint32_t gap_left, OpsPut &out) {
+HERO_HD int32_t band_walk(const BandSeg &s, const Codes &codes, uint32_t gap_up, uint32_t gap_left, OpsPut &out) {
     using T = PairTags<AFFINE>;
-    int32_t i = s.R, j = s.C;
-    if (TYPE == BT_LEFT && i - j > s.base + NB - 1) {  // rows of column C above the window
-        const int32_t k = i - j - (s.base + NB - 1);
-        out.put(gap_up, uint32_t(k));
+    constexpr int32_t AHEAD = 8;
+    const int32_t end = out.p;
+    int32_t i = s.R, j = s.C, c = i - j - s.base;
+    if (TYPE == BT_LEFT) {  // column C: the rows above the window, then its climb inside
+        int32_t k = c > NB - 1 ? c - (NB - 1) : 0;
+        while (c - k > 0 && ((codes.get(j, (c - k) >> 3) >> (2 * ((c - k) & 7))) & 3u) == uint32_t(T::up)) k++;
+        if (k > i) k = i;
+        out.run(gap_up, uint32_t(k));
         i -= k;
+        c -= k;
     }
     while (i > 0 && j > 0) {
-        const int32_t c = i - j - s.base;
-        if (uint32_t(c) >= uint32_t(NB)) return false;
-        const uint32_t code = (codes.get(j, c >> 3) >> (2 * (c & 7))) & 3u;
-        if (code == uint32_t(T::diag)) {
-            out.put((pack16(s.row, i - 1) ^ pack16(s.col, j - 1)) & 3u ? uint32_t(OP_X) : uint32_t(OP_M), 1u);
+        if (uint32_t(c) >= uint32_t(NB)) return -1;
+        const int32_t k = c >> 3, sh = 2 * (c & 7), n = i < j ? (i < AHEAD ? i : AHEAD) : (j < AHEAD ? j : AHEAD);
+        uint32_t code[AHEAD];
+#pragma unroll
+        for (int t = 0; t < AHEAD; t++) code[t] = t < n ? (codes.get(j - t, k) >> sh) & 3u : 3u;
+        int32_t run = 0;
+        uint32_t stop = 3u;  // the code that ends the run (3: none in these columns)
+#pragma unroll
+        for (int t = AHEAD - 1; t >= 0; t--)
+            if (code[t] != uint32_t(T::diag)) {
+                run = t;
+                stop = code[t];
+            }
+        if (stop == 3u) run = n;
+        if (run > 0) {
+            i -= run;
+            j -= run;
+            out.fields(mismatch16(pack16(s.row, i), pack16(s.col, j)) & ops_mask(0, uint32_t(run - 1)), uint32_t(run));
+        }
+        if (stop == uint32_t(T::up)) {
+            out.fields(gap_up, 1u);
             i--;
+            c--;
+        } else if (stop == uint32_t(T::left)) {
+            out.fields(gap_left, 1u);
             j--;
-        } else if (code == uint32_t(T::up)) {
-            out.put(gap_up, 1u);
-            i--;
-        } else {
-            out.put(gap_left, 1u);
-            j--;
+            c++;
         }
     }
-    out.put(gap_up, uint32_t(i));
-    out.put(gap_left, uint32_t(j));
-    return true;
+    out.run(gap_up, uint32_t(i));
+    out.run(gap_left, uint32_t(j));
+    out.flush();
+    return end - out.p;
 }
 
 // row (0-based) at which the main diagonal starts: the free run of an
 // align-right segment lies before it, that of an align-left one behind it
 HERO_HD int32_t main_row(int type, int32_t R, int32_t C) { return type == BT_RIGHT ? R - C : 0; }
 
-// mismatches on the main diagonal, counted up to `most`
-HERO_HD int32_t main_mismatches(const PackSeq &row, const PackSeq &col, int32_t r0, int32_t C, int32_t most) {
+// mismatches on the main diagonal, counted up to `most` (or a few more); first:
+// the column (0-based) of the first
+HERO_HD int32_t main_mismatches(const PackSeq &row, const PackSeq &col, int32_t r0, int32_t C, int32_t most,
+                                int32_t &first) {
     int32_t e = 0;
+    first = C;
     for (int32_t t = 0; t < C && e < most; t += 16) {
         uint32_t x = mismatch16(pack16(row, r0 + t), pack16(col, t));
         if (C - t < 16) x &= ops_mask(0, uint32_t(C - t - 1));
+        if (x && first == C) first = t + (low_bit(x) >> 1);
         e += popc32(x);
     }
     return e;
+}
+
+// a mismatch among columns [a, b) (0-based) against the rows r0 + column
+HERO_HD bool any_mismatch(const PackSeq &row, const PackSeq &col, int32_t r0, int32_t a, int32_t b) {
+    for (int32_t t = a; t < b; t += 16) {
+        uint32_t x = mismatch16(pack16(row, r0 + t), pack16(col, t));
+        if (b - t < 16) x &= ops_mask(0, uint32_t(b - t - 1));
+        if (x) return true;
+    }
+    return false;
+}
+
+// One mismatch on the main diagonal, at column f: is the straight path the
+// traceback's?  Its deficit is 5, so only paths of one gap and no mismatch
+// compete.  Anchored at the end (align-right): rows skipped after a start one
+// row higher (deficit 4; two rows higher, 5, wins its tie for the affine
+// aligner), with every column up to f matching there.  Anchored at the start:
+// one row skipped before f (deficit 4) with the rest matching; or, a tie the
+// affine aligner gives to the free climb, one column skipped with the rest
+// matching and at least one match behind it.  Anchored on both ends a gap needs
+// its opposite, and both cost at least 6.
+template <bool AFFINE>
+HERO_HD bool one_mismatch_straight(const PackSeq &row, const PackSeq &col, int type, int32_t R, int32_t C, int32_t f) {
+    const int32_t d = R - C;
+    if (type == BT_RIGHT)
+        return (d < 1 || any_mismatch(row, col, d - 1, 0, f + 1)) &&
+               (!AFFINE || d < 2 || any_mismatch(row, col, d - 2, 0, f + 1));
+    if (type == BT_LEFT)
+        return (d < 1 || any_mismatch(row, col, 1, f, C)) &&
+               (!AFFINE || (C > 1 && any_mismatch(row, col, -1, f + 1 < C ? f + 1 : C - 1, C)));
+    return true;
 }
 
 // Ops of the straight path, right-aligned in `stride` words: the main diagonal's

@@ -80,6 +80,28 @@ struct Count {
     uint64_t *c;  // segments, certified, straight, wrong ops, wrong summaries, wrong straight ops
 };
 
+// the segments the screen finishes: no mismatch, or one that one_mismatch_straight accepts
+template <bool AFFINE>
+void screen_run(const Seg &g, int type, Count n) {
+    const int32_t d = g.b.R - g.b.C;
+    if (type == BT_NONE && d > 0) return;
+    int32_t f = 0;
+    const int32_t e = main_mismatches(g.b.row, g.b.col, main_row(type, g.b.R, g.b.C), g.b.C, 4, f);
+    n.c[0]++;
+    if (e > 1 || (e == 1 && !one_mismatch_straight<AFFINE>(g.b.row, g.b.col, type, g.b.R, g.b.C, f))) return;
+    n.c[1]++;
+    n.c[2] += e == 0;
+    DpSum want, sum;
+    const std::vector<uint8_t> ops = whole(g.v, AFFINE, want);
+    const uint32_t stride = uint32_t((g.b.R + g.b.C + 15) / 16);
+    std::vector<uint32_t> w(stride + 1, 0xffffffffu);
+    straight_ops(g.b.row, g.b.col, type, g.b.R, g.b.C, g.rev ? OP_I : OP_D, w.data(), stride, sum);
+    bool same = int(ops.size()) == g.b.R;
+    for (size_t k = 0; same && k < ops.size(); k++) same = ops_field(w.data(), uint32_t(stride * 16 - ops.size() + k)) == ops[k];
+    n.c[3] += !same;
+    n.c[4] += memcmp(&sum, &want, sizeof(sum)) != 0;
+}
+
 template <bool AFFINE, int NB, int TYPE, bool MASK>
 void pair_run(Seg &a, Seg &b, Count n) {
     a.b.base = band_base<AFFINE, NB, TYPE>(a.b.R - a.b.C);
@@ -101,9 +123,9 @@ void pair_run(Seg &a, Seg &b, Count n) {
         std::vector<uint32_t> w(stride + 1, 0xffffffffu);
         const uint32_t up = g.rev ? OP_I : OP_D, left = g.rev ? OP_D : OP_I;
         OpsPut put{w.data(), int32_t(stride * 16)};
-        bool ok = band_walk<AFFINE, NB, TYPE>(g.b, Codes{st, h}, up, left, put);
-        put.finish(sum);
-        ok = ok && put.n == ops.size();
+        const int32_t np = band_walk<AFFINE, NB, TYPE>(g.b, Codes{st, h}, up, left, put);
+        bool ok = np == int32_t(ops.size());
+        if (ok) ops_summary(w.data(), stride * 16 - uint32_t(np), uint32_t(np), sum);
         for (size_t k = 0; ok && k < ops.size(); k++) ok = ops_field(w.data(), uint32_t(stride * 16 - ops.size() + k)) == ops[k];
         n.c[3] += !ok;
         n.c[4] += memcmp(&sum, &want, sizeof(sum)) != 0;
@@ -133,6 +155,10 @@ bool takes(int nb, bool mask, const Seg &g, int type) {
 }
 
 void pair_any(bool affine, int nb, int type, bool mask, Seg &a, Seg &b, Count n) {
+    if (nb == 0) {  // the screen alone
+        for (const Seg *g : {&a, &b}) affine ? screen_run<true>(*g, type, n) : screen_run<false>(*g, type, n);
+        return;
+    }
     if (!takes(nb, mask, a, type) || !takes(nb, mask, b, type)) return;
     if (affine) {
         if (nb == 4) pair_type<true, 4>(type, mask, a, b, n);
@@ -202,7 +228,7 @@ void band_random(int affine, int nb, int mask, uint64_t seed, uint64_t pairs, in
                 row.insert(type == BT_RIGHT ? row.begin() : row.end(), c);
             }
             while (int(row.size()) < C) row.push_back(uint8_t(rng_next(x) & 3));
-            if (type == BT_NONE && int(row.size()) > C + nb - 2) row.resize(C);
+            if (type == BT_NONE && int(row.size()) > C + (nb > 2 ? nb - 2 : 0)) row.resize(C);
             const bool swap = (rng_next(x) & 1) && int(row.size()) > C;  // the query on the rows
             const int64_t band = band_max > 0 ? int64_t(rng_next(x) % uint64_t(band_max)) : 65535;
             const auto &s = swap ? col : row, &q = swap ? row : col;

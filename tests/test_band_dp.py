@@ -34,7 +34,8 @@ def _clean(counts):
     return segments, certified, straight
 
 
-@pytest.mark.parametrize("affine,nb", [(1, 4), (1, 8), (1, 16), (0, 4), (0, 8)])
+# nb 0: the segments finished without a window (at most one mismatch on the main diagonal)
+@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 4), (1, 8), (1, 16), (0, 0), (0, 4), (0, 8)])
 @pytest.mark.parametrize("kind", [0, 1, 2], ids=["both", "right", "left"])
 def test_every_short_segment(band, affine, nb, kind):
     n = np.zeros(3, np.int64)
@@ -45,10 +46,10 @@ def test_every_short_segment(band, affine, nb, kind):
                     c = (C.c_uint64 * 6)()
                     band.band_exhaustive(affine, nb, kind, mask, letters, rows, cols, C.c_int64(m), c)
                     n += _clean(list(c))
-    assert n[0] > n[2] > 0 and n[1] > n[0] // 4  # the certificate accepts, and not only straight paths
+    assert n[1] > n[2] > 0 and n[1] > n[0] // (4 if nb else 50)  # it accepts, and not only the plainest paths
 
 
-@pytest.mark.parametrize("affine,nb", [(1, 8), (1, 16), (1, 24), (1, 40), (0, 8), (0, 16)])
+@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 8), (1, 16), (1, 24), (1, 40), (0, 0), (0, 8), (0, 16)])
 @pytest.mark.parametrize("cmax", [5, 40, 250, 1023])
 def test_random_segments(band, affine, nb, cmax):
     for mask, m in ((0, 0), (1, 4), (1, 30)):
