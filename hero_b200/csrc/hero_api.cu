@@ -62,8 +62,7 @@ struct hero_ctx {
         cs_gnch, cs_gbest, cs_gkept, cs_gkeys, cs_gdp;
     DBuf ch_subj, ch_query, ch_key_off, ch_seg_off, ch_nkeys, ch_nseg, ch_orient, ch_status,
         ch_win, ch_rate, ch_len;
-    DBuf keys, segs, sums, cells, ops, perm, bins, bin_off, tb, bnd, dp_tasks, winners;
-    DBuf win_sorted, win_bins;  // winners sorted by chain shape, and the sort's bins
+    DBuf keys, segs, sums, cells, ops, perm, bins, bin_off, tb, bnd, dp_tasks;
     DBuf scan_tmp, counters;
     // alignment output: record lists, text units and the batch's text
     DBuf a_list, a_n, a_roff, a_unit, a_len, a_pre, a_cig, a_uoff, a_text;
@@ -113,9 +112,9 @@ struct hero_ctx {
                         &cs_gnch, &cs_gbest, &cs_gkept, &cs_gkeys, &cs_gdp, &ch_subj, &ch_query,
                         &ch_key_off, &ch_seg_off, &ch_nkeys, &ch_nseg, &ch_orient, &ch_status,
                         &ch_win, &ch_rate, &ch_len, &keys, &segs, &sums, &cells, &ops, &perm,
-                        &bins, &bin_off, &tb, &bnd, &dp_tasks, &winners, &scan_tmp, &counters, &x_cnt, &x_koff,
+                        &bins, &bin_off, &tb, &bnd, &dp_tasks, &scan_tmp, &counters, &x_cnt, &x_koff,
                         &x_klo, &x_khi, &x_kval, &x_owner, &x_count, &x_slot_of, &x_start,
-                        &x_fill, &x_tmp, &q_job, &win_sorted, &win_bins, &a_list, &a_n,
+                        &x_fill, &x_tmp, &q_job, &a_list, &a_n,
                         &a_roff, &a_unit, &a_len, &a_pre, &a_cig, &a_uoff, &a_text, &q_ext,
                         &m_seq, &m_len, &map_hist, &map_max, &wcache, &q_pack, &s_pack,
                         &w_key, &w_order, &w_rest, &w_bin, &w_codes};
@@ -685,8 +684,8 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         if ((r = c->ensure(c->scan_tmp, scan_tmp_bytes(std::max<uint64_t>(nseg + 1, kDpBins + 1)), "scan"))) break;
         // zero the per-batch counters that size buffers (keep the running totals)
         if ((r = c->cuda(cudaMemsetAsync(ctr + C_NC, 0, sizeof(unsigned long long) * (C_MAXC - C_NC + 1), c->st), "batch: counters"))) break;
-        static_assert(C_WIN == C_OVERFLOW + 1 && C_REST == C_WIN + 1, "cleared together");
-        if ((r = c->cuda(cudaMemsetAsync(ctr + C_OVERFLOW, 0, 3 * sizeof(unsigned long long), c->st), "batch: counters"))) break;
+        static_assert(C_REST == C_OVERFLOW + 1, "cleared together");
+        if ((r = c->cuda(cudaMemsetAsync(ctr + C_OVERFLOW, 0, 2 * sizeof(unsigned long long), c->st), "batch: counters"))) break;
         // the count pass leaves the slot of every window (2 x 8 bytes a subject base) for the emit pass
         if ((r = c->ensure(c->wcache, std::max<uint64_t>(nbases, 1) * 16, "probe windows"))) break;
         uint2 *wc = P_<uint2>(c->wcache);
@@ -786,26 +785,19 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
             rec(5);
             if ((r = aln_batch(c, subj, nsub, q, ch, NC, stride))) break;
         } else {
-            if ((r = c->ensure(c->winners, std::max<uint64_t>(NC, 1) * 4, "winners"))) break;
-            if ((r = c->ensure(c->win_sorted, std::max<uint64_t>(NC, 1) * 4, "winners"))) break;
-            if ((r = c->ensure(c->win_bins, kWinScratch * 4, "winners"))) break;
             if (c->mapping) {
                 if ((r = c->ensure(c->a_list, std::max<uint64_t>(NC, 1) * 4, "mapping lists"))) break;
                 launch_map_choose(c->p, nsub, P_<uint32_t>(c->seg_cstart), P_<uint32_t>(c->seg_ccount),
                                   ch, P_<uint32_t>(c->keys), subj, q, P_<DpSum>(c->sums),
-                                  P_<uint32_t>(c->a_list), P_<uint32_t>(c->winners), ctr, c->st);
-            } else {
-                launch_dedupe(nsub, P_<uint32_t>(c->seg_cstart), P_<uint32_t>(c->seg_ccount), ch,
-                              P_<uint32_t>(c->winners), ctr, c->st);
+                                  P_<uint32_t>(c->a_list), ctr, c->st);
             }
             rec(5);
-            launch_vote(c->p, NC, ch, P_<uint32_t>(c->winners), P_<uint32_t>(c->win_sorted),
-                        P_<uint32_t>(c->win_bins), P_<uint32_t>(c->keys), subj, q,
-                        P_<uint32_t>(c->ops), stride, P_<DpSum>(c->sums), P_<uint32_t>(c->cov),
-                        P_<int32_t>(c->mdiff), ctr, c->st);
+            launch_vote(c->p, c->mapping, NC, ch, P_<uint32_t>(c->seg_cstart), P_<uint32_t>(c->seg_ccount),
+                        P_<uint32_t>(c->keys), subj, q, P_<uint32_t>(c->ops), stride, P_<DpSum>(c->sums),
+                        P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff), ctr, c->st);
             if (c->merge)
-                launch_vote_overhang(c->p, NC, ch, P_<uint32_t>(c->winners), P_<uint32_t>(c->keys),
-                                     subj, q, P_<DpSum>(c->sums), P_<uint32_t>(c->q_ext), ctr, c->st);
+                launch_vote_overhang(c->p, NC, ch, P_<uint32_t>(c->keys), subj, q, P_<DpSum>(c->sums),
+                                     P_<uint32_t>(c->q_ext), c->st);
         }
         if ((r = c->check_launch("record/vote"))) break;
         if (cap) break;

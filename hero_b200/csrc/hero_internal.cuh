@@ -76,7 +76,6 @@ enum Counter : int {
     C_CELLS_ALL,    // band cells of every segment computed
     C_ANOMALY,
     C_OVERFLOW,
-    C_WIN,          // winners of the current batch (compacted list length)
     C_REST,         // DP segments of the current batch the window DP left to the whole-matrix kernels
     C_OVERFLOW_ALL, // overflows over the context's life (C_OVERFLOW is cleared per batch)
     C_CELLS_PAIR,   // band cells computed in 16-bit pairs (of C_CELLS_ALL's)
@@ -139,7 +138,7 @@ void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView 
 void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
                        const uint32_t *ccount, ChainArrays ch, const uint32_t *keys,
                        ReadsView subj, ReadsView q, const DpSum *sums, uint32_t *alist,
-                       uint32_t *winners, unsigned long long *counters, cudaStream_t st);
+                       unsigned long long *counters, cudaStream_t st);
 void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
                      unsigned long long *hist, unsigned long long *maxc, cudaStream_t st);
 void launch_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits, cudaStream_t st);
@@ -241,15 +240,9 @@ uint64_t dp_threads(int device);
 void launch_assemble(const Params &p, uint64_t nc, ChainArrays ch, const uint32_t *keys,
                      ReadsView subj, ReadsView q, const DpSum *sums, const uint32_t *cells,
                      unsigned long long *counters, cudaStream_t st);
-// winners (one per subject x query) are appended to `winners`; the count is
-// counters[C_WIN]
-void launch_dedupe(uint64_t nsub, const uint32_t *seg_chain_start,
-                   const uint32_t *seg_chain_count, ChainArrays ch, uint32_t *winners,
-                   unsigned long long *counters, cudaStream_t st);
 // Votes.  A mismatch votes the subject base into cov[pos][4]; a run of matches
 // votes the query's own base, recorded as +1/-1 at the run's ends in mdiff
 // (a per-read difference array, summed by the consensus).
-constexpr uint32_t kWinScratch = 3 * 512;  // uint32 bins, offsets and cursors of the winner sort
 constexpr uint32_t kUnitSubject = 0x80000000u;  // header unit: kUnitSubject | subject
 constexpr uint32_t kUnitEnd = 0xffffffffu;      // closing newline of a subject
 constexpr uint32_t kUnitChainLimit = kUnitSubject;  // chains and subjects of a batch stay below
@@ -271,19 +264,18 @@ void launch_aln_write(const Params &p, uint64_t nunit, const uint32_t *unit, con
                       ChainArrays ch, const uint32_t *keys, ReadsView subj, ReadsView q,
                       const uint32_t *ops, uint32_t stride, const DpSum *sums,
                       const uint32_t *upre, const uint32_t *ucig, char *text, cudaStream_t st);
-// --merge: overhang votes of the batch's winners (after launch_vote; ext is
+// --merge: overhang votes of the batch's kept records (after launch_vote; ext is
 // uint32 [query reads][kOverhang][4]), and the pair merge after the consensus
-void launch_vote_overhang(const Params &p, uint64_t max_winners, ChainArrays ch,
-                          const uint32_t *winners, const uint32_t *keys, ReadsView subj,
-                          ReadsView q, const DpSum *sums, uint32_t *ext,
-                          const unsigned long long *counters, cudaStream_t st);
+void launch_vote_overhang(const Params &p, uint64_t nc, ChainArrays ch, const uint32_t *keys, ReadsView subj,
+                          ReadsView q, const DpSum *sums, uint32_t *ext, cudaStream_t st);
 void launch_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_t *corrected,
                         const uint32_t *ext, uint8_t *merged, uint32_t *merged_len,
                         cudaStream_t st);
-void launch_vote(const Params &p, uint64_t max_winners, ChainArrays ch, const uint32_t *winners,
-                 uint32_t *sorted, uint32_t *win_bins, const uint32_t *keys, ReadsView subj,
-                 ReadsView q, const uint32_t *ops, uint32_t stride, const DpSum *sums,
-                 uint32_t *cov, int32_t *mdiff, unsigned long long *counters, cudaStream_t st);
+// chosen: the records flagged in ch.win vote; else those SubjectRead::addAlignment keeps (and flags)
+void launch_vote(const Params &p, bool chosen, uint64_t nc, ChainArrays ch, const uint32_t *cstart,
+                 const uint32_t *ccount, const uint32_t *keys, ReadsView subj, ReadsView q,
+                 const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov, int32_t *mdiff,
+                 unsigned long long *counters, cudaStream_t st);
 void launch_consensus(const Params &p, ReadsView q, const uint32_t *cov, const int32_t *mdiff,
                       uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
                       uint32_t *imax, double *mis, cudaStream_t st);

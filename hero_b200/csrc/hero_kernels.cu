@@ -10,8 +10,8 @@
 //   BandAligner::calculateAlignment                   k_band_* (hero_band.cu), then for the
 //                                                     segments they leave: k_dp_scatter, k_dp*
 //   AlignmentRecord scoring + early exits             k_assemble
-//   SubjectRead::addAlignment                         k_dedupe
-//   SubjectRead::updateQueryCoverage                  k_vote
+//   SubjectRead::addAlignment,
+//   SubjectRead::updateQueryCoverage                  k_vote (record_wins, VoteVisitor)
 //   QueryRead::callConsensus + coverage statistics    k_consensus
 #include <cuda_runtime.h>
 
@@ -1563,37 +1563,40 @@ __global__ void k_assemble(Params p, uint64_t nc, ChainArrays ch, const uint32_t
     }
 }
 
-// SubjectRead::addAlignment (SubjectRead.cpp:25-79): one record per (subject,
-// query); forward chains arrive before reverse-complement chains.
-__global__ void k_dedupe(uint64_t nsub, const uint32_t *seg_chain_start,
-                         const uint32_t *seg_chain_count, ChainArrays ch, uint32_t *winners,
-                         unsigned long long *counters) {
-    unsigned long long kept = 0;
-    for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < nsub;
-         s += uint64_t(gridDim.x) * blockDim.x) {
-        uint32_t i = seg_chain_start[2 * s], ie = i + seg_chain_count[2 * s];
-        uint32_t j = seg_chain_start[2 * s + 1], je = j + seg_chain_count[2 * s + 1];
-        while (i < ie || j < je) {
-            const uint32_t qi = i < ie ? ch.query[i] : 0xffffffffu;
-            const uint32_t qj = j < je ? ch.query[j] : 0xffffffffu;
-            const uint32_t qq = qi < qj ? qi : qj;
-            int64_t best = -1;
-            auto consider = [&](uint32_t c) {
-                if (ch.status[c] != CH_ACCEPTED) return;
-                if (best < 0 || record_better(ch.rate[c], ch.len[c], ch.rate[best], ch.len[best]))
-                    best = c;
-            };
-            while (i < ie && ch.query[i] == qq) consider(i++);
-            while (j < je && ch.query[j] == qq) consider(j++);
-            if (best >= 0) {
-                ch.win[best] = 1;
-                winners[atomicAdd(&counters[C_WIN], 1ull)] = uint32_t(best);
-                kept++;
-            }
+// SubjectRead::addAlignment (SubjectRead.cpp:25-79) keeps one record per
+// (subject, query): the first in arrival order -- forward chains, then
+// reverse-complement chains, each list sorted by query -- among the best
+// (record_better is a strict weak order).  So a chain settles its own fate: no
+// earlier record of its query may be as good, no later one better.  Its own
+// list holds those beside it; the other orientation's are found by bisection.
+__device__ __forceinline__ bool record_wins(const ChainArrays &ch, uint32_t c, const uint32_t *cstart,
+                                            const uint32_t *ccount) {
+    const uint32_t q = ch.query[c], o = ch.orient[c], seg = 2u * ch.subj[c] + o;
+    const double rs = ch.rate[c], ln = ch.len[c];
+    auto earlier = [&](uint32_t e) {  // an earlier record that c does not replace
+        return ch.status[e] == CH_ACCEPTED && !record_better(rs, ln, ch.rate[e], ch.len[e]);
+    };
+    auto later = [&](uint32_t e) {  // a later record that replaces c
+        return ch.status[e] == CH_ACCEPTED && record_better(ch.rate[e], ch.len[e], rs, ln);
+    };
+    const uint32_t b = cstart[seg], e = b + ccount[seg];
+    for (uint32_t j = c; j > b && ch.query[j - 1] == q; j--)
+        if (earlier(j - 1)) return false;
+    for (uint32_t j = c + 1; j < e && ch.query[j] == q; j++)
+        if (later(j)) return false;
+    uint32_t lo = cstart[seg ^ 1u], hi = lo + ccount[seg ^ 1u];
+    const uint32_t end = hi;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (ch.query[mid] < q) {
+            lo = mid + 1u;
+        } else {
+            hi = mid;
         }
     }
-    kept = warp_sum(kept);
-    if (lane_id() == 0) atomicAdd(&counters[C_KEPT], kept);
+    for (; lo < end && ch.query[lo] == q; lo++)
+        if (o ? earlier(lo) : later(lo)) return false;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1644,11 +1647,11 @@ __global__ void k_aln_list(uint64_t nsub, const uint32_t *cstart, const uint32_t
 // accepted records in arrival order kept as SubjectRead::addAlignment keeps
 // them in consensus mode (keyed by the query's inner id, list_add), then
 // chooseQueryWithBestAlignment (SubjectRead.cpp:463-500, map_choose) picks the
-// records that vote; they become the batch's winners for k_vote.
+// records that vote (ch.win, which k_vote<true> reads).
 __global__ void k_map_choose(Params p, uint64_t nsub, const uint32_t *cstart,
                              const uint32_t *ccount, ChainArrays ch, const uint32_t *keys,
                              ReadsView subj, ReadsView q, const DpSum *sums, uint32_t *alist,
-                             uint32_t *winners, unsigned long long *counters) {
+                             unsigned long long *counters) {
     unsigned long long kept = 0;
     for (uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; s < nsub;
          s += uint64_t(gridDim.x) * blockDim.x) {
@@ -1694,7 +1697,6 @@ __global__ void k_map_choose(Params p, uint64_t nsub, const uint32_t *cstart,
         for (uint32_t i = 0; i < n_keep; i++) {
             const uint32_t c = L.get(n_keep == 1 && best >= 0 ? uint32_t(best) : i);
             ch.win[c] = 1;
-            winners[atomicAdd(&counters[C_WIN], 1ull)] = c;
         }
         kept += n_keep;
     }
@@ -1855,18 +1857,18 @@ struct VoteVisitor {
     uint32_t stride;
     const DpSum *sums;
     uint32_t seg;       // segment index of the next DP piece
-    int64_t ps = 0, pq = 0;
-    int64_t open = -1;  // start of the open match run
-    unsigned long long anomalies = 0;
+    int32_t ps = 0, pq = 0;
+    int32_t open = -1;  // start of the open match run
+    uint32_t anomalies = 0;
 
-    __device__ __forceinline__ uint8_t subj_code(int64_t i) const {
+    __device__ __forceinline__ uint8_t subj_code(int32_t i) const {
         return orient ? uint8_t(sc[Ls - 1 - i] ^ 2u) : sc[i];
     }
     __device__ __forceinline__ void close() {
         if (open < 0) return;
-        int64_t e = pq;
+        int32_t e = pq;
         if (e > Lq) {  // match votes past the read (the reference reads out of range)
-            anomalies += uint64_t(e - (open > Lq ? open : Lq));
+            anomalies += uint32_t(e - (open > Lq ? open : Lq));
             e = Lq;
         }
         if (open < e) {
@@ -1875,7 +1877,7 @@ struct VoteVisitor {
         }
         open = -1;
     }
-    __device__ __forceinline__ void match(int64_t c) {
+    __device__ __forceinline__ void match(int32_t c) {
         if (open < 0) open = pq;
         pq += c;
         ps += c;
@@ -1893,127 +1895,95 @@ struct VoteVisitor {
     }
     __device__ void begin(int64_t, int64_t, int64_t) {}
     __device__ void position(int64_t p) {
-        ps = p;
+        ps = int32_t(p);
         pq = 0;
     }
     __device__ void run(uint8_t t, int64_t c) {
         if (t == OP_M) {
-            match(c);
+            match(int32_t(c));
         } else {
-            close();
-            if (t == OP_I) {
-                pq += c;
-            } else {
-                ps += c;
-            }
+            gap(t, uint32_t(int32_t(c)));
         }
     }
+    // c skipped query (I) or subject (D) bases
+    __device__ __forceinline__ void gap(uint32_t op, uint32_t c) {
+        close();
+        if (op == OP_I) {
+            pq += c;
+        } else {
+            ps += c;
+        }
+    }
+    // The piece's first and last runs come from its summary -- the free run of an
+    // end piece alone is as long as the reads' overhang -- and its op words are
+    // read only when something between them is not a match.  (One op at a time
+    // through those runs took 37 ms of the 150 bp affine workload's 475.)
     __device__ void dp(int64_t, int64_t, int64_t, int64_t, uint32_t, int64_t) {
         const DpSum s = sums[seg];
         const uint32_t P = uint32_t(s.tot[0]) + s.tot[1] + s.tot[2] + s.tot[3];
-        if (s.tot[OP_M] == P) {  // one match run
-            match(P);
+        const uint32_t lead = s.ft >= OP_I ? s.fc : 0u;
+        const uint32_t tail = s.nruns >= 2 && s.lt >= OP_I ? s.lc : 0u;
+        if (lead) gap(s.ft, lead);
+        if (s.tot[OP_M] + lead + tail == P) {
+            if (s.tot[OP_M]) match(s.tot[OP_M]);
         } else {
             // ops a word (16) at a time: match stretches advance at once, the
             // other ops are found by their non-zero 2-bit fields (OP_M is 0)
             const uint32_t *w = ops + uint64_t(seg) * stride;
-            const uint32_t end = stride * 16u;
-            for (uint32_t pos = end - P; pos < end;) {
-                const uint32_t f0 = pos & 15u, nf = 16u - f0;  // fields left in this word
+            const uint32_t end = stride * 16u - tail;
+            for (uint32_t pos = stride * 16u - P + lead; pos < end;) {
+                const uint32_t f0 = pos & 15u, nf = min(16u - f0, end - pos);  // fields left in this word
                 const uint32_t word = w[pos >> 4] >> (2 * f0);
-                uint32_t nm = (word | (word >> 1)) & 0x55555555u;
+                uint32_t nm = (word | (word >> 1)) & ops_mask(0, nf - 1u);
                 uint32_t done = 0;
                 while (nm) {
                     const uint32_t b = uint32_t(__ffs(int(nm))) - 1u, fi = b >> 1;
-                    if (fi > done) match(int64_t(fi - done));
+                    if (fi > done) match(int32_t(fi - done));
                     const uint32_t op = (word >> b) & 3u;
                     if (op == OP_X) {
                         mismatch();
                     } else {
-                        close();
-                        if (op == OP_I) {
-                            pq++;
-                        } else {
-                            ps++;
-                        }
+                        gap(op, 1u);
                     }
                     done = fi + 1u;
                     nm &= nm - 1u;
                 }
-                if (nf > done) match(int64_t(nf - done));
+                if (nf > done) match(int32_t(nf - done));
                 pos += nf;
             }
         }
+        if (tail) gap(s.lt, tail);
         seg++;
     }
     __device__ bool check(int64_t, int64_t) { return true; }
     __device__ void finish() { close(); }
 };
 
-// Winners sorted by chain shape (DP pieces, keys) before the votes: a warp then
-// walks chains of one shape, and its lanes stay together (a counting sort over
-// kWinBins shapes; order inside a shape is free, votes commute).
-constexpr uint32_t kWinBins = 512;
-
-__device__ __forceinline__ uint32_t win_key(const ChainArrays &ch, uint32_t c) {
-    const uint32_t ns = ch.nseg[c], nk = ch.nkeys[c];
-    return ((ns < 31u ? ns : 31u) << 4) | (nk < 15u ? nk : 15u);
-}
-
-__global__ void k_win_hist(const unsigned long long *counters, ChainArrays ch,
-                           const uint32_t *winners, uint32_t *bins) {
-    __shared__ uint32_t h[kWinBins];
-    for (uint32_t i = threadIdx.x; i < kWinBins; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    const uint64_t nw = counters[C_WIN];
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nw;
-         i += uint64_t(gridDim.x) * blockDim.x)
-        atomicAdd(&h[win_key(ch, winners[i])], 1u);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kWinBins; i += blockDim.x)
-        if (h[i]) atomicAdd(&bins[i], h[i]);
-}
-
-// bins -> first slot of each shape (exclusive scan); cursors start at zero
-__global__ void k_win_offsets(const uint32_t *bins, uint32_t *off, uint32_t *cursor) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        uint32_t t = 0;
-        for (uint32_t i = 0; i < kWinBins; i++) {
-            off[i] = t;
-            t += bins[i];
-            cursor[i] = 0;
+// One thread a chain, in chain order: a warp's chains are neighbours, mostly of
+// one subject, so their arrays, summaries and ops are read as they lie.  The
+// rest is the scattered votes (atomics without a result), bound by the sectors
+// of the vote state they touch.  Sorting the records by shape first, so that a
+// warp's lanes agree, cost more in scattered reads (1.8 KB of DRAM a record)
+// and passes than it saved.  1.67 M x 150 bp, 80 M records: 51 -> 26 ms with
+// the selection and the sort.
+// CHOSEN: the records are flagged in ch.win (--mapping), else the kept ones vote
+// (and are flagged, for k_vote_overhang).
+template <bool CHOSEN>
+__global__ void __launch_bounds__(128)
+    k_vote(Params p, uint64_t nc, ChainArrays ch, const uint32_t *cstart, const uint32_t *ccount,
+           const uint32_t *keys, ReadsView subj, ReadsView q, const uint32_t *ops, uint32_t stride,
+           const DpSum *sums, uint32_t *cov, int32_t *mdiff, unsigned long long *counters) {
+    unsigned long long anomalies = 0, kept = 0;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nc;
+         i += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t ci = uint32_t(i);
+        if (CHOSEN) {
+            if (!ch.win[ci]) continue;
+        } else {
+            if (ch.status[ci] != CH_ACCEPTED || !record_wins(ch, ci, cstart, ccount)) continue;
+            ch.win[ci] = 1;
+            kept++;
         }
-    }
-}
-
-__global__ void k_win_scatter(const unsigned long long *counters, ChainArrays ch,
-                              const uint32_t *winners, const uint32_t *off, uint32_t *cursor,
-                              uint32_t *sorted) {
-    const uint32_t lane = lane_id();
-    const uint64_t nw = counters[C_WIN];
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < nw;
-         b += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t i = b + lane;
-        const uint32_t w = i < nw ? winners[i] : 0u;
-        const uint32_t key = i < nw ? win_key(ch, w) : 0xffffffffu;
-        const uint32_t same = __match_any_sync(0xffffffffu, key);
-        const uint32_t leader = uint32_t(__ffs(int(same))) - 1u;
-        uint32_t base = 0;
-        if (i < nw && lane == leader) base = atomicAdd(&cursor[key], uint32_t(__popc(same)));
-        base = __shfl_sync(0xffffffffu, base, int(leader));
-        if (i < nw) sorted[off[key] + base + __popc(same & ((1u << lane) - 1u))] = w;
-    }
-}
-
-__global__ void k_vote(Params p, const unsigned long long *counters_in, ChainArrays ch,
-                       const uint32_t *winners, const uint32_t *keys, ReadsView subj, ReadsView q,
-                       const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov,
-                       int32_t *mdiff, unsigned long long *counters) {
-    unsigned long long anomalies = 0;
-    const uint64_t nw = counters_in[C_WIN];
-    for (uint64_t wi = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; wi < nw;
-         wi += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t ci = winners[wi];
         const uint32_t s = ch.subj[ci], qid = ch.query[ci];
         VoteVisitor v;
         v.sc = subj.code + subj.off[s];
@@ -2031,7 +2001,11 @@ __global__ void k_vote(Params p, const unsigned long long *counters_in, ChainArr
         anomalies += v.anomalies;
     }
     anomalies = warp_sum(anomalies);
-    if (lane_id() == 0 && anomalies) atomicAdd(&counters[C_ANOMALY], anomalies);
+    kept = warp_sum(kept);
+    if (lane_id() == 0) {
+        if (anomalies) atomicAdd(&counters[C_ANOMALY], anomalies);
+        if (kept) atomicAdd(&counters[C_KEPT], kept);
+    }
 }
 
 // --merge: per kept record, the subject bases past its end voted into the
@@ -2039,13 +2013,11 @@ __global__ void k_vote(Params p, const unsigned long long *counters_in, ChainArr
 // SubjectRead.cpp:332-462; QueryRead::updateExtraCoverageMatrix,
 // QueryRead.cpp:352-369).  A second, light walk of each winner (positions and
 // DP totals only); k_vote is unchanged.
-__global__ void k_vote_overhang(Params p, const unsigned long long *counters_in, ChainArrays ch,
-                                const uint32_t *winners, const uint32_t *keys, ReadsView subj,
+__global__ void k_vote_overhang(Params p, uint64_t nc, ChainArrays ch, const uint32_t *keys, ReadsView subj,
                                 ReadsView q, const DpSum *sums, uint32_t *ext) {
-    const uint64_t nw = counters_in[C_WIN];
-    for (uint64_t wi = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; wi < nw;
-         wi += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t ci = winners[wi];
+    for (uint64_t ci = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; ci < nc;
+         ci += uint64_t(gridDim.x) * blockDim.x) {
+        if (!ch.win[ci]) continue;
         const uint32_t s = ch.subj[ci], qid = ch.query[ci];
         const DpSum *sm = sums + ch.seg_off[ci];
         auto piece = [sm](uint32_t i) { return sm[i]; };
@@ -2458,24 +2430,14 @@ void launch_assemble(const Params &p, uint64_t nc, ChainArrays ch, const uint32_
     }
 }
 
-void launch_dedupe(uint64_t nsub, const uint32_t *seg_chain_start,
-                   const uint32_t *seg_chain_count, ChainArrays ch, uint32_t *winners,
-                   unsigned long long *counters, cudaStream_t st) {
-    if (nsub) {
-        counted();
-        k_dedupe<<<grid_1d(nsub, 128), 128, 0, st>>>(nsub, seg_chain_start, seg_chain_count, ch,
-                                                     winners, counters);
-    }
-}
-
 void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
                        const uint32_t *ccount, ChainArrays ch, const uint32_t *keys,
                        ReadsView subj, ReadsView q, const DpSum *sums, uint32_t *alist,
-                       uint32_t *winners, unsigned long long *counters, cudaStream_t st) {
+                       unsigned long long *counters, cudaStream_t st) {
     if (!nsub) return;
     counted();
     k_map_choose<<<grid_1d(nsub, 128), 128, 0, st>>>(p, nsub, cstart, ccount, ch, keys, subj, q,
-                                                     sums, alist, winners, counters);
+                                                     sums, alist, counters);
 }
 
 void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
@@ -2523,33 +2485,25 @@ void launch_aln_write(const Params &p, uint64_t nunit, const uint32_t *unit, con
                                                      stride, sums, upre, ucig, text);
 }
 
-void launch_vote(const Params &p, uint64_t max_winners, ChainArrays ch, const uint32_t *winners,
-                 uint32_t *sorted, uint32_t *win_bins, const uint32_t *keys, ReadsView subj,
-                 ReadsView q, const uint32_t *ops, uint32_t stride, const DpSum *sums,
-                 uint32_t *cov, int32_t *mdiff, unsigned long long *counters, cudaStream_t st) {
-    if (!max_winners) return;
-    uint32_t *bins = win_bins, *off = win_bins + kWinBins, *cursor = win_bins + 2 * kWinBins;
-    cudaMemsetAsync(bins, 0, kWinBins * sizeof(uint32_t), st);
-    const unsigned g = grid_1d(max_winners, 256, 148u * 8u);
+void launch_vote(const Params &p, bool chosen, uint64_t nc, ChainArrays ch, const uint32_t *cstart,
+                 const uint32_t *ccount, const uint32_t *keys, ReadsView subj, ReadsView q,
+                 const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov, int32_t *mdiff,
+                 unsigned long long *counters, cudaStream_t st) {
+    if (!nc) return;
     counted();
-    k_win_hist<<<g, 256, 0, st>>>(counters, ch, winners, bins);
-    counted();
-    k_win_offsets<<<1, 32, 0, st>>>(bins, off, cursor);
-    counted();
-    k_win_scatter<<<g, 256, 0, st>>>(counters, ch, winners, off, cursor, sorted);
-    counted();
-    k_vote<<<grid_1d(max_winners, 128), 128, 0, st>>>(p, counters, ch, sorted, keys, subj, q, ops,
-                                                      stride, sums, cov, mdiff, counters);
+    const unsigned g = grid_1d(nc, 128);
+    if (chosen) {
+        k_vote<true><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, cov, mdiff, counters);
+    } else {
+        k_vote<false><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, cov, mdiff, counters);
+    }
 }
 
-void launch_vote_overhang(const Params &p, uint64_t max_winners, ChainArrays ch,
-                          const uint32_t *winners, const uint32_t *keys, ReadsView subj,
-                          ReadsView q, const DpSum *sums, uint32_t *ext,
-                          const unsigned long long *counters, cudaStream_t st) {
-    if (!max_winners) return;
+void launch_vote_overhang(const Params &p, uint64_t nc, ChainArrays ch, const uint32_t *keys, ReadsView subj,
+                          ReadsView q, const DpSum *sums, uint32_t *ext, cudaStream_t st) {
+    if (!nc) return;
     counted();
-    k_vote_overhang<<<grid_1d(max_winners, 128), 128, 0, st>>>(p, counters, ch, winners, keys, subj,
-                                                               q, sums, ext);
+    k_vote_overhang<<<grid_1d(nc, 128), 128, 0, st>>>(p, nc, ch, keys, subj, q, sums, ext);
 }
 
 void launch_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_t *corrected,
