@@ -58,8 +58,7 @@ struct hero_ctx {
     DBuf s_raw, s_code, s_off, s_len, s_uid, s_good;
     // batch buffers
     DBuf seg_hits, hit_off, hits, seg_cstart, seg_ccount;
-    DBuf cs_grp, cs_chain_of, cs_first, cs_last, cs_prev, cs_size, cs_coff, cs_ckeys, cs_kl,
-        cs_gnch, cs_gbest, cs_gkept, cs_gkeys, cs_gdp;
+    DBuf cs_grp, cs_chain_of, cs_first, cs_last, cs_prev, cs_ckeys, cs_kl;
     DBuf ch_subj, ch_query, ch_key_off, ch_seg_off, ch_nkeys, ch_nseg, ch_orient, ch_status,
         ch_win, ch_rate, ch_len;
     DBuf keys, segs, sums, cells, ops, perm, bins, bin_off, tb, bnd, dp_tasks;
@@ -108,8 +107,7 @@ struct hero_ctx {
                         &t_slots, &t_vals, &cov, &mdiff, &out_seq, &colsum, &o_imin, &o_imed, &o_imax,
                         &o_mis, &s_raw, &s_code, &s_off, &s_len, &s_uid, &s_good, &seg_hits,
                         &hit_off, &hits, &seg_cstart, &seg_ccount, &cs_grp, &cs_chain_of,
-                        &cs_first, &cs_last, &cs_prev, &cs_size, &cs_coff, &cs_ckeys, &cs_kl,
-                        &cs_gnch, &cs_gbest, &cs_gkept, &cs_gkeys, &cs_gdp, &ch_subj, &ch_query,
+                        &cs_first, &cs_last, &cs_prev, &cs_ckeys, &cs_kl, &ch_subj, &ch_query,
                         &ch_key_off, &ch_seg_off, &ch_nkeys, &ch_nseg, &ch_orient, &ch_status,
                         &ch_win, &ch_rate, &ch_len, &keys, &segs, &sums, &cells, &ops, &perm,
                         &bins, &bin_off, &tb, &bnd, &dp_tasks, &scan_tmp, &counters, &x_cnt, &x_koff,
@@ -710,9 +708,8 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
             DBuf *b;
             size_t per;
         } hb[] = {{&c->cs_grp, 4},     {&c->cs_chain_of, 4}, {&c->cs_first, 4}, {&c->cs_last, 4},
-                  {&c->cs_prev, 4},    {&c->cs_size, 4},     {&c->cs_coff, 4},  {&c->cs_ckeys, 4},
-                  {&c->cs_kl, 8},      {&c->cs_gnch, 4},     {&c->cs_gbest, 8}, {&c->cs_gkept, 4},
-                  {&c->cs_gkeys, 4},   {&c->cs_gdp, 4},      {&c->ch_subj, 4},  {&c->ch_query, 4},
+                  {&c->cs_prev, 4},    {&c->cs_ckeys, 4},    {&c->cs_kl, 8},
+                  {&c->ch_subj, 4},    {&c->ch_query, 4},
                   {&c->ch_key_off, 4}, {&c->ch_seg_off, 4},  {&c->ch_nkeys, 2}, {&c->ch_nseg, 2},
                   {&c->ch_orient, 1},  {&c->ch_status, 1},   {&c->ch_win, 1},   {&c->ch_rate, 8},
                   {&c->ch_len, 8},     {&c->keys, 4}};
@@ -720,18 +717,16 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
             if ((r = c->ensure(*x.b, Hc * x.per, "chains"))) break;
         if (r) break;
         if ((r = c->ensure(c->segs, 2 * Hc * sizeof(DpSeg), "DP segments"))) break;
-        ChainScratch sc{P_<uint32_t>(c->cs_grp),  P_<uint32_t>(c->cs_chain_of), P_<int32_t>(c->cs_first),
-                        P_<int32_t>(c->cs_last),  P_<int32_t>(c->cs_prev),      P_<int32_t>(c->cs_size),
-                        P_<int32_t>(c->cs_coff),  P_<int32_t>(c->cs_ckeys),     P_<int64_t>(c->cs_kl),
-                        P_<int32_t>(c->cs_gnch),  P_<int64_t>(c->cs_gbest),     P_<uint32_t>(c->cs_gkept),
-                        P_<uint32_t>(c->cs_gkeys), P_<uint32_t>(c->cs_gdp)};
+        ChainScratch sc{P_<uint32_t>(c->cs_grp), P_<uint32_t>(c->cs_chain_of), P_<int32_t>(c->cs_first),
+                        P_<int32_t>(c->cs_last), P_<int32_t>(c->cs_prev), P_<int32_t>(c->cs_ckeys),
+                        P_<int64_t>(c->cs_kl)};
         ChainArrays ch{P_<uint32_t>(c->ch_subj),   P_<uint32_t>(c->ch_query), P_<uint32_t>(c->ch_key_off),
                        P_<uint32_t>(c->ch_seg_off), P_<uint16_t>(c->ch_nkeys), P_<uint16_t>(c->ch_nseg),
                        P_<uint8_t>(c->ch_orient),  P_<uint8_t>(c->ch_status), P_<uint8_t>(c->ch_win),
                        P_<double>(c->ch_rate),     P_<double>(c->ch_len)};
-        launch_chain(c->p, nseg, subj, q, P_<uint64_t>(c->hit_off), P_<uint64_t>(c->hits), sc,
+        launch_chain(c->p, nsub, subj, q, P_<uint64_t>(c->hit_off), P_<uint64_t>(c->hits), sc,
                      P_<uint32_t>(c->seg_cstart), P_<uint32_t>(c->seg_ccount), ch,
-                     P_<uint32_t>(c->keys), P_<DpSeg>(c->segs), Hc, Hc, 2 * Hc, ctr, c->st);
+                     P_<uint32_t>(c->keys), P_<DpSeg>(c->segs), Hc, 2 * Hc, ctr, c->st);
         if ((r = c->check_launch("chain"))) break;
         if (!cap) {
             unsigned long long h_ctr[C_COUNT];

@@ -321,7 +321,7 @@ uint64_t band_warps(int device, uint64_t nd) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const uint64_t full = uint64_t(sms) * kBandBlocks;
-    const uint64_t need = (nd + kBandWarps - 1) / kBandWarps;  // a task holds one segment at least
+    const uint64_t need = (nd + 32 * kBandWarps - 1) / (32 * kBandWarps);  // half a task a warp
     return kBandWarps * (need < full ? (need ? need : 1) : full);
 }
 

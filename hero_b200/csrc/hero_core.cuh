@@ -363,6 +363,24 @@ HERO_HD bool walk_chain(const Params &p, int64_t Lq, int64_t Ls, const KeyAt &ke
     return true;
 }
 
+// BandAligner calls walk_chain makes for a chain, without walking it: the start
+// piece when the first key leaves bases on both reads, one per step that leaves
+// a gap on both, the end piece when bases are left on both.
+template <class KeyAt>
+HERO_HD uint32_t chain_dp_count(const Params &p, int32_t Lq, int32_t Ls, const KeyAt &keys, int32_t n) {
+    int32_t posQ = hit_posQ(keys(0)), posS = hit_posS(keys(0));
+    const int32_t ov = (posQ < posS ? posQ : posS) + (Lq - posQ < Ls - posS ? Lq - posQ : Ls - posS);
+    if (ov < p.l) return 0;
+    uint32_t dp = posQ != 0 && posS != 0;
+    for (int32_t i = 1; i < n; i++) {
+        const int32_t cQ = hit_posQ(keys(i)), cS = hit_posS(keys(i));
+        dp += posS + p.k < cS && posQ + p.k < cQ;
+        posQ = cQ;
+        posS = cS;
+    }
+    return dp + (posQ + p.k < Lq && posS + p.k != Ls);
+}
+
 // ---------------------------------------------------------------------------
 // record score: AlignmentRecord::addCigar + calculateScore (AlignmentRecord.cpp:35-100)
 // Only the first and last runs are treated specially (leading/trailing I or D

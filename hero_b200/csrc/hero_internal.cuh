@@ -64,7 +64,6 @@ enum Counter : int {
     C_HITS,
     C_CHAINS,
     C_NC,           // chains kept (allocated)
-    C_NK,           // chain keys
     C_ND,           // DP segments
     C_MAXR,
     C_MAXC,
@@ -93,15 +92,13 @@ struct ChainArrays {
 };
 enum : uint8_t { CH_NONE = 0, CH_REJECTED = 1, CH_ACCEPTED = 2 };
 
-// scratch parallel to the hit array used by the chaining kernel
+// scratch parallel to the hit array, for the groups that are not one chain
 struct ChainScratch {
-    uint32_t *grp;       // group starts
+    uint32_t *grp;       // group starts past those a warp keeps in shared memory
     uint32_t *chain_of;  // chain of each hit
-    int32_t *first, *last, *prev, *size, *coff, *ckeys;
-    int64_t *kl;
-    int32_t *g_nch;
-    int64_t *g_best;
-    uint32_t *g_kept, *g_keys, *g_dp;
+    int32_t *first, *last;  // ends of a group's chains, then their sizes and places
+    int32_t *prev, *ckeys;  // cursors; hits by chain
+    int64_t *kl;            // key lengths
 };
 
 // kernels launched through the launchers below since the library was loaded
@@ -142,11 +139,11 @@ void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
 void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
                      unsigned long long *hist, unsigned long long *maxc, cudaStream_t st);
 void launch_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits, cudaStream_t st);
-void launch_chain(const Params &p, uint64_t nseg, ReadsView subj, ReadsView q,
+void launch_chain(const Params &p, uint64_t nsub, ReadsView subj, ReadsView q,
                   const uint64_t *hit_off, const uint64_t *hits, ChainScratch sc,
                   uint32_t *seg_chain_start, uint32_t *seg_chain_count, ChainArrays ch,
-                  uint32_t *keys, DpSeg *segs, uint64_t cap_chains, uint64_t cap_keys,
-                  uint64_t cap_segs, unsigned long long *counters, cudaStream_t st);
+                  uint32_t *keys, DpSeg *segs, uint64_t cap_chains, uint64_t cap_segs,
+                  unsigned long long *counters, cudaStream_t st);
 
 constexpr uint32_t kShapeStripShift = 14;  // shape key: strips << 14 | align-left column << 10 | rows
 constexpr uint32_t kDpBins = 1u << 20;

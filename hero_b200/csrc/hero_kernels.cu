@@ -549,18 +549,9 @@ __global__ void __launch_bounds__(kSortThreads)
 
 // ---------------------------------------------------------------------------
 // chaining + record layout: processOneSubjectRead2 (SubjectReadAligner.cpp:805-852)
-// One warp per (subject, orientation); lane g takes query groups g, g+32, ...
+// One warp a subject, both orientations together; lane g takes query groups g,
+// g + 32, ... of its hits.
 // ---------------------------------------------------------------------------
-struct CountDp {
-    uint32_t n = 0;
-    HERO_HD void begin(int64_t, int64_t, int64_t) {}
-    HERO_HD void position(int64_t) {}
-    HERO_HD void run(uint8_t, int64_t) {}
-    HERO_HD void dp(int64_t, int64_t, int64_t, int64_t, uint32_t, int64_t) { n++; }
-    HERO_HD bool check(int64_t, int64_t) { return true; }
-    HERO_HD void finish() {}
-};
-
 struct EmitDp {
     DpSeg *out;
     uint32_t subj, query, orient;
@@ -592,177 +583,211 @@ struct EmitDp {
     HERO_HD void finish() {}
 };
 
-__global__ void __launch_bounds__(256)
-    k_chain(Params p, uint64_t nseg, ReadsView subj, ReadsView q, const uint64_t *hit_off,
+// Where a group's kept chains lie.  Nearly every group is one chain of all its
+// hits: that is settled from the hits alone, and the chain's keys are the hits.
+// Others go through the scratch arrays, which lie along the hits.
+struct GroupChains {
+    uint32_t kept, ndp;
+    int32_t nch;   // 0: one chain of all hits
+    int64_t best;  // key length of the kept chains (nch > 0)
+};
+
+__device__ __forceinline__ GroupChains group_chains(const Params &p, const uint64_t *G, int32_t gn, int32_t Lq,
+                                                    int32_t Ls, const ChainScratch &sc, uint64_t off) {
+    const int32_t q0 = hit_posQ(G[0]), s0 = hit_posS(G[0]);
+    int32_t eq = q0, es = s0, h = 1;
+    for (; h < gn; h++) {
+        const int32_t q = hit_posQ(G[h]), s = hit_posS(G[h]);
+        if (!same_alignment(p, q, s, q0, s0, eq, es)) break;
+        eq = q;
+        es = s;
+    }
+    auto hit = [G](int32_t i) { return G[i]; };
+    if (h == gn) return GroupChains{1u, chain_dp_count(p, Lq, Ls, hit, gn), 0, 0};
+    GroupChains r{0, 0, 0, 0};
+    r.nch = chain_group(p, hit, gn, sc.chain_of + off, sc.first + off, sc.last + off);
+    r.best = chain_key_lengths(p, hit, gn, sc.chain_of + off, r.nch, sc.kl + off, sc.prev + off);
+    // bucket the hits by chain, in order (first and last are free: sizes and places)
+    int32_t *size = sc.first + off, *place = sc.last + off, *cursor = sc.prev + off;
+    for (int32_t c = 0; c < r.nch; c++) size[c] = 0;
+    for (int32_t i = 0; i < gn; i++) size[sc.chain_of[off + i]]++;
+    int32_t run = 0;
+    for (int32_t c = 0; c < r.nch; c++) {
+        place[c] = cursor[c] = run;
+        run += size[c];
+    }
+    for (int32_t i = 0; i < gn; i++) sc.ckeys[off + cursor[sc.chain_of[off + i]]++] = i;
+    for (int32_t c = 0; c < r.nch; c++) {
+        if (sc.kl[off + c] != r.best) continue;
+        const int32_t *ck = sc.ckeys + off + place[c];
+        auto key = [G, ck](int32_t i) { return G[ck[i]]; };
+        r.kept++;
+        r.ndp += chain_dp_count(p, Lq, Ls, key, size[c]);
+    }
+    return r;
+}
+
+// A block takes eight subjects at a time: each warp finds its subject's groups
+// and counts their chains and DP pieces, one atomic places the eight subjects'
+// output, and each warp writes its own.  Chain keys lie at their group's hits
+// (a chain has no more keys than hits).  Bound by the latency of the hits and by
+// the output's 50 bytes a chain; with a warp an orientation, three atomics a
+// segment and every group in the scratch arrays it took 12.4 ms on 1.67 M x
+// 150 bp (80.7 M chains) and 1.77 ms on 300 k x 100 bp (6.1 M): now 7.4 ms
+// and 0.68 ms.
+constexpr int kChainWarps = 8;
+constexpr uint32_t kGroupStarts = 256;  // group starts a warp keeps in shared memory; more go to sc.grp
+
+__global__ void __launch_bounds__(kChainWarps * 32)
+    k_chain(Params p, uint64_t nsub, ReadsView subj, ReadsView q, const uint64_t *hit_off,
             const uint64_t *hits, ChainScratch sc, uint32_t *seg_chain_start,
             uint32_t *seg_chain_count, ChainArrays ch, uint32_t *keys, DpSeg *segs,
-            uint64_t cap_chains, uint64_t cap_keys, uint64_t cap_segs,
-            unsigned long long *counters) {
-    const uint32_t lane = lane_id();
-    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
+            uint64_t cap_chains, uint64_t cap_segs, unsigned long long *counters) {
+    __shared__ uint32_t starts[kChainWarps][kGroupStarts];
+    __shared__ uint32_t total[kChainWarps][2];
+    __shared__ unsigned long long at[2];
+    __shared__ int overflow;
+    const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     unsigned long long nchains_all = 0;
     int32_t maxr = 0, maxc = 0;
-    for (uint64_t seg = uint64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); seg < nseg;
-         seg += warps) {
-        const uint64_t base = hit_off[seg], n = hit_off[seg + 1] - base;
-        const uint32_t s = uint32_t(seg >> 1), orient = uint32_t(seg & 1);
-        if (n == 0) {
-            if (lane == 0) {
-                seg_chain_start[seg] = 0;
-                seg_chain_count[seg] = 0;
-            }
-            continue;
-        }
+    for (uint64_t s0 = uint64_t(blockIdx.x) * kChainWarps; s0 < nsub; s0 += uint64_t(gridDim.x) * kChainWarps) {
+        const uint64_t si = s0 + wib;
+        const uint32_t s = uint32_t(si);
+        const bool has = si < nsub;
+        const uint64_t base = has ? hit_off[2 * si] : 0;
+        const uint32_t n0 = has ? uint32_t(hit_off[2 * si + 1] - base) : 0u;  // forward hits
+        const uint32_t n = has ? uint32_t(hit_off[2 * si + 2] - base) : 0u;
         const uint64_t *H = hits + base;
-        // group starts (a group = hits of one query read)
-        uint32_t ng = 0;
-        for (uint64_t c0 = 0; c0 < n; c0 += 32) {
-            const uint64_t i = c0 + lane;
-            const bool flag = i < n && (i == 0 || hit_q(H[i]) != hit_q(H[i - 1]));
+        const int32_t Ls = has ? int32_t(subj.len[si]) : 0;
+        // group starts: a group is the hits of one query read in one orientation
+        uint32_t ng = 0, ng0 = 0;  // all, and the forward ones
+        for (uint32_t c0 = 0; c0 < n; c0 += 32) {
+            const uint32_t i = c0 + lane;
+            const bool flag = i < n && (i == 0 || i == n0 || hit_q(H[i]) != hit_q(H[i - 1]));
             const uint32_t m = __ballot_sync(0xffffffffu, flag);
-            if (flag) sc.grp[base + ng + __popc(m & ((1u << lane) - 1u))] = uint32_t(i);
+            if (flag) {
+                const uint32_t g = ng + __popc(m & ((1u << lane) - 1u));
+                if (g < kGroupStarts) starts[wib][g] = i;
+                else sc.grp[base + g] = i;
+            }
             ng += __popc(m);
+            ng0 += __popc(__ballot_sync(0xffffffffu, flag && i < n0));
         }
         __syncwarp();
-        const int32_t Ls = int32_t(subj.len[s]);
-        // pass A: chain every group, keep the results in the scratch
-        uint32_t tk = 0, tkeys = 0, tdp = 0;
+        auto start = [&](uint32_t g) { return g >= ng ? n : (g < kGroupStarts ? starts[wib][g] : sc.grp[base + g]); };
+        // count: the first 32 groups keep their result for the second pass
+        GroupChains mine{0, 0, 0, 0};
+        uint32_t tc = 0, tc0 = 0, td = 0;
         for (uint32_t g = lane; g < ng; g += 32) {
-            const uint32_t gs = sc.grp[base + g];
-            const uint32_t ge = (g + 1 < ng) ? sc.grp[base + g + 1] : uint32_t(n);
-            const int32_t gn = int32_t(ge - gs);
-            const uint64_t off = base + gs;
+            const uint32_t gs = start(g);
             const uint64_t *G = H + gs;
-            auto hit = [G](int32_t h) { return G[h]; };
-            const int32_t nch = chain_group(p, hit, gn, sc.chain_of + off, sc.first + off, sc.last + off);
-            const int64_t best = chain_key_lengths(p, hit, gn, sc.chain_of + off, nch, sc.kl + off, sc.prev + off);
-            // bucket the keys by chain, in order
-            for (int32_t c = 0; c < nch; c++) sc.size[off + c] = 0;
-            for (int32_t h = 0; h < gn; h++) sc.size[off + sc.chain_of[off + h]]++;
-            int32_t run = 0;
-            for (int32_t c = 0; c < nch; c++) {
-                sc.coff[off + c] = run;
-                sc.prev[off + c] = run;
-                run += sc.size[off + c];
-            }
-            for (int32_t h = 0; h < gn; h++) {
-                const uint32_t c = sc.chain_of[off + h];
-                sc.ckeys[off + sc.prev[off + c]++] = h;
-            }
-            const uint32_t qid = hit_q(G[0]);
-            const int64_t Lq = q.len[qid];
-            uint32_t kept = 0, nkeys = 0, ndp = 0;
-            for (int32_t c = 0; c < nch; c++) {
-                if (sc.kl[off + c] != best) continue;
-                kept++;
-                nkeys += uint32_t(sc.size[off + c]);
-                const int32_t *ck = sc.ckeys + off + sc.coff[off + c];
-                auto key = [G, ck](int32_t i) { return G[ck[i]]; };
-                CountDp cv;
-                walk_chain(p, Lq, Ls, key, sc.size[off + c], cv);
-                ndp += cv.n;
-            }
-            sc.g_nch[off] = nch;
-            sc.g_best[off] = best;
-            sc.g_kept[off] = kept;
-            sc.g_keys[off] = nkeys;
-            sc.g_dp[off] = ndp;
-            tk += kept;
-            tkeys += nkeys;
-            tdp += ndp;
-            nchains_all += uint64_t(nch);
+            const GroupChains r = group_chains(p, G, int32_t(start(g + 1) - gs), int32_t(q.len[hit_q(G[0])]), Ls, sc, base + gs);
+            if (g < 32) mine = r;
+            tc += r.kept;
+            tc0 += g < ng0 ? r.kept : 0u;
+            td += r.ndp;
+            nchains_all += uint64_t(r.nch ? r.nch : 1);
         }
-        tk = warp_sum(tk);
-        tkeys = warp_sum(tkeys);
-        tdp = warp_sum(tdp);
-        unsigned long long cs = 0, ks = 0, ds = 0;
-        int overflow = 0;
+        tc = warp_sum(tc);
+        tc0 = warp_sum(tc0);
+        td = warp_sum(td);
         if (lane == 0) {
-            cs = atomicAdd(&counters[C_NC], (unsigned long long)tk);
-            ks = atomicAdd(&counters[C_NK], (unsigned long long)tkeys);
-            ds = atomicAdd(&counters[C_ND], (unsigned long long)tdp);
-            if (cs + tk > cap_chains || ks + tkeys > cap_keys || ds + tdp > cap_segs) {
-                overflow = 1;
+            total[wib][0] = tc;
+            total[wib][1] = td;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t c = 0, d = 0;
+            for (int w = 0; w < kChainWarps; w++) {
+                c += total[w][0];
+                d += total[w][1];
+            }
+            at[0] = c ? atomicAdd(&counters[C_NC], (unsigned long long)c) : 0ull;
+            at[1] = d ? atomicAdd(&counters[C_ND], (unsigned long long)d) : 0ull;
+            overflow = (c && at[0] + c > cap_chains) || (d && at[1] + d > cap_segs);
+            if (overflow) {
                 atomicAdd(&counters[C_OVERFLOW], 1ull);
                 atomicAdd(&counters[C_OVERFLOW_ALL], 1ull);
             }
-            seg_chain_start[seg] = overflow ? 0u : uint32_t(cs);
-            seg_chain_count[seg] = overflow ? 0u : tk;
         }
-        overflow = __shfl_sync(0xffffffffu, overflow, 0);
-        if (overflow) continue;
-        cs = __shfl_sync(0xffffffffu, cs, 0);
-        ks = __shfl_sync(0xffffffffu, ks, 0);
-        ds = __shfl_sync(0xffffffffu, ds, 0);
-        // pass B: emit chains, keys and DP segments in (query, chain) order
-        for (uint32_t g0 = 0; g0 < ng; g0 += 32) {
+        __syncthreads();
+        uint64_t cs = at[0], ds = at[1];
+        for (uint32_t w = 0; w < wib; w++) {
+            cs += total[w][0];
+            ds += total[w][1];
+        }
+        const bool skip = overflow != 0;
+        if (has && lane == 0) {
+            seg_chain_start[2 * si] = skip ? 0u : uint32_t(cs);
+            seg_chain_count[2 * si] = skip ? 0u : tc0;
+            seg_chain_start[2 * si + 1] = skip ? 0u : uint32_t(cs + tc0);
+            seg_chain_count[2 * si + 1] = skip ? 0u : tc - tc0;
+        }
+        // write chains, keys and DP segments in (orientation, query, chain) order
+        for (uint32_t g0 = 0; g0 < (skip ? 0u : ng); g0 += 32) {
             const uint32_t g = g0 + lane;
-            const bool has = g < ng;
-            uint32_t gs = 0, gk = 0, gkeys = 0, gdp = 0;
-            if (has) {
-                gs = sc.grp[base + g];
-                gk = sc.g_kept[base + gs];
-                gkeys = sc.g_keys[base + gs];
-                gdp = sc.g_dp[base + gs];
-            }
-            uint32_t tot_c, tot_k, tot_d;
-            const uint32_t ec = warp_exclusive<uint32_t>(gk, &tot_c);
-            const uint32_t ek = warp_exclusive<uint32_t>(gkeys, &tot_k);
-            const uint32_t ed = warp_exclusive<uint32_t>(gdp, &tot_d);
-            if (has) {
-                const uint32_t ge = (g + 1 < ng) ? sc.grp[base + g + 1] : uint32_t(n);
-                const uint64_t off = base + gs;
-                const uint64_t *G = H + gs;
-                const uint32_t qid = hit_q(G[0]);
-                const int64_t Lq = q.len[qid];
-                const int32_t nch = sc.g_nch[off];
-                const int64_t best = sc.g_best[off];
-                (void)ge;
-                uint64_t ci = cs + ec, ki = ks + ek, di = ds + ed;
-                for (int32_t c = 0; c < nch; c++) {
-                    if (sc.kl[off + c] != best) continue;
-                    const int32_t sz = sc.size[off + c];
-                    const int32_t *ck = sc.ckeys + off + sc.coff[off + c];
-                    for (int32_t i = 0; i < sz; i++) {
-                        const uint64_t x = G[ck[i]];
-                        keys[ki + i] = (uint32_t(hit_posQ(x)) << 16) | uint32_t(hit_posS(x));
-                    }
-                    auto key = [G, ck](int32_t i) { return G[ck[i]]; };
-                    EmitDp ev;
-                    ev.out = segs + di;
-                    ev.subj = s;
-                    ev.query = qid;
-                    ev.orient = orient;
-                    ev.orient_shift = p.aln ? kSegQrcShift : kSegOrientShift;
-                    walk_chain(p, Lq, Ls, key, sz, ev);
-                    if (ev.maxr > maxr) maxr = ev.maxr;
-                    if (ev.maxc > maxc) maxc = ev.maxc;
-                    ch.subj[ci] = s;
-                    ch.query[ci] = qid;
-                    ch.key_off[ci] = uint32_t(ki);
-                    ch.seg_off[ci] = uint32_t(di);
-                    ch.nkeys[ci] = uint16_t(sz);
-                    ch.nseg[ci] = uint16_t(ev.n);
-                    ch.orient[ci] = uint8_t(orient);
-                    ch.status[ci] = CH_NONE;
-                    ch.win[ci] = 0;
-                    ci++;
-                    ki += uint32_t(sz);
-                    di += ev.n;
+            const bool on = g < ng;
+            const uint32_t gs = on ? start(g) : 0u;
+            const int32_t gn = on ? int32_t(start(g + 1) - gs) : 0;
+            const uint64_t *G = H + gs;
+            const uint64_t off = base + gs;
+            const uint32_t qid = on ? hit_q(G[0]) : 0u;
+            const int32_t Lq = on ? int32_t(q.len[qid]) : 0;
+            GroupChains r{0, 0, 0, 0};
+            if (on) r = g0 == 0 ? mine : group_chains(p, G, gn, Lq, Ls, sc, off);
+            uint32_t tot_c, tot_d;
+            uint64_t ci = cs + warp_exclusive<uint32_t>(r.kept, &tot_c);
+            uint64_t di = ds + warp_exclusive<uint32_t>(r.ndp, &tot_d);
+            cs += tot_c;
+            ds += tot_d;
+            if (!on) continue;
+            uint64_t ki = off;
+            auto emit = [&](int32_t sz, auto key) {
+                for (int32_t i = 0; i < sz; i++) {
+                    const uint64_t x = key(i);
+                    keys[ki + i] = (uint32_t(hit_posQ(x)) << 16) | uint32_t(hit_posS(x));
+                }
+                EmitDp ev;
+                ev.out = segs + di;
+                ev.subj = s;
+                ev.query = qid;
+                ev.orient = g < ng0 ? 0u : 1u;
+                ev.orient_shift = p.aln ? kSegQrcShift : kSegOrientShift;
+                walk_chain(p, int64_t(Lq), int64_t(Ls), key, sz, ev);
+                if (ev.maxr > maxr) maxr = ev.maxr;
+                if (ev.maxc > maxc) maxc = ev.maxc;
+                ch.subj[ci] = s;
+                ch.query[ci] = qid;
+                ch.key_off[ci] = uint32_t(ki);
+                ch.seg_off[ci] = uint32_t(di);
+                ch.nkeys[ci] = uint16_t(sz);
+                ch.nseg[ci] = uint16_t(ev.n);
+                ch.orient[ci] = uint8_t(ev.orient);
+                ch.status[ci] = CH_NONE;
+                ch.win[ci] = 0;
+                ci++;
+                ki += uint32_t(sz);
+                di += ev.n;
+            };
+            if (r.nch == 0) {
+                emit(gn, [G](int32_t i) { return G[i]; });
+            } else {
+                for (int32_t c = 0; c < r.nch; c++) {
+                    if (sc.kl[off + c] != r.best) continue;
+                    const int32_t *ck = sc.ckeys + off + sc.last[off + c];
+                    emit(sc.first[off + c], [G, ck](int32_t i) { return G[ck[i]]; });
                 }
             }
-            cs += tot_c;
-            ks += tot_k;
-            ds += tot_d;
         }
+        __syncthreads();  // starts, total and at are reused
     }
     nchains_all = warp_sum(nchains_all);
     maxr = warp_max(maxr);
     maxc = warp_max(maxc);
     if (lane == 0) {
-        atomicAdd(&counters[C_CHAINS], nchains_all);
-        atomicMax(&counters[C_MAXR], (unsigned long long)maxr);
-        atomicMax(&counters[C_MAXC], (unsigned long long)maxc);
+        if (nchains_all) atomicAdd(&counters[C_CHAINS], nchains_all);
+        if (maxr) atomicMax(&counters[C_MAXR], (unsigned long long)maxr);
+        if (maxc) atomicMax(&counters[C_MAXC], (unsigned long long)maxc);
     }
 }
 
@@ -2297,17 +2322,16 @@ void launch_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits, cu
     k_sort_hits<<<g, kSortThreads, 0, st>>>(nseg, hit_off, hits);
 }
 
-void launch_chain(const Params &p, uint64_t nseg, ReadsView subj, ReadsView q,
+void launch_chain(const Params &p, uint64_t nsub, ReadsView subj, ReadsView q,
                   const uint64_t *hit_off, const uint64_t *hits, ChainScratch sc,
                   uint32_t *seg_chain_start, uint32_t *seg_chain_count, ChainArrays ch,
-                  uint32_t *keys, DpSeg *segs, uint64_t cap_chains, uint64_t cap_keys,
-                  uint64_t cap_segs, unsigned long long *counters, cudaStream_t st) {
-    if (!nseg) return;
+                  uint32_t *keys, DpSeg *segs, uint64_t cap_chains, uint64_t cap_segs,
+                  unsigned long long *counters, cudaStream_t st) {
+    if (!nsub) return;
     counted();
-    k_chain<<<grid_1d(nseg, 8, 148u * 16u), 256, 0, st>>>(p, nseg, subj, q, hit_off, hits, sc,
-                                                        seg_chain_start, seg_chain_count, ch, keys,
-                                                        segs, cap_chains, cap_keys, cap_segs,
-                                                        counters);
+    k_chain<<<grid_1d(nsub, kChainWarps, 148u * 16u), kChainWarps * 32, 0, st>>>(
+        p, nsub, subj, q, hit_off, hits, sc, seg_chain_start, seg_chain_count, ch, keys, segs, cap_chains,
+        cap_segs, counters);
 }
 
 void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void *scan_tmp, cudaStream_t st) {

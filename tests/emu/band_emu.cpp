@@ -180,9 +180,44 @@ uint64_t rng_next(uint64_t &x) {
     return x * 0x2545f4914f6cdd1dull;
 }
 
+struct CountWalk {
+    uint32_t n = 0;
+    void begin(int64_t, int64_t, int64_t) {}
+    void position(int64_t) {}
+    void run(uint8_t, int64_t) {}
+    void dp(int64_t, int64_t, int64_t, int64_t, uint32_t, int64_t) { n++; }
+    bool check(int64_t, int64_t) { return true; }
+    void finish() {}
+};
+
 }  // namespace
 
 extern "C" {
+
+// random chains of increasing keys, with touching, overlapping and end-aligned
+// ones: chain_dp_count against the BandAligner calls of walk_chain
+uint64_t chain_counts(uint64_t seed, uint64_t chains) {
+    uint64_t x = seed * 0x9e3779b97f4a7c15ull + 1, wrong = 0;
+    for (uint64_t c = 0; c < chains; c++) {
+        Params p{int32_t(1 + rng_next(x) % 20), int32_t(rng_next(x) % 40), 1, 0, 1.0, double(rng_next(x) % 3) / 2, 0.6};
+        const int32_t n = 1 + int32_t(rng_next(x) % 5);
+        std::vector<uint64_t> keys;
+        int32_t q = int32_t(rng_next(x) % 4) * int32_t(rng_next(x) % 9), s = int32_t(rng_next(x) % 4) * int32_t(rng_next(x) % 9);
+        for (int32_t i = 0; i < n; i++) {
+            keys.push_back(hit_pack(0, uint32_t(q), uint32_t(s)));
+            const int32_t step = 1 + int32_t(rng_next(x) % uint64_t(2 * p.k));
+            q += rng_next(x) % 4 == 0 ? p.k : step;
+            s += rng_next(x) % 4 == 0 ? p.k : step + (rng_next(x) % 3 == 0 ? int32_t(rng_next(x) % 3) : 0);
+        }
+        const int32_t Lq = hit_posQ(keys.back()) + p.k + int32_t(rng_next(x) % 3) * int32_t(rng_next(x) % 20);
+        const int32_t Ls = hit_posS(keys.back()) + p.k + int32_t(rng_next(x) % 3) * int32_t(rng_next(x) % 20);
+        auto key = [&keys](int32_t i) { return keys[size_t(i)]; };
+        CountWalk w;
+        walk_chain(p, Lq, Ls, key, n, w);
+        wrong += w.n != chain_dp_count(p, Lq, Ls, key, n);
+    }
+    return wrong;
+}
 
 // every pair of strings of the first `letters` bases with R rows and C columns (codes 0..3)
 void band_exhaustive(int affine, int nb, int type, int mask, int letters, int R, int C, int64_t band, uint64_t *counts) {

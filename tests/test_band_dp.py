@@ -60,6 +60,11 @@ def test_random_segments(band, affine, nb, cmax):
         assert segments and certified > straight
 
 
+def test_dp_pieces_of_a_chain_counted_without_walking_it(band):
+    band.chain_counts.restype = C.c_uint64
+    assert band.chain_counts(C.c_uint64(3), C.c_uint64(200000)) == 0
+
+
 def _segments(rng, n):
     """(subject, query, band, flags): copies with e substitutions and at times an
     indel, on either side, with a free run on the anchored side's far end."""
