@@ -586,7 +586,7 @@ static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
     w.warps = band_warps(c->dev, a.nd);
     w.code_words = band_code_words(cmax, a.affine != 0);
     const size_t table = kBandBins * (sizeof(BandBin) + 4) + 16;
-    w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 4, "DP windows") &&
+    w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 8, "DP windows") &&
            c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 4, "DP windows") &&
            c->optional(b.bin, table, "DP windows") &&
            c->optional(b.codes, size_t(w.warps) * w.code_words * 4, "DP windows");
@@ -594,11 +594,11 @@ static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
     a.rest = w.on ? P_<uint32_t>(b.rest) : a.ops;
     a.perm = P_<uint32_t>(b.perm);
     if (w.on) {
-        w.key = P_<uint32_t>(b.key);
+        w.key = P_<uint2>(b.key);
         w.order = P_<uint32_t>(b.order);
         w.bin = P_<BandBin>(b.bin);
-        w.cursor = reinterpret_cast<uint32_t *>(w.bin + kBandBins);
-        w.head = w.cursor + kBandBins;
+        w.start = reinterpret_cast<uint32_t *>(w.bin + kBandBins);
+        w.head = w.start + kBandBins;
         w.codes = P_<uint32_t>(b.codes);
         w.count = a.bins + kDpBins;
     }

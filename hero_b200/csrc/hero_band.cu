@@ -37,18 +37,20 @@ __device__ __forceinline__ int band_type(const DpSeg &g) {
 
 // Window classes, widest first: 0..3 whole-band segments, 4..5 segments whose
 // band cuts the matrix.  A segment's mismatches on the main diagonal, e, bound
-// its deficit by 5 e, so few mismatches need only a narrow window (the limits
-// of 8, 16, 24 and 40 diagonals are 8, 13, 18 and 29 for the affine aligner, of
-// 8 and 16 diagonals 19 and 35 for the global one); from four on the cause is
-// mostly a gap, whose own deficit is small.
+// its deficit by 5 e, so few mismatches need only a narrow window: the limits
+// of 11, 19, 26 and 40 diagonals are 10, 16, 20 and 30 for the affine aligner, of
+// 8 and 16 diagonals 19 and 35 for the global one.  From five on the cause is
+// mostly a gap, whose own deficit is small: the widest certifies 83 % of them.
+// (Windows of 8, 16, 24 and 40 took 31 ms where these take 28.6.)
+constexpr int kBandMostMismatches = 5;
 template <bool AFFINE, int CLS>
 __host__ __device__ constexpr int band_width() {
-    return AFFINE ? (CLS == 0 ? 40 : CLS == 1 || CLS == 4 ? 24 : CLS == 2 || CLS == 5 ? 16 : 8)
+    return AFFINE ? (CLS == 0 ? 40 : CLS == 1 ? 26 : CLS == 2 ? 19 : CLS == 3 ? 11 : CLS == 4 ? 24 : 16)
                   : (CLS == 0 || CLS == 4 || CLS == 5 ? 16 : 8);
 }
 __device__ __forceinline__ int band_class(bool affine, bool masked, int32_t e) {
     if (masked) return affine && e > 2 ? 4 : 5;
-    if (affine) return e > 3 ? 0 : (e == 3 ? 1 : (e == 2 ? 2 : 3));
+    if (affine) return e > 4 ? 0 : (e == 4 ? 1 : (e == 3 ? 2 : 3));
     return e > 3 ? 0 : 3;
 }
 
@@ -82,38 +84,44 @@ __global__ void __launch_bounds__(256) k_band_screen(DpLaunch a, BandWork w) {
         const bool has = i < a.nd;
         DpSeg g{};
         uint32_t key = kBandNoKey;
-        bool rest = false;
+        bool rest = false, done = false, reversed = false;
+        int type = BT_NONE;
+        int32_t f = 0, e = kBandMostMismatches, R = 0, C = 0;
         if (has) {
             g = a.segs[i];
-            bool reversed;
-            BandSeg s = band_seg(a, g, reversed);
+            const BandSeg s = band_seg(a, g, reversed);
+            R = s.R;
+            C = s.C;
             if (a.cells) {
-                const uint64_t cl = band_cells(s.R, s.C, s.m);
+                const uint64_t cl = band_cells(R, C, s.m);
                 a.cells[i] = uint32_t(cl > 0xffffffffull ? 0xffffffffull : cl);
             }
-            const int type = band_type(g);
-            const int32_t d = s.R - s.C;
-            const bool masked = s.m < s.R, affine = a.affine != 0;
+            type = band_type(g);
+            const int32_t d = R - C;
+            const bool masked = s.m < R, affine = a.affine != 0;
             // both ends anchored on different diagonals: the widest window must hold both
             const int32_t most_d = affine ? (masked ? 12 : 24) : 8;
-            rest = !w.on || (g.flags & 3u) == 3u || s.C > kBandMaxC || (type == BT_NONE && d > most_d);
+            rest = !w.on || (g.flags & 3u) == 3u || C > kBandMaxC || (type == BT_NONE && d > most_d);
             if (!rest) {
-                int32_t f = 0, e = 4;
-                if (type != BT_NONE || d == 0) e = main_mismatches(s.row, s.col, main_row(type, s.R, s.C), s.C, 4, f);
-                if (e == 0 || (e == 1 && (affine ? one_mismatch_straight<true>(s.row, s.col, type, s.R, s.C, f)
-                                                 : one_mismatch_straight<false>(s.row, s.col, type, s.R, s.C, f)))) {
-                    DpSum sum;
-                    straight_ops(s.row, s.col, type, s.R, s.C, reversed ? uint32_t(OP_I) : uint32_t(OP_D),
-                                 a.ops + i * a.stride, a.stride, sum);
-                    a.sums[i] = sum;
-                } else {
-                    key = (uint32_t(band_class(affine, masked, e) * 3 + type) << kBandColBits) | uint32_t(kBandMaxC - s.C);
-                }
+                if (type != BT_NONE || d == 0)
+                    e = main_mismatches(s.row, s.col, main_row(type, R, C), C, kBandMostMismatches, f);
+                done = e == 0 || (e == 1 && (affine ? one_mismatch_straight<true>(s.row, s.col, type, R, C, f)
+                                                    : one_mismatch_straight<false>(s.row, s.col, type, R, C, f)));
+                if (!done) key = (uint32_t(band_class(affine, masked, e) * 3 + type) << kBandColBits) | uint32_t(kBandMaxC - C);
             }
         }
-        if (has && w.on) w.key[i] = key;
+        // the segment's place among those of its key: counted now, placed by k_band_scatter
         const uint32_t same = __match_any_sync(0xffffffffu, key);
-        if (key != kBandNoKey && lane == uint32_t(__ffs(int(same))) - 1u) atomicAdd(&w.count[key], uint32_t(__popc(same)));
+        const uint32_t leader = uint32_t(__ffs(int(same))) - 1u;
+        uint32_t rank = 0;
+        if (key != kBandNoKey && lane == leader) rank = atomicAdd(&w.count[key], uint32_t(__popc(same)));
+        if (done) {
+            DpSum sum;
+            plain_ops(type, R, C, e, f, reversed ? uint32_t(OP_I) : uint32_t(OP_D), a.ops + i * a.stride, a.stride, sum);
+            a.sums[i] = sum;
+        }
+        rank = __shfl_sync(0xffffffffu, rank, int(leader)) + __popc(same & ((1u << lane) - 1u));
+        if (has && w.on) w.key[i] = make_uint2(key, rank);
         rest_append(a, rest, uint32_t(i), g);
     }
 }
@@ -157,7 +165,7 @@ __global__ void __launch_bounds__(1024) k_band_tasks(BandWork w) {
         const uint32_t key = threadIdx.x * per + k;
         const uint32_t c = key < kBandBins ? w.count[key] : 0u;
         if (!c) continue;
-        w.cursor[key] = ex[0];
+        w.start[key] = ex[0];
         w.bin[ex[2]] = BandBin{key, ex[1], ex[0], c};
         ex[0] += c;
         ex[1] += (c + kTaskSegs - 1) / kTaskSegs;
@@ -171,17 +179,9 @@ __global__ void __launch_bounds__(1024) k_band_tasks(BandWork w) {
 }
 
 __global__ void __launch_bounds__(256) k_band_scatter(uint64_t nd, BandWork w) {
-    const uint32_t lane = lane_id();
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~uint64_t(31); b < nd;
-         b += uint64_t(gridDim.x) * blockDim.x) {
-        const uint64_t i = b + lane;
-        const uint32_t key = i < nd ? w.key[i] : kBandNoKey;
-        const uint32_t same = __match_any_sync(0xffffffffu, key);
-        const uint32_t leader = uint32_t(__ffs(int(same))) - 1u;
-        uint32_t at = 0;
-        if (key != kBandNoKey && lane == leader) at = atomicAdd(&w.cursor[key], uint32_t(__popc(same)));
-        at = __shfl_sync(0xffffffffu, at, int(leader));
-        if (key != kBandNoKey) w.order[at + __popc(same & ((1u << lane) - 1u))] = uint32_t(i);
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nd; i += uint64_t(gridDim.x) * blockDim.x) {
+        const uint2 k = w.key[i];
+        if (k.x != kBandNoKey) w.order[w.start[k.x] + k.y] = uint32_t(i);
     }
 }
 
@@ -277,9 +277,9 @@ __device__ __forceinline__ void band_dispatch(int type, const DpLaunch &a, const
 
 // Persistent warps fed by a queue of tasks.  Measured, DP stage of one
 // correction before (every matrix whole) and with the window: 5 Mbp affine,
-// 1.67 M x 150 bp, 109 M segments, 358 -> 55 ms; 1 Mbp global, 300 k x 100 bp,
-// 7.3 -> 1.6 ms; 300 kbp affine with -i 2 (bands of a few diagonals), 80 k x
-// 150 bp, 34.5 -> 1.8 ms.
+// 1.67 M x 150 bp, 109 M segments, 358 -> 42 ms; 1 Mbp global, 300 k x 100 bp,
+// 7.3 -> 1.0 ms; 300 kbp affine with -i 2 (bands of a few diagonals), 80 k x
+// 150 bp, 34.5 -> 1.5 ms.
 constexpr int kBandWarps = 4, kBandBlocks = 3;  // 12 warps an SM: 168 registers hold the widest window
 
 template <bool AFFINE>

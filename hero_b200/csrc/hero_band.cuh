@@ -67,6 +67,32 @@ HERO_HD uint32_t pack16(const PackSeq &s, int32_t t) {
     return s.dir > 0 ? x : reverse_fields(x) ^ 0xaaaaaaaau;
 }
 
+// pack16 at t0, t0 + 16, ... of a stretch, one word loaded a call
+struct PackStream {
+    const uint32_t *p;
+    uint32_t cur, sh;
+    int32_t step;
+    HERO_HD PackStream(const PackSeq &s, int32_t t0) {
+        const int64_t at = s.dir > 0 ? s.at + t0 : s.at - t0 - 15;
+        const uint32_t *w = s.w + (at >> 4);
+        step = s.dir;
+        sh = uint32_t(at & 15) * 2u;
+        cur = w[step > 0 ? 0 : 1];
+        p = w + (step > 0 ? 1 : 0);
+    }
+    HERO_HD uint32_t next() {
+        const uint32_t n = *p, lo = step > 0 ? cur : n, hi = step > 0 ? n : cur;
+        p += step;
+        cur = n;
+#if defined(__CUDA_ARCH__)
+        const uint32_t x = __funnelshift_r(lo, hi, sh);
+#else
+        const uint32_t x = uint32_t(((uint64_t(hi) << 32) | lo) >> sh);
+#endif
+        return step > 0 ? x : reverse_fields(x) ^ 0xaaaaaaaau;
+    }
+};
+
 // 01 in every field where two packed words differ: OP_X there, OP_M elsewhere
 HERO_HD uint32_t mismatch16(uint32_t a, uint32_t b) {
     const uint32_t x = a ^ b;
@@ -473,8 +499,9 @@ HERO_HD int32_t main_mismatches(const PackSeq &row, const PackSeq &col, int32_t 
                                 int32_t &first) {
     int32_t e = 0;
     first = C;
+    PackStream a(row, r0), b(col, 0);
     for (int32_t t = 0; t < C && e < most; t += 16) {
-        uint32_t x = mismatch16(pack16(row, r0 + t), pack16(col, t));
+        uint32_t x = mismatch16(a.next(), b.next());
         if (C - t < 16) x &= ops_mask(0, uint32_t(C - t - 1));
         if (x && first == C) first = t + (low_bit(x) >> 1);
         e += popc32(x);
@@ -484,8 +511,9 @@ HERO_HD int32_t main_mismatches(const PackSeq &row, const PackSeq &col, int32_t 
 
 // a mismatch among columns [a, b) (0-based) against the rows r0 + column
 HERO_HD bool any_mismatch(const PackSeq &row, const PackSeq &col, int32_t r0, int32_t a, int32_t b) {
+    PackStream u(row, r0 + a), v(col, a);
     for (int32_t t = a; t < b; t += 16) {
-        uint32_t x = mismatch16(pack16(row, r0 + t), pack16(col, t));
+        uint32_t x = mismatch16(u.next(), v.next());
         if (b - t < 16) x &= ops_mask(0, uint32_t(b - t - 1));
         if (x) return true;
     }
@@ -522,16 +550,47 @@ HERO_HD void straight_ops(const PackSeq &row, const PackSeq &col, int type, int3
     const int32_t end = int32_t(stride) * 16, first = end - R;  // R = d + C ops
     const int32_t ds = type == BT_RIGHT ? first + d : first, de = ds + C;
     const int32_t gs = type == BT_RIGHT ? first : de;           // the gap's range [gs, gs + d)
+    PackStream u(row, r0 + (first & ~15) - ds), v(col, (first & ~15) - ds);
     for (int32_t k = first >> 4; k < int32_t(stride); k++) {
         const int32_t p0 = k * 16;
+        const uint32_t m = mismatch16(u.next(), v.next());
         uint32_t x = 0;
         const int32_t a = ds > p0 ? ds - p0 : 0, b = de - p0 < 16 ? de - p0 : 16;  // the diagonal's fields [a, b)
-        if (a < b) x = mismatch16(pack16(row, r0 + p0 - ds), pack16(col, p0 - ds)) & ops_mask(uint32_t(a), uint32_t(b - 1));
+        if (a < b) x = m & ops_mask(uint32_t(a), uint32_t(b - 1));
         const int32_t g = gs > p0 ? gs - p0 : 0, h = gs + d - p0 < 16 ? gs + d - p0 : 16;
         if (g < h) x |= gap_up * ops_mask(uint32_t(g), uint32_t(h - 1));
         w[k] = x;
     }
     ops_summary(w, uint32_t(first), uint32_t(R), sum);
+}
+
+// straight_ops of a diagonal with no mismatch (e = 0) or one, at column f: the
+// words and the summary follow without reading the bases again
+HERO_HD void plain_ops(int type, int32_t R, int32_t C, int32_t e, int32_t f, uint32_t gap_up, uint32_t *w,
+                       uint32_t stride, DpSum &sum) {
+    const int32_t d = R - C, end = int32_t(stride) * 16, first = end - R;
+    const int32_t ds = type == BT_RIGHT ? first + d : first;
+    const int32_t gs = type == BT_RIGHT ? first : end - d;
+    const int32_t px = e ? ds + f : -1;
+    for (int32_t k = first >> 4; k < int32_t(stride); k++) {
+        const int32_t p0 = k * 16;
+        uint32_t x = (px >> 4) == k ? 1u << (2 * (px & 15)) : 0u;
+        const int32_t g = gs > p0 ? gs - p0 : 0, h = gs + d - p0 < 16 ? gs + d - p0 : 16;
+        if (g < h) x |= gap_up * ops_mask(uint32_t(g), uint32_t(h - 1));
+        w[k] = x;
+    }
+    const bool lead = type == BT_RIGHT && d > 0, tail = type != BT_RIGHT && d > 0;
+    const bool fx = e && f == 0, lx = e && f == C - 1;
+    for (int i = 0; i < 4; i++) sum.tot[i] = 0;
+    sum.tot[OP_M] = uint16_t(C - e);
+    sum.tot[OP_X] = uint16_t(e);
+    if (d > 0) sum.tot[gap_up] = uint16_t(d);
+    sum.ft = uint8_t(lead ? gap_up : fx ? uint32_t(OP_X) : uint32_t(OP_M));
+    sum.fc = uint16_t(lead ? d : fx ? 1 : e ? f : C);
+    sum.lt = uint8_t(tail ? gap_up : lx ? uint32_t(OP_X) : uint32_t(OP_M));
+    sum.lc = uint16_t(tail ? d : lx ? 1 : e ? C - 1 - f : C);
+    sum.nruns = sum.fc == R ? 1 : 2;
+    sum.pad = 0;
 }
 
 }  // namespace hero

@@ -206,10 +206,10 @@ struct BandBin {
 };
 struct BandWork {
     bool on;           // false: every segment goes to the whole-matrix kernels
-    uint32_t *key;     // a segment's key (kBandNoKey: done, or not for the window)
+    uint2 *key;        // a segment's key (kBandNoKey: done, or not for the window) and place in it
     uint32_t *order;   // segments by key
     uint32_t *count;   // kBandBins segment counts (zeroed before launch_band)
-    uint32_t *cursor;  // kBandBins next positions
+    uint32_t *start;   // first position of each key
     BandBin *bin;      // the non-empty keys
     uint32_t *head;    // their number, the number of tasks, the next task
     uint32_t *codes;   // traceback codes, code_words a warp

@@ -95,7 +95,7 @@ void screen_run(const Seg &g, int type, Count n) {
     const std::vector<uint8_t> ops = whole(g.v, AFFINE, want);
     const uint32_t stride = uint32_t((g.b.R + g.b.C + 15) / 16);
     std::vector<uint32_t> w(stride + 1, 0xffffffffu);
-    straight_ops(g.b.row, g.b.col, type, g.b.R, g.b.C, g.rev ? OP_I : OP_D, w.data(), stride, sum);
+    plain_ops(type, g.b.R, g.b.C, e, f, g.rev ? OP_I : OP_D, w.data(), stride, sum);
     bool same = int(ops.size()) == g.b.R;
     for (size_t k = 0; same && k < ops.size(); k++) same = ops_field(w.data(), uint32_t(stride * 16 - ops.size() + k)) == ops[k];
     n.c[3] += !same;
@@ -164,7 +164,10 @@ void pair_any(bool affine, int nb, int type, bool mask, Seg &a, Seg &b, Count n)
         if (nb == 4) pair_type<true, 4>(type, mask, a, b, n);
         if (nb == 8) pair_type<true, 8>(type, mask, a, b, n);
         if (nb == 16) pair_type<true, 16>(type, mask, a, b, n);
+        if (nb == 11) pair_type<true, 11>(type, mask, a, b, n);
+        if (nb == 19) pair_type<true, 19>(type, mask, a, b, n);
         if (nb == 24) pair_type<true, 24>(type, mask, a, b, n);
+        if (nb == 26) pair_type<true, 26>(type, mask, a, b, n);
         if (nb == 40) pair_type<true, 40>(type, mask, a, b, n);
     } else {
         if (nb == 4) pair_type<false, 4>(type, mask, a, b, n);

@@ -49,7 +49,7 @@ def test_every_short_segment(band, affine, nb, kind):
     assert n[1] > n[2] > 0 and n[1] > n[0] // (4 if nb else 50)  # it accepts, and not only the plainest paths
 
 
-@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 8), (1, 16), (1, 24), (1, 40), (0, 0), (0, 8), (0, 16)])
+@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 11), (1, 16), (1, 19), (1, 24), (1, 26), (1, 40), (0, 0), (0, 8), (0, 16)])
 @pytest.mark.parametrize("cmax", [5, 40, 250, 1023])
 def test_random_segments(band, affine, nb, cmax):
     for mask, m in ((0, 0), (1, 4), (1, 30)):
