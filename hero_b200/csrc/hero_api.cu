@@ -82,7 +82,6 @@ struct hero_ctx {
     std::vector<uint8_t> aln_host;  // .aln text of every subject aligned since the last take
     // index build temporaries (kept between builds)
     DBuf x_cnt, x_koff, x_klo, x_khi, x_kval, x_owner, x_count, x_slot_of, x_start, x_fill, x_tmp;
-    uint64_t dp_T = 0;
 
     hero_stats stats{};
     unsigned long long ctr[C_COUNT] = {};
@@ -327,7 +326,6 @@ extern "C" int hero_create(const hero_params *p, hero_ctx **out) {
         }
         c->own_stream = true;
     }
-    c->dp_T = dp_threads(c->dev);
     if (c->ensure(c->counters, sizeof(unsigned long long) * C_COUNT, "counters")) {
         delete c;
         return HERO_E_OOM;
@@ -583,13 +581,12 @@ struct DpBufs {
 static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
     if (!a.nd) return HERO_OK;
     BandWork w{};
-    w.warps = band_warps(c->dev, a.nd);
-    w.code_words = band_code_words(cmax, a.affine != 0);
-    const size_t table = kBandBins * (sizeof(BandBin) + 4) + 16;
+    const size_t codes = band_sizes(c->dev, a.nd, a.rmax, cmax, a.affine != 0, w);
+    const size_t table = kBandBins * (sizeof(BandBin) + 4) + kBandHead * 4;
     w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 8, "DP windows") &&
-           c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 4, "DP windows") &&
+           c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 8, "DP windows") &&
            c->optional(b.bin, table, "DP windows") &&
-           c->optional(b.codes, size_t(w.warps) * w.code_words * 4, "DP windows");
+           c->optional(b.codes, codes, "DP windows");
     a.bins = P_<uint32_t>(b.bins);
     a.rest = w.on ? P_<uint32_t>(b.rest) : a.ops;
     a.perm = P_<uint32_t>(b.perm);
@@ -600,6 +597,7 @@ static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
         w.start = reinterpret_cast<uint32_t *>(w.bin + kBandBins);
         w.head = w.start + kBandBins;
         w.codes = P_<uint32_t>(b.codes);
+        w.again = a.rest + a.nd;
         w.count = a.bins + kDpBins;
     }
     HERO_TRY(c->cuda(cudaMemsetAsync(b.bins.p, 0, (kDpBins + kBandBins) * 4, c->st), "DP bins"));
@@ -752,19 +750,34 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         if ((r = c->ensure(c->ops, NDc * stride * 4, "DP ops"))) break;
         if ((r = c->ensure(c->bins, (kDpBins + kBandBins) * 4, "DP bins"))) break;
         if ((r = c->ensure(c->bin_off, (kDpBins + 1) * 8, "DP bins"))) break;
-        const int32_t nst = (cmax + kStripW - 1) / kStripW;
         if ((r = c->ensure(c->dp_tasks, kDpTaskWords * 8, "DP tasks"))) break;
+        DpLaunch a{};
+        const size_t long_bytes = dp_long_sizes(c->dev, rmax, cmax, a);
         if (dp_needs_scratch(rmax, cmax)) {
-            if ((r = c->ensure(c->tb, size_t(c->dp_T) * size_t(rmax) * size_t(nst) * 2, "DP traceback scratch"))) break;
-            if ((r = c->ensure(c->bnd, size_t(c->dp_T) * size_t(rmax + 1) * 3 * 4, "DP boundary scratch"))) break;
+            if ((r = c->ensure(c->tb, long_bytes, "DP traceback scratch"))) break;
+            if ((r = c->ensure(c->bnd, dp_long_bounds(rmax, a), "DP boundary scratch"))) break;
         }
         rec(3);
         if (cap) launch_stamp(P_<unsigned long long>(c->stamps) + 2 * c->batch_idx, c->st);
-        DpLaunch a{P_<DpSeg>(c->segs), P_<uint32_t>(c->perm), ND, subj.code, subj.off, subj.len,
-                   q.code, q.off, P_<uint32_t>(c->ops), stride, P_<DpSum>(c->sums),
-                   P_<uint32_t>(c->cells), P_<uint16_t>(c->tb), P_<int32_t>(c->bnd), c->dp_T, rmax,
-                   c->p.affine, 1,  // reads with a non-ACGT base never reach the DP
-                   0u, 0u, kStripsAll, 4, ctr + C_CELLS_PAIR};
+        a.segs = P_<DpSeg>(c->segs);
+        a.nd = ND;
+        a.scode = subj.code;
+        a.soff = subj.off;
+        a.slen = subj.len;
+        a.qcode = q.code;
+        a.qoff = q.off;
+        a.ops = P_<uint32_t>(c->ops);
+        a.stride = stride;
+        a.sums = P_<DpSum>(c->sums);
+        a.cells = P_<uint32_t>(c->cells);
+        a.tb = P_<uint16_t>(c->tb);
+        a.bnd = P_<int32_t>(c->bnd);
+        a.rmax = rmax;
+        a.affine = c->p.affine;
+        a.whole = 1;  // reads with a non-ACGT base never reach the DP
+        a.chunk_mask = kStripsAll;
+        a.warps = 4;
+        a.pair_cells = ctr + C_CELLS_PAIR;
         a.staged = ctr + C_STAGED;
         a.spack = subj.pack;
         a.qpack = q.pack;
@@ -1333,13 +1346,14 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
         if ((r = upload_reads(c, query, query_off, no_uid.data(), n_query, qraw, qcode, qpack, qoff, qlen,
                               quid, nullptr, nullptr, nullptr)))
             break;
-        const int32_t nst = (cmax + kStripW - 1) / kStripW;
+        DpLaunch a{};
+        const size_t long_bytes = dp_long_sizes(c->dev, rmax, cmax, a);
         if ((r = c->ensure(dsegs, n_seg * sizeof(DpSeg), "segments"))) break;
         if ((r = c->ensure(dsums, n_seg * sizeof(DpSum), "segments"))) break;
         if ((r = c->ensure(dops, n_seg * stride * 4, "segments"))) break;
         if (dp_needs_scratch(rmax, cmax)) {
-            if ((r = c->ensure(dtb, size_t(c->dp_T) * rmax * nst * 2, "scratch"))) break;
-            if ((r = c->ensure(dbnd, size_t(c->dp_T) * (rmax + 1) * 3 * 4, "scratch"))) break;
+            if ((r = c->ensure(dtb, long_bytes, "scratch"))) break;
+            if ((r = c->ensure(dbnd, dp_long_bounds(rmax, a), "scratch"))) break;
         }
         if ((r = c->ensure(dperm, n_seg * 4, "order"))) break;
         if ((r = c->ensure(dbins, (kDpBins + kBandBins) * 4, "bins"))) break;
@@ -1351,10 +1365,23 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
         if ((r = c->ensure(dn, n_seg * 4, "ops"))) break;
         cudaMemcpyAsync(dsegs.p, h.data(), n_seg * sizeof(DpSeg), cudaMemcpyHostToDevice, c->st);
         cudaMemcpyAsync(doo.p, ops_off, (n_seg + 1) * 8, cudaMemcpyHostToDevice, c->st);
-        DpLaunch a{P_<DpSeg>(dsegs), P_<uint32_t>(dperm), n_seg, P_<uint8_t>(scode), P_<uint64_t>(soff),
-                   P_<uint32_t>(slen), P_<uint8_t>(qcode), P_<uint64_t>(qoff), P_<uint32_t>(dops),
-                   stride, P_<DpSum>(dsums), nullptr, P_<uint16_t>(dtb), P_<int32_t>(dbnd),
-                   c->dp_T, rmax, affine ? 1 : 0, acgt ? 1 : 0, 0u, 0u, kStripsAll, 4};
+        a.segs = P_<DpSeg>(dsegs);
+        a.nd = n_seg;
+        a.scode = P_<uint8_t>(scode);
+        a.soff = P_<uint64_t>(soff);
+        a.slen = P_<uint32_t>(slen);
+        a.qcode = P_<uint8_t>(qcode);
+        a.qoff = P_<uint64_t>(qoff);
+        a.ops = P_<uint32_t>(dops);
+        a.stride = stride;
+        a.sums = P_<DpSum>(dsums);
+        a.tb = P_<uint16_t>(dtb);
+        a.bnd = P_<int32_t>(dbnd);
+        a.rmax = rmax;
+        a.affine = affine ? 1 : 0;
+        a.whole = acgt ? 1 : 0;
+        a.chunk_mask = kStripsAll;
+        a.warps = 4;
         a.spack = pack_words(spack);
         a.qpack = pack_words(qpack);
         a.n_rest = P_<unsigned long long>(dtasks) + kDpTaskWords;

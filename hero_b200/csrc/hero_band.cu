@@ -3,6 +3,8 @@
 // whole-matrix kernels of hero_kernels.cu.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "hero_band.cuh"
 #include "hero_internal.cuh"
 
@@ -175,6 +177,8 @@ __global__ void __launch_bounds__(1024) k_band_tasks(BandWork w) {
         w.head[0] = all[2];  // bins
         w.head[1] = all[1];  // tasks
         w.head[2] = 0;       // next task
+        w.head[3] = 0;       // segments for the wide window
+        w.head[4] = 0;       // next of its tasks
     }
 }
 
@@ -206,8 +210,8 @@ struct WarpCodes {
 // diagonal, the row selectors), so a cell costs six ALU instructions and a
 // column touches memory only for its code words.
 template <bool AFFINE, int NB, int TYPE, bool MASK>
-__device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order, uint32_t n, int32_t C,
-                                       uint32_t *codes) {
+__device__ __noinline__ void band_task(const DpLaunch &a, const BandWork &w, const uint32_t *order, uint32_t n,
+                                       int32_t C, uint32_t *codes) {
     constexpr int WORDS = (NB + 7) / 8;
     const uint32_t lane = lane_id();
     BandSeg s[2];
@@ -229,7 +233,7 @@ __device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order,
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const bool has = lane + 32u * h < n;
-        const bool sure = has && C - e[h].v <= band_limit<AFFINE, NB, TYPE>(s[h]);
+        const bool sure = has && C - e[h].v <= band_limit<AFFINE, TYPE>(s[h], NB);
         if (sure && e[h].straight) {
             DpSum sum;
             straight_ops(s[h].row, s[h].col, TYPE, s[h].R, C, rev[h] ? uint32_t(OP_I) : uint32_t(OP_D),
@@ -237,7 +241,15 @@ __device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order,
             a.sums[si[h]] = sum;
         }
         walk[h] = __ballot_sync(0xffffffffu, sure && !e[h].straight);
-        rest_append(a, has && !sure, si[h], a.segs[si[h]]);
+        const bool wide = has && !sure && !MASK && s[h].R >= w.wide_min;  // whole bands only
+        rest_append(a, has && !sure && !wide, si[h], a.segs[si[h]]);
+        const uint32_t m = __ballot_sync(0xffffffffu, wide);
+        if (m) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&w.head[3], uint32_t(__popc(m)));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (wide) w.again[at + __popc(m & ((1u << lane) - 1u))] = si[h];
+        }
     }
     __syncwarp();  // the codes of every lane are written
     // the paths with gaps, one a lane: lane l traces the l-th of them
@@ -262,16 +274,16 @@ __device__ __noinline__ void band_task(const DpLaunch &a, const uint32_t *order,
 }
 
 template <bool AFFINE, int CLS>
-__device__ __forceinline__ void band_dispatch(int type, const DpLaunch &a, const uint32_t *order, uint32_t n,
-                                              int32_t C, uint32_t *codes) {
+__device__ __forceinline__ void band_dispatch(int type, const DpLaunch &a, const BandWork &w, const uint32_t *order,
+                                              uint32_t n, int32_t C, uint32_t *codes) {
     constexpr int NB = band_width<AFFINE, CLS>();
     constexpr bool MASK = CLS >= 4;
     if (type == BT_RIGHT) {
-        band_task<AFFINE, NB, BT_RIGHT, MASK>(a, order, n, C, codes);
+        band_task<AFFINE, NB, BT_RIGHT, MASK>(a, w, order, n, C, codes);
     } else if (type == BT_LEFT) {
-        band_task<AFFINE, NB, BT_LEFT, MASK>(a, order, n, C, codes);
+        band_task<AFFINE, NB, BT_LEFT, MASK>(a, w, order, n, C, codes);
     } else {
-        band_task<AFFINE, NB, BT_NONE, MASK>(a, order, n, C, codes);
+        band_task<AFFINE, NB, BT_NONE, MASK>(a, w, order, n, C, codes);
     }
 }
 
@@ -305,29 +317,118 @@ __global__ void __launch_bounds__(kBandWarps * 32, kBandBlocks) k_band(DpLaunch 
         const uint32_t ct = b.key >> kBandColBits;
         const int type = int(ct % 3u);
         switch (ct / 3u) {
-            case 0: band_dispatch<AFFINE, 0>(type, a, order, n, C, codes); break;
-            case 1: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 1 : 0>(type, a, order, n, C, codes); break;
-            case 2: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 2 : 0>(type, a, order, n, C, codes); break;
-            case 3: band_dispatch<AFFINE, 3>(type, a, order, n, C, codes); break;
-            case 4: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 4 : 5>(type, a, order, n, C, codes); break;
-            default: band_dispatch<AFFINE, 5>(type, a, order, n, C, codes); break;
+            case 0: band_dispatch<AFFINE, 0>(type, a, w, order, n, C, codes); break;
+            case 1: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 1 : 0>(type, a, w, order, n, C, codes); break;
+            case 2: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 2 : 0>(type, a, w, order, n, C, codes); break;
+            case 3: band_dispatch<AFFINE, 3>(type, a, w, order, n, C, codes); break;
+            case 4: if (AFFINE) band_dispatch<AFFINE, AFFINE ? 4 : 5>(type, a, w, order, n, C, codes); break;
+            default: band_dispatch<AFFINE, 5>(type, a, w, order, n, C, codes); break;
         }
+    }
+}
+
+// The wide window of what the register windows left, 64 segments a warp in list
+// order (theirs: class, type, columns).  One-warp blocks; the strips' edges in
+// shared memory (18 KB for 64 diagonals, 26 KB for 96).  Bound by its serial chain, a row of
+// eight cells after the other; what it replaces -- the whole matrix -- took 31 of
+// 33 ms on 300-600 bp reads and 8 of 38 ms on 75-250 bp ones: now 2.2 and 2.7 ms.
+// A task is 71 rows a strip after strip where the whole-matrix wavefront is one
+// pass down the rows, so batches of up to 128 rows, and those too small to fill
+// the device with tasks, stay with that (1.67 M x 150 bp: 42.4 ms of DP without
+// the wide window, 44.5 with; 4310 reads of 75-250 bp: 0.95 and 1.65 ms), as do
+// single segments below 64 rows.
+constexpr int32_t kWideBatchRows = 128, kWideMinRows = 64;
+constexpr uint64_t kWideMinSegments = 4000000;  // below it only batches with columns past 256, where
+                                                // the whole matrices are k_dp_long's
+struct SmemEdge {
+    uint32_t *p;  // + lane
+    __device__ __forceinline__ uint32_t &m(int32_t t) { return p[t * 64]; }
+    __device__ __forceinline__ uint32_t &l(int32_t t) { return p[t * 64 + 32]; }
+};
+struct WideStore {
+    uint32_t *p;  // + lane
+    int32_t rows;
+    __device__ __forceinline__ void put(int32_t k, int32_t t, uint32_t bits) { p[size_t(k * rows + t) * 32] = bits; }
+};
+struct WideCodes {
+    const uint32_t *p;  // + lane of the segment
+    int32_t rows;
+    uint32_t shift;
+    __device__ __forceinline__ uint32_t get(int32_t k, int32_t t) const {
+        return (p[size_t(k * rows + t) * 32] >> shift) & 0xffffu;
+    }
+};
+
+template <bool AFFINE>
+__global__ void __launch_bounds__(32) k_band_wide(DpLaunch a, BandWork w) {
+    extern __shared__ uint32_t edges[];
+    const uint32_t lane = threadIdx.x;
+    const int32_t nb = w.wide_nb, rows = wide_rows(nb);
+    uint32_t *codes = w.codes + size_t(blockIdx.x) * w.wide_words;
+    const uint32_t count = w.head[3];
+    for (;;) {
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(&w.head[4], 1u);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= (count + kTaskSegs - 1) / kTaskSegs) break;
+        const uint32_t *list = w.again + size_t(q) * kTaskSegs;
+        const uint32_t n = min(count - q * kTaskSegs, uint32_t(kTaskSegs));
+        BandSeg s[2];
+        uint32_t si[2];
+        int type[2];
+        bool rev[2];
+        int32_t v[2], cmax = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t k = lane + 32u * h;
+            si[h] = list[k < n ? k : 0u];
+            const DpSeg g = a.segs[si[h]];
+            s[h] = band_seg(a, g, rev[h]);
+            type[h] = band_type(g);
+            s[h].base = wide_base(AFFINE, nb, type[h], s[h].R - s[h].C);
+            cmax = max(cmax, s[h].C);
+        }
+        cmax = __reduce_max_sync(0xffffffffu, cmax);
+        SmemEdge edge{edges + lane};
+        WideStore st{codes + lane, rows};
+        wide_fill<AFFINE>(s[0], s[1], type[0], type[1], nb, cmax, edge, st, v[0], v[1]);
+        __syncwarp();
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            const bool has = lane + 32u * h < n;
+            const bool sure = has && s[h].C - v[h] <= wide_limit<AFFINE>(s[h], type[h], nb);
+            if (sure) {
+                OpsPut put{a.ops + uint64_t(si[h]) * a.stride, int32_t(a.stride * 16u)};
+                DpSum sum;
+                const uint32_t up = rev[h] ? uint32_t(OP_I) : uint32_t(OP_D), left = rev[h] ? uint32_t(OP_D) : uint32_t(OP_I);
+                const int32_t np = wide_walk<AFFINE>(s[h], type[h], nb, WideCodes{codes + lane, rows, h ? 16u : 0u}, up, left, put);
+                ops_summary(put.w, a.stride * 16u - uint32_t(np), uint32_t(np), sum);
+                a.sums[si[h]] = sum;
+            }
+            rest_append(a, has && !sure, si[h], a.segs[si[h]]);
+        }
+        __syncwarp();
     }
 }
 
 }  // namespace
 
-uint64_t band_warps(int device, uint64_t nd) {
+// Resident warps for nd segments (half a task each at least), the code words of
+// each -- and, in the same words, the wide window's blocks, which need more each.
+size_t band_sizes(int device, uint64_t nd, int32_t rmax, int32_t cmax, bool affine, BandWork &w) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const uint64_t full = uint64_t(sms) * kBandBlocks;
-    const uint64_t need = (nd + 32 * kBandWarps - 1) / (32 * kBandWarps);  // half a task a warp
-    return kBandWarps * (need < full ? (need ? need : 1) : full);
-}
-
-uint32_t band_code_words(int32_t cmax, bool affine) {
     const uint32_t c = uint32_t(cmax < kBandMaxC ? cmax : kBandMaxC);
-    return c * 32u * (affine ? 5u : 2u);
+    const uint64_t full = uint64_t(sms) * kBandBlocks, need = (nd + 32 * kBandWarps - 1) / (32 * kBandWarps);
+    w.warps = kBandWarps * (need < full ? need : full);
+    w.code_words = c * 32u * (affine ? 5u : 2u);
+    w.wide_nb = c <= 256u ? 64 : 96;
+    const bool wide = rmax > kWideBatchRows && (cmax > 256 || nd >= kWideMinSegments);
+    w.wide_min = wide ? kWideMinRows : 1 << 30;
+    w.wide_words = (c + kWideStrip - 1) / kWideStrip * uint32_t(wide_rows(w.wide_nb)) * 32u;
+    const uint64_t words = std::max<uint64_t>(w.warps * w.code_words, wide ? w.wide_words : 0u);
+    w.wide_blocks = wide ? std::min<uint64_t>(words / w.wide_words, uint64_t(sms) * (w.wide_nb > 64 ? 8 : 12)) : 0u;
+    return words * 4;
 }
 
 void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
@@ -347,6 +448,14 @@ void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
         k_band<true><<<blocks, kBandWarps * 32, 0, st>>>(a, w);
     } else {
         k_band<false><<<blocks, kBandWarps * 32, 0, st>>>(a, w);
+    }
+    if (!w.wide_blocks) return;
+    count_launch();
+    const size_t wide_smem = size_t(wide_rows(w.wide_nb)) * 64 * 4;
+    if (a.affine) {
+        k_band_wide<true><<<unsigned(w.wide_blocks), 32, wide_smem, st>>>(a, w);
+    } else {
+        k_band_wide<false><<<unsigned(w.wide_blocks), 32, wide_smem, st>>>(a, w);
     }
 }
 

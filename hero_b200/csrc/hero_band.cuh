@@ -135,10 +135,10 @@ HERO_HD int32_t band_base(int32_t d) {
 // up for the affine aligner, not for the global one), below it the free climb
 // would carry its score to the cells of the traceback.  The limits are the
 // deficits of those paths, less one where a tie would change a move.
-template <bool AFFINE, int NB, int TYPE>
-HERO_HD int32_t band_limit(const BandSeg &s) {
+template <bool AFFINE, int TYPE>
+HERO_HD int32_t band_limit(const BandSeg &s, int32_t nb) {
     constexpr int32_t kNone = 1 << 20;
-    const int32_t d = s.R - s.C, lo = s.base, hi = s.base + NB - 1;
+    const int32_t d = s.R - s.C, lo = s.base, hi = s.base + nb - 1;
     const int32_t v1 = AFFINE ? 1 : 4, h1 = AFFINE ? 2 : 5, open = AFFINE ? 3 : 0;
     int32_t below = kNone, above = kNone;
     if (lo > -s.m && lo > -s.C) {
@@ -481,6 +481,193 @@ HERO_HD int32_t band_walk(const BandSeg &s, const Codes &codes, uint32_t gap_up,
             out.fields(gap_left, 1u);
             j--;
             c++;
+        }
+    }
+    out.run(gap_up, uint32_t(i));
+    out.run(gap_left, uint32_t(j));
+    out.flush();
+    return end - out.p;
+}
+
+// ---------------------------------------------------------------------------
+// The wide window: NB diagonals at run time, for the segments whose deficit the
+// register windows cannot certify.  Strips of eight columns, the strip's columns
+// in registers, its last column's M and next IY kept by row for the next strip
+// (edge.m(t), edge.l(t)).  A strip's row t is row first column + base + t, so
+// cell (t, w) lies on window diagonal t - w; rows 0 .. NB + 6 hold the window and
+// some cells beside it, whose values are paths' all the same.  The two segments
+// of a pair may differ in type and columns.
+// ---------------------------------------------------------------------------
+constexpr int kWideStrip = 8;
+HERO_HD constexpr int wide_rows(int nb) { return nb + kWideStrip - 1; }
+
+HERO_HD int wide_near(bool affine, int nb) { return affine ? (nb - 1) / 3 : (nb - 1) / 2; }
+HERO_HD int32_t wide_base(bool affine, int nb, int type, int32_t d) {
+    const int near = wide_near(affine, nb);
+    return type == BT_RIGHT ? d - (nb - 1 - near) : type == BT_LEFT ? -near : -((nb - 1 - d) / 2);
+}
+
+template <bool AFFINE>
+HERO_HD int32_t wide_limit(const BandSeg &s, int type, int32_t nb) {
+    return type == BT_RIGHT ? band_limit<AFFINE, BT_RIGHT>(s, nb)
+         : type == BT_LEFT ? band_limit<AFFINE, BT_LEFT>(s, nb) : band_limit<AFFINE, BT_NONE>(s, nb);
+}
+
+// scores of column 0 at row i: M, and IY of (i, 1)
+template <bool AFFINE>
+HERO_HD int32_t wide_col0(int type, int32_t i) {
+    return type == BT_RIGHT ? band_col0<AFFINE, BT_RIGHT>(i) : band_col0<AFFINE, BT_LEFT>(i);
+}
+
+// one row of a strip; ENDS: column C of a segment is in the strip (free: the
+// halves of align-left ones, whose rows cost nothing there)
+template <bool AFFINE, bool ENDS>
+HERO_HD uint32_t wide_row(uint32_t (&m)[kWideStrip], uint32_t (&xn)[kWideStrip], const uint32_t (&sel)[kWideStrip],
+                          uint32_t ta, uint32_t tb, uint32_t dm, uint32_t &y, const uint32_t (&free)[kWideStrip],
+                          uint32_t (&mts)[kWideStrip], uint32_t (&fxs)[kWideStrip]) {
+    using K = BandCost<AFFINE>;
+    uint32_t acc = 0;
+#pragma unroll
+    for (int w = 0; w < kWideStrip; w++) {
+        const uint32_t f = add2(dm, byte_sel(ta, tb, sel[w]));
+        const uint32_t x = xn[w];
+        uint32_t mt;
+        if (AFFINE) {
+            mt = max3_2(f, x, y);
+            if (ENDS) fxs[w] = max3_2(f, x, x);
+            y = add_max2(f, K::right, y);
+            xn[w] = add_max2(f, K::down, x);
+            if (ENDS) xn[w] = (xn[w] & ~free[w]) | (add_max2(f, K::free_open, add2(x, K::free_more)) & free[w]);
+        } else {  // xn: the clean score of the row above plus the row's cost
+            mt = add_max2(y, K::right, max3_2(f, x, x));
+            if (ENDS) fxs[w] = mt;
+            y = mt & ~kTagMask2;
+            xn[w] = add2(y, K::down);
+            if (ENDS) xn[w] = (xn[w] & ~free[w]) | (add2(y, K::free_open) & free[w]);
+        }
+        const uint32_t tg = mt & kTagMask2;
+        if (ENDS) mts[w] = mt;
+        dm = m[w];
+        m[w] = mt & ~kTagMask2;
+        acc += tg << (2 * w);
+    }
+    return acc;
+}
+
+HERO_HD bool any_lane(bool x) {
+#if defined(__CUDA_ARCH__)
+    return __any_sync(0xffffffffu, x);
+#else
+    return x;
+#endif
+}
+
+// cmax: the most columns of the warp's segments; st.put(strip, row, codes)
+template <bool AFFINE, class Edge, class Store>
+HERO_HD void wide_fill(const BandSeg &a, const BandSeg &b, int type_a, int type_b, int32_t nb, int32_t cmax,
+                       Edge &edge, Store &st, int32_t &va, int32_t &vb) {
+    using K = BandCost<AFFINE>;
+    const uint32_t dead = band_half2(kBandDead);
+    const int32_t rows = wide_rows(nb), da = a.R - a.C, db = b.R - b.C;
+    const int32_t cea = da - a.base < nb - 1 ? da - a.base : nb - 1, ceb = db - b.base < nb - 1 ? db - b.base : nb - 1;
+    va = vb = kBandDead;
+    // column 0, rows base .. base + nb - 1, as the last column of a strip before the first
+    for (int32_t t = kWideStrip - 1; t < rows; t++) {
+        const int32_t u = t - (kWideStrip - 1), ia = a.base + u, ib = b.base + u;
+        edge.m(t) = pack2(ia >= 0 ? 4 * (wide_col0<AFFINE>(type_a, ia) + K::pot * u) : kBandDead,
+                          ib >= 0 ? 4 * (wide_col0<AFFINE>(type_b, ib) + K::pot * u) : kBandDead);
+        if (AFFINE) {
+            const int32_t la = type_a == BT_RIGHT ? band_col0_right<BT_RIGHT>(ia) : band_col0_right<BT_LEFT>(ia);
+            const int32_t lb = type_b == BT_RIGHT ? band_col0_right<BT_RIGHT>(ib) : band_col0_right<BT_LEFT>(ib);
+            edge.l(t) = pack2(ia >= 0 ? 4 * (la + u + 1) : kBandDead, ib >= 0 ? 4 * (lb + u + 1) : kBandDead);
+        }
+    }
+    uint32_t wca = 0, wcb = 0;
+    for (int32_t j0 = 1, k = 0; j0 <= cmax; j0 += kWideStrip, k++) {
+        uint32_t m[kWideStrip], xn[kWideStrip], sel[kWideStrip], free[kWideStrip], mts[kWideStrip], fxs[kWideStrip];
+        const int32_t ja = j0 < a.C ? j0 : a.C, jb = j0 < b.C ? j0 : b.C;  // no reads past a shorter segment's end
+        if ((k & 1) == 0) {
+            wca = pack16(a.col, ja - 1);
+            wcb = pack16(b.col, jb - 1);
+        }
+#pragma unroll
+        for (int w = 0; w < kWideStrip; w++) {
+            m[w] = xn[w] = dead;
+            sel[w] = band_sel(wca & 3u, wcb & 3u);
+            wca >>= 2;
+            wcb >>= 2;
+            free[w] = (type_a == BT_LEFT && j0 + w == a.C ? 0xffffu : 0u) |
+                      (type_b == BT_LEFT && j0 + w == b.C ? 0xffff0000u : 0u);
+        }
+        const bool ends = any_lane((a.C >= j0 && a.C < j0 + kWideStrip) || (b.C >= j0 && b.C < j0 + kWideStrip));
+        PackStream sa(a.row, ja + a.base - 1), sb(b.row, jb + b.base - 1);
+        uint32_t ra = 0, rb = 0, dm = edge.m(kWideStrip - 1);
+        for (int32_t t = 0; t < rows; t++) {
+            if ((t & 15) == 0) {
+                ra = sa.next();
+                rb = sb.next();
+            }
+            const bool in = t + kWideStrip < rows;  // the strip before has this row
+            uint32_t y = in ? (AFFINE ? edge.l(t + kWideStrip) : edge.m(t + kWideStrip)) : dead;
+            const uint32_t next = in ? edge.m(t + kWideStrip) : dead;
+            const uint32_t ta = band_table<AFFINE>(ra & 3u), tb = band_table<AFFINE>(rb & 3u);
+            ra >>= 2;
+            rb >>= 2;
+            uint32_t acc;
+            // row 0: its IX equal its IY, which a row's gap extensions leave as they are
+            const uint32_t row0 = (j0 + a.base + t == 0 ? 0xffffu : 0u) | (j0 + b.base + t == 0 ? 0xffff0000u : 0u);
+            const uint32_t y0 = y + 0x00020002u;
+            if (ends) {
+                acc = wide_row<AFFINE, true>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
+#pragma unroll
+                for (int w = 0; w < kWideStrip; w++) {
+                    // above the window an align-left path climbs freely: its row, or the window's last
+                    const int32_t pot = K::pot * (2 * (j0 + w) + t - w);
+                    if (j0 + w == a.C && t - w == cea) va = (half_lo(da - a.base > cea ? fxs[w] : mts[w]) >> 2) - pot;
+                    if (j0 + w == b.C && t - w == ceb) vb = (half_hi(db - b.base > ceb ? fxs[w] : mts[w]) >> 2) - pot;
+                }
+            } else {
+                acc = wide_row<AFFINE, false>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
+            }
+            if (AFFINE && row0) {
+#pragma unroll
+                for (int w = 0; w < kWideStrip; w++) xn[w] = (xn[w] & ~row0) | (add2(y0, free[w] & K::free_more) & row0);
+            }
+            st.put(k, t, acc);
+            edge.m(t) = m[kWideStrip - 1];
+            if (AFFINE) edge.l(t) = y;
+            dm = next;
+        }
+    }
+}
+
+// band_walk over the wide window's codes: codes.get(strip, row) holds the
+// strip's eight cells of a row
+template <bool AFFINE, class Codes>
+HERO_HD int32_t wide_walk(const BandSeg &s, int type, int32_t nb, const Codes &codes, uint32_t gap_up,
+                          uint32_t gap_left, OpsPut &out) {
+    using T = PairTags<AFFINE>;
+    const int32_t end = out.p;
+    int32_t i = s.R, j = s.C;
+    if (type == BT_LEFT && i - j - s.base > nb - 1) {
+        const int32_t k = i - j - s.base - (nb - 1);
+        out.run(gap_up, uint32_t(k));
+        i -= k;
+    }
+    while (i > 0 && j > 0) {
+        if (uint32_t(i - j - s.base) >= uint32_t(nb)) return -1;
+        const int32_t k = (j - 1) >> 3, w = (j - 1) & 7;
+        const uint32_t code = (codes.get(k, i - (kWideStrip * k + 1) - s.base) >> (2 * w)) & 3u;
+        if (code == uint32_t(T::diag)) {
+            i--;
+            j--;
+            out.fields((pack16(s.row, i) ^ pack16(s.col, j)) & 3u ? 1u : 0u, 1u);
+        } else if (code == uint32_t(T::up)) {
+            i--;
+            out.fields(gap_up, 1u);
+        } else {
+            j--;
+            out.fields(gap_left, 1u);
         }
     }
     out.run(gap_up, uint32_t(i));

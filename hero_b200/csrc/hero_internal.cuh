@@ -160,9 +160,8 @@ struct DpLaunch {
     uint32_t stride;
     DpSum *sums;
     uint32_t *cells;        // reference band cells per segment (may be NULL)
-    uint16_t *tb;           // traceback scratch: threads * rmax * nstrips
-    int32_t *bnd;           // boundary scratch: threads * 3 * (rmax + 1)
-    uint64_t threads;       // resident threads the scratch is laid out for
+    uint16_t *tb;           // traceback codes of k_dp_long, long_codes a warp
+    int32_t *bnd;           // its panel boundaries, 3 (rmax + 1) a warp
     int32_t rmax;
     int32_t affine;
     int32_t whole;          // 1: every base is A/C/G/T, the whole-band rows may run
@@ -174,6 +173,7 @@ struct DpLaunch {
     int32_t regs;           // registers a thread of the wavefront kernel: 128 (0 too) or 168
     unsigned long long *staged = nullptr;  // counters: C_STAGED, then C_STAGE_FAIL (may be NULL)
     uint32_t stage_extra = 0;  // bytes a warp's code area has past its rmax rows (set by launch_dp)
+    uint64_t long_codes = 0, long_blocks = 1;  // k_dp_long's code words a warp and blocks (dp_long_sizes)
     // the window DP (launch_band) and what it leaves to the whole-matrix kernels
     const uint32_t *spack = nullptr, *qpack = nullptr;  // 2-bit codes of subjects and queries
     uint32_t *rest = nullptr;                // segments for the whole-matrix kernels, in any order
@@ -211,20 +211,24 @@ struct BandWork {
     uint32_t *count;   // kBandBins segment counts (zeroed before launch_band)
     uint32_t *start;   // first position of each key
     BandBin *bin;      // the non-empty keys
-    uint32_t *head;    // their number, the number of tasks, the next task
-    uint32_t *codes;   // traceback codes, code_words a warp
-    uint32_t code_words;
-    uint64_t warps;
+    uint32_t *head;    // their number, the number of tasks, the next task; wide: segments, next task
+    uint32_t *again;   // segments for the wide window
+    uint32_t *codes;   // traceback codes: code_words a warp, then wide_words a block
+    uint32_t code_words, wide_words;
+    int32_t wide_nb;   // diagonals of the wide window
+    int32_t wide_min;  // rows from which a segment takes it
+    uint64_t warps, wide_blocks;
 };
-uint64_t band_warps(int device, uint64_t nd);              // resident warps for nd segments
-uint32_t band_code_words(int32_t cmax, bool affine);       // code words a warp
+constexpr int kBandHead = 8;
+// sets warps, wide_blocks and their words; returns the bytes of `codes`
+size_t band_sizes(int device, uint64_t nd, int32_t rmax, int32_t cmax, bool affine, BandWork &w);
 // fills ops, sums and cells of the segments it certifies; a.rest, a.n_rest (zeroed
 // before) and a.bins (zeroed before) get the others
 void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st);
 // order (a.nd entries) and bin offsets of the listed segments, for launch_dp
 void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void *scan_tmp, cudaStream_t st);
 // needs the shape sort (perm, bin_off); tasks: kDpTaskWords uint64 of device scratch.
-// The per-thread scratch (tb, bnd) is only used when dp_needs_scratch().
+// k_dp_long's scratch (tb, bnd) is only used when dp_needs_scratch().
 constexpr uint32_t kDpTaskWords = 128;
 void launch_dp(const DpLaunch &a, const uint64_t *bin_off, uint64_t *tasks, int32_t cmax,
                cudaStream_t st);
@@ -232,7 +236,8 @@ bool dp_wave_fits(int32_t rmax);
 inline bool dp_needs_scratch(int32_t rmax, int32_t cmax) {
     return !dp_wave_fits(rmax) || cmax > 32 * kStripW;
 }
-uint64_t dp_threads(int device);
+size_t dp_long_sizes(int device, int32_t rmax, int32_t cmax, DpLaunch &a);  // bytes of tb
+size_t dp_long_bounds(int32_t rmax, const DpLaunch &a);                     // bytes of bnd
 
 void launch_assemble(const Params &p, uint64_t nc, ChainArrays ch, const uint32_t *keys,
                      ReadsView subj, ReadsView q, const DpSum *sums, const uint32_t *cells,

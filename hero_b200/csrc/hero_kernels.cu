@@ -792,25 +792,9 @@ __global__ void __launch_bounds__(kChainWarps * 32)
 }
 
 // ---------------------------------------------------------------------------
-// banded DP (BandAligner.cpp:56-419), one thread per segment
+// banded DP (BandAligner.cpp:56-419) of whole matrices, for the segments the
+// window DP leaves
 // ---------------------------------------------------------------------------
-struct DevScratch {
-    uint16_t *tb;
-    int32_t *bnd;
-    uint64_t T;
-    int32_t rmax;
-    uint64_t t;
-    __device__ __forceinline__ void tb_set(int32_t s, int32_t i, uint32_t bits) {
-        tb[(uint64_t(s) * uint64_t(rmax) + uint64_t(i - 1)) * T + t] = uint16_t(bits);
-    }
-    __device__ __forceinline__ uint32_t tb_get(int32_t s, int32_t i) const {
-        return tb[(uint64_t(s) * uint64_t(rmax) + uint64_t(i - 1)) * T + t];
-    }
-    __device__ __forceinline__ int32_t &b(int32_t st, int32_t i) {
-        return bnd[(uint64_t(st) * uint64_t(rmax + 1) + uint64_t(i)) * T + t];
-    }
-};
-
 struct OpsWriter {
     uint32_t *base;
     int32_t p;
@@ -847,27 +831,6 @@ __global__ void k_dp_scatter(DpLaunch a, uint32_t *cursor, const uint64_t *bin_o
         if (i < n && lane == leader) base = atomicAdd(&cursor[key], uint32_t(__popc(same)));
         base = __shfl_sync(0xffffffffu, base, int(leader));
         if (i < n) perm[bin_off[key] + base + __popc(same & ((1u << lane) - 1u))] = si;
-    }
-}
-
-constexpr int kDpThreads = 128;
-
-template <bool AFFINE>
-__global__ void __launch_bounds__(kDpThreads) k_dp(DpLaunch a) {
-    const uint64_t T = uint64_t(gridDim.x) * blockDim.x;
-    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    DevScratch sc{a.tb, a.bnd, T, a.rmax, t};
-    const uint64_t n = *a.n_rest;
-    for (uint64_t idx = t; idx < n; idx += T) {
-        const uint32_t si = a.perm[idx];
-        const DpSeg g = a.segs[si];
-        const SegView v = dpseg_view(g, a.scode, a.soff, a.slen, a.qcode, a.qoff);
-        dp_fill<kStripW, AFFINE>(v, sc);
-        OpsWriter w{a.ops + uint64_t(si) * a.stride, int32_t(a.stride * 16u)};
-        DpSum sum;
-        dp_traceback<kStripW>(v, sc, w, sum);
-        w.flush();
-        a.sums[si] = sum;
     }
 }
 
@@ -917,7 +880,7 @@ __global__ void k_dp_tasks(const uint64_t *bin_off, uint64_t *tasks, uint32_t pa
         t += (e - b + S - 1) / S;
     }
     tasks[33] = t;
-    tasks[0] = bin_off[uint32_t(33) << kShapeStripShift];  // first segment for the per-thread kernel
+    tasks[0] = bin_off[uint32_t(33) << kShapeStripShift];  // first segment for k_dp_long
     tasks[kTaskQueue] = 0;  // work queue head of k_dp_wave
 }
 
@@ -1496,23 +1459,88 @@ __global__ void __launch_bounds__(WARPS * 32, kWaveRegBlocks(WARPS, TIER))
     }
 }
 
-// per-thread kernel for the segments wider than 32 strips (after the wavefront ranges)
+// Segments wider than 32 strips, or of batches whose rows exceed the shared
+// memory codes: a warp each.  The wavefront runs in panels of 32 strips; the
+// last lane's states of a panel are the next one's left boundary (global
+// memory, as the codes, which lie as the lanes write them: step by step).
+// One thread a segment, before, left one long serial chain per segment (16 ms
+// for the few of them among 300-600 bp reads; now 0.8) and laid 12 GB of
+// scratch out for them.
+constexpr int kLongWarps = 4;
+
+struct LongCodes {
+    const uint16_t *tb;
+    int32_t steps;  // steps a panel has room for
+    __device__ __forceinline__ uint32_t tb_get(int32_t st, int32_t i) const {
+        const int32_t s = st & 31;
+        return tb[(size_t(st >> 5) * size_t(steps) + size_t(i - 1 + s)) * 32u + size_t(s)];
+    }
+};
+
 template <bool AFFINE>
-__global__ void __launch_bounds__(kDpThreads) k_dp_wide(DpLaunch a, const uint64_t *tasks) {
-    const uint64_t T = uint64_t(gridDim.x) * blockDim.x;
-    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    DevScratch sc{a.tb, a.bnd, T, a.rmax, t};
-    const uint64_t n = *a.n_rest;
-    for (uint64_t idx = tasks[0] + t; idx < n; idx += T) {
-        const uint32_t si = a.perm[idx];
-        const DpSeg g = a.segs[si];
-        const SegView v = dpseg_view(g, a.scode, a.soff, a.slen, a.qcode, a.qoff);
-        dp_fill<kStripW, AFFINE>(v, sc);
-        OpsWriter w{a.ops + uint64_t(si) * a.stride, int32_t(a.stride * 16u)};
-        DpSum sum;
-        dp_traceback<kStripW>(v, sc, w, sum);
-        w.flush();
-        a.sums[si] = sum;
+__global__ void __launch_bounds__(kLongWarps * 32) k_dp_long(DpLaunch a, const uint64_t *tasks) {
+    const int lane = int(threadIdx.x & 31u);
+    const uint64_t nw = uint64_t(gridDim.x) * kLongWarps, wid = uint64_t(blockIdx.x) * kLongWarps + (threadIdx.x >> 5);
+    const int32_t steps = a.rmax + 31;
+    uint16_t *tb = a.tb + wid * a.long_codes;
+    int32_t *bnd = a.bnd + wid * uint64_t(3 * (a.rmax + 1));
+    const uint64_t first = tasks ? tasks[0] : 0u, n = *a.n_rest;
+    for (uint64_t k = wid; first + k < n; k += nw) {
+        const uint32_t si = a.perm[n - 1 - k];  // the widest first
+        const SegView v = seg_view(a, si);
+        const int32_t R = v.R, nst = (v.C + kStripW - 1) / kStripW;
+        for (int32_t p = 0; p * 32 < nst; p++) {
+            const int32_t j0 = (p * 32 + lane) * kStripW, G = nst - p * 32 < 32 ? nst - p * 32 : 32;
+            const bool active = lane < G;
+            uint8_t bc[kStripW];
+            int32_t uf[kStripW], ux[kStripW], uy[kStripW];
+            Cell3 prev{0, 0, 0}, pub{kNEG, kNEG, kNEG};
+            bool full = false;
+            int32_t wlast = -1;
+            uint8_t ch = 0;
+            if (active) {
+                dp_strip_init<kStripW, AFFINE>(v, j0, bc, uf, ux, uy);
+                prev = dp_row0<AFFINE>(v, j0);
+                full = dp_strip_full(v, j0, kStripW);
+                wlast = dp_strip_wlast(v, j0, kStripW);
+                ch = v.row(1);
+            }
+            const bool hand_on = lane == 31 && (p + 1) * 32 < nst;
+            uint16_t *row = tb + size_t(p) * size_t(steps) * 32u + lane;
+#pragma unroll 1
+            for (int32_t t = 0; t < R + G - 1; t++) {
+                Cell3 in;
+                in.f = __shfl_up_sync(0xffffffffu, pub.f, 1);
+                in.x = __shfl_up_sync(0xffffffffu, pub.x, 1);
+                in.y = __shfl_up_sync(0xffffffffu, pub.y, 1);
+                const int32_t i = t - lane + 1;
+                if (active && i >= 1 && i <= R) {
+                    const uint8_t base = ch;
+                    if (i < R) ch = v.row(i + 1);
+                    Cell3 left = in;
+                    if (lane == 0) left = p == 0 ? dp_col0<AFFINE>(v, i) : Cell3{bnd[3 * i], bnd[3 * i + 1], bnd[3 * i + 2]};
+                    const Cell3 lb = left;
+                    row[size_t(t) * 32u] = uint16_t(dp_strip_row_any<kStripW, AFFINE>(full, wlast, v, i, j0, base, bc, uf, ux, uy, left, prev));
+                    pub = left;
+                    prev = lb;
+                    if (hand_on) {  // read by lane 0 in the next panel; its own reads of this row are 31 steps past
+                        bnd[3 * i] = left.f;
+                        bnd[3 * i + 1] = left.x;
+                        bnd[3 * i + 2] = left.y;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (lane == 0) {
+            OpsWriter w{a.ops + uint64_t(si) * a.stride, int32_t(a.stride * 16u)};
+            const int32_t np = dp_walk<kStripW>(v, LongCodes{tb, steps}, w);
+            w.flush();
+            DpSum sum;
+            ops_summary(a.ops + uint64_t(si) * a.stride, a.stride * 16u - uint32_t(np), uint32_t(np), sum);
+            a.sums[si] = sum;
+        }
+        __syncwarp();
     }
 }
 
@@ -2342,10 +2370,19 @@ void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void 
     k_dp_scatter<<<grid_1d(a.nd, 256), 256, 0, st>>>(a, a.bins, bin_off, order);
 }
 
-uint64_t dp_threads(int device) {
+// Warps of k_dp_long and their scratch: the resident ones, fewer where the codes
+// of long reads would take more than 2 GB (a read of 32767 bases: 270 MB a warp).
+size_t dp_long_sizes(int device, int32_t rmax, int32_t cmax, DpLaunch &a) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    return uint64_t(sms) * 8u * kDpThreads;
+    const uint64_t panels = (uint64_t((cmax + kStripW - 1) / kStripW) + 31) / 32;
+    a.long_codes = panels * uint64_t(rmax + 31) * 32u;
+    const uint64_t fit = (uint64_t(1) << 31) / (a.long_codes * 2);
+    a.long_blocks = std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(sms) * 3, fit / kLongWarps));
+    return size_t(a.long_blocks * kLongWarps * a.long_codes * 2);
+}
+size_t dp_long_bounds(int32_t rmax, const DpLaunch &a) {
+    return size_t(a.long_blocks) * kLongWarps * size_t(rmax + 1) * 3 * 4;
 }
 
 // shared memory of a wavefront block: per warp, the lanes' strip tables and
@@ -2385,13 +2422,13 @@ void launch_dp(const DpLaunch &a_in, const uint64_t *bin_off, uint64_t *tasks, i
     // pairs need 32-bit code rows; without the room none run
     if (wave_smem(a.rmax, 4, a.warps) > 200u * 1024u) a.pair_mask = 0;
     a.tb_bytes = a.pair_mask ? 4u : 2u;
+    const unsigned gl = unsigned(a.long_blocks);
     if (!dp_wave_fits(a.rmax)) {  // rows too long for the shared-memory codes
-        const unsigned g = unsigned(a.threads / kDpThreads);
         counted();
         if (a.affine) {
-            k_dp<true><<<g, kDpThreads, 0, st>>>(a);
+            k_dp_long<true><<<gl, kLongWarps * 32, 0, st>>>(a, nullptr);
         } else {
-            k_dp<false><<<g, kDpThreads, 0, st>>>(a);
+            k_dp_long<false><<<gl, kLongWarps * 32, 0, st>>>(a, nullptr);
         }
         return;
     }
@@ -2435,12 +2472,11 @@ void launch_dp(const DpLaunch &a_in, const uint64_t *bin_off, uint64_t *tasks, i
     counted();
     fn<<<g, unsigned(32 * a.warps), smem, st>>>(a, tasks);
     if (cmax > 32 * kStripW) {
-        const unsigned gw = unsigned(a.threads / kDpThreads);
         counted();
         if (a.affine) {
-            k_dp_wide<true><<<gw, kDpThreads, 0, st>>>(a, tasks);
+            k_dp_long<true><<<gl, kLongWarps * 32, 0, st>>>(a, tasks);
         } else {
-            k_dp_wide<false><<<gw, kDpThreads, 0, st>>>(a, tasks);
+            k_dp_long<false><<<gl, kLongWarps * 32, 0, st>>>(a, tasks);
         }
     }
 }

@@ -115,7 +115,7 @@ void pair_run(Seg &a, Seg &b, Count n) {
     for (int h = 0; h < 2; h++) {
         const Seg &g = h ? b : a;
         n.c[0]++;
-        if (g.b.C - e[h].v > band_limit<AFFINE, NB, TYPE>(g.b)) continue;
+        if (g.b.C - e[h].v > band_limit<AFFINE, TYPE>(g.b, NB)) continue;
         n.c[1]++;
         DpSum want, sum;
         const std::vector<uint8_t> ops = whole(g.v, AFFINE, want);
@@ -139,6 +139,53 @@ void pair_run(Seg &a, Seg &b, Count n) {
     }
 }
 
+struct Edge {
+    std::vector<uint32_t> a, b;
+    uint32_t &m(int32_t t) { return a[size_t(t)]; }
+    uint32_t &l(int32_t t) { return b[size_t(t)]; }
+};
+struct WideStore {
+    int rows;
+    std::vector<uint32_t> w;
+    void put(int32_t k, int32_t t, uint32_t bits) { w[size_t(k) * rows + t] = bits; }
+};
+struct WideCodes {
+    const WideStore &s;
+    int half;
+    uint32_t get(int32_t k, int32_t t) const { return (s.w[size_t(k) * s.rows + t] >> (16 * half)) & 0xffffu; }
+};
+
+// the wide window; b may be of another type and size
+template <bool AFFINE>
+void wide_pair(int nb, int ta, int tb, Seg &a, Seg &b, Count n) {
+    a.b.base = wide_base(AFFINE, nb, ta, a.b.R - a.b.C);
+    b.b.base = wide_base(AFFINE, nb, tb, b.b.R - b.b.C);
+    const int32_t cmax = a.b.C > b.b.C ? a.b.C : b.b.C;
+    Edge edge;
+    edge.a.assign(wide_rows(nb), 0x12345678u);
+    edge.b.assign(wide_rows(nb), 0x12345678u);
+    WideStore st{wide_rows(nb), std::vector<uint32_t>(size_t(wide_rows(nb)) * ((cmax + 7) / 8), 0u)};
+    int32_t v[2];
+    wide_fill<AFFINE>(a.b, b.b, ta, tb, nb, cmax, edge, st, v[0], v[1]);
+    for (int h = 0; h < 2; h++) {
+        const Seg &g = h ? b : a;
+        n.c[0]++;
+        if (g.b.C - v[h] > wide_limit<AFFINE>(g.b, h ? tb : ta, nb)) continue;
+        n.c[1]++;
+        DpSum want, sum{};
+        const std::vector<uint8_t> ops = whole(g.v, AFFINE, want);
+        const uint32_t stride = uint32_t((g.b.R + g.b.C + 15) / 16);
+        std::vector<uint32_t> w(stride + 1, 0xffffffffu);
+        OpsPut put{w.data(), int32_t(stride * 16)};
+        const int32_t np = wide_walk<AFFINE>(g.b, h ? tb : ta, nb, WideCodes{st, h}, g.rev ? OP_I : OP_D, g.rev ? OP_D : OP_I, put);
+        bool ok = np == int32_t(ops.size());
+        if (ok) ops_summary(w.data(), stride * 16 - uint32_t(np), uint32_t(np), sum);
+        for (size_t k = 0; ok && k < ops.size(); k++) ok = ops_field(w.data(), uint32_t(stride * 16 - ops.size() + k)) == ops[k];
+        n.c[3] += !ok;
+        n.c[4] += memcmp(&sum, &want, sizeof(sum)) != 0;
+    }
+}
+
 template <bool AFFINE, int NB>
 void pair_type(int type, bool mask, Seg &a, Seg &b, Count n) {
 #define HERO_RUN(T) (mask ? pair_run<AFFINE, NB, T, true>(a, b, n) : pair_run<AFFINE, NB, T, false>(a, b, n))
@@ -157,6 +204,23 @@ bool takes(int nb, bool mask, const Seg &g, int type) {
 void pair_any(bool affine, int nb, int type, bool mask, Seg &a, Seg &b, Count n) {
     if (nb == 0) {  // the screen alone
         for (const Seg *g : {&a, &b}) affine ? screen_run<true>(*g, type, n) : screen_run<false>(*g, type, n);
+        return;
+    }
+    if (nb < 0) {  // the wide window of -nb diagonals: a segment beside the one before it
+        static Seg before;
+        static int before_type = -1, before_nb = 0;
+        if (before_nb != nb) before_type = -1;
+        before_nb = nb;
+        for (Seg *g : {&a, &b}) {
+            if (g->b.m < g->b.R || (type == BT_NONE && g->b.R - g->b.C >= -nb - 1)) continue;
+            if (before_type >= 0) affine ? wide_pair<true>(-nb, before_type, type, before, *g, n) : wide_pair<false>(-nb, before_type, type, before, *g, n);
+            before = *g;
+            before.b.row.w = before.rp.data() + kPackPad;
+            before.b.col.w = before.cp.data() + kPackPad;
+            before.v.row_base = before.rowc.data();
+            before.v.col_base = before.colc.data();
+            before_type = type;
+        }
         return;
     }
     if (!takes(nb, mask, a, type) || !takes(nb, mask, b, type)) return;
@@ -266,7 +330,7 @@ void band_random(int affine, int nb, int mask, uint64_t seed, uint64_t pairs, in
                 row.insert(type == BT_RIGHT ? row.begin() : row.end(), c);
             }
             while (int(row.size()) < C) row.push_back(uint8_t(rng_next(x) & 3));
-            if (type == BT_NONE && int(row.size()) > C + (nb > 2 ? nb - 2 : 0)) row.resize(C);
+            if (type == BT_NONE && int(row.size()) > C + (nb > 2 ? nb - 2 : nb < -2 ? -nb - 2 : 0)) row.resize(C);
             const bool swap = (rng_next(x) & 1) && int(row.size()) > C;  // the query on the rows
             const int64_t band = band_max > 0 ? int64_t(rng_next(x) % uint64_t(band_max)) : 65535;
             const auto &s = swap ? col : row, &q = swap ? row : col;

@@ -34,8 +34,9 @@ def _clean(counts):
     return segments, certified, straight
 
 
-# nb 0: the segments finished without a window (at most one mismatch on the main diagonal)
-@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 4), (1, 8), (1, 16), (0, 0), (0, 4), (0, 8)])
+# nb 0: the segments finished without a window (at most one mismatch on the main diagonal);
+# nb < 0: the wide window of -nb diagonals
+@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 4), (1, 8), (1, 16), (1, -4), (1, -7), (0, 0), (0, 4), (0, 8), (0, -4)])
 @pytest.mark.parametrize("kind", [0, 1, 2], ids=["both", "right", "left"])
 def test_every_short_segment(band, affine, nb, kind):
     n = np.zeros(3, np.int64)
@@ -46,13 +47,14 @@ def test_every_short_segment(band, affine, nb, kind):
                     c = (C.c_uint64 * 6)()
                     band.band_exhaustive(affine, nb, kind, mask, letters, rows, cols, C.c_int64(m), c)
                     n += _clean(list(c))
-    assert n[1] > n[2] > 0 and n[1] > n[0] // (4 if nb else 50)  # it accepts, and not only the plainest paths
+    assert n[1] > n[2] and n[1] > n[0] // (4 if nb else 50)  # it accepts, and not only the plainest paths
 
 
-@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 11), (1, 16), (1, 19), (1, 24), (1, 26), (1, 40), (0, 0), (0, 8), (0, 16)])
+@pytest.mark.parametrize("affine,nb", [(1, 0), (1, 11), (1, 16), (1, 19), (1, 24), (1, 26), (1, 40), (1, -24), (1, -96), (0, 0), (0, 8),
+                                       (0, 16), (0, -24), (0, -96)])
 @pytest.mark.parametrize("cmax", [5, 40, 250, 1023])
 def test_random_segments(band, affine, nb, cmax):
-    for mask, m in ((0, 0), (1, 4), (1, 30)):
+    for mask, m in ((0, 0), (1, 4), (1, 30)) if nb >= 0 else ((0, 0),):  # the wide window takes whole bands
         c = (C.c_uint64 * 6)()
         band.band_random(affine, nb, mask, C.c_uint64(nb * 1000 + cmax), C.c_uint64(200000 // (cmax + 100)), cmax,
                          C.c_int64(m), c)
@@ -90,11 +92,35 @@ def _segments(rng, n):
     return out
 
 
+def _long_segments(rng, n):
+    """Segments of up to 800 rows and 600 columns: copies with many mismatches and
+    gaps (the wide window), and unrelated strings (whole matrices, in panels)."""
+    out = []
+    for i in range(n):
+        c = int(rng.choice([100, 129, 255, 256, 257, 263, 264, 511, 512, 513, 600]))
+        kind = int(rng.integers(0, 3))
+        col = ACGT[rng.integers(0, 4, c)]
+        row = col.copy() if i % 4 else ACGT[rng.integers(0, 4, c)]
+        for p in rng.integers(0, c, int(rng.integers(0, 25))):
+            row[p] = ACGT[rng.integers(0, 4)]
+        for _ in range(int(rng.integers(0, 5))):
+            p, k = int(rng.integers(0, len(row))), int(rng.integers(1, 12))
+            row = np.concatenate([row[:p], ACGT[rng.integers(0, 4, k)], row[p:]]) if rng.random() < 0.5 \
+                else np.delete(row, slice(p, p + k))
+        d = int(rng.integers(0, 200)) if kind else 0
+        free = ACGT[rng.integers(0, 4, d)]
+        row = np.concatenate([free, row] if kind == 1 else [row, free])
+        s, q = (row, col) if rng.random() < 0.5 else (col, row)
+        out.append((bytes(s), bytes(q), int(rng.choice([20, 900, 900])), kind))
+    return out
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("affine", [0, 1])
-def test_gpu_segments_at_the_edges_of_the_classes(gpu_lib, oracle, affine):
+@pytest.mark.parametrize("make,count", [(_segments, 5000), (_long_segments, 300), (_long_segments, 7)])
+def test_gpu_segments_at_the_edges_of_the_classes(gpu_lib, oracle, affine, make, count):
     from hero_b200 import Hero
-    seg = _segments(np.random.default_rng(40 + affine), 5000)
+    seg = make(np.random.default_rng(40 + affine), count)
     n = len(seg)
     off = [np.zeros(n + 1, np.uint64) for _ in range(2)]
     for h in range(2):
