@@ -1760,8 +1760,16 @@ __global__ void k_map_choose(Params p, uint64_t nsub, const uint32_t *cstart,
 // --mapping: QueryDataset::getCoverageAndWriteResults (QueryDataset.cpp:560-599)
 // -- per query base the sum of its four vote counts (no self vote), counted
 // into hist[min(sum, bins - 1)]; the largest sum goes to *maxc.  One warp per read.
-__global__ void k_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
+// A block counts sums below kHistSmem in shared memory -- nearly all, a sum is
+// about the coverage -- and adds its counts once: a global atomic a base, all on
+// a few dozen bins, took 3.6 ms for 6 Mbp of queries.
+constexpr uint32_t kHistSmem = 4096;
+
+__global__ void __launch_bounds__(256) k_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
                            unsigned long long *hist, unsigned long long *maxc) {
+    __shared__ uint32_t part[kHistSmem];
+    for (uint32_t i = threadIdx.x; i < kHistSmem; i += blockDim.x) part[i] = 0;
+    __syncthreads();
     const uint32_t lane = lane_id();
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
     unsigned long long mx = 0;
@@ -1779,13 +1787,20 @@ __global__ void k_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdif
             if (i < Lr) {
                 const uint64_t sum = uint64_t(cov[(b + i) * 4]) + cov[(b + i) * 4 + 1] +
                                      cov[(b + i) * 4 + 2] + cov[(b + i) * 4 + 3] + uint64_t(run);
-                atomicAdd(&hist[sum < bins ? sum : bins - 1], 1ull);
+                if (sum < kHistSmem && sum < bins) {
+                    atomicAdd(&part[sum], 1u);
+                } else {
+                    atomicAdd(&hist[sum < bins ? sum : bins - 1], 1ull);
+                }
                 mx = sum > mx ? sum : mx;
             }
         }
     }
     mx = warp_max(mx);
     if (lane == 0) atomicMax(maxc, mx);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kHistSmem; i += blockDim.x)
+        if (part[i]) atomicAdd(&hist[i], (unsigned long long)part[i]);
 }
 
 // one thread per subject: its units (rec_off = exclusive scan of alist_n)
@@ -2504,7 +2519,7 @@ void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uin
                      unsigned long long *hist, unsigned long long *maxc, cudaStream_t st) {
     if (!q.n) return;
     counted();
-    k_map_hist<<<grid_1d(q.n * 32, 256), 256, 0, st>>>(q, cov, mdiff, bins, hist, maxc);
+    k_map_hist<<<grid_1d(q.n * 32, 256, 148u * 8u), 256, 0, st>>>(q, cov, mdiff, bins, hist, maxc);
 }
 
 void launch_aln_list(uint64_t nsub, const uint32_t *cstart, const uint32_t *ccount,
