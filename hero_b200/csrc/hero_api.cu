@@ -581,7 +581,7 @@ struct DpBufs {
 static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
     if (!a.nd) return HERO_OK;
     BandWork w{};
-    const size_t codes = band_sizes(c->dev, a.nd, a.rmax, cmax, a.affine != 0, w);
+    const size_t codes = band_sizes(c->dev, a.nd, cmax, a.affine != 0, w);
     const size_t table = kBandBins * (sizeof(BandBin) + 4) + kBandHead * 4;
     w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 8, "DP windows") &&
            c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 8, "DP windows") &&

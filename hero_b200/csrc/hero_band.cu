@@ -241,7 +241,7 @@ __device__ __noinline__ void band_task(const DpLaunch &a, const BandWork &w, con
             a.sums[si[h]] = sum;
         }
         walk[h] = __ballot_sync(0xffffffffu, sure && !e[h].straight);
-        const bool wide = has && !sure && !MASK && s[h].R >= w.wide_min;  // whole bands only
+        const bool wide = has && !sure && !MASK;  // whole bands only
         rest_append(a, has && !sure && !wide, si[h], a.segs[si[h]]);
         const uint32_t m = __ballot_sync(0xffffffffu, wide);
         if (m) {
@@ -327,107 +327,127 @@ __global__ void __launch_bounds__(kBandWarps * 32, kBandBlocks) k_band(DpLaunch 
     }
 }
 
-// The wide window of what the register windows left, 64 segments a warp in list
-// order (theirs: class, type, columns).  One-warp blocks; the strips' edges in
-// shared memory (18 KB for 64 diagonals, 26 KB for 96).  Bound by its serial chain, a row of
-// eight cells after the other; what it replaces -- the whole matrix -- took 31 of
-// 33 ms on 300-600 bp reads and 8 of 38 ms on 75-250 bp ones: now 2.2 and 2.7 ms.
-// A task is 71 rows a strip after strip where the whole-matrix wavefront is one
-// pass down the rows, so batches of up to 128 rows, and those too small to fill
-// the device with tasks, stay with that (1.67 M x 150 bp: 42.4 ms of DP without
-// the wide window, 44.5 with; 4310 reads of 75-250 bp: 0.95 and 1.65 ms), as do
-// single segments below 64 rows.
-constexpr int32_t kWideBatchRows = 128, kWideMinRows = 64;
-constexpr uint64_t kWideMinSegments = 4000000;  // below it only batches with columns past 256, where
-                                                // the whole matrices are k_dp_long's
-struct SmemEdge {
-    uint32_t *p;  // + lane
-    __device__ __forceinline__ uint32_t &m(int32_t t) { return p[t * 64]; }
-    __device__ __forceinline__ uint32_t &l(int32_t t) { return p[t * 64 + 32]; }
-};
-struct WideStore {
-    uint32_t *p;  // + lane
-    int32_t rows;
-    __device__ __forceinline__ void put(int32_t k, int32_t t, uint32_t bits) { p[size_t(k * rows + t) * 32] = bits; }
-};
+// The wide window of what the register windows left: a group of 8 lanes (64
+// diagonals; 16 and 136 for small batches and columns past 256) a pair of segments,
+// in list order (theirs: class, type, columns).  Bound by the chain down the
+// strips, nine steps a strip; a thread a pair, strip after strip, was six times
+// that chain and slower than whole matrices for all but large batches.  What it
+// replaces -- the whole matrix -- took 31 of 33 ms on 300-600 bp reads, 8 of 38 ms
+// on 75-250 bp ones and 0.38 ms on 4310 such reads: now 2.1, 4.6 and 0.32
+// with what it leaves to them.
 struct WideCodes {
-    const uint32_t *p;  // + lane of the segment
-    int32_t rows;
+    const uint32_t *p;  // + first lane of the group
+    int32_t lanes;
     uint32_t shift;
     __device__ __forceinline__ uint32_t get(int32_t k, int32_t t) const {
-        return (p[size_t(k * rows + t) * 32] >> shift) & 0xffffu;
+        return (p[size_t(kWideLag * k + t) * 32 + (k & (lanes - 1))] >> shift) & 0xffffu;
     }
 };
 
-template <bool AFFINE>
-__global__ void __launch_bounds__(32) k_band_wide(DpLaunch a, BandWork w) {
-    extern __shared__ uint32_t edges[];
-    const uint32_t lane = threadIdx.x;
-    const int32_t nb = w.wide_nb, rows = wide_rows(nb);
-    uint32_t *codes = w.codes + size_t(blockIdx.x) * w.wide_words;
+constexpr int kWideWarps = 4;
+// A batch with enough work runs 64 diagonals, and whole matrices what that
+// leaves; a smaller one waits for its longest chain, so it takes 136, which leave
+// almost nothing to a second chain.
+constexpr uint64_t kWideManySegments = 300000;
+
+template <bool AFFINE, int LANES>
+__global__ void __launch_bounds__(kWideWarps * 32) k_band_wide(DpLaunch a, BandWork w) {
+    constexpr int NB = wide_diagonals(LANES), ROWS = wide_rows(NB);
+    constexpr uint32_t SEGS = 64 / LANES;  // segments a task
+    const uint32_t lane = lane_id(), gl = lane % LANES, gbase = lane - gl;
+    uint32_t *codes = w.codes + size_t(blockIdx.x * kWideWarps + (threadIdx.x >> 5)) * w.wide_words;
     const uint32_t count = w.head[3];
     for (;;) {
         uint32_t q = 0;
         if (lane == 0) q = atomicAdd(&w.head[4], 1u);
         q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= (count + kTaskSegs - 1) / kTaskSegs) break;
-        const uint32_t *list = w.again + size_t(q) * kTaskSegs;
-        const uint32_t n = min(count - q * kTaskSegs, uint32_t(kTaskSegs));
+        if (q >= (count + SEGS - 1) / SEGS) break;
+        const uint32_t *list = w.again + size_t(q) * SEGS;
+        const uint32_t n = min(count - q * SEGS, SEGS);
         BandSeg s[2];
         uint32_t si[2];
         int type[2];
         bool rev[2];
-        int32_t v[2], cmax = 0;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const uint32_t k = lane + 32u * h;
+            const uint32_t k = 2u * (lane / LANES) + uint32_t(h);
             si[h] = list[k < n ? k : 0u];
             const DpSeg g = a.segs[si[h]];
             s[h] = band_seg(a, g, rev[h]);
             type[h] = band_type(g);
-            s[h].base = wide_base(AFFINE, nb, type[h], s[h].R - s[h].C);
-            cmax = max(cmax, s[h].C);
+            s[h].base = wide_base(AFFINE, NB, type[h], s[h].R - s[h].C);
         }
-        cmax = __reduce_max_sync(0xffffffffu, cmax);
-        SmemEdge edge{edges + lane};
-        WideStore st{codes + lane, rows};
-        wide_fill<AFFINE>(s[0], s[1], type[0], type[1], nb, cmax, edge, st, v[0], v[1]);
-        __syncwarp();
+        const int32_t strips = (max(s[0].C, s[1].C) + kWideStrip - 1) / kWideStrip;
+        const int32_t most = __reduce_max_sync(0xffffffffu, strips);
+        const int32_t steps = kWideLag * (most - 1) + ROWS;
+        WideLane<AFFINE, LANES> x{int(gl)};
+        const int src = int(gbase + (gl + LANES - 1) % LANES);
+        uint32_t *out = codes + lane;
 #pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-            const bool has = lane + 32u * h < n;
-            const bool sure = has && s[h].C - v[h] <= wide_limit<AFFINE>(s[h], type[h], nb);
-            if (sure) {
-                OpsPut put{a.ops + uint64_t(si[h]) * a.stride, int32_t(a.stride * 16u)};
-                DpSum sum;
-                const uint32_t up = rev[h] ? uint32_t(OP_I) : uint32_t(OP_D), left = rev[h] ? uint32_t(OP_D) : uint32_t(OP_I);
-                const int32_t np = wide_walk<AFFINE>(s[h], type[h], nb, WideCodes{codes + lane, rows, h ? 16u : 0u}, up, left, put);
-                ops_summary(put.w, a.stride * 16u - uint32_t(np), uint32_t(np), sum);
-                a.sums[si[h]] = sum;
-            }
-            rest_append(a, has && !sure, si[h], a.segs[si[h]]);
+        for (int32_t t = 0; t < steps; t++, out += 32) {
+            const uint32_t in_m = __shfl_sync(0xffffffffu, x.out_m, src);
+            const uint32_t in_y = AFFINE ? __shfl_sync(0xffffffffu, x.out_y, src) : 0u;
+            const int32_t u = t - kWideLag * x.k;
+            const bool on = u >= 0 && u < ROWS && x.k < strips;
+            if (on && u == 0) x.begin(s[0], s[1], type[0], type[1]);
+            if ((t & 15) == 0 && on) x.refill(s[0], s[1]);
+            const bool any_ends = __any_sync(0xffffffffu, on && x.ends);
+            if (on) *out = x.row(s[0], s[1], type[0], type[1], in_m, in_y, any_ends);
+            if (u == ROWS) x.k += LANES;
+            x.last_m = in_m;
         }
+        int32_t v[2];
+        v[0] = __shfl_sync(0xffffffffu, x.va, int(gbase) + ((s[0].C - 1) / kWideStrip) % LANES);
+        v[1] = __shfl_sync(0xffffffffu, x.vb, int(gbase) + ((s[1].C - 1) / kWideStrip) % LANES);
+        __syncwarp();  // the codes of every lane are written
+        // lanes 0 and 1 of a group trace its two segments
+        const int h = int(gl & 1u);
+        const BandSeg sh = h ? s[1] : s[0];
+        const int th = h ? type[1] : type[0];
+        const uint32_t sih = h ? si[1] : si[0];
+        const bool has = gl < 2u && 2u * (lane / LANES) + uint32_t(h) < n;
+        const bool sure = has && sh.C - (h ? v[1] : v[0]) <= wide_limit<AFFINE>(sh, th, NB);
+        if (sure) {
+            const bool reversed = h ? rev[1] : rev[0];
+            OpsPut put{a.ops + uint64_t(sih) * a.stride, int32_t(a.stride * 16u)};
+            DpSum sum;
+            const int32_t np = wide_walk<AFFINE>(sh, th, NB, WideCodes{codes + gbase, LANES, h ? 16u : 0u},
+                                                 reversed ? uint32_t(OP_I) : uint32_t(OP_D),
+                                                 reversed ? uint32_t(OP_D) : uint32_t(OP_I), put);
+            ops_summary(put.w, a.stride * 16u - uint32_t(np), uint32_t(np), sum);
+            a.sums[sih] = sum;
+        }
+        rest_append(a, has && !sure, sih, a.segs[sih]);
         __syncwarp();
+    }
+}
+
+template <bool AFFINE>
+void wide_launch(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
+    const unsigned g = unsigned(w.wide_blocks);
+    if (w.wide_lanes == 8) {
+        k_band_wide<AFFINE, 8><<<g, kWideWarps * 32, 0, st>>>(a, w);
+    } else {
+        k_band_wide<AFFINE, 16><<<g, kWideWarps * 32, 0, st>>>(a, w);
     }
 }
 
 }  // namespace
 
 // Resident warps for nd segments (half a task each at least), the code words of
-// each -- and, in the same words, the wide window's blocks, which need more each.
-size_t band_sizes(int device, uint64_t nd, int32_t rmax, int32_t cmax, bool affine, BandWork &w) {
+// each -- and, in the same words, the wide window's blocks, whose warps need others.
+size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &w) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const uint32_t c = uint32_t(cmax < kBandMaxC ? cmax : kBandMaxC);
     const uint64_t full = uint64_t(sms) * kBandBlocks, need = (nd + 32 * kBandWarps - 1) / (32 * kBandWarps);
     w.warps = kBandWarps * (need < full ? need : full);
     w.code_words = c * 32u * (affine ? 5u : 2u);
-    w.wide_nb = c <= 256u ? 64 : 96;
-    const bool wide = rmax > kWideBatchRows && (cmax > 256 || nd >= kWideMinSegments);
-    w.wide_min = wide ? kWideMinRows : 1 << 30;
-    w.wide_words = (c + kWideStrip - 1) / kWideStrip * uint32_t(wide_rows(w.wide_nb)) * 32u;
-    const uint64_t words = std::max<uint64_t>(w.warps * w.code_words, wide ? w.wide_words : 0u);
-    w.wide_blocks = wide ? std::min<uint64_t>(words / w.wide_words, uint64_t(sms) * (w.wide_nb > 64 ? 8 : 12)) : 0u;
+    w.wide_lanes = c <= 256u && nd >= kWideManySegments ? 8 : 16;
+    w.wide_words = uint32_t(kWideLag * ((c + kWideStrip - 1) / kWideStrip - 1) + wide_rows(wide_diagonals(w.wide_lanes))) * 32u;
+    const uint64_t block = uint64_t(w.wide_words) * kWideWarps;
+    const uint64_t words = std::max<uint64_t>(w.warps * w.code_words, block);
+    w.wide_blocks = std::min<uint64_t>(words / block, full);
     return words * 4;
 }
 
@@ -449,13 +469,11 @@ void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
     } else {
         k_band<false><<<blocks, kBandWarps * 32, 0, st>>>(a, w);
     }
-    if (!w.wide_blocks) return;
     count_launch();
-    const size_t wide_smem = size_t(wide_rows(w.wide_nb)) * 64 * 4;
     if (a.affine) {
-        k_band_wide<true><<<unsigned(w.wide_blocks), 32, wide_smem, st>>>(a, w);
+        wide_launch<true>(a, w, st);
     } else {
-        k_band_wide<false><<<unsigned(w.wide_blocks), 32, wide_smem, st>>>(a, w);
+        wide_launch<false>(a, w, st);
     }
 }
 

@@ -490,16 +490,20 @@ HERO_HD int32_t band_walk(const BandSeg &s, const Codes &codes, uint32_t gap_up,
 }
 
 // ---------------------------------------------------------------------------
-// The wide window: NB diagonals at run time, for the segments whose deficit the
-// register windows cannot certify.  Strips of eight columns, the strip's columns
-// in registers, its last column's M and next IY kept by row for the next strip
-// (edge.m(t), edge.l(t)).  A strip's row t is row first column + base + t, so
-// cell (t, w) lies on window diagonal t - w; rows 0 .. NB + 6 hold the window and
-// some cells beside it, whose values are paths' all the same.  The two segments
-// of a pair may differ in type and columns.
+// The wide window: for the segments whose deficit the register windows cannot
+// certify.  Strips of eight columns, one lane a strip, in turn: a strip's row t
+// is row first column + base + t, so cell (t, w) lies on window diagonal t - w,
+// and rows 0 .. nb + 6 hold the window and some cells beside it, whose values are
+// paths' all the same.  The strip before reaches a matrix row eight rows of its
+// own later and started nine steps earlier, so a group of lanes, strip k on lane
+// k mod lanes starting at step 9 k, passes each row's last M and next IY on by
+// one shuffle a step, and a lane is free again when its next strip starts.  The
+// two segments of a pair may differ in type and columns.
 // ---------------------------------------------------------------------------
 constexpr int kWideStrip = 8;
+constexpr int kWideLag = kWideStrip + 1;  // steps between the starts of neighbouring strips
 HERO_HD constexpr int wide_rows(int nb) { return nb + kWideStrip - 1; }
+HERO_HD constexpr int wide_diagonals(int lanes) { return kWideLag * lanes - kWideStrip; }  // one step of rest a strip
 
 HERO_HD int wide_near(bool affine, int nb) { return affine ? (nb - 1) / 3 : (nb - 1) / 2; }
 HERO_HD int32_t wide_base(bool affine, int nb, int type, int32_t d) {
@@ -554,101 +558,121 @@ HERO_HD uint32_t wide_row(uint32_t (&m)[kWideStrip], uint32_t (&xn)[kWideStrip],
     return acc;
 }
 
-HERO_HD bool any_lane(bool x) {
-#if defined(__CUDA_ARCH__)
-    return __any_sync(0xffffffffu, x);
-#else
-    return x;
-#endif
-}
-
-// cmax: the most columns of the warp's segments; st.put(strip, row, codes)
-template <bool AFFINE, class Edge, class Store>
-HERO_HD void wide_fill(const BandSeg &a, const BandSeg &b, int type_a, int type_b, int32_t nb, int32_t cmax,
-                       Edge &edge, Store &st, int32_t &va, int32_t &vb) {
+// A lane of the wide window: the strip it is on.
+template <bool AFFINE, int LANES>
+struct WideLane {
     using K = BandCost<AFFINE>;
-    const uint32_t dead = band_half2(kBandDead);
-    const int32_t rows = wide_rows(nb), da = a.R - a.C, db = b.R - b.C;
-    const int32_t cea = da - a.base < nb - 1 ? da - a.base : nb - 1, ceb = db - b.base < nb - 1 ? db - b.base : nb - 1;
-    va = vb = kBandDead;
-    // column 0, rows base .. base + nb - 1, as the last column of a strip before the first
-    for (int32_t t = kWideStrip - 1; t < rows; t++) {
-        const int32_t u = t - (kWideStrip - 1), ia = a.base + u, ib = b.base + u;
-        edge.m(t) = pack2(ia >= 0 ? 4 * (wide_col0<AFFINE>(type_a, ia) + K::pot * u) : kBandDead,
-                          ib >= 0 ? 4 * (wide_col0<AFFINE>(type_b, ib) + K::pot * u) : kBandDead);
-        if (AFFINE) {
-            const int32_t la = type_a == BT_RIGHT ? band_col0_right<BT_RIGHT>(ia) : band_col0_right<BT_LEFT>(ia);
-            const int32_t lb = type_b == BT_RIGHT ? band_col0_right<BT_RIGHT>(ib) : band_col0_right<BT_LEFT>(ib);
-            edge.l(t) = pack2(ia >= 0 ? 4 * (la + u + 1) : kBandDead, ib >= 0 ? 4 * (lb + u + 1) : kBandDead);
-        }
+    static constexpr int NB = wide_diagonals(LANES), ROWS = wide_rows(NB), PERIOD = kWideLag * LANES;
+    uint32_t m[kWideStrip], xn[kWideStrip], sel[kWideStrip], free[kWideStrip];
+    uint32_t ra = 0, rb = 0;      // the next rows' bases
+    uint32_t out_m, out_y;        // last column's M and next column's IY of the row done last
+    uint32_t last_m;              // the neighbour's M a step ago
+    int32_t k, t = 0;             // strip, row
+    int32_t va = kBandDead, vb = kBandDead;  // scores at the segments' ends, on the lanes that meet them
+    bool ends = false;            // a segment's column C is in the strip
+
+    HERO_HD explicit WideLane(int lane) : k(lane) { out_m = out_y = last_m = band_half2(kBandDead); }
+
+    // M of column 0 at the row of strip 0's row u (u >= -1), and IY of its right neighbour
+    HERO_HD static int32_t col0(int type, int32_t base, int32_t u) {
+        const int32_t i = base + 1 + u;
+        return i < 0 ? kBandDead : 4 * (wide_col0<AFFINE>(type, i) + K::pot * (u + 1));
     }
-    uint32_t wca = 0, wcb = 0;
-    for (int32_t j0 = 1, k = 0; j0 <= cmax; j0 += kWideStrip, k++) {
-        uint32_t m[kWideStrip], xn[kWideStrip], sel[kWideStrip], free[kWideStrip], mts[kWideStrip], fxs[kWideStrip];
+    HERO_HD static int32_t col0_right(int type, int32_t base, int32_t u) {
+        const int32_t i = base + 1 + u;
+        if (i < 0) return kBandDead;
+        if (!AFFINE) return col0(type, base, u);
+        return 4 * ((type == BT_RIGHT ? band_col0_right<BT_RIGHT>(i) : band_col0_right<BT_LEFT>(i)) + u + 2);
+    }
+
+    HERO_HD void begin(const BandSeg &a, const BandSeg &b, int type_a, int type_b) {
+        const uint32_t dead = band_half2(kBandDead);
+        const int32_t j0 = kWideStrip * k + 1;
         const int32_t ja = j0 < a.C ? j0 : a.C, jb = j0 < b.C ? j0 : b.C;  // no reads past a shorter segment's end
-        if ((k & 1) == 0) {
-            wca = pack16(a.col, ja - 1);
-            wcb = pack16(b.col, jb - 1);
-        }
+        uint32_t wa = pack16(a.col, ja - 1), wb = pack16(b.col, jb - 1);
+        ends = (a.C >= j0 && a.C < j0 + kWideStrip) || (b.C >= j0 && b.C < j0 + kWideStrip);
 #pragma unroll
         for (int w = 0; w < kWideStrip; w++) {
             m[w] = xn[w] = dead;
-            sel[w] = band_sel(wca & 3u, wcb & 3u);
-            wca >>= 2;
-            wcb >>= 2;
+            sel[w] = band_sel(wa & 3u, wb & 3u);
+            wa >>= 2;
+            wb >>= 2;
             free[w] = (type_a == BT_LEFT && j0 + w == a.C ? 0xffffu : 0u) |
                       (type_b == BT_LEFT && j0 + w == b.C ? 0xffff0000u : 0u);
         }
-        const bool ends = any_lane((a.C >= j0 && a.C < j0 + kWideStrip) || (b.C >= j0 && b.C < j0 + kWideStrip));
-        PackStream sa(a.row, ja + a.base - 1), sb(b.row, jb + b.base - 1);
-        uint32_t ra = 0, rb = 0, dm = edge.m(kWideStrip - 1);
-        for (int32_t t = 0; t < rows; t++) {
-            if ((t & 15) == 0) {
-                ra = sa.next();
-                rb = sb.next();
-            }
-            const bool in = t + kWideStrip < rows;  // the strip before has this row
-            uint32_t y = in ? (AFFINE ? edge.l(t + kWideStrip) : edge.m(t + kWideStrip)) : dead;
-            const uint32_t next = in ? edge.m(t + kWideStrip) : dead;
-            const uint32_t ta = band_table<AFFINE>(ra & 3u), tb = band_table<AFFINE>(rb & 3u);
-            ra >>= 2;
-            rb >>= 2;
-            uint32_t acc;
-            // row 0: its IX equal its IY, which a row's gap extensions leave as they are
-            const uint32_t row0 = (j0 + a.base + t == 0 ? 0xffffu : 0u) | (j0 + b.base + t == 0 ? 0xffff0000u : 0u);
-            const uint32_t y0 = y + 0x00020002u;
-            if (ends) {
-                acc = wide_row<AFFINE, true>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
-#pragma unroll
-                for (int w = 0; w < kWideStrip; w++) {
-                    // above the window an align-left path climbs freely: its row, or the window's last
-                    const int32_t pot = K::pot * (2 * (j0 + w) + t - w);
-                    if (j0 + w == a.C && t - w == cea) va = (half_lo(da - a.base > cea ? fxs[w] : mts[w]) >> 2) - pot;
-                    if (j0 + w == b.C && t - w == ceb) vb = (half_hi(db - b.base > ceb ? fxs[w] : mts[w]) >> 2) - pot;
-                }
-            } else {
-                acc = wide_row<AFFINE, false>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
-            }
-            if (AFFINE && row0) {
-#pragma unroll
-                for (int w = 0; w < kWideStrip; w++) xn[w] = (xn[w] & ~row0) | (add2(y0, free[w] & K::free_more) & row0);
-            }
-            st.put(k, t, acc);
-            edge.m(t) = m[kWideStrip - 1];
-            if (AFFINE) edge.l(t) = y;
-            dm = next;
-        }
+        t = 0;
+        refill(a, b);
     }
-}
+
+    // the bases of the next sixteen rows: at the strip's first row, and every
+    // sixteen steps of the warp, so that its lanes load together
+    HERO_HD void refill(const BandSeg &a, const BandSeg &b) {
+        const int32_t j0 = kWideStrip * k + 1;
+        ra = pack16(a.row, (j0 < a.C ? j0 : a.C) + a.base - 1 + t);
+        rb = pack16(b.row, (j0 < b.C ? j0 : b.C) + b.base - 1 + t);
+    }
+
+    // Row t of strip k; in_m, in_y: what the neighbour passed on.  any_ends: some
+    // lane of the warp has a column C in its strip.  Returns the row's codes.
+    HERO_HD uint32_t row(const BandSeg &a, const BandSeg &b, int type_a, int type_b, uint32_t in_m, uint32_t in_y,
+                         bool any_ends) {
+        const uint32_t dead = band_half2(kBandDead);
+        const int32_t j0 = kWideStrip * k + 1;
+        uint32_t dm = t + kWideStrip - 1 < ROWS ? last_m : dead;  // (row above, j0 - 1)
+        uint32_t y = t + kWideStrip < ROWS ? in_y : dead;
+        if (k == 0) {
+            dm = pack2(col0(type_a, a.base, t - 1), col0(type_b, b.base, t - 1));
+            y = pack2(col0_right(type_a, a.base, t), col0_right(type_b, b.base, t));
+            if (t + kWideStrip >= ROWS) y = dead;  // past the window
+            if (t + kWideStrip - 1 >= ROWS) dm = dead;
+        } else if (!AFFINE) {
+            y = t + kWideStrip < ROWS ? in_m : dead;
+        }
+        const uint32_t ta = band_table<AFFINE>(ra & 3u), tb = band_table<AFFINE>(rb & 3u);
+        ra >>= 2;
+        rb >>= 2;
+        // row 0: its IX equal its IY, which a row's gap extensions leave as they are
+        const uint32_t row0 = (j0 + a.base + t == 0 ? 0xffffu : 0u) | (j0 + b.base + t == 0 ? 0xffff0000u : 0u);
+        const uint32_t y0 = y + 0x00020002u;
+        uint32_t mts[kWideStrip], fxs[kWideStrip], acc;
+        if (any_ends) {
+            acc = wide_row<AFFINE, true>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
+            const int32_t da = a.R - a.C - a.base, db = b.R - b.C - b.base;  // the ends' window places
+            const int32_t cea = da < NB - 1 ? da : NB - 1, ceb = db < NB - 1 ? db : NB - 1;
+#pragma unroll
+            for (int w = 0; w < kWideStrip; w++) {
+                // above the window an align-left path climbs freely: its row, or the window's last
+                const int32_t pot = K::pot * (2 * (j0 + w) + t - w);
+                if (j0 + w == a.C && t - w == cea) va = (half_lo(da > cea ? fxs[w] : mts[w]) >> 2) - pot;
+                if (j0 + w == b.C && t - w == ceb) vb = (half_hi(db > ceb ? fxs[w] : mts[w]) >> 2) - pot;
+            }
+        } else {
+            acc = wide_row<AFFINE, false>(m, xn, sel, ta, tb, dm, y, free, mts, fxs);
+        }
+        if (AFFINE && row0) {
+#pragma unroll
+            for (int w = 0; w < kWideStrip; w++) xn[w] = (xn[w] & ~row0) | (add2(y0, free[w] & K::free_more) & row0);
+        }
+        out_m = m[kWideStrip - 1];
+        out_y = y;
+        t++;
+        return acc;
+    }
+};
 
 // band_walk over the wide window's codes: codes.get(strip, row) holds the
-// strip's eight cells of a row
+// strip's eight cells of a row.  Diagonal runs are found eight cells at a time.
 template <bool AFFINE, class Codes>
 HERO_HD int32_t wide_walk(const BandSeg &s, int type, int32_t nb, const Codes &codes, uint32_t gap_up,
                           uint32_t gap_left, OpsPut &out) {
     using T = PairTags<AFFINE>;
+    constexpr int32_t AHEAD = 8;
     const int32_t end = out.p;
     int32_t i = s.R, j = s.C;
+    auto code_at = [&](int32_t ci, int32_t cj) {
+        const int32_t k = (cj - 1) >> 3;
+        return (codes.get(k, ci - (kWideStrip * k + 1) - s.base) >> (2 * ((cj - 1) & 7))) & 3u;
+    };
     if (type == BT_LEFT && i - j - s.base > nb - 1) {
         const int32_t k = i - j - s.base - (nb - 1);
         out.run(gap_up, uint32_t(k));
@@ -656,18 +680,30 @@ HERO_HD int32_t wide_walk(const BandSeg &s, int type, int32_t nb, const Codes &c
     }
     while (i > 0 && j > 0) {
         if (uint32_t(i - j - s.base) >= uint32_t(nb)) return -1;
-        const int32_t k = (j - 1) >> 3, w = (j - 1) & 7;
-        const uint32_t code = (codes.get(k, i - (kWideStrip * k + 1) - s.base) >> (2 * w)) & 3u;
-        if (code == uint32_t(T::diag)) {
-            i--;
-            j--;
-            out.fields((pack16(s.row, i) ^ pack16(s.col, j)) & 3u ? 1u : 0u, 1u);
-        } else if (code == uint32_t(T::up)) {
-            i--;
+        const int32_t n = i < j ? (i < AHEAD ? i : AHEAD) : (j < AHEAD ? j : AHEAD);
+        uint32_t code[AHEAD];
+#pragma unroll
+        for (int t = 0; t < AHEAD; t++) code[t] = t < n ? code_at(i - t, j - t) : 3u;
+        int32_t run = 0;
+        uint32_t stop = 3u;
+#pragma unroll
+        for (int t = AHEAD - 1; t >= 0; t--)
+            if (code[t] != uint32_t(T::diag)) {
+                run = t;
+                stop = code[t];
+            }
+        if (stop == 3u) run = n;
+        if (run > 0) {
+            i -= run;
+            j -= run;
+            out.fields(mismatch16(pack16(s.row, i), pack16(s.col, j)) & ops_mask(0, uint32_t(run - 1)), uint32_t(run));
+        }
+        if (stop == uint32_t(T::up)) {
             out.fields(gap_up, 1u);
-        } else {
-            j--;
+            i--;
+        } else if (stop == uint32_t(T::left)) {
             out.fields(gap_left, 1u);
+            j--;
         }
     }
     out.run(gap_up, uint32_t(i));

@@ -213,15 +213,14 @@ struct BandWork {
     BandBin *bin;      // the non-empty keys
     uint32_t *head;    // their number, the number of tasks, the next task; wide: segments, next task
     uint32_t *again;   // segments for the wide window
-    uint32_t *codes;   // traceback codes: code_words a warp, then wide_words a block
+    uint32_t *codes;   // traceback codes: code_words a warp, then wide_words a warp
     uint32_t code_words, wide_words;
-    int32_t wide_nb;   // diagonals of the wide window
-    int32_t wide_min;  // rows from which a segment takes it
+    int32_t wide_lanes;  // lanes a pair of the wide window
     uint64_t warps, wide_blocks;
 };
 constexpr int kBandHead = 8;
 // sets warps, wide_blocks and their words; returns the bytes of `codes`
-size_t band_sizes(int device, uint64_t nd, int32_t rmax, int32_t cmax, bool affine, BandWork &w);
+size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &w);
 // fills ops, sums and cells of the segments it certifies; a.rest, a.n_rest (zeroed
 // before) and a.bins (zeroed before) get the others
 void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st);

@@ -139,34 +139,46 @@ void pair_run(Seg &a, Seg &b, Count n) {
     }
 }
 
-struct Edge {
-    std::vector<uint32_t> a, b;
-    uint32_t &m(int32_t t) { return a[size_t(t)]; }
-    uint32_t &l(int32_t t) { return b[size_t(t)]; }
-};
-struct WideStore {
-    int rows;
-    std::vector<uint32_t> w;
-    void put(int32_t k, int32_t t, uint32_t bits) { w[size_t(k) * rows + t] = bits; }
-};
 struct WideCodes {
-    const WideStore &s;
-    int half;
-    uint32_t get(int32_t k, int32_t t) const { return (s.w[size_t(k) * s.rows + t] >> (16 * half)) & 0xffffu; }
+    const std::vector<uint32_t> &w;
+    int lanes, half;
+    uint32_t get(int32_t k, int32_t t) const {
+        return (w[size_t(kWideLag * k + t) * lanes + k % lanes] >> (16 * half)) & 0xffffu;
+    }
 };
 
 // the wide window; b may be of another type and size
-template <bool AFFINE>
-void wide_pair(int nb, int ta, int tb, Seg &a, Seg &b, Count n) {
+template <bool AFFINE, int LANES>
+void wide_pair(int ta, int tb, Seg &a, Seg &b, Count n) {
+    constexpr int nb = wide_diagonals(LANES);
     a.b.base = wide_base(AFFINE, nb, ta, a.b.R - a.b.C);
     b.b.base = wide_base(AFFINE, nb, tb, b.b.R - b.b.C);
-    const int32_t cmax = a.b.C > b.b.C ? a.b.C : b.b.C;
-    Edge edge;
-    edge.a.assign(wide_rows(nb), 0x12345678u);
-    edge.b.assign(wide_rows(nb), 0x12345678u);
-    WideStore st{wide_rows(nb), std::vector<uint32_t>(size_t(wide_rows(nb)) * ((cmax + 7) / 8), 0u)};
+    const int32_t cmax = a.b.C > b.b.C ? a.b.C : b.b.C, strips = (cmax + 7) / 8;
+    const int32_t steps = kWideLag * (strips - 1) + wide_rows(nb);
+    std::vector<uint32_t> codes(size_t(steps) * LANES, 0u);
+    std::vector<WideLane<AFFINE, LANES>> lane;
+    for (int l = 0; l < LANES; l++) lane.emplace_back(l);
+    for (int32_t s = 0; s < steps; s++) {  // the lanes of a step read what the step before left
+        std::vector<uint32_t> in_m(LANES), in_y(LANES);
+        for (int l = 0; l < LANES; l++) {
+            in_m[l] = lane[(l + LANES - 1) % LANES].out_m;
+            in_y[l] = lane[(l + LANES - 1) % LANES].out_y;
+        }
+        for (int l = 0; l < LANES; l++) {
+            WideLane<AFFINE, LANES> &w = lane[l];
+            const int32_t u = s - kWideLag * w.k;
+            if (u == 0 && w.k < strips) w.begin(a.b, b.b, ta, tb);
+            if (u >= 0 && u < wide_rows(nb) && w.k < strips && (s & 15) == 0) w.refill(a.b, b.b);
+            if (u >= 0 && u < wide_rows(nb) && w.k < strips)
+                codes[size_t(s) * LANES + l] = w.row(a.b, b.b, ta, tb, in_m[l], in_y[l], w.ends);
+            if (u == wide_rows(nb)) w.k += LANES;
+            w.last_m = in_m[l];
+        }
+    }
     int32_t v[2];
-    wide_fill<AFFINE>(a.b, b.b, ta, tb, nb, cmax, edge, st, v[0], v[1]);
+    const int ka = ((a.b.C - 1) / 8) % LANES, kb = ((b.b.C - 1) / 8) % LANES;
+    v[0] = lane[ka].va;
+    v[1] = lane[kb].vb;
     for (int h = 0; h < 2; h++) {
         const Seg &g = h ? b : a;
         n.c[0]++;
@@ -177,7 +189,7 @@ void wide_pair(int nb, int ta, int tb, Seg &a, Seg &b, Count n) {
         const uint32_t stride = uint32_t((g.b.R + g.b.C + 15) / 16);
         std::vector<uint32_t> w(stride + 1, 0xffffffffu);
         OpsPut put{w.data(), int32_t(stride * 16)};
-        const int32_t np = wide_walk<AFFINE>(g.b, h ? tb : ta, nb, WideCodes{st, h}, g.rev ? OP_I : OP_D, g.rev ? OP_D : OP_I, put);
+        const int32_t np = wide_walk<AFFINE>(g.b, h ? tb : ta, nb, WideCodes{codes, LANES, h}, g.rev ? OP_I : OP_D, g.rev ? OP_D : OP_I, put);
         bool ok = np == int32_t(ops.size());
         if (ok) ops_summary(w.data(), stride * 16 - uint32_t(np), uint32_t(np), sum);
         for (size_t k = 0; ok && k < ops.size(); k++) ok = ops_field(w.data(), uint32_t(stride * 16 - ops.size() + k)) == ops[k];
@@ -213,7 +225,14 @@ void pair_any(bool affine, int nb, int type, bool mask, Seg &a, Seg &b, Count n)
         before_nb = nb;
         for (Seg *g : {&a, &b}) {
             if (g->b.m < g->b.R || (type == BT_NONE && g->b.R - g->b.C >= -nb - 1)) continue;
-            if (before_type >= 0) affine ? wide_pair<true>(-nb, before_type, type, before, *g, n) : wide_pair<false>(-nb, before_type, type, before, *g, n);
+            if (before_type >= 0) {
+                if (affine && nb == -10) wide_pair<true, 2>(before_type, type, before, *g, n);
+                if (affine && nb == -64) wide_pair<true, 8>(before_type, type, before, *g, n);
+                if (affine && nb == -136) wide_pair<true, 16>(before_type, type, before, *g, n);
+                if (!affine && nb == -10) wide_pair<false, 2>(before_type, type, before, *g, n);
+                if (!affine && nb == -64) wide_pair<false, 8>(before_type, type, before, *g, n);
+                if (!affine && nb == -136) wide_pair<false, 16>(before_type, type, before, *g, n);
+            }
             before = *g;
             before.b.row.w = before.rp.data() + kPackPad;
             before.b.col.w = before.cp.data() + kPackPad;
