@@ -685,7 +685,7 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         // the count pass leaves the slot of every window (2 x 8 bytes a subject base) for the emit pass
         if ((r = c->ensure(c->wcache, std::max<uint64_t>(nbases, 1) * 16, "probe windows"))) break;
         uint2 *wc = P_<uint2>(c->wcache);
-        launch_probe(false, c->p.aln != 0, subj, nsub, q, t, c->p.k, wc, P_<uint32_t>(c->seg_hits), nullptr, nullptr, ctr, c->st);
+        launch_probe(false, c->p.aln != 0, subj, nsub, q, t, c->p.k, c->p.l, wc, P_<uint32_t>(c->seg_hits), nullptr, nullptr, ctr, c->st);
         launch_scan_u32(P_<uint32_t>(c->seg_hits), P_<uint64_t>(c->hit_off), nseg, c->scan_tmp.p, c->st);
         uint64_t H = 0;
         if (cap) {
@@ -697,7 +697,7 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         }
         const uint64_t Hc = std::max<uint64_t>(H, 1);
         if ((r = c->ensure(c->hits, Hc * 8, "hits"))) break;
-        launch_probe(true, c->p.aln != 0, subj, nsub, q, t, c->p.k, wc, nullptr, P_<uint64_t>(c->hit_off), P_<uint64_t>(c->hits), ctr, c->st);
+        launch_probe(true, c->p.aln != 0, subj, nsub, q, t, c->p.k, c->p.l, wc, nullptr, P_<uint64_t>(c->hit_off), P_<uint64_t>(c->hits), ctr, c->st);
         launch_sort_hits(nseg, P_<uint64_t>(c->hit_off), P_<uint64_t>(c->hits), c->st);
         if ((r = c->check_launch("seed"))) break;
         rec(1);

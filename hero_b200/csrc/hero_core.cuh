@@ -100,6 +100,39 @@ HERO_HD void kmer_push_front(Kmer &m, uint32_t code, int k) {
     }
 }
 
+// k-mer keys of a window from its packed 2-bit codes (base t at bits 2t of the
+// 128-bit value {w[0], w[1], w[2], w[3]}, bits above 2k arbitrary): the key of the
+// window is the value with its digits reversed, that of its reverse complement
+// the value with every base complemented.
+HERO_HD uint64_t reverse_digits(uint64_t x) {  // the thirty-two 2-bit digits in reverse order
+#if defined(__CUDA_ARCH__)
+    x = __brevll(x);
+    return ((x >> 1) & 0x5555555555555555ull) | ((x & 0x5555555555555555ull) << 1);
+#else
+    uint64_t r = 0;
+    for (int i = 0; i < 32; i++) r |= ((x >> (2 * i)) & 3ull) << (2 * (31 - i));
+    return r;
+#endif
+}
+HERO_HD void kmer_from_window(const uint32_t (&w)[4], int k, Kmer &forward, Kmer &reverse) {
+    uint64_t lo = (uint64_t(w[1]) << 32) | w[0], hi = (uint64_t(w[3]) << 32) | w[2];
+    const int b = 2 * k;
+    const uint64_t ml = b >= 64 ? ~0ull : (1ull << b) - 1ull, mh = b > 64 ? (1ull << (b - 64)) - 1ull : 0ull;
+    lo &= ml;
+    hi &= mh;
+    reverse.lo = (lo ^ 0xaaaaaaaaaaaaaaaaull) & ml;
+    reverse.hi = (hi ^ 0xaaaaaaaaaaaaaaaaull) & mh;
+    const uint64_t rl = reverse_digits(hi), rh = reverse_digits(lo);  // 128 bits reversed, to shift right by 128 - b
+    const int s = 128 - b;
+    if (s >= 64) {
+        forward.lo = s == 64 ? rh : rh >> (s - 64);
+        forward.hi = 0;
+    } else {
+        forward.lo = (rl >> s) | (rh << (64 - s));
+        forward.hi = rh >> s;
+    }
+}
+
 // Jobs served together share one k-mer table: a key carries its job above the
 // 2k k-mer bits, so keys of different jobs never compare equal (job must fit
 // in the 128 - 2k bits left: kmer_job_bits).

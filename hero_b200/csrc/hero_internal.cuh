@@ -130,7 +130,7 @@ void launch_table_finalize(const uint64_t *klo, const uint64_t *khi, const uint3
 
 // aln: the alignment output's positions (seed_hit)
 void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView q, TableView t, int32_t k,
-                  uint2 *wcache, uint32_t *seg_hits, const uint64_t *hit_off, uint64_t *hits,
+                  int32_t l, uint2 *wcache, uint32_t *seg_hits, const uint64_t *hit_off, uint64_t *hits,
                   unsigned long long *counters, cudaStream_t st);
 void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
                        const uint32_t *ccount, ChainArrays ch, const uint32_t *keys,

@@ -107,24 +107,24 @@ __global__ void k_codes(const uint8_t *raw, uint64_t n, uint8_t *code, uint32_t 
 // QueryDataset::qualityFilter (QueryDataset.cpp:60-75), the good-read tests of
 // QueryDataset.cpp:226 (query) and SubjectDataset.cpp:157-162 (subject), and
 // QueryRead::setGcContent (QueryRead.cpp:73-81)
-__global__ void k_read_flags(const uint8_t *code, const uint64_t *off, uint64_t n, uint32_t *len,
-                             uint8_t *gq, uint8_t *gs, double *gc, int32_t l) {
-    for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n;
-         r += uint64_t(gridDim.x) * blockDim.x) {
+// One warp a read, 32 bases a step, counted by ballots (a thread a read chased
+// its bytes one at a time: 1.08 ms for 1.67 M x 150 bp, 21 us for 300 reads; now
+// 0.62 ms and 5 us).
+__global__ void __launch_bounds__(256)
+    k_read_flags(const uint8_t *code, const uint64_t *off, uint64_t n, uint32_t *len, uint8_t *gq,
+                 uint8_t *gs, double *gc, int32_t l) {
+    const uint32_t lane = lane_id();
+    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
+    for (uint64_t r = uint64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps) {
         const uint64_t b = off[r], L = off[r + 1] - b;
-        uint64_t cnt[4] = {0, 0, 0, 0};
-        bool valid = true;
-        uint64_t ngc = 0;
-        for (uint64_t i = 0; i < L; i++) {
-            const uint8_t c = code[b + i];
-            if (c >= 4) {
-                valid = false;
-            } else {
-                cnt[c]++;
-                ngc += (c & 1u);  // C (1) or G (3)
-            }
+        uint32_t cnt[4] = {0, 0, 0, 0};
+        for (uint64_t i0 = 0; i0 < L; i0 += 32) {
+            const uint32_t c = i0 + lane < L ? code[b + i0 + lane] : 255u;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) cnt[k] += uint32_t(__popc(__ballot_sync(0xffffffffu, c == k)));
         }
-        bool qf = valid;
+        if (lane != 0) continue;
+        bool qf = uint64_t(cnt[0]) + cnt[1] + cnt[2] + cnt[3] == L;  // no other letter
         if (qf) {
             const uint64_t thr = uint64_t(__dmul_rn(double(L), 0.8));
             if (cnt[0] >= thr || cnt[1] >= thr || cnt[2] >= thr || cnt[3] >= thr) qf = false;
@@ -133,7 +133,7 @@ __global__ void k_read_flags(const uint8_t *code, const uint64_t *off, uint64_t 
         len[r] = uint32_t(L);
         if (gq) gq[r] = (L > lu && qf) ? 1 : 0;
         if (gs) gs[r] = (L < lu || qf) ? 1 : 0;
-        if (gc) gc[r] = __ddiv_rn(double(ngc), double(L));
+        if (gc) gc[r] = __ddiv_rn(double(cnt[1] + cnt[3]), double(L));  // C (1) or G (3)
     }
 }
 
@@ -220,6 +220,28 @@ void scan_rec(const T *in, uint64_t *out, uint64_t n, uint64_t *tmp, cudaStream_
 // ---------------------------------------------------------------------------
 // k-mer table (HashTableLongKey.cpp:41-68, 250-342)
 // ---------------------------------------------------------------------------
+// the packed codes of bases at .. at + 63 of the read array (words of the window
+// that k needs; without packed codes from the bytes)
+__device__ __forceinline__ void window_words(const ReadsView &v, uint64_t at, int32_t k, uint32_t (&w)[4]) {
+    const int n = (2 * k + 31) / 32;
+    if (v.pack) {
+        const uint32_t *p = v.pack + (at >> 4);
+        const uint32_t sh = uint32_t(at & 15u) * 2u;
+        uint32_t cur = p[0];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t next = i < n ? p[i + 1] : 0u;
+            w[i] = __funnelshift_r(cur, next, sh);
+            cur = next;
+        }
+    } else {
+        for (int i = 0; i < 4; i++) {
+            w[i] = 0;
+            for (int j = 0; j < 16 && 16 * i + j < k; j++) w[i] |= uint32_t(v.code[at + 16 * i + j] & 3u) << (2 * j);
+        }
+    }
+}
+
 __global__ void k_key_count(ReadsView q, int32_t k, uint32_t *count) {
     for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < q.n;
          r += uint64_t(gridDim.x) * blockDim.x)
@@ -233,13 +255,14 @@ __global__ void k_key_emit(ReadsView q, int32_t k, const uint64_t *key_off, uint
         if (!q.good[r]) continue;
         const int64_t L = q.len[r];
         const int32_t nk = query_key_count(L, k);
-        const uint8_t *c = q.code + q.off[r];
         uint64_t e = key_off[r];
         const uint32_t tag = uid_tag(q.uid[r]);
         for (int32_t i = 0; i < nk; i++, e++) {
             const int64_t pos = query_key_pos(L, k, i);
-            Kmer m{0, 0};
-            for (int32_t t = 0; t < k; t++) kmer_push(m, c[pos + t] & 3u, k);
+            uint32_t w[4];
+            window_words(q, q.off[r] + uint64_t(pos), k, w);
+            Kmer m, rc;
+            kmer_from_window(w, k, m, rc);
             if (q.job) kmer_tag(m, q.job[r], k);
             klo[e] = m.lo;
             khi[e] = m.hi;
@@ -301,40 +324,45 @@ __global__ void k_table_finalize(const uint64_t *klo, const uint64_t *khi, const
 }
 
 // exact multimap lookup (HashTableLongKey::getListOfReads, HashTableLongKey.cpp:79-99)
-__device__ __forceinline__ bool table_find(const TableView &t, const Kmer &m, uint32_t &start,
-                                           uint32_t &count) {
-    uint64_t h = kmer_hash(m) & t.mask;
+// of a window's two keys: their first slots are loaded together
+struct SlotAt {
+    uint4 a, b;
+};
+__device__ __forceinline__ SlotAt slot_load(const TableView &t, uint64_t h) {
+    const uint4 *p = reinterpret_cast<const uint4 *>(&t.slots[h]);
+    return SlotAt{__ldg(p), __ldg(p + 1)};
+}
+// the slot's (start, count) for key m, walking on from slot h already loaded
+__device__ __forceinline__ uint2 slot_find(const TableView &t, const Kmer &m, uint64_t h, SlotAt s) {
     for (uint64_t it = 0; it <= t.mask; it++) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(&t.slots[h]));
-        const uint4 b = __ldg(reinterpret_cast<const uint4 *>(&t.slots[h]) + 1);
-        const uint32_t cnt = b.y;
-        if (cnt == 0) return false;
-        const uint64_t lo = (uint64_t(a.y) << 32) | a.x, hi = (uint64_t(a.w) << 32) | a.z;
-        if (lo == m.lo && hi == m.hi) {
-            start = b.x;
-            count = cnt;
-            return true;
-        }
+        if (s.b.y == 0) break;
+        const uint64_t lo = (uint64_t(s.a.y) << 32) | s.a.x, hi = (uint64_t(s.a.w) << 32) | s.a.z;
+        if (lo == m.lo && hi == m.hi) return make_uint2(s.b.x, s.b.y);
         h = (h + 1) & t.mask;
+        s = slot_load(t, h);
     }
-    return false;
+    return make_uint2(0u, 0u);
 }
 
 // ---------------------------------------------------------------------------
 // seeding: SubjectReadAligner::searchHashTable2 (SubjectReadAligner.cpp:444-491)
-// Count pass: one warp per subject read; lane f takes the contiguous windows
-// [fa, fb), so both k-mers roll one base per window (the forward window at f
-// and the reverse-complement window at L-k-f are the same bases).  It probes
-// the table for each window and orientation, counts the hits of each
-// (subject, orientation) and leaves the slot it found (start, count) in the
-// window cache, indexed by the window's base in the batch: 2 entries a base.
-// Emit pass: the same warps read the cache (lanes interleaved, so the reads
-// are coalesced) and write the hits without probing the table again.
+// Count pass: one warp per subject read, lane f windows f, f + 32, ...  Both keys
+// of a window come from its packed codes (the reverse-complement window at L-k-f
+// is the same bases), so a window costs the same wherever it lies.  It probes
+// the table for each orientation, counts the hits of each (subject,
+// orientation) and leaves the slots it found (start, count) in the window cache,
+// indexed by the window's base in the batch: 2 entries a base.
+// Emit pass: the same warps read the cache and write the hits without probing
+// the table again.
+// The count pass is bound by its scattered slots and values in L2.  Rolling the
+// keys base by base, a lane a stretch of windows, pushed k - 1 bases to fill the
+// first window of three or four: 14.9 ms for 1.67 M x 150 bp and 1.23 ms for
+// 300 k x 100 bp; now 13.6 (the table is four times the L2) and 0.84.
 // ---------------------------------------------------------------------------
 constexpr int kProbeWarps = 8;
 
 __global__ void __launch_bounds__(kProbeWarps * 32)
-    k_probe_count(ReadsView subj, uint64_t nsub, ReadsView q, TableView t, int32_t k, uint2 *wcache,
+    k_probe_count(ReadsView subj, uint64_t nsub, ReadsView q, TableView t, int32_t k, int32_t l, uint2 *wcache,
                   uint32_t *seg_hits, unsigned long long *counters) {
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     const uint64_t warps = uint64_t(gridDim.x) * kProbeWarps;
@@ -342,44 +370,39 @@ __global__ void __launch_bounds__(kProbeWarps * 32)
     unsigned long long probes = 0, nhits = 0;
     for (uint64_t s = uint64_t(blockIdx.x) * kProbeWarps + wib; s < nsub; s += warps) {
         const int32_t L = int32_t(subj.len[s]);
-        const int64_t su = subj.uid[s];
-        const uint32_t stag = uid_tag(su);
-        const uint8_t *c = subj.code + subj.off[s];
-        uint2 *wc = wcache + 2 * (subj.off[s] - base0);
         uint32_t c0 = 0, c1 = 0;
         if (subj.good[s] && L >= k) {
+            const int64_t su = subj.uid[s];
+            const uint32_t stag = uid_tag(su), job = subj.job ? subj.job[s] : 0u;
+            const uint64_t off = subj.off[s];
+            uint4 *wc = reinterpret_cast<uint4 *>(wcache) + (off - base0);
+            // a good subject holds another letter only if it is shorter than l
+            // (SubjectDataset.cpp:157-162): only there are the windows looked through
+            const bool letters = L < int32_t(uint16_t(l));
             const int32_t P = L - k + 1;
             if (lane == 0) probes += 2ull * uint64_t(P);
-            // nbad counts the non-ACGT bases in the window
-            const int32_t fa = int32_t(int64_t(P) * lane / 32), fb = int32_t(int64_t(P) * (lane + 1) / 32);
-            Kmer fr{0, 0}, rr{0, 0};
-            int32_t nbad = 0;
-            if (fa < fb)
-                for (int32_t i = 0; i < k - 1; i++) {
-                    const uint8_t x = c[fa + i];
-                    nbad += x >= 4;
-                    kmer_push(fr, x & 3u, k);
-                    kmer_push_front(rr, (x & 3u) ^ 2u, k);
-                }
-            for (int32_t f = fa; f < fb; f++) {
-                const uint8_t x = c[f + k - 1];
-                nbad += x >= 4;
-                if (f > fa) nbad -= c[f - 1] >= 4;
-                kmer_push(fr, x & 3u, k);
-                kmer_push_front(rr, (x & 3u) ^ 2u, k);
+            for (int32_t f = int32_t(lane); f < P; f += 32) {
+                bool bad = false;
+                if (letters)
+                    for (int32_t i = 0; i < k; i++) bad = bad || subj.code[off + uint64_t(f + i)] >= 4;
                 uint2 found[2] = {make_uint2(0, 0), make_uint2(0, 0)};
-                if (!nbad) {
-                    Kmer fm = fr, rm = rr;
+                if (!bad) {
+                    uint32_t w[4];
+                    window_words(subj, off + uint64_t(f), k, w);
+                    Kmer fm, rm;
+                    kmer_from_window(w, k, fm, rm);
                     if (subj.job) {
-                        kmer_tag(fm, subj.job[s], k);
-                        kmer_tag(rm, subj.job[s], k);
+                        kmer_tag(fm, job, k);
+                        kmer_tag(rm, job, k);
                     }
-                    for (int o = 0; o < 2; o++) {
-                        uint32_t st = 0, cnt = 0;
-                        if (!table_find(t, o ? rm : fm, st, cnt)) continue;
-                        found[o] = make_uint2(st, cnt);
-                        for (uint32_t e = 0; e < cnt; e++) {
-                            const uint64_t v = __ldg(&t.vals[st + e]);
+                    const uint64_t h0 = kmer_hash(fm) & t.mask, h1 = kmer_hash(rm) & t.mask;
+                    const SlotAt s0 = slot_load(t, h0), s1 = slot_load(t, h1);
+                    found[0] = slot_find(t, fm, h0, s0);
+                    found[1] = slot_find(t, rm, h1, s1);
+#pragma unroll
+                    for (int o = 0; o < 2; o++)
+                        for (uint32_t e = 0; e < found[o].y; e++) {
+                            const uint64_t v = __ldg(&t.vals[found[o].x + e]);
                             // self hit (SubjectReadAligner.cpp:463-465): ids compared
                             // only where their folds agree
                             if (value_tag(v) == stag && __ldg(&q.uid[value_query(v)]) == su) continue;
@@ -389,9 +412,8 @@ __global__ void __launch_bounds__(kProbeWarps * 32)
                                 c0++;
                             }
                         }
-                    }
                 }
-                reinterpret_cast<uint4 *>(wc)[f] = make_uint4(found[0].x, found[0].y, found[1].x, found[1].y);
+                wc[f] = make_uint4(found[0].x, found[0].y, found[1].x, found[1].y);
             }
         }
         c0 = warp_sum(c0);
@@ -2294,7 +2316,7 @@ void launch_prep_reads(const uint8_t *raw, uint64_t nbases, uint8_t *code, uint3
     }
     if (n) {
         counted();
-        k_read_flags<<<grid_1d(n, 128), 128, 0, st>>>(code, off, n, len, good_query, good_subject, gc, l);
+        k_read_flags<<<grid_1d(n, 8, 148u * 8u), 256, 0, st>>>(code, off, n, len, good_query, good_subject, gc, l);
     }
 }
 
@@ -2343,7 +2365,7 @@ void launch_table_finalize(const uint64_t *klo, const uint64_t *khi, const uint3
 }
 
 void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView q, TableView t, int32_t k,
-                  uint2 *wcache, uint32_t *seg_hits, const uint64_t *hit_off, uint64_t *hits,
+                  int32_t l, uint2 *wcache, uint32_t *seg_hits, const uint64_t *hit_off, uint64_t *hits,
                   unsigned long long *counters, cudaStream_t st) {
     if (!nsub) return;
     const unsigned g = grid_1d(nsub, kProbeWarps, 148u * 16u);
@@ -2351,7 +2373,7 @@ void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView 
     if (emit) {
         k_probe_emit<<<g, kProbeWarps * 32, 0, st>>>(subj, nsub, q, t, k, aln, wcache, hit_off, hits);
     } else {
-        k_probe_count<<<g, kProbeWarps * 32, 0, st>>>(subj, nsub, q, t, k, wcache, seg_hits, counters);
+        k_probe_count<<<g, kProbeWarps * 32, 0, st>>>(subj, nsub, q, t, k, l, wcache, seg_hits, counters);
     }
 }
 

@@ -280,6 +280,25 @@ struct CountWalk {
 
 extern "C" {
 
+// keys of random windows: from packed codes against base by base, for every k
+uint64_t window_keys(uint64_t seed) {
+    uint64_t x = seed * 0x9e3779b97f4a7c15ull + 1, wrong = 0;
+    for (int32_t k = 1; k <= 63; k++)
+        for (int rep = 0; rep < 50; rep++) {
+            uint32_t w[4];
+            for (uint32_t &v : w) v = uint32_t(rng_next(x) >> 16);  // bits above 2k arbitrary
+            Kmer f{0, 0}, r{0, 0}, gf, gr;
+            for (int32_t t = 0; t < k; t++) {
+                const uint32_t c = (w[t >> 4] >> (2 * (t & 15))) & 3u;
+                kmer_push(f, c, k);
+                kmer_push_front(r, c ^ 2u, k);
+            }
+            kmer_from_window(w, k, gf, gr);
+            wrong += gf.lo != f.lo || gf.hi != f.hi || gr.lo != r.lo || gr.hi != r.hi;
+        }
+    return wrong;
+}
+
 // random chains of increasing keys, with touching, overlapping and end-aligned
 // ones: chain_dp_count against the BandAligner calls of walk_chain
 uint64_t chain_counts(uint64_t seed, uint64_t chains) {

@@ -67,6 +67,11 @@ def test_dp_pieces_of_a_chain_counted_without_walking_it(band):
     assert band.chain_counts(C.c_uint64(3), C.c_uint64(200000)) == 0
 
 
+def test_keys_of_packed_windows(band):
+    band.window_keys.restype = C.c_uint64
+    assert band.window_keys(C.c_uint64(5)) == 0
+
+
 def _segments(rng, n):
     """(subject, query, band, flags): copies with e substitutions and at times an
     indel, on either side, with a free run on the anchored side's far end."""
