@@ -9,6 +9,8 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -79,7 +81,15 @@ struct hero_ctx {
     DBuf w_key, w_order, w_rest, w_bin, w_codes;
     bool window = true;             // off from an allocation that did not fit until the next query set
     bool consensus_done = false;  // out_seq holds the consensus of the current votes
-    std::vector<uint8_t> aln_host;  // .aln text of every subject aligned since the last take
+    // .aln text of every subject aligned since the last take: the batches' in host
+    // memory, except the last one's, which stays in a_text until the next batch
+    // needs it or a take copies it out
+    struct Text {
+        std::unique_ptr<uint8_t[]> p;
+        uint64_t n;
+    };
+    std::vector<Text> aln_host;
+    uint64_t aln_dev = 0;
     // index build temporaries (kept between builds)
     DBuf x_cnt, x_koff, x_klo, x_khi, x_kval, x_owner, x_count, x_slot_of, x_start, x_fill, x_tmp;
 
@@ -616,6 +626,14 @@ static int aln_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, ReadsView q,
     unsigned long long *ctr = P_<unsigned long long>(c->counters);
     if (NC >= uint64_t(kUnitChainLimit) || nsub >= uint64_t(kUnitChainLimit))
         return c->fail(HERO_E_INPUT, "too many chains or subjects in a batch");
+    if (c->aln_dev) {  // the batch before this one
+        hero_ctx::Text t{std::unique_ptr<uint8_t[]>(new (std::nothrow) uint8_t[c->aln_dev]), c->aln_dev};
+        if (!t.p) return c->fail(HERO_E_OOM, "host allocation failed for alignment text");
+        HERO_TRY(c->cuda(cudaMemcpyAsync(t.p.get(), c->a_text.p, t.n, cudaMemcpyDeviceToHost, c->st), "alignment text"));
+        HERO_TRY(c->cuda(cudaStreamSynchronize(c->st), "alignment text"));
+        c->aln_host.push_back(std::move(t));
+        c->aln_dev = 0;
+    }
     HERO_TRY(c->ensure(c->a_list, std::max<uint64_t>(NC, 1) * 4, "alignment lists"));
     HERO_TRY(c->ensure(c->a_n, nsub * 4 + 4, "alignment lists"));
     HERO_TRY(c->ensure(c->a_roff, (nsub + 1) * 8, "alignment lists"));
@@ -650,11 +668,9 @@ static int aln_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, ReadsView q,
                      P_<DpSum>(c->sums), P_<uint32_t>(c->a_pre), P_<uint32_t>(c->a_cig),
                      P_<char>(c->a_text), c->st);
     HERO_TRY(c->check_launch("alignment text"));
-    const size_t o = c->aln_host.size();
-    c->aln_host.resize(o + B);
-    if (B)
-        HERO_TRY(c->cuda(cudaMemcpyAsync(c->aln_host.data() + o, c->a_text.p, B, cudaMemcpyDeviceToHost, c->st), "alignment text"));
-    return c->cuda(cudaStreamSynchronize(c->st), "alignment text");
+    HERO_TRY(c->cuda(cudaStreamSynchronize(c->st), "alignment text"));
+    c->aln_dev = B;
+    return HERO_OK;
 }
 
 // runs every stage for subjects [0, nsub) of the given reads
@@ -1221,17 +1237,28 @@ extern "C" int hero_get_overhang(hero_ctx *c, uint32_t *out) {
 extern "C" int hero_alignments_size(hero_ctx *c, uint64_t *bytes) {
     if (!c || !bytes) return HERO_E_INPUT;
     if (!c->p.aln) return c->fail(HERO_E_STATE, "not an alignment-output context");
-    *bytes = c->aln_host.size();
+    *bytes = c->aln_dev;
+    for (const auto &t : c->aln_host) *bytes += t.n;
     return HERO_OK;
 }
 
 extern "C" int hero_alignments_take(hero_ctx *c, uint8_t *out, uint64_t cap) {
-    if (!c) return HERO_E_INPUT;
-    if (!c->p.aln) return c->fail(HERO_E_STATE, "not an alignment-output context");
-    const uint64_t n = c->aln_host.size();
+    uint64_t n = 0;
+    const int r = hero_alignments_size(c, &n);
+    if (r != HERO_OK) return r;
     if (cap < n || (n && !out)) return c->fail(HERO_E_INPUT, "output buffer too small");
-    if (n) std::memcpy(out, c->aln_host.data(), n);
-    std::vector<uint8_t>().swap(c->aln_host);
+    cudaSetDevice(c->dev);
+    if (c->aln_dev) {
+        HERO_TRY(c->cuda(cudaMemcpyAsync(out + (n - c->aln_dev), c->a_text.p, c->aln_dev, cudaMemcpyDeviceToHost, c->st),
+                         "alignment text"));
+        HERO_TRY(c->cuda(cudaStreamSynchronize(c->st), "alignment text"));
+    }
+    for (const auto &t : c->aln_host) {
+        std::memcpy(out, t.p.get(), t.n);
+        out += t.n;
+    }
+    std::vector<hero_ctx::Text>().swap(c->aln_host);
+    c->aln_dev = 0;
     return HERO_OK;
 }
 

@@ -572,10 +572,8 @@ HERO_HD uint32_t list_add(List &list, uint32_t n, uint64_t &largest, uint32_t id
 // decimal text of integers, as ostream prints them
 HERO_HD uint32_t dec_len(uint64_t v) {
     uint32_t n = 1;
-    while (v >= 10) {
-        v /= 10;
-        n++;
-    }
+    for (; v >> 32; v /= 10) n++;
+    for (uint32_t x = uint32_t(v); x >= 10u; x /= 10u) n++;  // most numbers: 32-bit steps
     return n;
 }
 HERO_HD uint32_t dec_len_signed(int64_t v) {
@@ -583,10 +581,9 @@ HERO_HD uint32_t dec_len_signed(int64_t v) {
 }
 HERO_HD char *dec_put(char *o, uint64_t v) {
     const uint32_t n = dec_len(v);
-    for (uint32_t i = n; i > 0; i--) {
-        o[i - 1] = char('0' + v % 10);
-        v /= 10;
-    }
+    uint32_t i = n;
+    for (; v >> 32; v /= 10) o[--i] = char('0' + v % 10);
+    for (uint32_t x = uint32_t(v); i > 0; x /= 10u) o[--i] = char('0' + x % 10u);
     return o + n;
 }
 HERO_HD char *dec_put_signed(char *o, int64_t v) {
@@ -604,8 +601,8 @@ HERO_HD char *dec_put_signed(char *o, int64_t v) {
 // AlignmentRecord::addCigar (AlignmentRecord.cpp:35-48) merges every equal
 // neighbour, whichever piece it came from.  "inserted" holds the query bases
 // of every I entry except the first and the last entry.  Driven by walk_chain
-// through a piece source: src.each(piece, f) calls f(op) for the ops of DP
-// piece `piece` in order.  Count mode (cig == nullptr) only sizes the text.
+// through a piece source: src.each(piece, f) calls f(op) or f(op, n) for the ops
+// of DP piece `piece` in order.  Count mode (cig == nullptr) only sizes the text.
 template <class Src>
 struct AlnText {
     Src src;
@@ -649,20 +646,18 @@ struct AlnText {
         }
         if (type != 'D') pq += n;
     }
-    HERO_HD void op(uint8_t o) {
-        if (o == OP_M) {
-            add('M', 1);
-        } else if (o == OP_X) {
-            add(qbase(pq), 1);
+    HERO_HD void op(uint8_t o, int64_t n) {  // n equal ops
+        if (o == OP_X) {
+            for (; n > 0; n--) add(qbase(pq), 1);
         } else {
-            add(o == OP_I ? 'I' : 'D', 1);
+            add(o == OP_M ? 'M' : o == OP_I ? 'I' : 'D', n);
         }
     }
     HERO_HD void begin(int64_t, int64_t, int64_t) {}
     HERO_HD void position(int64_t p) { pos = p; }
     HERO_HD void run(uint8_t o, int64_t n) { add(o == OP_M ? 'M' : o == OP_I ? 'I' : 'D', n); }
     HERO_HD void dp(int64_t, int64_t, int64_t, int64_t, uint32_t, int64_t) {
-        src.each(piece++, [this](uint8_t o) { op(o); });
+        src.each(piece++, [this](uint8_t o, int64_t n = 1) { op(o, n); });
     }
     HERO_HD bool check(int64_t, int64_t) { return true; }
     HERO_HD void finish() {
