@@ -46,7 +46,7 @@ struct hero_ctx {
     std::vector<DBuf *> all;
 
     // query set
-    uint64_t nq = 0, nqb = 0;
+    uint64_t nq = 0, nqb = 0, q_longest = 0;
     DBuf q_raw, q_code, q_off, q_len, q_uid, q_good, q_sgood, q_gc;
     DBuf q_job;            // job of each query read (jobs served together)
     bool tagged = false;   // q_job holds the reads' jobs
@@ -415,6 +415,8 @@ extern "C" int hero_set_queries(hero_ctx *c, const uint8_t *seq, const uint64_t 
     c->nq = n;
     c->nqb = n ? off[n] : 0;
     c->q_off_h.assign(off, off + (n ? n + 1 : 0));
+    c->q_longest = 0;
+    for (uint64_t i = 0; i < n; i++) c->q_longest = std::max(c->q_longest, off[i + 1] - off[i]);
     c->have_index = false;
     c->consensus_done = false;
     c->tagged = false;
@@ -956,7 +958,7 @@ extern "C" int hero_consensus_range(hero_ctx *c, uint64_t first, uint64_t count,
     cudaSetDevice(c->dev);
     const uint64_t n = c->nq, nb = c->nqb;
     HERO_TRY(c->ensure(c->out_seq, nb, "consensus"));
-    HERO_TRY(c->ensure(c->colsum, nb * 4, "consensus"));
+    HERO_TRY(c->ensure(c->colsum, c->q_longest > kConsensusRead ? nb * 4 : 0, "consensus"));
     HERO_TRY(c->ensure(c->o_imin, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imed, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imax, n * 4, "consensus"));
@@ -1025,7 +1027,7 @@ extern "C" int hero_consensus(hero_ctx *c, uint8_t *seq_out, uint32_t *imin, uin
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     HERO_TRY(c->ensure(c->out_seq, nb, "consensus"));
-    HERO_TRY(c->ensure(c->colsum, nb * 4, "consensus"));
+    HERO_TRY(c->ensure(c->colsum, c->q_longest > kConsensusRead ? nb * 4 : 0, "consensus"));
     HERO_TRY(c->ensure(c->o_imin, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imed, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imax, n * 4, "consensus"));
@@ -1069,7 +1071,7 @@ extern "C" int hero_reset_votes(hero_ctx *c) {
 static int consensus_device(hero_ctx *c) {
     const uint64_t n = c->nq, nb = c->nqb;
     HERO_TRY(c->ensure(c->out_seq, nb, "consensus"));
-    HERO_TRY(c->ensure(c->colsum, nb * 4, "consensus"));
+    HERO_TRY(c->ensure(c->colsum, c->q_longest > kConsensusRead ? nb * 4 : 0, "consensus"));
     HERO_TRY(c->ensure(c->o_imin, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imed, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_imax, n * 4, "consensus"));

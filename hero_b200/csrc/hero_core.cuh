@@ -1753,6 +1753,10 @@ HERO_HD int32_t column_consensus(const uint32_t c[4], double thr) {
         }
     }
     if (id < 0) return -1;  // no count above 0: the reference keeps id -1 too
+    // away from the threshold the difference of the counts decides: the fractions'
+    // difference is within a few roundings of it
+    const double d = HERO_DSUB(double(largest - larger), HERO_DMUL(thr, sum));
+    if (HERO_FABS(d) > HERO_DMUL(1e-9, sum)) return d > 0 ? id : -1;
     const double fLargest = HERO_DDIV(double(largest), sum);
     const double fLarger = HERO_DDIV(double(larger), sum);
     if (HERO_DSUB(fLargest, fLarger) >= thr) return id;

@@ -277,6 +277,8 @@ void launch_vote(const Params &p, bool chosen, uint64_t nc, ChainArrays ch, cons
                  const uint32_t *ccount, const uint32_t *keys, ReadsView subj, ReadsView q,
                  const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov, int32_t *mdiff,
                  unsigned long long *counters, cudaStream_t st);
+constexpr uint32_t kConsensusRead = 1024;  // longest read whose column sums stay in shared memory;
+                                           // colsum (a word a base) is only used beyond it
 void launch_consensus(const Params &p, ReadsView q, const uint32_t *cov, const int32_t *mdiff,
                       uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
                       uint32_t *imax, double *mis, cudaStream_t st);

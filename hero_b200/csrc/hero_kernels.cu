@@ -529,7 +529,7 @@ __device__ __forceinline__ void bitonic_warp(uint64_t *a, uint32_t n, uint32_t l
     }
 }
 
-// small segments: one warp each, in shared memory
+// small segments: one warp each, in registers (up to 32 hits) or shared memory
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_hits_warp(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits) {
     __shared__ uint64_t sm[kSortThreads / 32][kWarpSort];
@@ -538,6 +538,22 @@ __global__ void __launch_bounds__(kSortThreads)
          seg += uint64_t(gridDim.x) * (kSortThreads / 32)) {
         const uint64_t b = hit_off[seg], n = hit_off[seg + 1] - b;
         if (n < 2 || n > uint64_t(kWarpSort)) continue;
+        if (n <= 32) {  // in registers: the same network by shuffles, lanes past n at the end
+            uint64_t x = lane < uint32_t(n) ? hits[b + lane] : ~0ull;
+#pragma unroll
+            for (uint32_t k = 2; k <= 32; k <<= 1) {
+                if (k / 2 >= uint32_t(n)) break;
+#pragma unroll
+                for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                    // mirror step of the stage, then half cleaners: all ascending
+                    const uint32_t other = j == k >> 1 ? lane ^ (k - 1u) : lane ^ j;
+                    const uint64_t y = __shfl_sync(0xffffffffu, x, int(other));
+                    x = (lane < other) == (x < y) ? x : y;
+                }
+            }
+            if (lane < uint32_t(n)) hits[b + lane] = x;
+            continue;
+        }
         uint32_t lgN = 0;
         while ((1u << lgN) < uint32_t(n)) lgN++;
         uint64_t *a = sm[wib];
@@ -549,23 +565,35 @@ __global__ void __launch_bounds__(kSortThreads)
     }
 }
 
+// the segments of more than kWarpSort hits, a block each: it looks for them 256
+// segments at a time (one after the other took 0.12 ms a batch to find none)
 __global__ void __launch_bounds__(kSortThreads)
     k_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits) {
     __shared__ uint64_t sm[kSortSmem];
-    for (uint64_t seg = blockIdx.x; seg < nseg; seg += gridDim.x) {
-        const uint64_t b = hit_off[seg], n = hit_off[seg + 1] - b;
-        if (n <= uint64_t(kWarpSort)) continue;  // sorted by k_sort_hits_warp
-        uint64_t N = 1;
-        while (N < n) N <<= 1;
-        if (n <= uint64_t(kSortSmem)) {
-            for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = hits[b + i];
-            __syncthreads();
-            bitonic(sm, n, N);
-            for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) hits[b + i] = sm[i];
-            __syncthreads();
-        } else {
-            bitonic(hits + b, n, N);
-        }
+    for (uint64_t s0 = uint64_t(blockIdx.x) * kSortThreads; s0 < nseg; s0 += uint64_t(gridDim.x) * kSortThreads) {
+        const uint64_t mine = s0 + threadIdx.x;
+        const bool big = mine < nseg && hit_off[mine + 1] - hit_off[mine] > uint64_t(kWarpSort);
+        __shared__ uint32_t found[kSortThreads / 32];
+        const uint32_t m = __ballot_sync(0xffffffffu, big);
+        if ((threadIdx.x & 31u) == 0) found[threadIdx.x >> 5] = m;
+        if (!__syncthreads_or(big)) continue;
+        for (uint32_t w = 0; w < kSortThreads / 32; w++)
+            for (uint32_t left = found[w]; left; left &= left - 1u) {
+                const uint64_t seg = s0 + 32u * w + uint32_t(__ffs(int(left))) - 1u;
+                const uint64_t b = hit_off[seg], n = hit_off[seg + 1] - b;
+                uint64_t N = 1;
+                while (N < n) N <<= 1;
+                if (n <= uint64_t(kSortSmem)) {
+                    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) sm[i] = hits[b + i];
+                    __syncthreads();
+                    bitonic(sm, n, N);
+                    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) hits[b + i] = sm[i];
+                    __syncthreads();
+                } else {
+                    bitonic(hits + b, n, N);
+                }
+            }
+        __syncthreads();  // found is reused
     }
 }
 
@@ -890,20 +918,20 @@ __device__ __forceinline__ bool pair_strips(uint32_t mask, int n) {
 __global__ void k_dp_tasks(const uint64_t *bin_off, uint64_t *tasks, uint32_t pair_mask) {
     // tasks[n] (n = 1..33): first task of segments with n strips; tasks[34+n]:
     // first sorted segment with n strips; tasks[68+n]: one past the last.
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint64_t t = 0;
-    for (int n = 1; n <= 32; n++) {
-        const uint64_t b = bin_off[uint32_t(n) << kShapeStripShift];
-        const uint64_t e = bin_off[uint32_t(n + 1) << kShapeStripShift];
-        tasks[n] = t;
-        tasks[34 + n] = b;
-        tasks[68 + n] = e;
-        const uint64_t S = uint64_t(32 / n) * (pair_strips(pair_mask, n) ? 2u : 1u);  // segments a task
-        t += (e - b + S - 1) / S;
+    if (threadIdx.x >= 32 || blockIdx.x != 0) return;
+    const int n = int(threadIdx.x) + 1;
+    const uint64_t b = bin_off[uint32_t(n) << kShapeStripShift];
+    const uint64_t e = bin_off[uint32_t(n + 1) << kShapeStripShift];
+    tasks[34 + n] = b;
+    tasks[68 + n] = e;
+    const uint64_t S = uint64_t(32 / n) * (pair_strips(pair_mask, n) ? 2u : 1u);  // segments a task
+    uint64_t total;
+    tasks[n] = warp_exclusive<uint64_t>((e - b + S - 1) / S, &total);
+    if (n == 1) {
+        tasks[33] = total;
+        tasks[0] = bin_off[uint32_t(33) << kShapeStripShift];  // first segment for k_dp_long
+        tasks[kTaskQueue] = 0;  // work queue head of k_dp_wave
     }
-    tasks[33] = t;
-    tasks[0] = bin_off[uint32_t(33) << kShapeStripShift];  // first segment for k_dp_long
-    tasks[kTaskQueue] = 0;  // work queue head of k_dp_wave
 }
 
 // the wavefront over one warp's segments; FULL / LEFT are warp-uniform.  The
@@ -2188,9 +2216,11 @@ __global__ void k_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_
 
 // ---------------------------------------------------------------------------
 // consensus: QueryRead::callConsensus + calculateCoverageStatistic
-// (QueryRead.cpp:148-212); one warp per query read
+// (QueryRead.cpp:148-212); one warp per query read.  Bound by the votes read (20
+// bytes a base) and the work a column: two divisions a column and reductions by
+// shuffles took 4.0 ms for 250 Mbp, 0.6 for 30; now 3.0 and 0.45.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kConsWarps = 8, kConsSmem = 1024;  // column sums of reads up to 1024 bases
+constexpr uint32_t kConsWarps = 8, kConsSmem = kConsensusRead;  // column sums of reads up to that
 
 __global__ void __launch_bounds__(kConsWarps * 32)
     k_consensus(Params p, ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint8_t *out,
@@ -2223,9 +2253,10 @@ __global__ void __launch_bounds__(kConsWarps * 32)
             carry += tot;
             if (i < L) {
                 const uint8_t own = q.code[b + i];
-                uint32_t c[4];
-                for (int j = 0; j < 4; j++) c[j] = cov[(b + i) * 4 + j];
-                c[own] += uint32_t(run) + 1u;  // match votes + the read's own vote
+                const uint4 v = reinterpret_cast<const uint4 *>(cov)[b + i];
+                const uint32_t more = uint32_t(run) + 1u;  // match votes + the read's own vote
+                const uint32_t c[4] = {v.x + (own == 0 ? more : 0u), v.y + (own == 1 ? more : 0u),
+                                       v.z + (own == 2 ? more : 0u), v.w + (own == 3 ? more : 0u)};
                 const int32_t id = column_consensus(c, p.thr);
                 uint8_t nb = own;
                 if (id >= 0) {
@@ -2239,9 +2270,9 @@ __global__ void __launch_bounds__(kConsWarps * 32)
                 mx = sm > mx ? sm : mx;
             }
         }
-        changed = warp_sum(changed);
-        mn = warp_min(mn);
-        mx = warp_max(mx);
+        changed = __reduce_add_sync(0xffffffffu, changed);
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        mx = __reduce_max_sync(0xffffffffu, mx);
         __syncwarp();
         // median of the column sums (QueryRead.cpp:204-211: the sorted sums'
         // middle one, or the mean of the middle two): the p-th smallest value by
@@ -2251,7 +2282,7 @@ __global__ void __launch_bounds__(kConsWarps * 32)
         auto count_le = [&](uint32_t v) {
             uint32_t c = 0;
             for (uint32_t i = lane; i < L; i += 32) c += cs[i] <= v;
-            return warp_sum(c);
+            return __reduce_add_sync(0xffffffffu, c);
         };
         auto select = [&](uint32_t p, uint32_t lo, uint32_t hi) {
             while (lo < hi) {
@@ -2422,7 +2453,7 @@ void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView 
 
 void launch_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits, cudaStream_t st) {
     if (!nseg) return;
-    const unsigned g = unsigned(nseg < 148u * 16u ? nseg : 148u * 16u);
+    const unsigned g = grid_1d(nseg, kSortThreads, 148u * 16u);
     counted();
     k_sort_hits_warp<<<grid_1d(nseg, kSortThreads / 32, 148u * 8u), kSortThreads, 0, st>>>(
         nseg, hit_off, hits);
