@@ -160,7 +160,8 @@ struct hero_ctx {
         b.pooled = false;
     }
     // gives the window DP's buffers back (work that reads them is queued before
-    // the stream-ordered frees); false when there are none
+    // the stream-ordered frees; views taken before drop their packed codes, see
+    // still()); false when there are none
     bool shed() {
         bool any = false;
         for (DBuf *b : {&q_pack, &s_pack, &w_key, &w_order, &w_rest, &w_bin, &w_codes}) {
@@ -256,6 +257,11 @@ static size_t pack_bytes(uint64_t nb) { return size_t((nb + 15) / 16 + 2 * kPack
 static ReadsView query_view(hero_ctx *c) {
     return ReadsView{P_<uint8_t>(c->q_code), P_<uint64_t>(c->q_off), P_<uint32_t>(c->q_len),
                      P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_good), c->nq, job_tags(c), pack_words(c->q_pack)};
+}
+
+// a view taken before buffers grew: without its packed codes if they were given back
+static void still(const hero_ctx *c, ReadsView &v) {
+    if (!c->window) v.pack = nullptr;
 }
 
 // kernel shape of a DP launch from the tuning table (first class covering rmax)
@@ -553,6 +559,7 @@ extern "C" int hero_build_index(hero_ctx *c) {
         if ((r = c->ensure(c->t_slots, slots * sizeof(Slot), "table"))) break;
         if ((r = c->ensure(c->t_vals, nkeys * 8, "table values"))) break;
         if ((r = c->ensure(tmp, scan_tmp_bytes(slots + 1), "scan"))) break;
+        still(c, q);
         launch_key_emit(q, c->p.k, P_<uint64_t>(koff), P_<uint64_t>(klo), P_<uint64_t>(khi),
                         P_<uint64_t>(kval), c->st);
         if ((r = c->check_launch("index: key emit"))) break;
@@ -703,6 +710,7 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         // the count pass leaves the slot of every window (2 x 8 bytes a subject base) for the emit pass
         if ((r = c->ensure(c->wcache, std::max<uint64_t>(nbases, 1) * 16, "probe windows"))) break;
         uint2 *wc = P_<uint2>(c->wcache);
+        still(c, subj);
         launch_probe(false, c->p.aln != 0, subj, nsub, q, t, c->p.k, c->p.l, wc, P_<uint32_t>(c->seg_hits), nullptr, nullptr, ctr, c->st);
         launch_scan_u32(P_<uint32_t>(c->seg_hits), P_<uint64_t>(c->hit_off), nseg, c->scan_tmp.p, c->st);
         uint64_t H = 0;

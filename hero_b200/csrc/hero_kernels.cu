@@ -54,15 +54,6 @@ __device__ __forceinline__ T warp_max(T v) {
     }
     return v;
 }
-template <class T>
-__device__ __forceinline__ T warp_min(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        T w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
-}
 // exclusive prefix over lanes; *total receives the warp total
 template <class T>
 __device__ __forceinline__ T warp_exclusive(T v, T *total) {

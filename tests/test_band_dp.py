@@ -141,3 +141,38 @@ def test_gpu_segments_at_the_edges_of_the_classes(gpu_lib, oracle, affine, make,
         want, _ = oracle.align(affine, s, q, m, kind == 1, kind == 2)
         got = ops[int(oo[i]):int(oo[i]) + int(nops[i])]
         assert np.array_equal(got, want), (i, len(s), len(q), m, kind)
+
+
+def _correct(h, rs):
+    h.set_queries(rs.seq, rs.off, rs.names)
+    h.build_index()
+    h.align_self()
+    return h.consensus()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["c1_20k", "c2_30k"])
+def test_gpu_budgets_without_room_for_the_windows(gpu_lib, oracle, name):
+    """Whatever buffer meets the budget first, the windows' memory goes and the
+    result stays, or the job is refused."""
+    from fixtures import FIXTURES, params, upper
+    from hero_b200 import Hero, HeroError
+    from hero_testlib import assert_same_consensus
+    gen, flags = FIXTURES[name]
+    rs, kw = upper(gen()), params(flags)
+    want = oracle.correct(rs, **kw)
+    with Hero(subject_batch=500, **kw) as h:
+        _correct(h, rs)
+        peak, pairs = h.stats()["device_bytes_peak"], h.stats()["dp_cells_pairs"]
+    done = without = 0
+    for f in np.linspace(0.30, 1.0, 36):
+        with Hero(subject_batch=500, device_memory_budget=int(peak * f), **kw) as h:
+            try:
+                got = _correct(h, rs)
+            except HeroError as e:
+                assert "OOM" in str(e)
+                continue
+            assert_same_consensus(want, got, f"{f:.2f} of the peak")
+            done += 1
+            without += h.stats()["dp_cells_pairs"] > pairs
+    assert done and without
