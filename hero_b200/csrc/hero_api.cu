@@ -159,6 +159,11 @@ struct hero_ctx {
         b.external = false;
         b.pooled = false;
     }
+    // a buffer of a captured round moved or went: the round is planned and captured again
+    void unplan() {
+        plan_ok = false;
+        drop_graph();
+    }
     // gives the window DP's buffers back (work that reads them is queued before
     // the stream-ordered frees; views taken before drop their packed codes, see
     // still()); false when there are none
@@ -169,7 +174,7 @@ struct hero_ctx {
             release(*b);
         }
         window = false;
-        if (any) plan_ok = false;  // a captured round reads them
+        if (any) unplan();
         return any;
     }
     // a buffer of the window DP: one that does not fit turns the window off
@@ -192,6 +197,7 @@ struct hero_ctx {
         if (b.cap >= need) return HERO_OK;
         if (b.external) return fail(HERO_E_INPUT, std::string("caller's buffer too small for ") + what);
         const auto t0 = std::chrono::steady_clock::now();
+        if (b.p) unplan();
         release(b);
         size_t want = need + need / 4 + 256;
         if (P.device_memory_budget && bytes + want > P.device_memory_budget) {
@@ -1142,15 +1148,17 @@ extern "C" int hero_round(hero_ctx *c, uint32_t flags) {
         c->consensus_done = true;
         return HERO_OK;
     }
-    // eager round: runs the work and records the per-batch plan
+    // eager round: runs the work and records the per-batch plan; a graph of an
+    // earlier plan goes
+    if (!c->plan_ok || c->plan_fp != c->qfp) c->drop_graph();
     HERO_TRY(round_body(c));
     HERO_TRY(c->cuda(cudaStreamSynchronize(c->st), "round"));
+    if (graph) HERO_TRY(c->ensure(c->stamps, 16 * c->plan.size(), "stamps"));
     c->plan_fp = c->qfp;
     c->plan_ok = true;
     if (!graph) return HERO_OK;
     // capture the same round (every size from the plan, no host syncs)
     c->drop_graph();
-    HERO_TRY(c->ensure(c->stamps, 16 * c->plan.size(), "stamps"));
     c->capturing = true;
     cudaError_t e = cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal);
     int r = e == cudaSuccess ? round_body(c) : c->cuda(e, "begin capture");

@@ -176,3 +176,27 @@ def test_gpu_budgets_without_room_for_the_windows(gpu_lib, oracle, name):
             done += 1
             without += h.stats()["dp_cells_pairs"] > pairs
     assert done and without
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("plain", [False, True])
+def test_gpu_graph_rounds_after_buffers_moved(gpu_lib, oracle, plain):
+    """A captured round is captured again once a larger job has moved its buffers."""
+    from fixtures import FIXTURES, upper
+    from hero_b200 import Hero
+    from hero_testlib import assert_same_consensus
+    a, b = upper(FIXTURES["c1_20k"][0]()), upper(FIXTURES["mix"][0]())
+    want = oracle.correct(a)
+    with Hero() as h:
+        h.set_queries(a.seq, a.off, a.names)
+        h.round(graph=True)
+        h.round(graph=True)
+        off = np.concatenate([np.zeros(1, np.uint64)] + [b.off[1:] + np.uint64(i) * b.off[-1] for i in range(3)])
+        h.align_subjects(np.tile(b.seq, 3), off, np.tile(b.names, 3))
+        if plain:
+            h.round(graph=False)
+            assert_same_consensus(want, h.fetch(), "plain")
+        for i in range(3):
+            h.round(graph=True)
+            assert_same_consensus(want, h.fetch(), f"round {i}")
+        assert h.stats()["graph_rounds"] >= 3
