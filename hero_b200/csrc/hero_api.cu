@@ -265,6 +265,11 @@ static ReadsView query_view(hero_ctx *c) {
                      P_<int64_t>(c->q_uid), P_<uint8_t>(c->q_good), c->nq, job_tags(c), pack_words(c->q_pack)};
 }
 
+// the votes; in a caller's buffer the state is the exchanged one at any time
+static VoteState vote_state(const hero_ctx *c) {
+    return VoteState{static_cast<uint32_t *>(c->cov.p), static_cast<int32_t *>(c->mdiff.p), !c->cov.external};
+}
+
 // a view taken before buffers grew: without its packed codes if they were given back
 static void still(const hero_ctx *c, ReadsView &v) {
     if (!c->window) v.pack = nullptr;
@@ -834,7 +839,7 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
             rec(5);
             launch_vote(c->p, c->mapping, NC, ch, P_<uint32_t>(c->seg_cstart), P_<uint32_t>(c->seg_ccount),
                         P_<uint32_t>(c->keys), subj, q, P_<uint32_t>(c->ops), stride, P_<DpSum>(c->sums),
-                        P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff), ctr, c->st);
+                        vote_state(c), ctr, c->st);
             if (c->merge)
                 launch_vote_overhang(c->p, NC, ch, P_<uint32_t>(c->keys), subj, q, P_<DpSum>(c->sums),
                                      P_<uint32_t>(c->q_ext), c->st);
@@ -927,7 +932,12 @@ extern "C" int hero_votes_save(hero_ctx *c, void *dst) {
     cudaSetDevice(c->dev);
     uint8_t *d = static_cast<uint8_t *>(dst);
     HERO_TRY(c->cuda(cudaMemcpyAsync(d, c->cov.p, c->nqb * 16, cudaMemcpyDeviceToDevice, c->st), "votes save"));
-    HERO_TRY(c->cuda(cudaMemcpyAsync(d + c->nqb * 16, c->mdiff.p, c->nqb * 4, cudaMemcpyDeviceToDevice, c->st), "votes save"));
+    // the runs end at mismatches for the copy
+    const VoteState vs = vote_state(c);
+    if (vs.inside) launch_vote_runs(query_view(c), vs.cov, vs.mdiff, -1, c->st);
+    HERO_TRY(c->cuda(cudaMemcpyAsync(d + c->nqb * 16, vs.mdiff, c->nqb * 4, cudaMemcpyDeviceToDevice, c->st), "votes save"));
+    if (vs.inside) launch_vote_runs(query_view(c), vs.cov, vs.mdiff, 1, c->st);
+    HERO_TRY(c->check_launch("votes save"));
     return c->cuda(cudaStreamSynchronize(c->st), "votes save");
 }
 
@@ -942,6 +952,11 @@ extern "C" int hero_votes_load(hero_ctx *c, const void *src) {
     c->consensus_done = false;
     HERO_TRY(c->cuda(cudaMemcpyAsync(c->cov.p, s, c->nqb * 16, cudaMemcpyDeviceToDevice, c->st), "votes load"));
     HERO_TRY(c->cuda(cudaMemcpyAsync(c->mdiff.p, s + c->nqb * 16, c->nqb * 4, cudaMemcpyDeviceToDevice, c->st), "votes load"));
+    const VoteState vs = vote_state(c);
+    if (vs.inside) {
+        launch_vote_runs(query_view(c), vs.cov, vs.mdiff, 1, c->st);
+        HERO_TRY(c->check_launch("votes load"));
+    }
     return c->cuda(cudaStreamSynchronize(c->st), "votes load");
 }
 
@@ -989,7 +1004,7 @@ extern "C" int hero_consensus_range(hero_ctx *c, uint64_t first, uint64_t count,
     v.good += first;
     v.n = count;
     v.job = nullptr;
-    launch_consensus(c->p, v, P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff), os, P_<uint32_t>(c->colsum),
+    launch_consensus(c->p, v, vote_state(c), os, P_<uint32_t>(c->colsum),
                      P_<uint32_t>(c->o_imin) + first, P_<uint32_t>(c->o_imed) + first,
                      P_<uint32_t>(c->o_imax) + first, P_<double>(c->o_mis) + first, c->st);
     HERO_TRY(c->check_launch("consensus"));
@@ -1048,7 +1063,7 @@ extern "C" int hero_consensus(hero_ctx *c, uint8_t *seq_out, uint32_t *imin, uin
     HERO_TRY(c->ensure(c->o_mis, n * 8, "consensus"));
     cudaEventRecord(e0, c->st);
     if (nb) cudaMemcpyAsync(c->out_seq.p, c->q_raw.p, nb, cudaMemcpyDeviceToDevice, c->st);
-    launch_consensus(c->p, query_view(c), P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff),
+    launch_consensus(c->p, query_view(c), vote_state(c),
                      P_<uint8_t>(c->out_seq),
                      P_<uint32_t>(c->colsum), P_<uint32_t>(c->o_imin), P_<uint32_t>(c->o_imed),
                      P_<uint32_t>(c->o_imax), P_<double>(c->o_mis), c->st);
@@ -1091,7 +1106,7 @@ static int consensus_device(hero_ctx *c) {
     HERO_TRY(c->ensure(c->o_imax, n * 4, "consensus"));
     HERO_TRY(c->ensure(c->o_mis, n * 8, "consensus"));
     if (nb) cudaMemcpyAsync(c->out_seq.p, c->q_raw.p, nb, cudaMemcpyDeviceToDevice, c->st);
-    launch_consensus(c->p, query_view(c), P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff),
+    launch_consensus(c->p, query_view(c), vote_state(c),
                      P_<uint8_t>(c->out_seq), P_<uint32_t>(c->colsum), P_<uint32_t>(c->o_imin),
                      P_<uint32_t>(c->o_imed), P_<uint32_t>(c->o_imax), P_<double>(c->o_mis), c->st);
     c->consensus_done = true;
@@ -1226,7 +1241,7 @@ extern "C" int hero_mapping_histogram(hero_ctx *c, uint64_t *hist, uint64_t cap,
         HERO_TRY(c->ensure(c->map_max, 8, "mapping histogram"));
         HERO_TRY(c->cuda(cudaMemsetAsync(c->map_hist.p, 0, bins * 8, c->st), "mapping histogram"));
         HERO_TRY(c->cuda(cudaMemsetAsync(c->map_max.p, 0, 8, c->st), "mapping histogram"));
-        launch_map_hist(q, P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff), bins,
+        launch_map_hist(q, vote_state(c), bins,
                         P_<unsigned long long>(c->map_hist), P_<unsigned long long>(c->map_max), c->st);
         HERO_TRY(c->check_launch("mapping histogram"));
         HERO_TRY(c->cuda(cudaMemcpyAsync(&maxc, c->map_max.p, 8, cudaMemcpyDeviceToHost, c->st), "mapping histogram"));
@@ -1287,8 +1302,7 @@ extern "C" int hero_get_votes(hero_ctx *c, uint32_t *cov) {
     DBuf tmp;
     int r = c->ensure(tmp, c->nqb * 16, "votes");
     if (r == HERO_OK) {
-        launch_expand_votes(query_view(c), P_<uint32_t>(c->cov), P_<int32_t>(c->mdiff),
-                            P_<uint32_t>(tmp), c->st);
+        launch_expand_votes(query_view(c), vote_state(c), P_<uint32_t>(tmp), c->st);
         r = c->check_launch("votes");
         if (r == HERO_OK)
             r = c->cuda(cudaMemcpyAsync(cov, tmp.p, c->nqb * 16, cudaMemcpyDeviceToHost, c->st), "votes");

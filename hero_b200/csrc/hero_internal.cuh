@@ -128,6 +128,17 @@ void launch_table_finalize(const uint64_t *klo, const uint64_t *khi, const uint3
                            const uint32_t *count, const uint64_t *start, uint64_t nslots,
                            Slot *slots, cudaStream_t st);
 
+// Votes.  A mismatch votes the subject base into cov[pos][4]; a run of matches
+// votes the query's own base, recorded as +1/-1 at the run's ends in mdiff
+// (a per-read difference array, summed by the consensus).  inside: the runs go
+// on over mismatches, so a column's own votes are its runs less its mismatch
+// votes; the state that contexts exchange ends them there.
+struct VoteState {
+    uint32_t *cov;
+    int32_t *mdiff;
+    bool inside;
+};
+
 // aln: the alignment output's positions (seed_hit)
 void launch_probe(bool emit, bool aln, ReadsView subj, uint64_t nsub, ReadsView q, TableView t, int32_t k,
                   int32_t l, uint2 *wcache, uint32_t *seg_hits, const uint64_t *hit_off, uint64_t *hits,
@@ -136,7 +147,7 @@ void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
                        const uint32_t *ccount, ChainArrays ch, const uint32_t *keys,
                        ReadsView subj, ReadsView q, const DpSum *sums, uint32_t *alist,
                        unsigned long long *counters, cudaStream_t st);
-void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
+void launch_map_hist(ReadsView q, const VoteState &vs, uint64_t bins,
                      unsigned long long *hist, unsigned long long *maxc, cudaStream_t st);
 void launch_sort_hits(uint64_t nseg, const uint64_t *hit_off, uint64_t *hits, cudaStream_t st);
 void launch_chain(const Params &p, uint64_t nsub, ReadsView subj, ReadsView q,
@@ -241,9 +252,6 @@ size_t dp_long_bounds(int32_t rmax, const DpLaunch &a);                     // b
 void launch_assemble(const Params &p, uint64_t nc, ChainArrays ch, const uint32_t *keys,
                      ReadsView subj, ReadsView q, const DpSum *sums, const uint32_t *cells,
                      unsigned long long *counters, cudaStream_t st);
-// Votes.  A mismatch votes the subject base into cov[pos][4]; a run of matches
-// votes the query's own base, recorded as +1/-1 at the run's ends in mdiff
-// (a per-read difference array, summed by the consensus).
 constexpr uint32_t kUnitSubject = 0x80000000u;  // header unit: kUnitSubject | subject
 constexpr uint32_t kUnitEnd = 0xffffffffu;      // closing newline of a subject
 constexpr uint32_t kUnitChainLimit = kUnitSubject;  // chains and subjects of a batch stay below
@@ -275,16 +283,16 @@ void launch_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_t *cor
 // chosen: the records flagged in ch.win vote; else those SubjectRead::addAlignment keeps (and flags)
 void launch_vote(const Params &p, bool chosen, uint64_t nc, ChainArrays ch, const uint32_t *cstart,
                  const uint32_t *ccount, const uint32_t *keys, ReadsView subj, ReadsView q,
-                 const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov, int32_t *mdiff,
+                 const uint32_t *ops, uint32_t stride, const DpSum *sums, const VoteState &vs,
                  unsigned long long *counters, cudaStream_t st);
 constexpr uint32_t kConsensusRead = 1024;  // longest read whose column sums stay in shared memory;
                                            // colsum (a word a base) is only used beyond it
-void launch_consensus(const Params &p, ReadsView q, const uint32_t *cov, const int32_t *mdiff,
-                      uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
+void launch_consensus(const Params &p, ReadsView q, const VoteState &vs, uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
                       uint32_t *imax, double *mis, cudaStream_t st);
 // full vote matrix (cov + match runs), as the reference's coverage matrix
-void launch_expand_votes(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint32_t *out,
-                         cudaStream_t st);
+void launch_expand_votes(ReadsView q, const VoteState &vs, uint32_t *out, cudaStream_t st);
+// runs ended at mismatches (sign -1) or taken on over them (+1)
+void launch_vote_runs(ReadsView q, const uint32_t *cov, int32_t *mdiff, int32_t sign, cudaStream_t st);
 void launch_stamp(unsigned long long *out, cudaStream_t st);
 void launch_fingerprint(const uint8_t *raw, uint64_t nb, const uint64_t *off, const int64_t *uid,
                         uint64_t n, unsigned long long *out, cudaStream_t st);

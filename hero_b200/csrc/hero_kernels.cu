@@ -1806,7 +1806,7 @@ __global__ void k_map_choose(Params p, uint64_t nsub, const uint32_t *cstart,
 // a few dozen bins, took 3.6 ms for 6 Mbp of queries.
 constexpr uint32_t kHistSmem = 4096;
 
-__global__ void __launch_bounds__(256) k_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
+__global__ void __launch_bounds__(256) k_map_hist(ReadsView q, VoteState vs, uint64_t bins,
                            unsigned long long *hist, unsigned long long *maxc) {
     __shared__ uint32_t part[kHistSmem];
     for (uint32_t i = threadIdx.x; i < kHistSmem; i += blockDim.x) part[i] = 0;
@@ -1821,13 +1821,14 @@ __global__ void __launch_bounds__(256) k_map_hist(ReadsView q, const uint32_t *c
         int32_t carry = 0;  // match-run votes entering the current chunk
         for (uint32_t c0 = 0; c0 < Lr; c0 += 32) {
             const uint32_t i = c0 + lane;
-            const int32_t d = i < Lr ? mdiff[b + i] : 0;
+            const int32_t d = i < Lr ? vs.mdiff[b + i] : 0;
             int32_t tot;
             const int32_t run = carry + warp_exclusive<int32_t>(d, &tot) + d;
             carry += tot;
             if (i < Lr) {
-                const uint64_t sum = uint64_t(cov[(b + i) * 4]) + cov[(b + i) * 4 + 1] +
-                                     cov[(b + i) * 4 + 2] + cov[(b + i) * 4 + 3] + uint64_t(run);
+                uint64_t sum = uint64_t(run);
+                if (!vs.inside)
+                    for (int k = 0; k < 4; k++) sum += vs.cov[(b + i) * 4 + k];
                 if (sum < kHistSmem && sum < bins) {
                     atomicAdd(&part[sum], 1u);
                 } else {
@@ -1996,10 +1997,19 @@ __global__ void __launch_bounds__(kTextWarps * 32)
     }
 }
 
+// a column's votes for its own base: of the runs over it those that are no mismatches
+__device__ __forceinline__ uint32_t run_own_votes(const VoteState &vs, int32_t run, const uint4 &v) {
+    return uint32_t(run) - (vs.inside ? v.x + v.y + v.z + v.w : 0u);
+}
+
 // SubjectRead::updateQueryCoverage (SubjectRead.cpp:208-330): M votes the
 // query's own base, a mismatch votes the subject base, I/D only move.  Runs of
 // M are kept open across pieces and land as two difference-array updates.
+// inside: runs go on over mismatches, which then cost their own vote alone
+// (run_own_votes takes them off again), where three updates of two arrays
+// closed and reopened a run: votes of 1.67 M x 150 bp 18.2 -> 15.8 ms.
 struct VoteVisitor {
+    bool inside;
     const uint8_t *sc;  // subject codes (forward)
     int32_t Ls, orient;
     int32_t Lq;
@@ -2035,9 +2045,14 @@ struct VoteVisitor {
         ps += c;
     }
     __device__ __forceinline__ void mismatch() {
-        close();
         const uint8_t code = (ps >= 0 && ps < Ls) ? subj_code(ps) : uint8_t(kBad);
-        if (pq < 0 || pq >= Lq || code >= 4) {
+        const bool out = pq < 0 || pq >= Lq || code >= 4;
+        if (!inside || out) {
+            close();
+        } else if (open < 0) {
+            open = pq;
+        }
+        if (out) {
             anomalies++;
         } else {
             atomicAdd(&cov[pq * 4 + code], 1u);
@@ -2116,15 +2131,15 @@ struct VoteVisitor {
 // rest is the scattered votes (atomics without a result), bound by the sectors
 // of the vote state they touch.  Sorting the records by shape first, so that a
 // warp's lanes agree, cost more in scattered reads (1.8 KB of DRAM a record)
-// and passes than it saved.  1.67 M x 150 bp, 80 M records: 51 -> 26 ms with
-// the selection and the sort.
+// and passes than it saved.  1.67 M x 150 bp, 80 M records: 51 ms with the
+// selection and the sort, 26 in chain order; now 15.8.
 // CHOSEN: the records are flagged in ch.win (--mapping), else the kept ones vote
 // (and are flagged, for k_vote_overhang).
 template <bool CHOSEN>
 __global__ void __launch_bounds__(128)
     k_vote(Params p, uint64_t nc, ChainArrays ch, const uint32_t *cstart, const uint32_t *ccount,
            const uint32_t *keys, ReadsView subj, ReadsView q, const uint32_t *ops, uint32_t stride,
-           const DpSum *sums, uint32_t *cov, int32_t *mdiff, unsigned long long *counters) {
+           const DpSum *sums, VoteState vs, unsigned long long *counters) {
     unsigned long long anomalies = 0, kept = 0;
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nc;
          i += uint64_t(gridDim.x) * blockDim.x) {
@@ -2142,8 +2157,9 @@ __global__ void __launch_bounds__(128)
         v.Ls = int32_t(subj.len[s]);
         v.orient = ch.orient[ci];
         v.Lq = int32_t(q.len[qid]);
-        v.cov = cov + q.off[qid] * 4;
-        v.md = mdiff + q.off[qid];
+        v.inside = vs.inside;
+        v.cov = vs.cov + q.off[qid] * 4;
+        v.md = vs.mdiff + q.off[qid];
         v.ops = ops;
         v.stride = stride;
         v.sums = sums;
@@ -2214,7 +2230,7 @@ __global__ void k_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_
 constexpr uint32_t kConsWarps = 8, kConsSmem = kConsensusRead;  // column sums of reads up to that
 
 __global__ void __launch_bounds__(kConsWarps * 32)
-    k_consensus(Params p, ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint8_t *out,
+    k_consensus(Params p, ReadsView q, VoteState vs, uint8_t *out,
                 uint32_t *colsum, uint32_t *imin, uint32_t *imed, uint32_t *imax, double *mis) {
     __shared__ uint32_t sums[kConsWarps][kConsSmem];
     const uint32_t lane = lane_id();
@@ -2238,14 +2254,14 @@ __global__ void __launch_bounds__(kConsWarps * 32)
         int32_t carry = 0;  // match-run coverage entering the current chunk
         for (uint32_t c0 = 0; c0 < L; c0 += 32) {
             const uint32_t i = c0 + lane;
-            const int32_t d = i < L ? mdiff[b + i] : 0;
+            const int32_t d = i < L ? vs.mdiff[b + i] : 0;
             int32_t tot;
             const int32_t run = carry + warp_exclusive<int32_t>(d, &tot) + d;
             carry += tot;
             if (i < L) {
                 const uint8_t own = q.code[b + i];
-                const uint4 v = reinterpret_cast<const uint4 *>(cov)[b + i];
-                const uint32_t more = uint32_t(run) + 1u;  // match votes + the read's own vote
+                const uint4 v = reinterpret_cast<const uint4 *>(vs.cov)[b + i];
+                const uint32_t more = run_own_votes(vs, run, v) + 1u;  // + the read's own vote
                 const uint32_t c[4] = {v.x + (own == 0 ? more : 0u), v.y + (own == 1 ? more : 0u),
                                        v.z + (own == 2 ? more : 0u), v.w + (own == 3 ? more : 0u)};
                 const int32_t id = column_consensus(c, p.thr);
@@ -2297,8 +2313,7 @@ __global__ void __launch_bounds__(kConsWarps * 32)
     }
 }
 
-__global__ void k_expand_votes(ReadsView q, const uint32_t *cov, const int32_t *mdiff,
-                               uint32_t *out) {
+__global__ void k_expand_votes(ReadsView q, VoteState vs, uint32_t *out) {
     const uint32_t lane = lane_id();
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
     for (uint64_t r = uint64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < q.n;
@@ -2308,18 +2323,36 @@ __global__ void k_expand_votes(ReadsView q, const uint32_t *cov, const int32_t *
         int32_t carry = 0;
         for (uint32_t c0 = 0; c0 < L; c0 += 32) {
             const uint32_t i = c0 + lane;
-            const int32_t d = i < L ? mdiff[b + i] : 0;
+            const int32_t d = i < L ? vs.mdiff[b + i] : 0;
             int32_t tot;
             const int32_t run = carry + warp_exclusive<int32_t>(d, &tot) + d;
             carry += tot;
             if (i < L) {
                 const uint8_t own = q.code[b + i];
-                for (int j = 0; j < 4; j++) {
-                    uint32_t v = cov[(b + i) * 4 + j];
-                    if (j == own) v += uint32_t(run);
-                    out[(b + i) * 4 + j] = v;
-                }
+                const uint4 v = reinterpret_cast<const uint4 *>(vs.cov)[b + i];
+                const uint32_t more = run_own_votes(vs, run, v);
+                const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+                for (int j = 0; j < 4; j++) out[(b + i) * 4 + j] = c[j] + (j == own ? more : 0u);
             }
+        }
+    }
+}
+
+// The state as contexts exchange it, whose runs end at mismatches: differences
+// of a column's and the one before's mismatch votes off (sign -1) or back on
+// (+1).  One warp a read.
+__global__ void __launch_bounds__(256)
+    k_vote_runs(ReadsView q, const uint32_t *cov, int32_t *mdiff, int32_t sign) {
+    const uint32_t lane = lane_id();
+    const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
+    for (uint64_t r = uint64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < q.n; r += warps) {
+        const uint64_t b = q.off[r];
+        const uint32_t L = q.len[r];
+        for (uint32_t i = lane; i < L; i += 32) {
+            const uint4 *v = reinterpret_cast<const uint4 *>(cov) + b + i;
+            const uint32_t before = i ? v[-1].x + v[-1].y + v[-1].z + v[-1].w : 0u;
+            const uint32_t d = v->x + v->y + v->z + v->w - before;
+            mdiff[b + i] = int32_t(uint32_t(mdiff[b + i]) + (sign < 0 ? 0u - d : d));
         }
     }
 }
@@ -2602,11 +2635,11 @@ void launch_map_choose(const Params &p, uint64_t nsub, const uint32_t *cstart,
                                                      sums, alist, counters);
 }
 
-void launch_map_hist(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint64_t bins,
+void launch_map_hist(ReadsView q, const VoteState &vs, uint64_t bins,
                      unsigned long long *hist, unsigned long long *maxc, cudaStream_t st) {
     if (!q.n) return;
     counted();
-    k_map_hist<<<grid_1d(q.n * 32, 256, 148u * 8u), 256, 0, st>>>(q, cov, mdiff, bins, hist, maxc);
+    k_map_hist<<<grid_1d(q.n * 32, 256, 148u * 8u), 256, 0, st>>>(q, vs, bins, hist, maxc);
 }
 
 void launch_aln_list(uint64_t nsub, const uint32_t *cstart, const uint32_t *ccount,
@@ -2649,15 +2682,15 @@ void launch_aln_write(const Params &p, uint64_t nunit, const uint32_t *unit, con
 
 void launch_vote(const Params &p, bool chosen, uint64_t nc, ChainArrays ch, const uint32_t *cstart,
                  const uint32_t *ccount, const uint32_t *keys, ReadsView subj, ReadsView q,
-                 const uint32_t *ops, uint32_t stride, const DpSum *sums, uint32_t *cov, int32_t *mdiff,
+                 const uint32_t *ops, uint32_t stride, const DpSum *sums, const VoteState &vs,
                  unsigned long long *counters, cudaStream_t st) {
     if (!nc) return;
     counted();
     const unsigned g = grid_1d(nc, 128);
     if (chosen) {
-        k_vote<true><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, cov, mdiff, counters);
+        k_vote<true><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, vs, counters);
     } else {
-        k_vote<false><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, cov, mdiff, counters);
+        k_vote<false><<<g, 128, 0, st>>>(p, nc, ch, cstart, ccount, keys, subj, q, ops, stride, sums, vs, counters);
     }
 }
 
@@ -2677,21 +2710,26 @@ void launch_merge_pairs(uint64_t npairs, const uint64_t *off, const uint8_t *cor
                                                         merged_len);
 }
 
-void launch_consensus(const Params &p, ReadsView q, const uint32_t *cov, const int32_t *mdiff,
-                      uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
+void launch_consensus(const Params &p, ReadsView q, const VoteState &vs, uint8_t *out, uint32_t *colsum, uint32_t *imin, uint32_t *imed,
                       uint32_t *imax, double *mis, cudaStream_t st) {
     if (q.n) {
         counted();
-        k_consensus<<<grid_1d(q.n, 8, 148u * 32u), 256, 0, st>>>(p, q, cov, mdiff, out, colsum,
+        k_consensus<<<grid_1d(q.n, 8, 148u * 32u), 256, 0, st>>>(p, q, vs, out, colsum,
                                                                  imin, imed, imax, mis);
     }
 }
 
-void launch_expand_votes(ReadsView q, const uint32_t *cov, const int32_t *mdiff, uint32_t *out,
-                         cudaStream_t st) {
+void launch_vote_runs(ReadsView q, const uint32_t *cov, int32_t *mdiff, int32_t sign, cudaStream_t st) {
     if (q.n) {
         counted();
-        k_expand_votes<<<grid_1d(q.n, 8, 148u * 32u), 256, 0, st>>>(q, cov, mdiff, out);
+        k_vote_runs<<<grid_1d(q.n, 8, 148u * 32u), 256, 0, st>>>(q, cov, mdiff, sign);
+    }
+}
+
+void launch_expand_votes(ReadsView q, const VoteState &vs, uint32_t *out, cudaStream_t st) {
+    if (q.n) {
+        counted();
+        k_expand_votes<<<grid_1d(q.n, 8, 148u * 32u), 256, 0, st>>>(q, vs, out);
     }
 }
 
