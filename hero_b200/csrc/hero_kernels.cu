@@ -1930,7 +1930,7 @@ __global__ void k_aln_size(Params p, uint64_t nunit, const uint32_t *unit, Chain
 // One thread a unit.  The text of a warp's 32 units lies together: it is put
 // together in shared memory and stored sixteen bytes at a time (longer texts go
 // out byte by byte).  Bytes of 32 scattered texts an instruction, one op and one
-// 64-bit division at a time, took 12.3 ms for 53 k reads and 2 M records; now 3.8.
+// 64-bit division at a time, took 12.3 ms for 53 k reads and 2 M records; now 0.74.
 constexpr int kTextWarps = 4;
 constexpr uint32_t kTextSmem = 4096;
 
@@ -2127,9 +2127,9 @@ struct VoteVisitor {
 };
 
 // One thread a chain, in chain order: a warp's chains are neighbours, mostly of
-// one subject, so their arrays, summaries and ops are read as they lie.  The
-// rest is the scattered votes (atomics without a result), bound by the sectors
-// of the vote state they touch.  Sorting the records by shape first, so that a
+// one subject, so their arrays, summaries and ops are read as they lie.  Bound
+// by the walk's instructions (issue slots 64 % busy, five thousand a warp of 32
+// records) and the wait for those reads.  Sorting the records by shape first, so that a
 // warp's lanes agree, cost more in scattered reads (1.8 KB of DRAM a record)
 // and passes than it saved.  1.67 M x 150 bp, 80 M records: 51 ms with the
 // selection and the sort, 26 in chain order; now 15.8.

@@ -125,13 +125,15 @@ typedef struct {
     double ms_dp_kernel;       /* device time of the DP kernels alone */
     double ms_align_wall;      /* host wall time inside the align calls */
     uint64_t graph_rounds;     /* rounds replayed from a CUDA graph */
-    uint64_t dp_cells_computed; /* band cells of every DP segment computed on the device */
+    uint64_t dp_cells_computed; /* band cells of every DP segment of the device, certified
+                                   without being computed or not */
     uint64_t dp_rows_max;      /* longest DP side (the row count of a segment) seen so far;
                                   the key of hero_dp_tuning classes */
-    uint64_t dp_cells_pairs;   /* of dp_cells_computed, the cells computed as 16-bit pairs */
+    uint64_t dp_cells_pairs;   /* of dp_cells_computed, the cells of whole matrices computed as
+                                  16-bit pairs (segments that the window DP left) */
     uint64_t buffer_allocs;    /* device buffers grown (allocated stream-ordered) */
     double ms_alloc;           /* host time spent growing device buffers */
-    uint64_t dp_tasks_staged;  /* DP wavefront tasks whose row bases the bulk copy engine
+    uint64_t dp_tasks_staged;  /* whole-matrix DP tasks whose row bases the bulk copy engine
                                   staged in shared memory */
     uint64_t dp_stage_timeouts; /* staging waits that ran out (those rows were read from
                                    global memory instead; results are unaffected) */
@@ -252,7 +254,8 @@ int hero_get_votes(hero_ctx *ctx, uint32_t *cov);
 
 int hero_get_stats(hero_ctx *ctx, hero_stats *out);
 
-/* Shapes of the banded-DP kernel per class of subject batch, chosen by the
+/* Shapes of the whole-matrix DP kernel (what the window DP leaves; without the
+ * memory for the windows, every segment) per class of subject batch, chosen by the
  * project's autotuner (hero_b200/autotune.py: it times each candidate on a
  * sample of a workload and records the fastest per class in a JSON file that
  * the Python binding loads).  A batch whose longest DP side is at most
