@@ -773,13 +773,14 @@ HERO_HD void straight_ops(const PackSeq &row, const PackSeq &col, int type, int3
     const int32_t end = int32_t(stride) * 16, first = end - R;  // R = d + C ops
     const int32_t ds = type == BT_RIGHT ? first + d : first, de = ds + C;
     const int32_t gs = type == BT_RIGHT ? first : de;           // the gap's range [gs, gs + d)
-    PackStream u(row, r0 + (first & ~15) - ds), v(col, (first & ~15) - ds);
+    // bases are read for the diagonal's words alone: the free run may be longer
+    // than the room around a read array
+    PackStream u(row, r0 + (ds & ~15) - ds), v(col, (ds & ~15) - ds);
     for (int32_t k = first >> 4; k < int32_t(stride); k++) {
         const int32_t p0 = k * 16;
-        const uint32_t m = mismatch16(u.next(), v.next());
         uint32_t x = 0;
         const int32_t a = ds > p0 ? ds - p0 : 0, b = de - p0 < 16 ? de - p0 : 16;  // the diagonal's fields [a, b)
-        if (a < b) x = m & ops_mask(uint32_t(a), uint32_t(b - 1));
+        if (a < b) x = mismatch16(u.next(), v.next()) & ops_mask(uint32_t(a), uint32_t(b - 1));
         const int32_t g = gs > p0 ? gs - p0 : 0, h = gs + d - p0 < 16 ? gs + d - p0 : 16;
         if (g < h) x |= gap_up * ops_mask(uint32_t(g), uint32_t(h - 1));
         w[k] = x;

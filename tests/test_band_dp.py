@@ -200,3 +200,15 @@ def test_gpu_graph_rounds_after_buffers_moved(gpu_lib, oracle, plain):
             h.round(graph=True)
             assert_same_consensus(want, h.fetch(), f"round {i}")
         assert h.stats()["graph_rounds"] >= 3
+
+
+def test_bases_are_read_inside_the_packed_arrays(tmp_path):
+    """Segments at the ends of their read arrays, with free runs longer than the
+    arrays' room, under address checking."""
+    exe = str(tmp_path / "band_bounds")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=address", "-o", exe,
+                    os.path.join(ROOT, "tests", "emu", "band_bounds.cpp")], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr[:3000]
+    segments, certified, straight = map(int, r.stdout.split()[:3])
+    assert certified > segments // 2 and straight > 1000
