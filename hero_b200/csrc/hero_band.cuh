@@ -28,8 +28,12 @@ namespace hero {
 enum : int { BT_NONE = 0, BT_RIGHT = 1, BT_LEFT = 2 };  // anchored at both ends, at the end, at the start
 
 constexpr int32_t kBandMaxC = 1023;   // columns of a window segment: 16-bit values hold 4 * 5 * C
-constexpr int32_t kBandDead = -12000; // outside the matrix or the aligner's band: 3000 below any value
-                                      // the certificate accepts, at every column
+// Start of what lies outside the matrix or the aligner's band.  Such a cell may
+// match on along its diagonal, where a value rises as the potential does, so a
+// path through it keeps a deficit of at least 3000 at every column: the
+// certificate takes no larger one, whatever the window holds.
+constexpr int32_t kBandDead = -12000;
+constexpr int32_t kBandMostDeficit = -kBandDead / 4 - 1;
 constexpr int kPackPad = 8;           // words (128 bases) before and after packed reads that fetches may touch
 
 // ---------------------------------------------------------------------------
@@ -134,13 +138,14 @@ HERO_HD int32_t band_base(int32_t d) {
 // moves there are still up while its deficit is no smaller than D (a tie goes
 // up for the affine aligner, not for the global one), below it the free climb
 // would carry its score to the cells of the traceback.  The limits are the
-// deficits of those paths, less one where a tie would change a move.
+// deficits of those paths, less one where a tie would change a move, and at most
+// what cells outside the aligner's band cannot reach (kBandMostDeficit), which
+// alone counts where the window holds the whole band.
 template <bool AFFINE, int TYPE>
 HERO_HD int32_t band_limit(const BandSeg &s, int32_t nb) {
-    constexpr int32_t kNone = 1 << 20;
     const int32_t d = s.R - s.C, lo = s.base, hi = s.base + nb - 1;
     const int32_t v1 = AFFINE ? 1 : 4, h1 = AFFINE ? 2 : 5, open = AFFINE ? 3 : 0;
-    int32_t below = kNone, above = kNone;
+    int32_t below = kBandMostDeficit, above = kBandMostDeficit;
     if (lo > -s.m && lo > -s.C) {
         const int32_t h = lo > 0 ? 0 : 1 - lo;  // columns skipped to get below the window
         if (TYPE == BT_RIGHT) below = open + h * h1 + (d - lo + 1) * v1 - 1;
@@ -152,7 +157,8 @@ HERO_HD int32_t band_limit(const BandSeg &s, int32_t nb) {
         if (TYPE == BT_LEFT) above = open + (hi + 1) * v1 + (hi < d ? (AFFINE ? 0 : -1) : h1 - 1);
         if (TYPE == BT_NONE) above = open + (hi + 1) * v1 + (hi + 1 - d) * h1 - 1;
     }
-    return below < above ? below : above;
+    const int32_t most = below < above ? below : above;
+    return most < kBandMostDeficit ? most : kBandMostDeficit;
 }
 
 // byte select with sign replication, as PRMT: nibble n of sel picks byte n & 7

@@ -377,4 +377,28 @@ void band_random(int affine, int nb, int mask, uint64_t seed, uint64_t pairs, in
         pair_any(affine != 0, nb, type, mask != 0, g[0], g[1], Count{counts});
     }
 }
+
+// segments whose band lies inside the window and whose path is bad, while a
+// diagonal beside the band matches: one side the other's bases moved by `shift`
+// rows (random ones, or a repeat of `period` bases), `free_rows` rows on the free
+// side of an anchored one
+void band_shifted(int affine, int nb, uint64_t seed, uint64_t pairs, int C, int64_t band, int shift, int period,
+                  int free_rows, uint64_t *counts) {
+    uint64_t x = seed * 0x9e3779b97f4a7c15ull + 1;
+    for (uint64_t k = 0; k < pairs; k++) {
+        const int type = int(k % 3), extra = type == BT_NONE ? 0 : free_rows;
+        Seg g[2];
+        for (int h = 0; h < 2; h++) {
+            std::vector<uint8_t> col(C), row;
+            for (int i = 0; i < C; i++) col[i] = period && i >= period ? col[i - period] : uint8_t(rng_next(x) & 3);
+            for (int i = 0; i < C; i++) {
+                const int j = h ? i + shift : i - shift;
+                row.push_back(j >= 0 && j < C ? col[j] : uint8_t(rng_next(x) & 3));
+            }
+            for (int i = 0; i < extra; i++) row.insert(type == BT_RIGHT ? row.begin() : row.end(), uint8_t(rng_next(x) & 3));
+            make(g[h], row.data(), int(row.size()), col.data(), C, band, type == BT_RIGHT, type == BT_LEFT, int(rng_next(x) & 15));
+        }
+        pair_any(affine != 0, nb, type, true, g[0], g[1], Count{counts});
+    }
+}
 }

@@ -212,3 +212,94 @@ def test_bases_are_read_inside_the_packed_arrays(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr[:3000]
     segments, certified, straight = map(int, r.stdout.split()[:3])
     assert certified > segments // 2 and straight > 1000
+
+
+# the 16-bit halves of cells outside the aligner's band: a path 3000 points worse
+# than all matches must not be certified, however much lies inside the window
+@pytest.mark.parametrize("affine,nb", [(1, 16), (1, 24), (0, 16)])
+@pytest.mark.parametrize("columns", [580, 620, 800, 900, 1023])
+def test_cut_bands_beside_a_matching_diagonal(band, affine, nb, columns):
+    n = np.zeros(3, np.int64)
+    for m in (0, 1, 2):
+        for shift in (m + 1, m + 2, m + 3):
+            for period in (0, 2, 3, 4):
+                for free in (0, 1):
+                    c = (C.c_uint64 * 6)()
+                    band.band_shifted(affine, nb, C.c_uint64(columns + 7 * shift + period), C.c_uint64(6), columns,
+                                      C.c_int64(m), shift, period, free, c)
+                    n += _clean(list(c))
+    assert n[0]
+
+
+def _check_segments(oracle, affine, seg, **kw):
+    """hero_align_segments on (subject, query, band, flags) tuples against the oracle; returns the stats."""
+    from hero_b200 import Hero
+    n = len(seg)
+    off = [np.zeros(n + 1, np.uint64) for _ in range(2)]
+    for h in range(2):
+        off[h][1:] = np.cumsum([len(x[h]) for x in seg])
+    seq = [np.frombuffer(b"".join(x[h] for x in seg), np.uint8) for h in range(2)]
+    idx, zeros = np.arange(n, dtype=np.uint32), np.zeros(n, np.int32)
+    with Hero(**kw) as h:
+        ops, oo, nops = h.align_segments(affine, seq[0], off[0], seq[1], off[1], idx, np.zeros(n, np.uint8), idx,
+                                         zeros, np.diff(off[0]).astype(np.int32), zeros,
+                                         np.diff(off[1]).astype(np.int32), np.array([x[3] for x in seg], np.uint8),
+                                         np.array([x[2] for x in seg], np.int64))
+        stats = h.stats()
+    for i, (s, q, m, kind) in enumerate(seg):
+        want, _ = oracle.align(affine, s, q, m, kind == 1, kind == 2)
+        got = ops[int(oo[i]):int(oo[i]) + int(nops[i])]
+        assert np.array_equal(got, want), (i, len(s), len(q), m, kind)
+    return stats
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("affine", [0, 1])
+def test_gpu_cut_bands_beside_a_matching_diagonal(gpu_lib, oracle, affine):
+    rng = np.random.default_rng(70 + affine)
+    seg = []
+    for c in (580, 620, 800, 900, 1023, 1024):
+        for m in (0, 1, 2):
+            for shift in (m + 1, m + 2, m + 3):
+                for period in (0, 2, 3, 4):
+                    kind = len(seg) % 3
+                    col = ACGT[rng.integers(0, 4, c)] if not period else np.resize(ACGT[rng.integers(0, 4, period)], c)
+                    new = ACGT[rng.integers(0, 4, shift)]
+                    row = np.concatenate([new, col[:-shift]]) if len(seg) % 2 else np.concatenate([col[shift:], new])
+                    free = ACGT[rng.integers(0, 4, len(seg) % 2 if kind else 0)]
+                    row = np.concatenate([free, row] if kind == 1 else [row, free])
+                    s, q = (row, col) if len(seg) % 5 else (col, row)
+                    seg.append((bytes(s), bytes(q), m, kind))
+    _check_segments(oracle, affine, seg)
+
+
+def _moved_reads():
+    """Pairs of 1000 bp reads: one the other with a base gone after 100, and behind
+    it a substitution every 25 bases, so that they share no key there."""
+    from hero_b200 import synth
+    rng = np.random.default_rng(77)
+    reads = []
+    for _ in range(6):
+        a = ACGT[rng.integers(0, 4, 1000)]
+        b = np.concatenate([a[:100], a[101:], ACGT[rng.integers(0, 4, 1)]])
+        for p in range(120, 1000, 25):
+            b[p] = ACGT[(int(np.searchsorted(ACGT, b[p])) + 1) % 4]
+        reads += [a, b, a, a]
+    off = np.zeros(len(reads) + 1, np.uint64)
+    off[1:] = np.cumsum([len(r) for r in reads])
+    return synth.ReadSet(np.concatenate(reads), off, np.arange(1, len(reads) + 1, dtype=np.int64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("aligner", ["affine", "global"])
+def test_gpu_correction_with_no_indels_of_long_reads(gpu_lib, oracle, aligner):
+    from hero_b200 import Hero
+    from hero_testlib import assert_same_consensus
+    rs, kw = _moved_reads(), dict(aligner=aligner, max_indel_rate=0.0)
+    want = oracle.correct(rs, keep_segments=True, **kw)
+    g = want["segments"]
+    side = np.minimum(g["s1"] - g["s0"], g["q1"] - g["q0"])
+    assert ((side > 800) & (side < 1000)).any()
+    with Hero(**kw) as h:
+        assert_same_consensus(want, _correct(h, rs), aligner)
+        assert np.array_equal(h.votes(), want["votes"])
