@@ -445,10 +445,13 @@ extern "C" int hero_set_queries(hero_ctx *c, const uint8_t *seq, const uint64_t 
                        P_<unsigned long long>(c->fp), c->st);
     if (c->vote_ext) {  // the caller's buffer: mismatch votes, then match-run differences
         if (c->vote_ext_bytes < c->nqb * 20) return c->fail(HERO_E_INPUT, "vote buffer smaller than 20 bytes a query base");
+        uint8_t *runs = static_cast<uint8_t *>(c->vote_ext) + c->nqb * 16;
+        // a captured round votes into the memory, and in the form, of its capture
+        if (c->cov.p != c->vote_ext || c->mdiff.p != runs) c->unplan();
         c->release(c->cov);
         c->release(c->mdiff);
         c->cov = DBuf{c->vote_ext, size_t(c->nqb * 16), true};
-        c->mdiff = DBuf{static_cast<uint8_t *>(c->vote_ext) + c->nqb * 16, size_t(c->nqb * 4), true};
+        c->mdiff = DBuf{runs, size_t(c->nqb * 4), true};
     }
     HERO_TRY(c->ensure(c->cov, c->nqb * 16, "vote matrix"));
     HERO_TRY(c->ensure(c->mdiff, c->nqb * 4, "vote matrix"));
@@ -968,7 +971,10 @@ extern "C" int hero_set_vote_buffer(hero_ctx *c, void *dev_ptr, uint64_t bytes) 
     c->vote_ext = dev_ptr;
     c->vote_ext_bytes = dev_ptr ? bytes : 0;
     if (!dev_ptr) {  // back to the context's own buffers at the next hero_set_queries
-        if (c->cov.external) c->release(c->cov);
+        if (c->cov.external) {
+            c->unplan();
+            c->release(c->cov);
+        }
         if (c->mdiff.external) c->release(c->mdiff);
         c->have_queries = false;
         c->have_index = false;

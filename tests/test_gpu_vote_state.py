@@ -41,3 +41,28 @@ def test_exchanged_words_are_the_votes(gpu_lib, oracle, name):
         votes[np.arange(a, b)[ok], own[ok]] += runs[ok]
         assert not runs[~ok].any()
     assert np.array_equal(votes.reshape(-1), np.asarray(want["votes"], np.uint32).reshape(-1))
+
+
+def test_captured_rounds_follow_the_vote_memory(gpu_lib, oracle):
+    """A round captured with the context's own votes is captured again when the
+    caller's memory takes their place, and the other way round, also with the
+    same reads."""
+    import torch
+    from hero_b200 import Hero
+    gen, flags = FIXTURES["c1_20k"]
+    rs, kw = upper(gen()), params(flags)
+    want = oracle.correct(rs, **kw)
+    nb = int(rs.off[-1])
+    ext = [torch.full((5 * nb,), 7, dtype=torch.int32, device="cuda") for _ in range(2)]
+    with Hero(**kw) as h:
+        for buf in (None, ext[0], ext[1], None, ext[0]):
+            before = [e.clone() for e in ext]
+            h.set_vote_buffer(buf.data_ptr() if buf is not None else 0, 20 * nb if buf is not None else 0)
+            h.set_queries(rs.seq, rs.off, rs.names)
+            for rnd in range(3):
+                h.round(graph=True)
+                assert_same_consensus(want, h.fetch(), f"round {rnd}")
+                assert np.array_equal(h.votes(), want["votes"])
+            for e, b in zip(ext, before):
+                assert e is buf or torch.equal(e, b)
+        assert h.stats()["graph_rounds"] == 10
