@@ -102,6 +102,7 @@ struct hero_ctx {
         int32_t rmax, cmax;
     };
     std::vector<BatchPlan> plan;
+    std::vector<BatchPlan> captured;  // of the captured round (other align calls plan anew)
     uint64_t plan_nkeys = 0, plan_fp = 0, qfp = 0;
     bool plan_ok = false, capturing = false;
     size_t batch_idx = 0;
@@ -1156,13 +1157,13 @@ extern "C" int hero_round(hero_ctx *c, uint32_t flags) {
             c->plan_ok = false;  // the next round runs eagerly and re-plans
             return c->fail(HERO_E_STATE, "graph round: chain buffer overflow (plan outgrown)");
         }
-        std::vector<unsigned long long> t(2 * c->plan.size());
+        std::vector<unsigned long long> t(2 * c->captured.size());
         HERO_TRY(c->cuda(cudaMemcpy(t.data(), c->stamps.p, t.size() * 8, cudaMemcpyDeviceToHost),
                          "graph stamps"));
-        for (size_t b = 0; b < c->plan.size(); b++) {
+        for (size_t b = 0; b < c->captured.size(); b++) {
             c->stats.ms_dp_kernel += double(t[2 * b + 1] - t[2 * b]) * 1e-6;
-            c->stats.dp_segments += c->plan[b].ND;
-            c->stats.chains_kept += c->plan[b].NC;
+            c->stats.dp_segments += c->captured[b].ND;
+            c->stats.chains_kept += c->captured[b].NC;
         }
         c->stats.subjects += c->nq;
         c->stats.graph_rounds++;
@@ -1193,6 +1194,7 @@ extern "C" int hero_round(hero_ctx *c, uint32_t flags) {
     if (e2 != cudaSuccess) return c->cuda(e2, "end capture");
     c->graph = g;
     HERO_TRY(c->cuda(cudaGraphInstantiate(&c->gexec, c->graph, 0), "graph instantiate"));
+    c->captured = c->plan;
     return HERO_OK;
 }
 
