@@ -434,18 +434,27 @@ void wide_launch(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
 
 }  // namespace
 
-// Resident warps for nd segments (half a task each at least), the code words of
-// each -- and, in the same words, the wide window's blocks, whose warps need others.
+// Warps of the window kernels and the code words of each -- and, in the same words,
+// the wide window's blocks, whose warps need others.  A job of a few hundred
+// thousand segments is over in one or two tasks a warp, and a new context pays for
+// the codes' memory: 135 KB a warp at 250 bp, 0.65 ms a 100 MB.  So a warp for
+// every 32 segments up to 400 warps, then for every 256 (the screen finishes
+// 61-85 % of them) up to the resident ones.  Affine, 75-250 bp, DP of 16 k, 52 k
+// and 213 k segments with a warp for every 32: 0.39, 0.61 and 0.80 ms; 64: 0.37,
+// 0.50, 0.83; 128: 0.50, 0.40, 0.74; 256: 0.79, 0.48, 0.61; from 0.6 M segments on
+// all are the same.  On 0.2 M segments the codes were 300 MB with one for every 32
+// and are 134 now; a new context's first pass 4.3 -> 3.0 ms (whole matrices: 3.8).
 size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &w) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const uint32_t c = uint32_t(cmax < kBandMaxC ? cmax : kBandMaxC);
-    const uint64_t full = uint64_t(sms) * kBandBlocks, need = (nd + 32 * kBandWarps - 1) / (32 * kBandWarps);
-    w.warps = kBandWarps * (need < full ? need : full);
+    const uint64_t full = uint64_t(sms) * kBandBlocks, few = 400;
     w.code_words = c * 32u * (affine ? 5u : 2u);
     w.wide_lanes = c <= 256u && nd >= kWideManySegments ? 8 : 16;
     w.wide_words = uint32_t(kWideLag * ((c + kWideStrip - 1) / kWideStrip - 1) + wide_rows(wide_diagonals(w.wide_lanes))) * 32u;
     const uint64_t block = uint64_t(w.wide_words) * kWideWarps;
+    const uint64_t warps = std::max(nd / 256, std::min((nd + 31) / 32, few));
+    w.warps = kBandWarps * std::min((warps + kBandWarps - 1) / kBandWarps, full);
     const uint64_t words = std::max<uint64_t>(w.warps * w.code_words, block);
     w.wide_blocks = std::min<uint64_t>(words / block, full);
     return words * 4;

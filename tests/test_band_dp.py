@@ -303,3 +303,23 @@ def test_gpu_correction_with_no_indels_of_long_reads(gpu_lib, oracle, aligner):
     with Hero(**kw) as h:
         assert_same_consensus(want, _correct(h, rs), aligner)
         assert np.array_equal(h.votes(), want["votes"])
+
+
+def _small_job():
+    """700 reads of 250 bases, 56 k segments of up to 211 columns."""
+    from hero_b200 import synth
+    return synth.Job(0, 0.0, 5, 5000, 250, 35.0).reads()
+
+
+@pytest.mark.gpu
+def test_gpu_small_jobs_take_little_window_memory(gpu_lib):
+    """The windows' codes follow the work: 400 warps of 135 KB and a quarter more
+    here, 68 MB beside about 45 of other buffers (a warp for every 32 segments:
+    272 MB)."""
+    from hero_b200 import Hero
+    rs = _small_job()
+    with Hero(aligner="affine") as h:
+        _correct(h, rs)
+        st = h.stats()
+    assert 20000 < st["dp_segments"] < 100000
+    assert st["device_bytes_peak"] < 160e6
