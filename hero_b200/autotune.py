@@ -1,10 +1,14 @@
-"""Autotuner of the banded-DP kernel shapes.
+"""Autotuner of the whole-matrix DP kernel's shapes.
 
 For each sample read length it builds a correction job with reads of that
-length, runs the DP kernel under every candidate shape -- warps per block,
+length, runs the DP under every candidate shape -- warps per block,
 16-bit pairs of segments, row-chunk tracebacks, registers a thread -- and records the
 fastest, with every candidate's time, in a JSON file (hero_b200/tuning.json by
-default), which hero_b200.Hero loads.  A class is keyed on the longest DP side
+default), which hero_b200.Hero loads.  The shapes are those of the kernel that
+computes whole matrices: of what the window DP leaves, and of everything where
+memory is too short for the windows.  The window DP would do nearly all of a
+sample's work and leave the times to chance, so the samples run in contexts
+whose memory budget has no room for it.  A class is keyed on the longest DP side
 the sample's batches showed (read length - k for reads that share a k-mer
 anchor, not the read length): its bound ``rows_max`` is the midpoint to the
 next sample's longest side, so a batch takes the class of the nearest sample
@@ -50,8 +54,38 @@ def sample(read_len: int, genome_bp: int, seed: int = 91):
     return synth.Job(0, 0.0, seed + read_len, genome_bp, read_len, 40.0).reads()
 
 
+def whole_matrices(reads, **kw):
+    """A context with these reads as its query set whose memory budget leaves the window DP
+    out: every matrix is computed whole."""
+    from hero_b200 import Hero, HeroError
+
+    def run(budget):
+        h = Hero(device_memory_budget=budget, **kw)
+        try:
+            h.set_queries(reads.seq, reads.off, reads.names)
+            h.build_index()
+            h.align_self()
+            h.consensus()
+        except HeroError:
+            h.close()
+            return None
+        return h
+
+    with run(0) as h:
+        most = int(h.stats()["device_bytes_peak"])
+    least = 0  # the smallest budget a correction fits, to 64 KB: less than the windows' tables
+    while most - least > 1 << 16:
+        h = run((least + most) // 2)
+        if h is None:
+            least = (least + most) // 2
+        else:
+            h.close()
+            most = (least + most) // 2
+    return run(most)
+
+
 def time_dp(h, reads, shape: dict, rounds: int = 2) -> float:
-    """Device time of the DP kernels of one correction under a shape (ms, best of rounds)."""
+    """Device time of the DP of one correction under a shape (ms, best of rounds)."""
     h.set_tuning([dict(shape, rows_max=ROWS_LAST)])
     best = None
     for _ in range(rounds):
@@ -71,7 +105,6 @@ def class_bounds(rows: list[int]) -> list[int]:
 
 def tune(genome_bp: int = 60_000, device: int = 0, read_lengths=READ_LENGTHS, log=print,
          aligner: str = "affine") -> dict:
-    from hero_b200 import Hero
     out = {"device": None, "genome_bp": genome_bp, "when": time.strftime("%Y-%m-%dT%H:%M:%SZ", time.gmtime()),
            "aligner": aligner, "classes": []}
     try:
@@ -81,8 +114,7 @@ def tune(genome_bp: int = 60_000, device: int = 0, read_lengths=READ_LENGTHS, lo
         pass
     for read_len in sorted(read_lengths):
         reads = sample(read_len, genome_bp)
-        with Hero(aligner=aligner, device=device, tuning=[]) as h:
-            h.set_queries(reads.seq, reads.off, reads.names)
+        with whole_matrices(reads, aligner=aligner, device=device, tuning=[]) as h:
             timings = []
             for shape in candidates():
                 ms = time_dp(h, reads, shape)

@@ -57,3 +57,27 @@ def test_tuner_records_the_fastest_candidate(tmp_path):
     p.write_text(json.dumps(rec))
     from hero_b200._lib import load_tuning
     assert load_tuning(str(p))[0]["warps_per_block"] in (1, 2, 4)
+
+
+@pytest.mark.parametrize("aligner,flags", [("affine", {}), ("global", {}), ("affine", dict(max_indel_rate=0.02))])
+def test_every_candidate_shape_on_whole_matrices(aligner, flags):
+    """Without the window DP the tuned kernel has every segment of a batch, and
+    gives the oracle's result under every shape."""
+    from hero_testlib import Oracle, assert_same_consensus
+    rs = upper(autotune.sample(150, 6_000))
+    kw = dict(aligner=aligner, **flags)
+    want = Oracle().correct(rs, **kw)
+    with autotune.whole_matrices(rs, tuning=[], **kw) as h:
+        whole = not flags  # bands cut the matrix: 32-bit rows, no pairs
+        for shape in autotune.candidates():
+            before = h.stats()
+            h.set_tuning([dict(shape, rows_max=100000)])
+            h.reset_votes()
+            h.build_index()
+            h.align_self()
+            assert_same_consensus(want, h.consensus(), str(shape))
+            after = h.stats()
+            cells, pairs = (after[f] - before[f] for f in ("dp_cells", "dp_cells_pairs"))
+            assert cells == want["stats"]["dp_cells"]
+            assert pairs > cells // 2 if whole and shape["pair_strips"] else pairs == 0 or not whole
+            assert after["dp_stage_timeouts"] == 0
