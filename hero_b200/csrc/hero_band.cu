@@ -436,14 +436,19 @@ void wide_launch(const DpLaunch &a, const BandWork &w, cudaStream_t st) {
 
 // Warps of the window kernels and the code words of each -- and, in the same words,
 // the wide window's blocks, whose warps need others.  A job of a few hundred
-// thousand segments is over in one or two tasks a warp, and a new context pays for
-// the codes' memory: 135 KB a warp at 250 bp, 0.65 ms a 100 MB.  So a warp for
-// every 32 segments up to 400 warps, then for every 256 (the screen finishes
-// 61-85 % of them) up to the resident ones.  Affine, 75-250 bp, DP of 16 k, 52 k
-// and 213 k segments with a warp for every 32: 0.39, 0.61 and 0.80 ms; 64: 0.37,
-// 0.50, 0.83; 128: 0.50, 0.40, 0.74; 256: 0.79, 0.48, 0.61; from 0.6 M segments on
-// all are the same.  On 0.2 M segments the codes were 300 MB with one for every 32
-// and are 134 now; a new context's first pass 4.3 -> 3.0 ms (whole matrices: 3.8).
+// thousand segments is over in a few tasks a warp: more warps then only spread the
+// codes (135 KB a warp at 250 bp, affine) past the L2, and a new context pays 0.65
+// ms for every 100 MB of them.  So a warp for every 32 segments up to 400 warps,
+// then for every 500 (affine; 256 for the global aligner, whose codes take 2/5) up
+// to the resident ones.  DP in ms with a warp for every 32 segments (as it was),
+// 256 and 600:
+//   affine  75-250 bp  0.2 M segments 0.80 0.60 0.54, 0.4 M 0.98 0.88 0.67, 1.3 M 1.60 1.60 1.64
+//           250 bp     0.2 M 0.91 0.69 0.79, 0.4 M 1.31 1.33 1.03
+//   global  250 bp     0.2 M 0.51 0.37 0.38, 0.4 M 0.57 0.48 0.47
+//           300-600    0.4 M - 1.14 1.38
+// (400 warps or more in each; on 23 k segments 200, 400 and 800 warps: 0.44 0.33
+// 0.39).  On 0.2 M segments of 75-250 bp reads the codes were 300 MB and are 71
+// now; a new context's first pass 4.3 -> 2.6 ms (whole matrices: 3.8).
 size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &w) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -453,7 +458,7 @@ size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &
     w.wide_lanes = c <= 256u && nd >= kWideManySegments ? 8 : 16;
     w.wide_words = uint32_t(kWideLag * ((c + kWideStrip - 1) / kWideStrip - 1) + wide_rows(wide_diagonals(w.wide_lanes))) * 32u;
     const uint64_t block = uint64_t(w.wide_words) * kWideWarps;
-    const uint64_t warps = std::max(nd / 256, std::min((nd + 31) / 32, few));
+    const uint64_t warps = std::max(nd / (affine ? 500 : 256), std::min((nd + 31) / 32, few));
     w.warps = kBandWarps * std::min((warps + kBandWarps - 1) / kBandWarps, full);
     const uint64_t words = std::max<uint64_t>(w.warps * w.code_words, block);
     w.wide_blocks = std::min<uint64_t>(words / block, full);
