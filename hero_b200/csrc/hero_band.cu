@@ -328,10 +328,10 @@ __global__ void __launch_bounds__(kBandWarps * 32, kBandBlocks) k_band(DpLaunch 
 }
 
 // The wide window of what the register windows left: a group of 8 lanes (64
-// diagonals; 16 and 136 for small batches and columns past 256) a pair of segments,
-// in list order (theirs: class, type, columns).  Bound by the chain down the
-// strips, nine steps a strip; a thread a pair, strip after strip, was six times
-// that chain and slower than whole matrices for all but large batches.  What it
+// diagonals; or 16 and 136, see wide_lanes) a pair of segments, in list order
+// (theirs: class, type, columns).  Bound by the chain down the strips, nine steps a
+// strip; a thread a pair, strip after strip, was six times that chain and slower
+// than whole matrices for all but large batches.  What it
 // replaces -- the whole matrix -- took 31 of 33 ms on 300-600 bp reads, 8 of 38 ms
 // on 75-250 bp ones and 0.38 ms on 4310 such reads: now 2.1, 4.6 and 0.32
 // with what it leaves to them.
@@ -345,10 +345,25 @@ struct WideCodes {
 };
 
 constexpr int kWideWarps = 4;
-// A batch with enough work runs 64 diagonals, and whole matrices what that
-// leaves; a smaller one waits for its longest chain, so it takes 136, which leave
-// almost nothing to a second chain.
-constexpr uint64_t kWideManySegments = 300000;
+// 64 diagonals on 8 lanes do a pair's work with half the lanes, but leave more to
+// whole matrices, a second chain; 136 on 16 leave almost nothing, which counts where
+// a batch only waits for its longest chains.  DP of one batch, 8 / 16 lanes, ms:
+//   global  250 bp  0.1 M segments 0.29 / 0.37, 0.4 M 0.48 / 0.56, 3.4 M 1.8 / 2.7
+//           75-250  0.1 M 0.27 / 0.30, 3.3 M 1.07 / 1.27; 100 and 150 bp alike
+//   affine  100 bp  0.1 M 0.21 / 0.23, 1 M 0.52 / 0.54, 2.9 M 0.76 / 0.82
+//           150 bp  0.2 M 0.58 / 0.39, 1.1 M 1.15 / 0.99, 3.3 M 1.56 / 1.52, batches
+//                   of 8.4 M 43 / 50 (13 of them)
+//           200 bp  0.2 M 0.81 / 0.57, 1.2 M 1.56 / 1.58, 3.4 M 2.6 / 3.1
+//           250 bp  0.2 M 0.95 / 0.67, 0.4 M 1.35 / 1.31, 0.6 M 1.61 / 1.71, 3.4 M 3.9 / 5.3
+//           75-250  0.2 M 0.81 / 0.60, 0.8 M 1.54 / 1.26, 1.7 M 1.66 / 1.62, 3.3 M 2.2 / 2.4
+// So 8 for the global aligner, and for the affine one where the longest matrix has
+// hardly more columns than its window diagonals (100 bp: 61) or segments x columns
+// squared, the cells left, pass 3e10: 2.4 M segments of 150 bp reads, 1.2 M of 200,
+// 0.7 M of 250.  Past 256 columns 16: a matrix left takes panels (k_dp_long).
+inline int wide_lanes(uint64_t nd, uint64_t columns, bool affine) {
+    if (columns > 256) return 16;
+    return !affine || columns <= 64 || nd * columns * columns >= 30000000000ull ? 8 : 16;
+}
 
 template <bool AFFINE, int LANES>
 __global__ void __launch_bounds__(kWideWarps * 32) k_band_wide(DpLaunch a, BandWork w) {
@@ -455,7 +470,7 @@ size_t band_sizes(int device, uint64_t nd, int32_t cmax, bool affine, BandWork &
     const uint32_t c = uint32_t(cmax < kBandMaxC ? cmax : kBandMaxC);
     const uint64_t full = uint64_t(sms) * kBandBlocks, few = 400;
     w.code_words = c * 32u * (affine ? 5u : 2u);
-    w.wide_lanes = c <= 256u && nd >= kWideManySegments ? 8 : 16;
+    w.wide_lanes = wide_lanes(nd, c, affine);
     w.wide_words = uint32_t(kWideLag * ((c + kWideStrip - 1) / kWideStrip - 1) + wide_rows(wide_diagonals(w.wide_lanes))) * 32u;
     const uint64_t block = uint64_t(w.wide_words) * kWideWarps;
     const uint64_t warps = std::max(nd / (affine ? 500 : 256), std::min((nd + 31) / 32, few));

@@ -323,3 +323,35 @@ def test_gpu_small_jobs_take_little_window_memory(gpu_lib):
         st = h.stats()
     assert 20000 < st["dp_segments"] < 100000
     assert st["device_bytes_peak"] < 160e6
+
+
+def _edited_segments(rng, n, columns):
+    """Segments of the given numbers of columns: copies with many mismatches and gaps,
+    every fourth an unrelated string."""
+    out = []
+    for i in range(n):
+        c, kind = int(rng.choice(columns)), i % 3
+        col = ACGT[rng.integers(0, 4, c)]
+        row = col.copy() if i % 4 else ACGT[rng.integers(0, 4, c)]
+        for p in rng.integers(0, c, int(rng.integers(4, 20))):
+            row[p] = ACGT[rng.integers(0, 4)]
+        for _ in range(int(rng.integers(1, 5))):
+            p, k = int(rng.integers(0, len(row))), int(rng.integers(1, 12))
+            row = np.concatenate([row[:p], ACGT[rng.integers(0, 4, k)], row[p:]])
+        if len(row) < c + 1 or not kind:
+            row = np.resize(row, c)
+        free = ACGT[rng.integers(0, 4, int(rng.integers(0, 30)) if kind else 0)]
+        row = np.concatenate([free, row] if kind == 1 else [row, free])
+        s, q = (row, col) if rng.random() < 0.5 else (col, row)
+        out.append((bytes(s), bytes(q), int(rng.choice([1500, 1500, 30])), kind))
+    return out
+
+
+# both widths of the wide window (8 lanes: the global aligner up to 256 columns, the
+# affine one up to 64), and the hand-over to whole matrices past 1023 columns
+@pytest.mark.gpu
+@pytest.mark.parametrize("affine", [0, 1])
+@pytest.mark.parametrize("columns,count", [([1, 8, 9, 63, 64], 1000), ([64, 65], 300), ([127, 128, 255, 256], 300),
+                                           ([255, 256, 257], 200), ([1022, 1023, 1024, 1025], 120)])
+def test_gpu_wide_windows_at_their_edges(gpu_lib, oracle, affine, columns, count):
+    _check_segments(oracle, affine, _edited_segments(np.random.default_rng(80 + affine), count, columns))
