@@ -79,6 +79,7 @@ struct hero_ctx {
     // the window DP's buffers: without room for them the whole-matrix kernels do all the work
     DBuf q_pack, s_pack;            // 2-bit codes of the reads, kPackPad words of room on both sides
     DBuf w_key, w_order, w_rest, w_bin, w_codes;
+    std::vector<DBuf *> window_bufs{&q_pack, &s_pack, &w_key, &w_order, &w_rest, &w_bin, &w_codes};
     bool window = true;             // off from an allocation that did not fit until the next query set
     bool consensus_done = false;  // out_seq holds the consensus of the current votes
     // .aln text of every subject aligned since the last take: the batches' in host
@@ -170,7 +171,7 @@ struct hero_ctx {
     // still()); false when there are none
     bool shed() {
         bool any = false;
-        for (DBuf *b : {&q_pack, &s_pack, &w_key, &w_order, &w_rest, &w_bin, &w_codes}) {
+        for (DBuf *b : window_bufs) {
             any = any || b->p;
             release(*b);
         }
@@ -616,7 +617,7 @@ static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
     if (!a.nd) return HERO_OK;
     BandWork w{};
     const size_t codes = band_sizes(c->dev, a.nd, cmax, a.affine != 0, w);
-    const size_t table = kBandBins * (sizeof(BandBin) + 4) + kBandHead * 4;
+    const size_t table = kBandBins * (sizeof(BandBin) + 8) + kBandHead * 4;
     w.on = a.whole && a.spack && a.qpack && c->optional(b.key, a.nd * 8, "DP windows") &&
            c->optional(b.order, a.nd * 4, "DP windows") && c->optional(b.rest, a.nd * 8, "DP windows") &&
            c->optional(b.bin, table, "DP windows") &&
@@ -632,9 +633,10 @@ static int run_dp(hero_ctx *c, DpLaunch &a, int32_t cmax, DpBufs b) {
         w.head = w.start + kBandBins;
         w.codes = P_<uint32_t>(b.codes);
         w.again = a.rest + a.nd;
-        w.count = a.bins + kDpBins;
+        w.count = w.head + kBandHead;
+        HERO_TRY(c->cuda(cudaMemsetAsync(w.count, 0, kBandBins * 4, c->st), "DP windows"));
     }
-    HERO_TRY(c->cuda(cudaMemsetAsync(b.bins.p, 0, (kDpBins + kBandBins) * 4, c->st), "DP bins"));
+    HERO_TRY(c->cuda(cudaMemsetAsync(b.bins.p, 0, kDpBins * 4, c->st), "DP bins"));
     apply_tuning(c, a);
     launch_band(a, w, c->st);
     launch_dp_sort(a, P_<uint32_t>(b.perm), P_<uint64_t>(b.bin_off), b.scan.p, c->st);
@@ -789,7 +791,7 @@ static int align_batch(hero_ctx *c, ReadsView subj, uint64_t nsub, uint64_t nbas
         if ((r = c->ensure(c->cells, NDc * 4, "DP cells"))) break;
         if ((r = c->ensure(c->perm, NDc * 4, "DP order"))) break;
         if ((r = c->ensure(c->ops, NDc * stride * 4, "DP ops"))) break;
-        if ((r = c->ensure(c->bins, (kDpBins + kBandBins) * 4, "DP bins"))) break;
+        if ((r = c->ensure(c->bins, kDpBins * 4, "DP bins"))) break;
         if ((r = c->ensure(c->bin_off, (kDpBins + 1) * 8, "DP bins"))) break;
         if ((r = c->ensure(c->dp_tasks, kDpTaskWords * 8, "DP tasks"))) break;
         DpLaunch a{};
@@ -1399,11 +1401,15 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
         for (uint64_t k = 0; k < rd.second && acgt; k++) acgt = base_code(rd.first[k]) < 4;
     DBuf sraw, scode, spack, soff, slen, suid, qraw, qcode, qpack, qoff, qlen, quid, dsegs, dsums, dops, dtb,
         dbnd, doo, dout, dn, dperm, dbins, dbinoff, dtasks, dtmp, dkey, dorder, drest, dbin, dcodes;
+    // what the windows take is given back like the context's when memory is short
+    const size_t own = c->window_bufs.size();
+    c->window_bufs.insert(c->window_bufs.end(), {&spack, &qpack, &dkey, &dorder, &drest, &dbin, &dcodes});
     auto cleanup = [&]() {
         for (DBuf *b : {&sraw, &scode, &soff, &slen, &suid, &qraw, &qcode, &qoff, &qlen, &quid,
                         &dsegs, &dsums, &dops, &dtb, &dbnd, &doo, &dout, &dn, &dperm, &dbins,
                         &dbinoff, &dtasks, &dtmp, &spack, &qpack, &dkey, &dorder, &drest, &dbin, &dcodes})
             c->release(*b);
+        c->window_bufs.resize(own);
     };
     int r = HERO_OK;
     do {
@@ -1423,9 +1429,9 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
             if ((r = c->ensure(dbnd, dp_long_bounds(rmax, a), "scratch"))) break;
         }
         if ((r = c->ensure(dperm, n_seg * 4, "order"))) break;
-        if ((r = c->ensure(dbins, (kDpBins + kBandBins) * 4, "bins"))) break;
+        if ((r = c->ensure(dbins, kDpBins * 4, "bins"))) break;
         if ((r = c->ensure(dbinoff, (kDpBins + 1) * 8, "bins"))) break;
-        if ((r = c->ensure(dtasks, (kDpTaskWords + 1) * 8, "tasks"))) break;
+        if ((r = c->ensure(dtasks, kDpTaskWords * 8, "tasks"))) break;
         if ((r = c->ensure(dtmp, scan_tmp_bytes(kDpBins + 1), "scan"))) break;
         if ((r = c->ensure(doo, (n_seg + 1) * 8, "ops"))) break;
         if ((r = c->ensure(dout, ops_off[n_seg], "ops"))) break;
@@ -1451,7 +1457,7 @@ extern "C" int hero_align_segments(hero_ctx *c, int affine, const uint8_t *subj,
         a.warps = 4;
         a.spack = pack_words(spack);
         a.qpack = pack_words(qpack);
-        a.n_rest = P_<unsigned long long>(dtasks) + kDpTaskWords;
+        a.n_rest = P_<unsigned long long>(dtasks) + kDpTaskRest;
         if ((r = c->cuda(cudaMemsetAsync(a.n_rest, 0, 8, c->st), "tasks"))) break;
         if ((r = run_dp(c, a, cmax, DpBufs{dbins, dbinoff, dperm, dtasks, dkey, dorder, drest, dbin, dcodes, dtmp}))) break;
         launch_unpack_ops(P_<uint32_t>(dops), stride, P_<DpSum>(dsums), n_seg, P_<uint64_t>(doo),

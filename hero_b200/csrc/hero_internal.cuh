@@ -239,7 +239,7 @@ void launch_band(const DpLaunch &a, const BandWork &w, cudaStream_t st);
 void launch_dp_sort(const DpLaunch &a, uint32_t *order, uint64_t *bin_off, void *scan_tmp, cudaStream_t st);
 // needs the shape sort (perm, bin_off); tasks: kDpTaskWords uint64 of device scratch.
 // k_dp_long's scratch (tb, bnd) is only used when dp_needs_scratch().
-constexpr uint32_t kDpTaskWords = 128;
+constexpr uint32_t kDpTaskWords = 128, kDpTaskRest = 126;  // kDpTaskRest: room for n_rest
 void launch_dp(const DpLaunch &a, const uint64_t *bin_off, uint64_t *tasks, int32_t cmax,
                cudaStream_t st);
 bool dp_wave_fits(int32_t rmax);

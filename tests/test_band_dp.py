@@ -355,3 +355,26 @@ def _edited_segments(rng, n, columns):
                                            ([255, 256, 257], 200), ([1022, 1023, 1024, 1025], 120)])
 def test_gpu_wide_windows_at_their_edges(gpu_lib, oracle, affine, columns, count):
     _check_segments(oracle, affine, _edited_segments(np.random.default_rng(80 + affine), count, columns))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,columns,free,budget", [(10, 50, 5, 13660160), (1000, 100, 20, 14622720), (20000, 100, 20, 35131392)])
+def test_gpu_segments_without_room_for_the_windows(gpu_lib, n, columns, free, budget):
+    """Segments take no more memory than whole matrices alone need (the budgets): what
+    the windows have is given back, and the ops are the same."""
+    from hero_b200 import Hero
+    rng = np.random.default_rng(3)
+    col = ACGT[rng.integers(0, 4, (n, columns))]
+    row = np.concatenate([ACGT[rng.integers(0, 4, (n, free))], col], 1)
+    col[:, ::9] = ACGT[rng.integers(0, 4, col[:, ::9].shape)]
+    seq = [np.ascontiguousarray(x).reshape(-1) for x in (row, col)]
+    off = [np.arange(n + 1, dtype=np.uint64) * np.uint64(x.shape[1]) for x in (row, col)]
+    idx, zeros = np.arange(n, dtype=np.uint32), np.zeros(n, np.int32)
+    got = []
+    for limit in (0, budget):
+        with Hero(device_memory_budget=limit) as h:
+            ops, oo, nops = h.align_segments(1, seq[0], off[0], seq[1], off[1], idx, np.zeros(n, np.uint8), idx, zeros,
+                                             np.diff(off[0]).astype(np.int32), zeros, np.diff(off[1]).astype(np.int32),
+                                             np.ones(n, np.uint8), np.full(n, 1000, np.int64))
+            got.append([bytes(ops[int(oo[i]):int(oo[i]) + int(nops[i])]) for i in range(n)])
+    assert got[0] == got[1]
