@@ -207,8 +207,9 @@ struct WarpCodes {
 
 // One task: up to 64 segments of one class, type and column count, two a lane
 // (positions lane and lane + 32).  Registers hold the window (M and IY of every
-// diagonal, the row selectors), so a cell costs six ALU instructions and a
-// column touches memory only for its code words.
+// diagonal, the row selectors): two cells take eight ALU instructions (affine: byte
+// select, add, two add-max, 3-way max, two masks, the code word's add) or seven
+// (global), and the move of a selector; a column touches memory only for its code words.
 template <bool AFFINE, int NB, int TYPE, bool MASK>
 __device__ __noinline__ void band_task(const DpLaunch &a, const BandWork &w, const uint32_t *order, uint32_t n,
                                        int32_t C, uint32_t *codes) {

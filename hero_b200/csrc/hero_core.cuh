@@ -303,7 +303,8 @@ HERO_HD bool walk_chain(const Params &p, int64_t Lq, int64_t Ls, const KeyAt &ke
     // the lanes of a warp reach together and visitors inline once.  (A branch with
     // its own calls for each of the seven kinds of piece made code that missed the
     // instruction cache, a third of the vote kernel's stalls: votes of 1.67 M x
-    // 150 bp 20.9 ms, .aln text of 53 k x 150 bp 4.3 ms; now 18.2 and 1.6.)
+    // 150 bp 20.9 -> 18.2 ms (15.8 with later steps), the four .aln kernels on 53 k x
+    // 150 bp 4.3 -> 1.5: lists 0.36, sizes 0.41, text 0.74.)
     for (int32_t i = 0; i <= n; i++) {
         int64_t s0 = 0, s1 = 0, q0 = 0, q1 = 0, gap = 0;
         uint32_t flags = 0;

@@ -81,3 +81,4 @@ def test_every_candidate_shape_on_whole_matrices(aligner, flags):
             assert cells == want["stats"]["dp_cells"]
             assert pairs > cells // 2 if whole and shape["pair_strips"] else pairs == 0 or not whole
             assert after["dp_stage_timeouts"] == 0
+        assert not whole or h.stats()["dp_tasks_staged"] > 0  # row bases by bulk copies, in the pairs' shapes
