@@ -66,8 +66,10 @@ def whole_matrices(reads, **kw):
             h.build_index()
             h.align_self()
             h.consensus()
-        except HeroError:
+        except HeroError as e:
             h.close()
+            if not budget or "HERO_E_OOM" not in str(e):
+                raise
             return None
         return h
 
